@@ -447,6 +447,15 @@ template <int P, class C> void launch_fft_full(const FullParamsT<C> &p, long ngr
 	QB_CUDA(cudaGetLastError());
 }
 
+template <class C> void launch_sum_slots(const SumSlotsT<C> &p, int ncells, cudaStream_t s) {
+	ProfScope ps("sum_slots", s);
+	k_sum_slots<C><<<dim3((unsigned)((p.len + 255) / 256), (unsigned)ncells), 256, 0, s>>>(p);
+	QB_CUDA(cudaGetLastError());
+}
+// partials a cell from which the sums get their own launch: below, the
+// assembly reads them faster than the launch costs
+constexpr int kSumSlots = 4;
+
 template <int P, class C> void launch_assemble(const AsmParamsT<C> &p, long ncells, cudaStream_t s) {
 	static DeviceFlag init;
 	if (!init) { set_smem(k_assemble<P, C>, smem_grids<P, C>(1)); init = true; }
@@ -621,7 +630,7 @@ template <int P, class C> struct Rhs {
 		}
 	}
 
-	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells) {
+	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells, cudaStream_t s) {
 		AsmParamsT<C> a{};
 		a.What = ws.What.as<C>();
 		a.FS = (parts & RHS_CC) ? ws.fs.as<C>() : nullptr;
@@ -629,6 +638,15 @@ template <int P, class C> struct Rhs {
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
 		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, q.i3->nterms, ncells);
+		const long slots = ch.i3_slots > 0 ? (long)ch.i3_slots : (long)ncells * ch.i3;
+		if ((parts & RHS_CD) && slots >= (long)kSumSlots * ncells && ncells <= 65535) {
+			SumSlotsT<C> p{};
+			p.rg = a.xrg; p.nx = ch.i3;
+			ws.i3s.ensure(sizeof(C) * 4 * ncells * PP);
+			p.in = ws.i3p.as<C>(); p.out = ws.i3s.as<C>(); p.len = (int)(4 * PP);
+			launch_sum_slots(p, ncells, s);
+			a.Xp = ws.i3s.as<C>(); a.nx = 1; a.xrg = TermRanges{};
+		}
 		a.s2 = 1.0 / (double)PP;
 		a.s1 = a.s2 * a.s2;
 		return a;
@@ -637,7 +655,7 @@ template <int P, class C> struct Rhs {
 	static void operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *cc, double2 *cd, cudaStream_t s) {
 		Chunks ch;
 		prepare(ws, q, ncells, W, parts, ch, s);
-		AsmParamsT<C> a = asm_params(ws, parts, ch, q, ncells);
+		AsmParamsT<C> a = asm_params(ws, parts, ch, q, ncells, s);
 		a.mode = 0; a.out_cc = cc; a.out_cd = cd;
 		launch_assemble<P>(a, ncells, s);
 	}
@@ -645,7 +663,7 @@ template <int P, class C> struct Rhs {
 	static void update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc, double2 *out, cudaStream_t s) {
 		Chunks ch;
 		prepare(ws, q, ncells, wcur, RHS_ALL, ch, s);
-		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, ncells);
+		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, ncells, s);
 		a.mode = 1; a.base = base; a.wcur = wcur; a.B = B; a.dtc = dtc; a.out = out;
 		launch_assemble<P>(a, ncells, s);
 	}

@@ -1035,14 +1035,57 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_fft_full(const FullParamsT<C> p)
 	init_twiddles<P>(tw);
 	const long b = blockIdx.x;
 	const C *in = p.in + b * p.grid_stride;
-	for (int i = threadIdx.x; i < P * P; i += G::NT) {
-		C s = in[i];
-		for (int k = 1; k < p.nparts; k++) s = cadd(s, in[k * p.part_stride + i]);
-		S[G::at(i / P, i % P)] = s;
+	{
+		// all of the thread's elements of one partial are loaded together: the sums
+		// wait for nparts memory latencies instead of nparts times the elements (one
+		// cell at N = 32, 16 partials: 23 -> 10 us)
+		C s[8];
+#pragma unroll
+		for (int e = 0; e < 8; e++) s[e] = in[threadIdx.x + e * G::NT];
+#pragma unroll 2
+		for (int k = 1; k < p.nparts; k++) {
+			const C *ik = in + k * p.part_stride + threadIdx.x;
+#pragma unroll
+			for (int e = 0; e < 8; e++) s[e] = cadd(s[e], ik[e * G::NT]);
+		}
+#pragma unroll
+		for (int e = 0; e < 8; e++) {
+			const int i = threadIdx.x + e * G::NT;
+			S[G::at(i / P, i % P)] = s[e];
+		}
 	}
 	__syncthreads();
 	fft2_smem<P, -1>(S, tw);
 	smem_to_global<P>(p.out + b * (long)P * P, S);
+}
+
+// ---------------------------------------------------------------------------
+// Sums of the I3 partials of each cell, in slot order: in[slot][len] (slots of
+// a cell as in the assembly) -> out[cell][len].  The assembly has four CTAs a
+// cell; with one cell and 74 partials it spent most of its time on them (N =
+// 32: 390 us, 20 us behind this kernel), which spreads them over the GPU.
+template <class C> struct SumSlotsT {
+	const C *in; C *out; int len, nx;       // nx: slots a cell when rg.nslots = 0
+	TermRanges rg;
+};
+template <class C>
+__global__ void __launch_bounds__(256) k_sum_slots(const SumSlotsT<C> p) {
+	const int i = blockIdx.x * 256 + threadIdx.x;
+	const long cell = blockIdx.y;
+	if (i >= p.len) return;
+	C s = czero<C>();
+	if (p.rg.nslots > 0) {
+		const TermRanges &g = p.rg;
+		const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
+		// after the first slot of a cell the others are the first of their cluster
+		s = cadd(s, p.in[((long)k0 * g.maxc + (cell - g.first_cell(k0))) * p.len + i]);
+#pragma unroll 8
+		for (int k = k0 + 1; k <= k1; k++) s = cadd(s, p.in[(long)k * g.maxc * p.len + i]);
+	} else {
+#pragma unroll 8
+		for (int k = 0; k < p.nx; k++) s = cadd(s, p.in[(cell * p.nx + k) * p.len + i]);
+	}
+	p.out[cell * p.len + i] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -1111,33 +1154,59 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 	}
 	// --- Cd ---
 	if (p.FS4 != nullptr || p.Qp != nullptr || p.Xp != nullptr) {
-		for (int i = threadIdx.x; i < PP; i += G::NT) {
-			C z = czero<C>();
-			if (p.Qp != nullptr) {
-				C q = czero<C>();
-				for (int ii = 0; ii < 4; ii++) {
-					const C *Q = p.Qp + ((cell * 4 + ii) * p.nq) * (long)PP + i;
-					C s = czero<C>();
-					for (int k = 0; k < p.nq; k++) s = cadd(s, Q[(long)k * PP]);
-					q.x += eta2[ii] * s.x; q.y += eta2[ii] * s.y;
-				}
-				C h; h.x = -Wh[j * PP + i].x; h.y = -Wh[j * PP + i].y;
+		// the partial sums of all the thread's elements together (as in k_fft_full)
+		C zs[8];
+#pragma unroll
+		for (int e = 0; e < 8; e++) zs[e] = czero<C>();
+		if (p.Qp != nullptr) {
+#pragma unroll 1
+			for (int ii = 0; ii < 4; ii++) {
+				const C *Q = p.Qp + ((cell * 4 + ii) * p.nq) * (long)PP + threadIdx.x;
+				C s[8];
+#pragma unroll
+				for (int e = 0; e < 8; e++) s[e] = czero<C>();
+#pragma unroll 1
+				for (int k = 0; k < p.nq; k++)
+#pragma unroll
+					for (int e = 0; e < 8; e++) s[e] = cadd(s[e], Q[(long)k * PP + e * G::NT]);
+#pragma unroll
+				for (int e = 0; e < 8; e++) { zs[e].x += eta2[ii] * s[e].x; zs[e].y += eta2[ii] * s[e].y; }
+			}
+#pragma unroll
+			for (int e = 0; e < 8; e++) {
+				C h = Wh[j * PP + threadIdx.x + e * G::NT];
+				h.x = -h.x; h.y = -h.y;
 				if (j == 0) h.x += (R)1.0;
-				const C v = cmul(h, q);
-				z.x += s2 * v.x; z.y += s2 * v.y;
+				const C v = cmul(h, zs[e]);
+				zs[e].x = s2 * v.x;
+				zs[e].y = s2 * v.y;
 			}
-			if (p.Xp != nullptr) {
-				C s = czero<C>();
-				if (p.xrg.nslots > 0) {
-					const TermRanges &g = p.xrg;
-					const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
-					for (int k = k0; k <= k1; k++)
-						s = cadd(s, p.Xp[(((long)k * g.maxc + (cell - g.first_cell(k))) * 4 + j) * (long)PP + i]);
-				} else {
-					for (int k = 0; k < p.nx; k++) s = cadd(s, p.Xp[((cell * p.nx + k) * 4 + j) * (long)PP + i]);
-				}
-				z.x -= eta2[j] * s1 * s.x; z.y -= eta2[j] * s1 * s.y;
+		}
+		if (p.Xp != nullptr) {
+			C s[8];
+#pragma unroll
+			for (int e = 0; e < 8; e++) s[e] = czero<C>();
+			auto add = [&](long slot) {
+				const C *X = p.Xp + (slot * 4 + j) * (long)PP + threadIdx.x;
+#pragma unroll
+				for (int e = 0; e < 8; e++) s[e] = cadd(s[e], X[e * G::NT]);
+			};
+			if (p.xrg.nslots > 0) {
+				const TermRanges &g = p.xrg;
+				const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
+#pragma unroll 1
+				for (int k = k0; k <= k1; k++) add((long)k * g.maxc + (cell - g.first_cell(k)));
+			} else {
+#pragma unroll 1
+				for (int k = 0; k < p.nx; k++) add(cell * p.nx + k);
 			}
+#pragma unroll
+			for (int e = 0; e < 8; e++) { zs[e].x -= eta2[j] * s1 * s[e].x; zs[e].y -= eta2[j] * s1 * s[e].y; }
+		}
+#pragma unroll
+		for (int e = 0; e < 8; e++) {
+			const int i = threadIdx.x + e * G::NT;
+			C z = zs[e];
 			if (p.FS4 != nullptr) {
 				const C *F4 = p.FS4 + cell * 4 * PP;
 				C v = cadd(cscale(cmul(Wh[i], F4[j * PP + i]), eta2[j]), cscale(cmul(Wh[j * PP + i], F4[i]), (R)2.0));
