@@ -326,7 +326,7 @@ inline TermRanges term_ranges(int slots, int nterms, int ncells) {
 }
 
 // the workspace's chunk multipliers applied to heuristic chunk counts
-inline void scale_chunks(const Workspace &ws, const QuadSet &q, Chunks &ch) {
+inline void scale_chunks(const Workspace &ws, const QuadSet &q, Chunks &ch, int i3_units) {
 	auto sc = [](int c, float f, int nterms, int cap) {
 		const int v = (int)std::lround((double)c * f);
 		return std::max(1, std::min(std::min(v, std::max(1, nterms)), cap));
@@ -335,7 +335,7 @@ inline void scale_chunks(const Workspace &ws, const QuadSet &q, Chunks &ch) {
 		if (q.i1) ch.i1 = sc(ch.i1, ws.chunk_scale12, q.i1->nterms, 64);
 		if (q.i2) ch.i2 = sc(ch.i2, ws.chunk_scale12, q.i2->nterms, 64);
 	}
-	if (ws.chunk_scale3 != 1.0f && q.i3) ch.i3 = sc(ch.i3, ws.chunk_scale3, q.i3->nterms, 256);
+	if (ws.chunk_scale3 != 1.0f && q.i3) ch.i3 = sc(ch.i3, ws.chunk_scale3, std::max(1, i3_units), 256);
 }
 
 constexpr double kRealFormBound = 1e-6;
@@ -563,15 +563,30 @@ template <int P, class C> struct Rhs {
 		launch_i2<P>(p, (long)ncells * 4 * nchunk, s);
 	}
 
+	// k_i3p and k_i3pr sum the terms of opposite shifts together (I3Units); each
+	// CTA of their clusters leaves its own partial of the Z sums
+	static constexpr int kZRanks = 2;
+	static bool pairs_units(const Workspace &) { return P == 64; }
+	static int i3_count(const Workspace &ws, const DevI3 &t) {
+		I3Units u;
+		if (pairs_units(ws)) u.M = t.pairM;
+		return u.count(t.nterms);
+	}
+
 	static void i3_sums(Workspace &ws, const DevI3 &t, int ncells, const double2 *W, const Chunks &ch, cudaStream_t s) {
 		const int nchunk = ch.i3;
 		I3ParamsT<C> p{};
-		p.nchunk = nchunk; p.nterms = t.nterms;
+		p.nchunk = nchunk; p.nterms = i3_count(ws, t);
+		if (pairs_units(ws)) p.un.M = t.pairM;
+		size_t slots = (size_t)ncells * nchunk;
 		if (ch.i3_slots > 0) {
-			p.rg = term_ranges(ch.i3_slots, t.nterms, ncells);
-			ws.i3p.ensure(sizeof(C) * (size_t)p.rg.nslots * p.rg.maxc * 4 * PP);
-		} else {
-			ws.i3p.ensure(sizeof(C) * ncells * nchunk * 4 * PP);
+			p.rg = term_ranges(ch.i3_slots, p.nterms, ncells);
+			slots = (size_t)p.rg.nslots * p.rg.maxc;
+		}
+		ws.i3p.ensure(sizeof(C) * slots * 4 * PP);
+		if (pairs_units(ws)) {
+			ws.i3z.ensure(sizeof(C) * slots * kZRanks * 4 * NN);
+			p.zout = ws.i3z.as<C>();
 		}
 		p.src = W; p.src_cell = 4 * NN;
 		for (int r = 0; r < 4; r++) p.src_comp[r] = r;
@@ -589,6 +604,8 @@ template <int P, class C> struct Rhs {
 			if constexpr (sizeof(C) == 8) {
 				if (use_real_form() && even_combos(p)) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
+					ws.i3zs.ensure(sizeof(C) * slots * kZRanks * 2 * (N + 1) * (N + 1));
+					p.zscr = ws.i3zs.as<C>();
 					int *kind = ws.i3kind.as<int>();
 					launch_nyquist_kind(P / 2, ncells, W, kRealFormBound, kind, ws.i3stats.as<unsigned long long>(), s);
 					launch_i3pr(p, (long)ncells * nchunk, kind, s);
@@ -610,17 +627,17 @@ template <int P, class C> struct Rhs {
 
 	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, Chunks &ch, cudaStream_t s) {
 		T::prepare(q, s);
-		ch = pick_chunks(N, ncells, q, (int)(8 * sizeof(typename CT<C>::R)));
+		ch = pick_chunks(N, ncells, q, (int)(8 * sizeof(typename CT<C>::R)), q.i3 ? i3_count(ws, *q.i3) : 0);
 		if (P == 32 && sizeof(C) == 8 && ws.i3_variant == 1 && q.i3) {
 			check_tmem_coresidency();
 			ch.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), num_sms(), 256, 0.15);      // one CTA per SM
 		}
-		scale_chunks(ws, q, ch);
+		scale_chunks(ws, q, ch, q.i3 ? i3_count(ws, *q.i3) : 0);
 		// FP64 at N = 32: every resident cluster of k_i3p takes one contiguous range
 		// of the (cell, term) work, one partial per cell it touches
 		const bool ranges = ws.i3_ranges >= 0 ? ws.i3_ranges == 1 : term_ranges_enabled();
 		if (P == 64 && sizeof(C) == 16 && q.i3 && q.i3->nterms > 0 && ranges)
-			ch.i3_slots = (int)std::min<long>(active_i3p_clusters<C>(), (long)ncells * q.i3->nterms);
+			ch.i3_slots = (int)std::min<long>(active_i3p_clusters<C>(), (long)ncells * i3_count(ws, *q.i3));
 		spectra(ws, ncells, W, s);
 		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s);
 		if (parts & RHS_CD) {
@@ -637,15 +654,23 @@ template <int P, class C> struct Rhs {
 		a.FS4 = (parts & RHS_CD) ? ws.fs4.as<C>() : nullptr;
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
-		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, q.i3->nterms, ncells);
+		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, i3_count(ws, *q.i3), ncells);
+		const bool zp = pairs_units(ws) && (parts & RHS_CD);
+		if (zp) { a.Zp = ws.i3z.as<C>(); a.nz = kZRanks; }
 		const long slots = ch.i3_slots > 0 ? (long)ch.i3_slots : (long)ncells * ch.i3;
 		if ((parts & RHS_CD) && slots >= (long)kSumSlots * ncells && ncells <= 65535) {
 			SumSlotsT<C> p{};
-			p.rg = a.xrg; p.nx = ch.i3;
+			p.rg = a.xrg; p.nx = ch.i3; p.per = 1;
 			ws.i3s.ensure(sizeof(C) * 4 * ncells * PP);
 			p.in = ws.i3p.as<C>(); p.out = ws.i3s.as<C>(); p.len = (int)(4 * PP);
 			launch_sum_slots(p, ncells, s);
 			a.Xp = ws.i3s.as<C>(); a.nx = 1; a.xrg = TermRanges{};
+			if (zp) {
+				ws.i3zsum.ensure(sizeof(C) * 4 * ncells * NN);
+				p.in = ws.i3z.as<C>(); p.out = ws.i3zsum.as<C>(); p.len = (int)(4 * NN); p.per = kZRanks;
+				launch_sum_slots(p, ncells, s);
+				a.Zp = ws.i3zsum.as<C>(); a.nz = 1;
+			}
 		}
 		a.s2 = 1.0 / (double)PP;
 		a.s1 = a.s2 * a.s2;
@@ -993,7 +1018,7 @@ template <class C> struct Rhs<128, C> {
 			const int act = (sizeof(C) == 8 && use_full128()) ? active_i3_full128_clusters() : active_i3_clusters128<C>();
 			ch.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), act, 256, 0.15);
 		}
-		scale_chunks(ws, q, ch);
+		scale_chunks(ws, q, ch, q.i3 ? q.i3->nterms : 0);
 		spectra(ws, ncells, W, s);
 		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s);
 		if (parts & RHS_CD) {
@@ -1010,7 +1035,6 @@ template <class C> struct Rhs<128, C> {
 		a.FS4 = (parts & RHS_CD) ? ws.fs4.as<C>() : nullptr;
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
-		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, q.i3->nterms, ncells);
 		a.s2 = 1.0 / (double)PP;
 		a.s1 = a.s2 * a.s2;
 		return a;
@@ -1073,7 +1097,7 @@ __global__ void k_rk4(long n, const double2 *__restrict__ W, double c, const dou
 
 }  // namespace
 
-Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec) {
+Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) {
 	Chunks c;
 	const int sms = num_sms();
 	if (q.i1) c.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), sms, 64);
@@ -1088,7 +1112,7 @@ Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec) {
 		}
 		// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written
 		// and read back at HBM speed; one term takes a cluster ~36 us there: 0.15
-		c.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), act, 256, 0.15);
+		c.i3 = best_chunks((long)ncells, std::max(1, i3_units), act, 256, 0.15);
 	}
 	return c;
 }

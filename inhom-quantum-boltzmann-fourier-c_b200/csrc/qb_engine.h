@@ -54,7 +54,8 @@ struct DevI1 { int N = 0, nterms = 0; DevBuf psi2, phi; mutable DevBuf psi2f, ph
 // I2-type: Q = sum_t FFT2(Pad(psi1_t f)) . FFT2(Pad(psi2_t g))
 struct DevI2 { int N = 0, nterms = 0; DevBuf psi1, psi2; mutable DevBuf psi1f, psi2f; };
 // I3-type: psi1_t complex N x N; psi2_t = scale[t] * table[idx[t]] (tables stored transposed)
-struct DevI3 { int N = 0, nterms = 0; DevBuf psi1, psi2T, idx, scale; mutable DevBuf psi1f, psi2Tf; };
+// pairM > 0: M = pairM terms an angle, with terms m and M - 1 - m of opposite shifts (FourierI3)
+struct DevI3 { int N = 0, nterms = 0, pairM = 0; DevBuf psi1, psi2T, idx, scale; mutable DevBuf psi1f, psi2Tf; };
 
 struct QuadSet { const DevI1 *i1 = nullptr; const DevI2 *i2 = nullptr; const DevI3 *i3 = nullptr; const DevI1 *i4 = nullptr; };
 
@@ -84,7 +85,7 @@ struct Workspace {
 	int prec = 64;                           // working precision of the collision operator: 64 (FP64) or 32 (FP32 form)
 	int conserve = 0;                        // restore the collision invariants after each velocity-space collision step
 	cudaStream_t stream = nullptr;           // own stream (upstream API calls)
-	DevBuf What, i1cc, i1i4, i2p, i3p, i3s, fs, fs4, wmid;      // collision scratch
+	DevBuf What, i1cc, i1i4, i2p, i3p, i3s, i3z, i3zsum, i3zs, fs, fs4, wmid;      // collision scratch
 	DevBuf fa, fb, va, vb;                   // state scratch (Fourier / velocity)
 	DevBuf io_in, io_out, bext, vgrid;       // staging for host-pointer calls
 	DevBuf aux, aux2;
@@ -142,7 +143,7 @@ struct Chunks {
 	int i1 = 1, i2 = 1, i3 = 1;
 	int i3_slots = 0;                        // > 0: the I3 sums run as that many contiguous (cell, term) ranges instead of chunks
 };
-Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec);
+Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units);
 
 // ---- operators (device pointers, stream-ordered) ------------------------------
 enum RhsParts { RHS_CC = 1, RHS_CD = 2, RHS_ALL = 3 };

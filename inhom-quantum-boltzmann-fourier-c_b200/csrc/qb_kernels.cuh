@@ -310,9 +310,33 @@ struct TermRanges {
 	__host__ __device__ long first_cell(int k) const { return start(k) / nterms; }
 };
 
+// Units of the I3 sums.  The radial nodes of FourierI3 are Gauss-Legendre on
+// [-R, R], so terms m and M - 1 - m of an angle have opposite shifts (psi1' =
+// conj psi1) and equal weights (and one psi2 table), and both follow from the
+// same chains T_ij = FFT2(psi2 . IFFT2(W^_i . P_j)):
+//   X_j  += sum_i eta_i P_i . T_ij                       (the shift a)
+//   Y_i   = sum_j eta_j W^_j . T_ij,
+//   Z_i  += conj(psi1) . Extract(IFFT2(Y_i))             (the shift -a)
+// because W_i(v) W_j(v - a) is W_i(v + a) W_j(v) shifted by a and psi2 commutes
+// with shifts.  No product of N-grids reaches the aliases of the extracted
+// points on the 2N grid, so the two forms agree for every W to rounding.  A
+// pair takes 16 chains of two transforms instead of 32 and one transform a
+// component more.  M = 0: the terms carry no such structure (caller-built
+// tables) and every unit is one term; the middle node of an odd M is alone.
+struct I3Units {
+	int M = 0;
+	__host__ __device__ int per_angle() const { return (M + 1) / 2; }
+	__host__ __device__ int count(int nterms) const { return M > 0 ? nterms / M * per_angle() : nterms; }
+	__device__ __forceinline__ int term(int u) const { return M > 0 ? u / per_angle() * M + u % per_angle() : u; }
+	__device__ __forceinline__ bool pair(int u) const { return M > 0 && 2 * (u % per_angle()) != M - 1; }
+};
+
 template <class C> struct I3ParamsT {
 	using R = typename CT<C>::R;
-	int nchunk, nterms;
+	int nchunk, nterms;                                   // nterms: terms, or units of `un` in the kernels that pair them
+	I3Units un;
+	C *zout;                                              // Z_i partials, layout given at each kernel (pairing kernels)
+	C *zscr;                                              // real forms: packed Z sums of the running cluster
 	TermRanges rg;                                        // nslots > 0: one term range per cluster (k_i3p)
 	const double2 *src; long src_cell; int src_comp[4];   // N x N grids (FP64 state)
 	const C *Ghat; long g_cell;                           // P x P grids, G_g at Ghat + cell*g_cell + g*P*P
@@ -574,7 +598,7 @@ template <class C> struct I3Tmem {
 	static constexpr unsigned PER_THREAD = 2 * 8 * WPC;       // columns of one thread's slice
 	static constexpr unsigned NCOLS = 4 * PER_THREAD;         // 4 warps share a lane quarter: 256 (FP64), 128 (FP32)
 	// after the accumulators each thread keeps its 8 psi2 values of the current
-	// term, its 8 values of the current P_j and (FP64) its twiddle powers w^1..w^4;
+	// term, 8 values of the current Y_i and (FP64) its twiddle powers w^1..w^4;
 	// columns a slot: 16 / 32 / 16 (FP64), 8 / 16 (FP32)
 	static constexpr unsigned ALLOC = sizeof(C) == 16 ? 512 : 256;
 	// column address of value e of output q of this thread
@@ -582,12 +606,12 @@ template <class C> struct I3Tmem {
 		const unsigned w = threadIdx.x >> 5;
 		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * PER_THREAD + (unsigned)(q * 8 + e) * WPC;
 	}
-	static constexpr unsigned PSI = 8 * WPC / 2, PJ = 8 * WPC;   // columns a slot
+	static constexpr unsigned PSI = 8 * WPC / 2, YI = 8 * WPC;   // columns a slot
 	__device__ __forceinline__ static unsigned lanes() { return (32u * ((threadIdx.x >> 5) & 3u)) << 16; }
 	__device__ __forceinline__ static unsigned slot() { return threadIdx.x >> 7; }
 	__device__ __forceinline__ static unsigned psiaddr(unsigned base) { return base + lanes() + NCOLS + slot() * PSI; }
-	__device__ __forceinline__ static unsigned pjaddr(unsigned base) { return base + lanes() + NCOLS + 4 * PSI + slot() * PJ; }
-	__device__ __forceinline__ static unsigned twaddr(unsigned base) { return base + lanes() + NCOLS + 4 * (PSI + PJ) + slot() * 16u; }
+	__device__ __forceinline__ static unsigned yaddr(unsigned base) { return base + lanes() + NCOLS + 4 * PSI + slot() * YI; }
+	__device__ __forceinline__ static unsigned twaddr(unsigned base) { return base + lanes() + NCOLS + 4 * (PSI + YI) + slot() * 16u; }
 };
 
 // FP32 at P = 64: each CTA of the pair pushes its P grids of the term into the
@@ -644,9 +668,14 @@ __device__ __forceinline__ void fence_async_smem_a() { asm volatile("fence.proxy
 // holding components 2r and 2r + 1: per term it computes both spectra
 // P_{t,c} = FFT2(Pad(psi1_t . W_c)) into its shared memory and, after a
 // cluster barrier, the 8 (pair, combo) chains of its two outputs
-//   X_j += eta_i P_i . FFT2(psi2_t . IFFT2(W^_i . P_j)),  j in {2r, 2r + 1}
+//   X_j += eta_i P_i . T_ij,  T_ij = FFT2(psi2_t . IFFT2(W^_i . P_j)),  j in {2r, 2r + 1}
 // with P_i of the partner's components read through distributed shared
-// memory.  The two 8-value accumulators of every thread live in TMEM, which
+// memory.  The chains run with i outermost: for a pair of opposite shifts
+// (I3Units) the CTA adds its two terms of Y_i = sum_j eta_j W^_j . T_ij, takes
+// IFFT2(Y_i) (every row, the columns that Extract keeps) and adds conj(psi1) .
+// Extract of it to its partial of Z_i; the two CTAs' partials are summed by
+// the assembly, which costs 4 extra transforms of 12 passes against 32 for the
+// chains but no exchange between the CTAs.  The two 8-value accumulators of every thread live in TMEM, which
 // frees their registers and lets 2-CTA clusters use all 148 SMs (4-CTA
 // clusters of k_i3 fit 33 of 37 four-SM slots).  The rest of the TMEM
 // allocation caches values each thread reuses at its own positions: its psi2
@@ -723,7 +752,22 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3p(const I3ParamsT<C> p, con
 		for (int e = 0; e < 8; e++) tmem_st(TM::addr(tbase, q, e), czero<C>());
 	tmem_wait_st();
 	const C *Gcell = p.Ghat + cell * p.g_cell;
-	for (int t = t0; t < t1; t++) {
+	// partial sums of this segment: slot (cluster, cell) of the ranges, or (cell, chunk)
+	const long slot = p.rg.nslots > 0 ? cid * p.rg.maxc + (cell - p.rg.first_cell((int)cid))
+	                                  : cell * p.nchunk + (int)(cid % p.nchunk);
+	// the extracted points of column `line` this thread owns: rows tau + 8 e, e = 0, 1, 6, 7
+	const bool zcol = G::src(line) >= 0;
+	const int zofs = tau * G::N + G::src(line);
+	C *zbase = p.zout + (slot * 2 + rank) * 4 * (long)G::N * G::N + zofs;
+	if (zcol) {
+#pragma unroll 1
+		for (int i = 0; i < 4; i++)
+#pragma unroll
+			for (int e = 0; e < 4; e++) zbase[(i * G::N + 8 * e) * G::N] = czero<C>();
+	}
+	for (int un = t0; un < t1; un++) {
+		const int t = p.un.term(un);
+		const bool pr = p.un.pair(un);
 #pragma unroll 1
 		for (int q = 0; q < 2; q++) {
 			const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank + q] * G::N * G::N;
@@ -752,32 +796,21 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3p(const I3ParamsT<C> p, con
 		}
 		if constexpr (kPush) push_wait(&pmbar, pphase, p.err);
 #pragma unroll 1
-		for (int q = 0; q < 2; q++) {
-			const int j = 2 * rank + q;
-			const C *Pj = Pq + q * G::GRID;
-			{
-				// this thread's 8 values of P_j (row line, columns tau + 8 r), read once from
-				// shared memory for the 4 chains of output j
-				C v[8];
-#pragma unroll
-				for (int r = 0; r < 8; r++) v[r] = Pj[G::at(line, tau + G::T * r)];
-				tmem_st8(TM::pjaddr(tbase), v);
-				tmem_wait_st();
-			}
+		for (int i = 0; i < 4; i++) {
+			const C *Gg = Gcell + (long)i * P * P;
+			const C *Pa = ((i >> 1) == rank ? Pq : (kPush ? Pr : Ppeer)) + (i & 1) * G::GRID;
+			const R coef = (R)(i == 0 ? 1.0 : -1.0);
+			C x[8];
 #pragma unroll 1
-			for (int c = 0; c < p.ncombo[j]; c++) {
-				const C *Gg = Gcell + (long)p.cgi[j][c] * P * P;
-				C x[8];
-				// rows: IFFT of G_g . P_j
+			for (int q = 0; q < 2; q++) {
+				const C *Pj = Pq + q * G::GRID;
+				// rows: IFFT of W^_i . P_j
 				{
-					C pj[8];
-					tmem_ld8(TM::pjaddr(tbase), pj);
 					C g[8];
 #pragma unroll
 					for (int r = 0; r < 8; r++) g[r] = Gg[line * P + tau + G::T * r];
-					tmem_wait_ld();
 #pragma unroll
-					for (int r = 0; r < 8; r++) x[r] = cmul(g[r], pj[r]);
+					for (int r = 0; r < 8; r++) x[r] = cmul(g[r], Pj[G::at(line, tau + G::T * r)]);
 				}
 				fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, twaddr);
 #pragma unroll
@@ -799,43 +832,77 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3p(const I3ParamsT<C> p, con
 #pragma unroll
 				for (int e = 0; e < 8; e++) Ug[G::at(Lp::out_pos(tau, e), line)] = x[e];
 				__syncthreads();
-				// rows: FFT, multiply by P_a (own or the partner's), accumulate in TMEM
+				// rows: FFT; X_j += eta_i P_i . T_ij in TMEM (P_i own or the partner's)
 #pragma unroll
 				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(line, tau + G::T * r)];
 				fft1d_lane<P, -1>(x, tau, G::row(Ug, line), wp, twaddr);
-				const int a = p.ca[j][c];
-				const C *Pa = ((a >> 1) == rank ? Pq : (kPush ? Pr : Ppeer)) + (a & 1) * G::GRID;
-				const R coef = (R)p.ccoef[j][c];
-				C acc[8];
-				if constexpr (sizeof(C) == 16) tmem_ld8(TM::addr(tbase, q, 0), acc);   // one load (FP64); FP32 per value measured faster
-				else {
+				{
+					C acc[8];
+					if constexpr (sizeof(C) == 16) tmem_ld8(TM::addr(tbase, q, 0), acc);   // one load (FP64); FP32 per value measured faster
+					else {
 #pragma unroll
-					for (int e = 0; e < 8; e++) tmem_ld(TM::addr(tbase, q, e), acc[e]);
+						for (int e = 0; e < 8; e++) tmem_ld(TM::addr(tbase, q, e), acc[e]);
+					}
+					tmem_wait_ld();
+#pragma unroll
+					for (int e = 0; e < 8; e++) {
+						const C v = cmul(Pa[G::at(line, Lp::out_pos(tau, e))], x[e]);
+						acc[e].x += coef * v.x;
+						acc[e].y += coef * v.y;
+					}
+					if constexpr (sizeof(C) == 16) tmem_st8(TM::addr(tbase, q, 0), acc);
+					else {
+#pragma unroll
+						for (int e = 0; e < 8; e++) tmem_st(TM::addr(tbase, q, e), acc[e]);
+					}
 				}
-				tmem_wait_ld();
+				// Y_i: the term of j = 2r waits in TMEM for that of j = 2r + 1
+				if (pr) {
+					const C *Wj = Gcell + (long)(2 * rank + q) * P * P + line * P + tau;
+					const R eta = (R)(2 * rank + q == 0 ? 1.0 : -1.0);
 #pragma unroll
-				for (int e = 0; e < 8; e++) {
-					const C v = cmul(Pa[G::at(line, Lp::out_pos(tau, e))], x[e]);
-					acc[e].x += coef * v.x;
-					acc[e].y += coef * v.y;
-				}
-				if constexpr (sizeof(C) == 16) tmem_st8(TM::addr(tbase, q, 0), acc);
-				else {
+					for (int e = 0; e < 8; e++) x[e] = cscale(cmul(Wj[G::T * e], x[e]), eta);
+					if (q == 0) {
+						tmem_st8(TM::yaddr(tbase), x);
+					} else {
+						C y[8];
+						tmem_ld8(TM::yaddr(tbase), y);
+						tmem_wait_ld();
 #pragma unroll
-					for (int e = 0; e < 8; e++) tmem_st(TM::addr(tbase, q, e), acc[e]);
+						for (int e = 0; e < 8; e++) x[e] = cadd(y[e], x[e]);
+					}
 				}
 				tmem_wait_st();
-				// no barrier here: the row passes that end this pair and begin the
+				// no barrier here: the row passes that end this chain and begin the
 				// next touch only the rows of their own 8-lane group, and the next
-				// column pass waits behind the next pair's first barrier
+				// column pass waits behind the next chain's first barrier
 			}
+			if (!pr) continue;
+			// Z_i += conj(psi1) . Extract(IFFT2(Y_i))
+			fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, twaddr);
+#pragma unroll
+			for (int e = 0; e < 8; e++) Ug[G::at(line, Lp::out_pos(tau, e))] = x[e];
+			__syncthreads();
+			if (zcol) {                                      // whole warps: lines 0 .. 15 and 48 .. 63
+				C z[4], w[4];
+				C *zi = zbase + (long)i * G::N * G::N;
+				const C *ps = p.psi1 + (long)t * G::N * G::N + zofs;
+#pragma unroll
+				for (int e = 0; e < 4; e++) { z[e] = zi[8 * e * G::N]; w[e] = ps[8 * e * G::N]; }
+#pragma unroll
+				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(tau + G::T * r, line)];
+				fft1d_lane<P, +1>(x, tau, G::col(Ug, line), wp, twaddr);
+#pragma unroll
+				for (int e = 0; e < 4; e++) {
+					w[e].y = -w[e].y;
+					zi[8 * e * G::N] = cadd(z[e], cmul(w[e], x[e < 2 ? e : e + 4]));
+				}
+			}
+			__syncthreads();                                 // the next chain's rows reuse Ug
 		}
 		if constexpr (kPush) push_release();              // the own P grids are read by the copy before they change
 		cluster.sync();
 	}
-	// partial sums of this segment: slot (cluster, cell) of the ranges, or (cell, chunk)
-	const long slot = p.rg.nslots > 0 ? cid * p.rg.maxc + (cell - p.rg.first_cell((int)cid))
-	                                  : cell * p.nchunk + (int)(cid % p.nchunk);
 #pragma unroll 1
 	for (int q = 0; q < 2; q++) {
 		C acc[8];
@@ -857,16 +924,16 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3p(const I3ParamsT<C> p, con
 // i W_2r+1) gives the real spectra P_2r (real part) and P_2r+1 (imaginary
 // part) in one shared grid; the chains of combos (i0, i1) of an output share
 // one complex transform of P_j . (W^_i0 + i W^_i1), and the real accumulators
-// take eta_i0 P_i0 . Re + eta_i1 P_i1 . Im.  Same shared-memory layout as k_i3p
-// (the second P grid unused); tensor memory: 2 x 8 real accumulators, 8 psi2
-// and 8 P_j values per thread.
+// take eta_i0 P_i0 . Re + eta_i1 P_i1 . Im; Y_i0 + i Y_i1 is packed the same way.
+// Same shared-memory layout as k_i3p (the second P grid unused); tensor memory:
+// 2 x 8 real accumulators, 8 psi2 values and 8 complex values of Y per thread.
 struct I3TmemR {
-	static constexpr unsigned PER_THREAD = 16, NCOLS = 64, PSI = 8, PJ = 8, ALLOC = 128;
+	static constexpr unsigned PER_THREAD = 16, NCOLS = 64, PSI = 8, YI = 16, ALLOC = 256;
 	__device__ __forceinline__ static unsigned lanes() { return (32u * ((threadIdx.x >> 5) & 3u)) << 16; }
 	__device__ __forceinline__ static unsigned slot() { return threadIdx.x >> 7; }
 	__device__ __forceinline__ static unsigned addr(unsigned base, int q) { return base + lanes() + (threadIdx.x >> 7) * PER_THREAD + (unsigned)q * 8; }
 	__device__ __forceinline__ static unsigned psiaddr(unsigned base) { return base + lanes() + NCOLS + slot() * PSI; }
-	__device__ __forceinline__ static unsigned pjaddr(unsigned base) { return base + lanes() + NCOLS + 4 * PSI + slot() * PJ; }
+	__device__ __forceinline__ static unsigned yaddr(unsigned base) { return base + lanes() + NCOLS + 4 * PSI + slot() * YI; }
 };
 
 template <int P>
@@ -907,9 +974,19 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3pr(const I3ParamsT<float2> 
 	}
 	const C *Gcell = p.Ghat + cell * p.g_cell;
 	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
+	// packed sums A_c = Z_2c + i Z_2c+1 on the frequencies -N/2 .. N/2 (both ends:
+	// separating the two real-grid parts needs the partner of -N/2)
+	constexpr int H = G::N / 2, ZA = (G::N + 1) * (G::N + 1);
+	const long slot = cell * p.nchunk + chunk;
+	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
+	for (int i = threadIdx.x; i < 2 * ZA; i += G::NT) za[i] = czero<C>();
+	const int zk = line <= H ? line : line - P;              // this thread's column as a frequency
+	const bool zcol = line <= H || line >= P - H;
 	push_init(&pmbar);
 	cluster.sync();                                          // the partner's mbarrier is initialised
-	for (int t = t0; t < t1; t++) {
+	for (int un = t0; un < t1; un++) {
+		const int t = p.un.term(un);
+		const bool pr = p.un.pair(un);
 		{
 			const double2 *sa = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank] * G::N * G::N;
 			const double2 *sb = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank + 1] * G::N * G::N;
@@ -929,35 +1006,27 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3pr(const I3ParamsT<float2> 
 		}
 		push_wait(&pmbar, pphase, p.err);
 #pragma unroll 1
-		for (int q = 0; q < 2; q++) {
-			const int j = 2 * rank + q;
-			{
-				float v[8];
-#pragma unroll
-				for (int r = 0; r < 8; r++) {
-					const C pv = Pq[G::at(line, tau + G::T * r)];
-					v[r] = q ? pv.y : pv.x;
-				}
-				tmem_st8r(TM::pjaddr(tbase), v);
-				tmem_wait_st();
-			}
+		for (int c = 0; c < 2; c++) {                        // the combos i = 2c (real part) and 2c + 1 (imaginary part)
+			const C *G0 = Gcell + (long)(2 * c) * P * P, *G1 = G0 + (long)P * P;
+			const C *Pa = (c == rank ? Pq : Pr);             // P_2c + i P_2c+1
+			const float c0 = c == 0 ? 1.f : -1.f;            // eta_2c; eta_2c+1 = -1
+			C x[8];
 #pragma unroll 1
-			for (int c = 0; c + 1 < p.ncombo[j]; c += 2) {
-				const C *G0 = Gcell + (long)p.cgi[j][c] * P * P, *G1 = Gcell + (long)p.cgi[j][c + 1] * P * P;
-				C x[8];
-				// rows: IFFT of P_j . (W^_i0 + i W^_i1)
+			for (int q = 0; q < 2; q++) {
+				// rows: IFFT of P_j . (W^_2c + i W^_2c+1)
 				{
-					float pj[8];
-					tmem_ld8r(TM::pjaddr(tbase), pj);
 					float g0[8], g1[8];
 #pragma unroll
 					for (int r = 0; r < 8; r++) {
 						g0[r] = G0[line * P + tau + G::T * r].x;
 						g1[r] = G1[line * P + tau + G::T * r].x;
 					}
-					tmem_wait_ld();
 #pragma unroll
-					for (int r = 0; r < 8; r++) x[r] = mk<C>(pj[r] * g0[r], pj[r] * g1[r]);
+					for (int r = 0; r < 8; r++) {
+						const C pv = Pq[G::at(line, tau + G::T * r)];
+						const float pj = q ? pv.y : pv.x;
+						x[r] = mk<C>(pj * g0[r], pj * g1[r]);
+					}
 				}
 				fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, 0u);
 #pragma unroll
@@ -979,30 +1048,84 @@ __global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3pr(const I3ParamsT<float2> 
 #pragma unroll
 				for (int e = 0; e < 8; e++) Ug[G::at(Lp::out_pos(tau, e), line)] = x[e];
 				__syncthreads();
-				// rows: FFT; the real part belongs to i0, the imaginary part to i1
+				// rows: FFT; the real part is T of i = 2c, the imaginary part of 2c + 1
 #pragma unroll
 				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(line, tau + G::T * r)];
 				fft1d_lane<P, -1>(x, tau, G::row(Ug, line), wp, 0u);
-				const int a0 = p.ca[j][c], a1 = p.ca[j][c + 1];
-				const C *Pa0 = ((a0 >> 1) == rank ? Pq : Pr), *Pa1 = ((a1 >> 1) == rank ? Pq : Pr);
-				const float c0 = (float)p.ccoef[j][c], c1 = (float)p.ccoef[j][c + 1];
-				float acc[8];
-				tmem_ld8r(TM::addr(tbase, q), acc);
-				tmem_wait_ld();
+				{
+					float acc[8];
+					tmem_ld8r(TM::addr(tbase, q), acc);
+					tmem_wait_ld();
 #pragma unroll
-				for (int e = 0; e < 8; e++) {
-					const int n = G::at(line, Lp::out_pos(tau, e));
-					const C v0 = Pa0[n], v1 = Pa1[n];
-					const float p0 = (a0 & 1) ? v0.y : v0.x, p1 = (a1 & 1) ? v1.y : v1.x;
-					acc[e] += c0 * (p0 * x[e].x) + c1 * (p1 * x[e].y);
+					for (int e = 0; e < 8; e++) {
+						const C pv = Pa[G::at(line, Lp::out_pos(tau, e))];
+						acc[e] += c0 * (pv.x * x[e].x) - pv.y * x[e].y;
+					}
+					tmem_st8r(TM::addr(tbase, q), acc);
 				}
-				tmem_st8r(TM::addr(tbase, q), acc);
+				// Y_2c + i Y_2c+1 += eta_j W^_j . T (W^_j real)
+				if (pr) {
+					const C *Wj = Gcell + (long)(2 * rank + q) * P * P + line * P + tau;
+					const float eta = 2 * rank + q == 0 ? 1.f : -1.f;
+#pragma unroll
+					for (int e = 0; e < 8; e++) x[e] = cscale(x[e], eta * Wj[G::T * e].x);
+					if (q == 0) {
+						tmem_st8(TM::yaddr(tbase), x);
+					} else {
+						C y[8];
+						tmem_ld8(TM::yaddr(tbase), y);
+						tmem_wait_ld();
+#pragma unroll
+						for (int e = 0; e < 8; e++) x[e] = cadd(y[e], x[e]);
+					}
+				}
 				tmem_wait_st();
 				// no barrier here, as in k_i3p
 			}
+			if (!pr) continue;
+			// A_c += conj(psi1) . IFFT2(Y_2c + i Y_2c+1) on the frequencies -N/2 .. N/2
+			fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, 0u);
+#pragma unroll
+			for (int e = 0; e < 8; e++) Ug[G::at(line, Lp::out_pos(tau, e))] = x[e];
+			__syncthreads();
+			if (line < H + 32 / G::T || line >= P - H) {     // whole warps; line H is the only one of its warp with zcol
+				const C *ps = p.psi1 + (long)t * G::N * G::N;
+#pragma unroll
+				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(tau + G::T * r, line)];
+				fft1d_lane<P, +1>(x, tau, G::col(Ug, line), wp, 0u);
+				if (zcol) {
+#pragma unroll
+					for (int e = 0; e < 8; e++) {
+						if (e > 2 && e < 6) continue;            // rows 24 .. 47
+						const int l = tau + G::T * e, zl = e < 3 ? l : l - P;
+						if (zl > H || (zl == H && zk == -H) || (zl == -H && zk == H)) continue;
+						// psi1 is tabulated on -N/2 .. N/2 - 1; at the upper end it is conj psi1(-k)
+						const bool up = zl == H || zk == H;
+						const int a = up ? -zl : zl, b = up ? -zk : zk;
+						C w = ps[(a < 0 ? a + G::N : a) * G::N + (b < 0 ? b + G::N : b)];
+						if (!up) w.y = -w.y;
+						C *z = za + c * ZA + (zl + H) * (G::N + 1) + zk + H;
+						*z = cadd(*z, cmul(w, x[e]));
+					}
+				}
+			}
+			__syncthreads();                                 // the next chain's rows reuse Ug
 		}
 		push_release();                                      // the own P grid is read by the copy before it changes
 		cluster.sync();
+	}
+	// A(k) = Z_2c(k) + i Z_2c+1(k) with both parts the transforms of real grids
+	{
+		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)G::N * G::N;
+		for (int i = threadIdx.x; i < 2 * G::N * G::N; i += G::NT) {
+			const int c = i / (G::N * G::N), n = i % (G::N * G::N);
+			int l = n / G::N, k = n % G::N;
+			l = l < H ? l : l - G::N;
+			k = k < H ? k : k - G::N;
+			const C u = za[c * ZA + (l + H) * (G::N + 1) + k + H], v = za[c * ZA + (H - l) * (G::N + 1) + H - k];
+			zo[(long)(2 * c) * G::N * G::N + n] = mk<C>(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
+			zo[(long)(2 * c + 1) * G::N * G::N + n] = mk<C>(0.5f * (u.y + v.y), -0.5f * (u.x - v.x));
+		}
 	}
 #pragma unroll 1
 	for (int q = 0; q < 2; q++) {
@@ -1066,6 +1189,7 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_fft_full(const FullParamsT<C> p)
 // 32: 390 us, 20 us behind this kernel), which spreads them over the GPU.
 template <class C> struct SumSlotsT {
 	const C *in; C *out; int len, nx;       // nx: slots a cell when rg.nslots = 0
+	int per;                                // partials a slot (in[slot][per][len])
 	TermRanges rg;
 };
 template <class C>
@@ -1074,16 +1198,27 @@ __global__ void __launch_bounds__(256) k_sum_slots(const SumSlotsT<C> p) {
 	const long cell = blockIdx.y;
 	if (i >= p.len) return;
 	C s = czero<C>();
+	long first = cell * p.nx, step = 1;
+	int n = p.nx;
 	if (p.rg.nslots > 0) {
-		const TermRanges &g = p.rg;
-		const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
 		// after the first slot of a cell the others are the first of their cluster
-		s = cadd(s, p.in[((long)k0 * g.maxc + (cell - g.first_cell(k0))) * p.len + i]);
+		const TermRanges &g = p.rg;
+		const int k0 = g.cluster_of(cell * (long)g.nterms);
+		n = g.cluster_of((cell + 1) * (long)g.nterms - 1) - k0 + 1;
+		const C *a = p.in + ((long)k0 * g.maxc + (cell - g.first_cell(k0))) * p.per * p.len + i;
+		for (int r = 0; r < p.per; r++) s = cadd(s, a[(long)r * p.len]);
+		first = (long)(k0 + 1) * g.maxc;
+		step = g.maxc;
+		n--;
+	}
+	const C *a = p.in + first * p.per * p.len + i;
+	step *= (long)p.per * p.len;
+	if (p.per == 1) {
 #pragma unroll 8
-		for (int k = k0 + 1; k <= k1; k++) s = cadd(s, p.in[(long)k * g.maxc * p.len + i]);
+		for (int k = 0; k < n; k++) s = cadd(s, a[k * step]);
 	} else {
 #pragma unroll 8
-		for (int k = 0; k < p.nx; k++) s = cadd(s, p.in[(cell * p.nx + k) * p.len + i]);
+		for (int m = 0; m < 2 * n; m++) s = cadd(s, a[(m >> 1) * step + (long)(m & 1) * p.len]);   // per = 2
 	}
 	p.out[cell * p.len + i] = s;
 }
@@ -1093,7 +1228,8 @@ __global__ void __launch_bounds__(256) k_sum_slots(const SumSlotsT<C> p) {
 //   Zcc_j = Wh_h . FS_g - Wh_g . FS_h          ((g,h) = (2,3),(3,1),(1,2); upstream collision.c:232-253)
 //   Zcd_j = s2 (-Wh_j + d_j0) . Q - eta2_j s1 X_j
 //         + s1 (eta2_j Wh_0 . FS4_j + 2 Wh_j . FS4_0) - d_j0 2 s1 sum_c Wh_c . FS4_c   (collision.c:95-167)
-//   Cc_j = s1 Extract(IFFT2(Zcc_j)), Cd_j = Extract(IFFT2(Zcd_j))
+//   Cc_j = s1 Extract(IFFT2(Zcc_j)), Cd_j = Extract(IFFT2(Zcd_j)) - eta2_j s1 Z_j
+// (Z_j: the already extracted sums of I3Units)
 // The spectra and transforms are in the working precision C; Cc and Cd are
 // widened to FP64 for the outputs.  mode 0 writes Cc and Cd; mode 1 writes
 // base + dtc (Cc + Cd + CB) in FP64 with the magnetic rotation CB of `wcur`
@@ -1105,6 +1241,7 @@ template <class C> struct AsmParamsT {
 	const C *Qp; int nq;              // [cell][4][nq][P*P] I2 partials, or null
 	const C *Xp; int nx;              // [cell][nx][4][P*P] I3 partials, or null
 	TermRanges xrg;                   // xrg.nslots > 0: Xp holds [slot][4][P*P] partials of term ranges
+	const C *Zp; int nz;              // extracted I3 sums of the opposite shifts, [slot of Xp][nz][4][N*N], or null
 	double s1, s2;
 	int mode;
 	double2 *out_cc, *out_cd;         // mode 0: [cell][4][N*N] (either may be null)
@@ -1113,6 +1250,27 @@ template <class C> struct AsmParamsT {
 	double2 *out;                     // mode 1
 };
 using AsmParams = AsmParamsT<double2>;
+
+// the sum of the Z partials of a cell at point q, in slot order
+template <class C>
+__device__ __forceinline__ double2 zsum(const AsmParamsT<C> &p, long cell, int j, int NN, int q) {
+	double2 z = czero();
+	auto add = [&](long slot) {
+		for (int r = 0; r < p.nz; r++) {
+			const C v = p.Zp[((slot * p.nz + r) * 4 + j) * NN + q];
+			z.x += (double)v.x;
+			z.y += (double)v.y;
+		}
+	};
+	if (p.xrg.nslots > 0) {
+		const TermRanges &g = p.xrg;
+		const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
+		for (int k = k0; k <= k1; k++) add((long)k * g.maxc + (cell - g.first_cell(k)));
+	} else {
+		for (int k = 0; k < p.nx; k++) add(cell * p.nx + k);
+	}
+	return z;
+}
 
 template <int P, class C>
 __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) {
@@ -1227,6 +1385,12 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 			if (q < NN) {
 				const C v = S[G::at(G::pad(q / N), G::pad(q % N))];
 				cd[u] = make_double2((double)v.x, (double)v.y);
+				if (p.Zp != nullptr) {
+					const double2 z = zsum(p, cell, j, NN, q);
+					const double f = (j == 0 ? 2.0 : -2.0) * p.s1;
+					cd[u].x -= f * z.x;
+					cd[u].y -= f * z.y;
+				}
 			}
 		}
 	}

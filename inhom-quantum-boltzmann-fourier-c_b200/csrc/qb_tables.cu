@@ -239,7 +239,7 @@ void build_i3(int N, int J, double L, double R, int M, DevI3 &dev, double *host_
 	xw.ensure(sizeof(double) * 2 * M);
 	scr.ensure(sizeof(double) * ((long)M * (M + 1) + 4 * M));
 	k_lgwt<<<1, 32, 0, s>>>(M, -R, R, xw.as<double>(), xw.as<double>() + M, scr.as<double>());
-	dev.N = N; dev.nterms = nt;
+	dev.N = N; dev.nterms = nt; dev.pairM = M;
 	dev.psi1.ensure(sizeof(double2) * nt * N * N);
 	dev.psi2T.ensure(sizeof(double) * J * P * P);
 	dev.idx.ensure(sizeof(int) * nt);
@@ -292,7 +292,7 @@ void upload_i2(int N, int num, const double *psiR1, const double *psiR2, DevI2 &
 
 void upload_i3(int N, int num, const double *psiR1, const double *psiR2, DevI3 &dev, cudaStream_t s) {
 	const long P = 2 * N;
-	dev.N = N; dev.nterms = num;
+	dev.N = N; dev.nterms = num; dev.pairM = 0;
 	dev.psi1.ensure(sizeof(double2) * num * N * N);
 	dev.psi2T.ensure(sizeof(double) * num * P * P);
 	dev.idx.ensure(sizeof(int) * num);
