@@ -203,27 +203,14 @@ template <class K> void set_smem(K kernel, size_t bytes) {
 
 template <int P, class C = double2> constexpr size_t smem_grids(int ngrids) { return sizeof(C) * ((size_t)ngrids * Geo<P, C>::GRID + P); }
 
-// active clusters of the I3 kernel (occupancy query, cached per P and C)
-template <int P, class C> int active_i3_clusters() {
+// resident CTAs of k_i3q on the GPU (occupancy query, cached per P and C)
+template <int P, class C> int active_i3q() {
 	static DeviceInt cached{-1};
 	if (cached < 0) {
-		auto kern = k_i3<P, 4, C>;
-		set_smem(kern, smem_grids<P, C>(2));
-		cudaLaunchConfig_t cfg = {};
-		cfg.gridDim = dim3(4);
-		cfg.blockDim = dim3(Geo<P>::NT);
-		cfg.dynamicSmemBytes = smem_grids<P, C>(2);
-		cudaLaunchAttribute attr;
-		attr.id = cudaLaunchAttributeClusterDimension;
-		attr.val.clusterDim.x = 4; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-		cfg.attrs = &attr;
-		cfg.numAttrs = 1;
+		set_smem(k_i3q<P, C>, I3q<P, C>::SMEM);
 		int n = 0;
-		if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-			cudaGetLastError();
-			n = std::max(1, num_sms() / 4);
-		}
-		cached = n;
+		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_i3q<P, C>, I3q<P, C>::NT, I3q<P, C>::SMEM));
+		cached = std::max(1, n) * num_sms();
 	}
 	return cached;
 }
@@ -264,6 +251,13 @@ template <int P, class C> void launch_i2(const I2ParamsT<C> &p, long nblocks, cu
 	if (!init) { set_smem(k_i2_terms<P, C>, smem_grids<P, C>(2)); init = true; }
 	ProfScope ps("i2_terms", s);
 	k_i2_terms<P, C><<<(unsigned)nblocks, Geo<P>::NT, smem_grids<P, C>(2), s>>>(p);
+	QB_CUDA(cudaGetLastError());
+}
+
+template <int P, class C> void launch_i3q(const I3ParamsT<C> &p, long nblocks, cudaStream_t s) {
+	active_i3q<P, C>();                        // shared-memory attribute
+	ProfScope ps("i3_cluster", s);
+	k_i3q<P, C><<<(unsigned)nblocks, I3q<P, C>::NT, I3q<P, C>::SMEM, s>>>(p);
 	QB_CUDA(cudaGetLastError());
 }
 
@@ -563,10 +557,11 @@ template <int P, class C> struct Rhs {
 		launch_i2<P>(p, (long)ncells * 4 * nchunk, s);
 	}
 
-	// k_i3p and k_i3pr sum the terms of opposite shifts together (I3Units); each
-	// CTA of their clusters leaves its own partial of the Z sums
-	static constexpr int kZRanks = 2;
-	static bool pairs_units(const Workspace &) { return P == 64; }
+	// the terms of opposite shifts are summed together (I3Units), except by the
+	// tensor-core form; each CTA of the clusters of k_i3p and k_i3pr leaves its
+	// own partial of the Z sums
+	static constexpr int kZRanks = P == 64 ? 2 : 1;
+	static bool pairs_units(const Workspace &ws) { return !(P == 32 && sizeof(C) == 8 && ws.i3_variant == 1); }
 	static int i3_count(const Workspace &ws, const DevI3 &t) {
 		I3Units u;
 		if (pairs_units(ws)) u.M = t.pairM;
@@ -621,7 +616,7 @@ template <int P, class C> struct Rhs {
 					return;
 				}
 			}
-			launch_i3<P, 4>(p, (long)ncells * nchunk, s);
+			launch_i3q<P>(p, (long)ncells * nchunk, s);
 		}
 	}
 
@@ -1106,8 +1101,8 @@ Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) 
 		int act = 0;
 		const bool f32 = prec == 32;
 		switch (N) {
-		case 8: act = f32 ? active_i3_clusters<16, float2>() : active_i3_clusters<16, double2>(); break;
-		case 16: act = f32 ? active_i3_clusters<32, float2>() : active_i3_clusters<32, double2>(); break;
+		case 8: act = f32 ? active_i3q<16, float2>() : active_i3q<16, double2>(); break;
+		case 16: act = f32 ? active_i3q<32, float2>() : active_i3q<32, double2>(); break;
 		default: act = f32 ? active_i3p_clusters<float2>() : active_i3p_clusters<double2>(); break;
 		}
 		// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written

@@ -291,7 +291,8 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_i2_terms(const I2ParamsT<C> p) {
 }
 
 // ---------------------------------------------------------------------------
-// K4: I3-type sums on a cluster of CS CTAs (one per source component).
+// K4: I3-type sums on a cluster of CS CTAs (one per source component), for the
+// single integrals.
 // CTA r of the cluster for (cell, chunk) computes P_r = FFT2(Pad(psi1_t . src_r))
 // into its shared memory; the other CTAs read it through distributed shared
 // memory.  For each of its combos (a, g, coef) it accumulates
@@ -422,6 +423,172 @@ __global__ void __launch_bounds__(Geo<P>::NT, Occ<C>::CTAS) k_i3(const I3ParamsT
 	C *o = p.out + ((cell * p.nchunk + chunk) * CS + rank) * (long)P * P + line * P;
 #pragma unroll
 	for (int e = 0; e < 8; e++) o[Lp::out_pos(tau, e)] = acc[e];
+}
+
+// ---------------------------------------------------------------------------
+// K4q: the I3 sums of the collision operator at P = 16 and 32, all four
+// components of a (cell, chunk) in one CTA of four groups of P T threads, group
+// j for component j.  Per unit group j forms P_j, then the groups run the 16
+// chains in four rounds, group j the chain of i = (j + round) % 4:
+//   X_j += eta_i P_i . T_ij  (registers),  Y_i += eta_j W^_j . T_ij  (shared memory)
+// In a round every i belongs to one group, so the Y sums need one CTA barrier
+// a round and no atomics; after the last round group j transforms its own Y_j
+// (see I3Units).  The P grids, work grids and Y sums of the four components
+// (12 grids: 203 KB in FP64 at P = 32) replace the distributed shared memory
+// of 4-CTA clusters, of which 33 fit the GPU (132 of 148 SMs), and a group's
+// barriers hold back its own warps only.  Out as k_i3 with CS = 4; zout:
+// [slot][4][N*N].
+// Bound by latency at 16 warps an SM: Strang step of 33 cells at N = 16,
+// J = 12, M = 9, FP64: 2.74 -> 1.70 ms (4-CTA clusters, term by term, before).
+template <int P, class C> struct I3q {
+	using G = Geo<P, C>;
+	static constexpr int NT = 4 * G::NT;
+	static constexpr size_t SMEM = sizeof(C) * (8 * (size_t)G::GRID + 4 * (size_t)P * P + P);
+	static constexpr int CTAS = P == 16 ? 4 : (sizeof(C) == 8 ? 2 : 1);    // resident an SM, by registers and shared memory
+};
+template <int NT> __device__ __forceinline__ void group_sync(int g) {
+	if constexpr (NT == 32) __syncwarp();
+	else asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(NT) : "memory");
+}
+template <int P, class C>
+__global__ void __launch_bounds__(I3q<P, C>::NT, I3q<P, C>::CTAS) k_i3q(const I3ParamsT<C> p) {
+	using G = Geo<P, C>;
+	using Lp = Len<P>;
+	using R = typename CT<C>::R;
+	constexpr int GT = G::NT, N = G::N, NN = N * N;
+	static_assert(P == 16 || P == 32, "P = 64 and up have kernels of their own");
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	C *Pg = reinterpret_cast<C *>(smem_raw), *Ug = Pg + 4 * G::GRID, *Yg = Ug + 4 * G::GRID, *tw = Yg + 4 * P * P;
+	const int j = threadIdx.x / GT, tid = threadIdx.x % GT;
+	const int line = tid / G::T, tau = tid % G::T;
+	const int chunk = (int)(blockIdx.x % p.nchunk);
+	const long cell = blockIdx.x / p.nchunk;
+	init_twiddles<P>(tw);
+	__syncthreads();
+	C *Pj = Pg + j * G::GRID, *U = Ug + j * G::GRID;
+	const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[j] * NN;
+	const C *What = p.Ghat + cell * p.g_cell;
+	const int u0 = (int)((long)chunk * p.nterms / p.nchunk), u1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
+	const R etaj = (R)(j == 0 ? 1.0 : -1.0);
+	const int zk = G::src(line);                             // the extracted column of this thread, or -1
+	C acc[8], z[4];                                          // z: the thread's four extracted rows of column zk
+#pragma unroll
+	for (int e = 0; e < 8; e++) acc[e] = czero<C>();
+#pragma unroll
+	for (int m = 0; m < 4; m++) z[m] = czero<C>();
+	// value index of the thread's m-th extracted row: T = 4: e = 0, 4 (rows below
+	// P / 4), 3, 7 (from 3P / 4 on); T = 2: e = 2 m + tau
+	auto zrow = [&](int m) { return G::src(Lp::out_pos(tau, P == 32 ? (m & 1) * 4 + (m >> 1) * 3 : 2 * m + tau)); };
+	for (int u = u0; u < u1; u++) {
+		const int t = p.un.term(u);
+		const bool pr = p.un.pair(u);
+		const C *psi1 = p.psi1 + (long)t * NN;
+		C x[8];
+		load_pad_row<P>(x, line, tau, src, MulCplx<C>{psi1});
+		fft1d_acc<P, -1>(x, tau, G::row(Pj, line), tw);
+#pragma unroll
+		for (int e = 0; e < 8; e++) Pj[G::at(line, Lp::out_pos(tau, e))] = x[e];
+		group_sync<GT>(j);
+#pragma unroll
+		for (int r = 0; r < 8; r++) x[r] = Pj[G::at(tau + G::T * r, line)];
+		fft1d_acc<P, -1>(x, tau, G::col(Pj, line), tw);
+#pragma unroll
+		for (int e = 0; e < 8; e++) Pj[G::at(Lp::out_pos(tau, e), line)] = x[e];
+		__syncthreads();
+		const R *psi2 = p.psi2T + (long)p.psi2_idx[t] * P * P + line * P;
+		const R sc = (R)p.psi2_scale[t];
+#pragma unroll 1
+		for (int c = 0; c < 4; c++) {
+			const int i = (j + c) & 3;
+			const C *Gg = What + i * P * P + line * P;
+			// rows: IFFT of W^_i . P_j
+#pragma unroll
+			for (int r = 0; r < 8; r++) {
+				const int k = tau + G::T * r;
+				x[r] = cmul(Gg[k], Pj[G::at(line, k)]);
+			}
+			fft1d_acc<P, +1>(x, tau, G::row(U, line), tw);
+#pragma unroll
+			for (int e = 0; e < 8; e++) U[G::at(line, Lp::out_pos(tau, e))] = x[e];
+			group_sync<GT>(j);
+			// columns: IFFT, multiply by psi2_t, FFT
+#pragma unroll
+			for (int r = 0; r < 8; r++) x[r] = U[G::at(tau + G::T * r, line)];
+			fft1d_acc<P, +1>(x, tau, G::col(U, line), tw);
+#pragma unroll
+			for (int e = 0; e < 8; e++) {
+				const R f = sc * psi2[Lp::out_pos(tau, e)];
+				x[e].x *= f;
+				x[e].y *= f;
+			}
+			out_to_in_acc<P>(x, tau, G::col(U, line));
+			fft1d_acc<P, -1>(x, tau, G::col(U, line), tw);
+#pragma unroll
+			for (int e = 0; e < 8; e++) U[G::at(Lp::out_pos(tau, e), line)] = x[e];
+			group_sync<GT>(j);
+			// rows: FFT, X_j += eta_i P_i . T_ij
+#pragma unroll
+			for (int r = 0; r < 8; r++) x[r] = U[G::at(line, tau + G::T * r)];
+			fft1d_acc<P, -1>(x, tau, G::row(U, line), tw);
+			const C *Pi = Pg + i * G::GRID;
+			const R coef = (R)(i == 0 ? 1.0 : -1.0);
+#pragma unroll
+			for (int e = 0; e < 8; e++) {
+				const C v = cmul(Pi[G::at(line, Lp::out_pos(tau, e))], x[e]);
+				acc[e].x += coef * v.x;
+				acc[e].y += coef * v.y;
+			}
+			if (pr) {
+				// Y_i in the order of the threads (every group maps a thread to the same points)
+				C *Y = Yg + i * P * P + tid;
+				const C *Wj = What + j * P * P + line * P;
+#pragma unroll
+				for (int e = 0; e < 8; e++) {
+					const C y = cscale(cmul(Wj[Lp::out_pos(tau, e)], x[e]), etaj);
+					Y[e * GT] = c == 0 ? y : cadd(Y[e * GT], y);
+				}
+				__syncthreads();
+			}
+		}
+		if (!pr) {
+			__syncthreads();                                 // the P grids are read
+			continue;
+		}
+		// Z_j += conj(psi1) . Extract(IFFT2(Y_j))
+#pragma unroll
+		for (int e = 0; e < 8; e++) x[e] = Yg[j * P * P + tid + e * GT];
+		out_to_in_acc<P>(x, tau, G::row(U, line));
+		fft1d_acc<P, +1>(x, tau, G::row(U, line), tw);
+#pragma unroll
+		for (int e = 0; e < 8; e++) U[G::at(line, Lp::out_pos(tau, e))] = x[e];
+		group_sync<GT>(j);
+		if (P == 16 || zk >= 0) {                            // P = 32: whole warps (lines 0 .. 7, 24 .. 31)
+#pragma unroll
+			for (int r = 0; r < 8; r++) x[r] = U[G::at(tau + G::T * r, line)];
+			fft1d_acc<P, +1>(x, tau, G::col(U, line), tw);
+			if (zk >= 0) {
+#pragma unroll
+				for (int m = 0; m < 4; m++) {
+					C w = psi1[zrow(m) * N + zk];
+					w.y = -w.y;
+					C v;
+					if constexpr (P == 32) v = x[(m & 1) * 4 + (m >> 1) * 3];
+					else v = tau ? x[2 * m + 1] : x[2 * m];
+					z[m] = cfma(w, v, z[m]);
+				}
+			}
+		}
+		group_sync<GT>(j);                                   // the next unit's chains reuse U
+	}
+	const long slot = cell * p.nchunk + chunk;
+	C *o = p.out + (slot * 4 + j) * (long)P * P + line * P;
+#pragma unroll
+	for (int e = 0; e < 8; e++) o[Lp::out_pos(tau, e)] = acc[e];
+	if (zk >= 0) {
+		C *zo = p.zout + (slot * 4 + j) * (long)NN + zk;
+#pragma unroll
+		for (int m = 0; m < 4; m++) zo[zrow(m) * N] = z[m];
+	}
 }
 
 // ---------------------------------------------------------------------------
