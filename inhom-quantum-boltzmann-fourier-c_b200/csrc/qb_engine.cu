@@ -449,6 +449,28 @@ template <class C> void launch_sum_slots(const SumSlotsT<C> &p, int ncells, cuda
 // partials a cell from which the sums get their own launch: below, the
 // assembly reads them faster than the launch costs
 constexpr int kSumSlots = 4;
+// the partial sums of X (a.Xp, lenx values a slot) and of Z (ws.i3z, zranks x
+// lenz values a slot; zranks = 0: none) as the assembly takes them: as they are, or
+// summed over the slots of each cell first
+template <class C>
+void sum_slots(Workspace &ws, AsmParamsT<C> &a, int ncells, long slots, long lenx, long lenz, int zranks, cudaStream_t s) {
+	if (zranks > 0) { a.Zp = ws.i3z.as<C>(); a.nz = zranks; }
+	if (slots < (long)kSumSlots * ncells || ncells > 65535) return;
+	SumSlotsT<C> p{};
+	p.rg = a.xrg; p.nx = a.nx; p.per = 1;
+	ws.i3s.ensure(sizeof(C) * ncells * lenx);
+	p.in = a.Xp; p.out = ws.i3s.as<C>(); p.len = (int)lenx;
+	launch_sum_slots(p, ncells, s);
+	a.Xp = ws.i3s.as<C>();
+	if (zranks > 0) {
+		ws.i3zsum.ensure(sizeof(C) * ncells * lenz);
+		p.in = a.Zp; p.out = ws.i3zsum.as<C>(); p.len = (int)lenz; p.per = zranks;
+		launch_sum_slots(p, ncells, s);
+		a.Zp = ws.i3zsum.as<C>(); a.nz = 1;
+	}
+	a.nx = 1;
+	a.xrg = TermRanges{};
+}
 
 template <int P, class C> void launch_assemble(const AsmParamsT<C> &p, long ncells, cudaStream_t s) {
 	static DeviceFlag init;
@@ -650,23 +672,8 @@ template <int P, class C> struct Rhs {
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
 		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, i3_count(ws, *q.i3), ncells);
-		const bool zp = pairs_units(ws) && (parts & RHS_CD);
-		if (zp) { a.Zp = ws.i3z.as<C>(); a.nz = kZRanks; }
 		const long slots = ch.i3_slots > 0 ? (long)ch.i3_slots : (long)ncells * ch.i3;
-		if ((parts & RHS_CD) && slots >= (long)kSumSlots * ncells && ncells <= 65535) {
-			SumSlotsT<C> p{};
-			p.rg = a.xrg; p.nx = ch.i3; p.per = 1;
-			ws.i3s.ensure(sizeof(C) * 4 * ncells * PP);
-			p.in = ws.i3p.as<C>(); p.out = ws.i3s.as<C>(); p.len = (int)(4 * PP);
-			launch_sum_slots(p, ncells, s);
-			a.Xp = ws.i3s.as<C>(); a.nx = 1; a.xrg = TermRanges{};
-			if (zp) {
-				ws.i3zsum.ensure(sizeof(C) * 4 * ncells * NN);
-				p.in = ws.i3z.as<C>(); p.out = ws.i3zsum.as<C>(); p.len = (int)(4 * NN); p.per = kZRanks;
-				launch_sum_slots(p, ncells, s);
-				a.Zp = ws.i3zsum.as<C>(); a.nz = 1;
-			}
-		}
+		if (parts & RHS_CD) sum_slots(ws, a, ncells, slots, 4 * PP, 4 * NN, pairs_units(ws) ? kZRanks : 0, s);
 		a.s2 = 1.0 / (double)PP;
 		a.s1 = a.s2 * a.s2;
 		return a;
@@ -809,12 +816,12 @@ int active_i3_full128_clusters() {
 	return cached;
 }
 
-void launch_i3_full128(const I3ParamsT<float2> &p, long nclusters, float2 *pscr, const int *kind, cudaStream_t s) {
+void launch_i3_full128(const I3ParamsT<float2> &p, long nclusters, float2 *pscr, float2 *yscr, const int *kind, cudaStream_t s) {
 	active_i3_full128_clusters();              // attribute + occupancy check
-	launch128(k_i3_full128<float2>, "i3_cluster", nclusters * 2, 2, kFull128Smem, s, p, pscr, kind);
+	launch128(k_i3_full128<float2>, "i3_cluster", nclusters * 2, 2, kFull128Smem, s, p, pscr, yscr, kind);
 }
 
-// the real form: same shared memory, 256 tensor-memory columns
+// the real form: same shared memory and tensor-memory columns
 void launch_i3_full128r(const I3ParamsT<float2> &p, long nclusters, float *pscr, const int *kind, cudaStream_t s) {
 	static DeviceFlag init;
 	if (!init) {
@@ -969,12 +976,26 @@ template <class C> struct Rhs<128, C> {
 		launch_i2_128(p, units, ws.scr128b.as<C>(), s);
 	}
 
+	// the whole-grid FP32 kernels sum the terms of opposite shifts together
+	// (I3Units), one partial of the Z sums per CTA of their clusters
+	static bool pairs_units() { return sizeof(C) == 8 && use_full128(); }
+	static int i3_count(const DevI3 &t) {
+		I3Units u;
+		if (pairs_units()) u.M = t.pairM;
+		return u.count(t.nterms);
+	}
+
 	static void i3_sums(Workspace &ws, const DevI3 &t, int ncells, const double2 *W, int nchunk, cudaStream_t s) {
 		const long ncl = (long)ncells * nchunk;
 		ws.i3p.ensure(sizeof(C) * ncl * 4 * PP);
 		ws.scr128a.ensure(sizeof(C) * ncl * 4 * PP);
 		I3ParamsT<C> p{};
-		p.nchunk = nchunk; p.nterms = t.nterms;
+		p.nchunk = nchunk; p.nterms = i3_count(t);
+		if (pairs_units()) {
+			p.un.M = t.pairM;
+			ws.i3z.ensure(sizeof(C) * ncl * 2 * 4 * NN);
+			p.zout = ws.i3z.as<C>();
+		}
 		p.src = W; p.src_cell = 4 * NN;
 		for (int r = 0; r < 4; r++) p.src_comp[r] = r;
 		p.Ghat = ws.What.as<C>(); p.g_cell = 4 * PP;
@@ -989,14 +1010,17 @@ template <class C> struct Rhs<128, C> {
 		p.err = ws.kerr.as<int>();
 		if constexpr (sizeof(C) == 8) {
 			if (use_full128()) {
+				ws.i3y.ensure(sizeof(C) * ncl * 2 * PP);
 				if (use_real_form() && even_combos(p)) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
+					ws.i3zs.ensure(sizeof(C) * ncl * 2 * 2 * (N + 1) * (N + 1));
+					p.zscr = ws.i3zs.as<C>();
 					int *kind = ws.i3kind.as<int>();
 					launch_nyquist_kind(N, ncells, W, kRealFormBound, kind, ws.i3stats.as<unsigned long long>(), s);
 					launch_i3_full128r(p, ncl, reinterpret_cast<float *>(ws.scr128a.as<C>()), kind, s);
-					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), kind, s);     // cells above the bound
+					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), ws.i3y.as<C>(), kind, s);     // cells above the bound
 				} else {
-					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), nullptr, s);
+					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), ws.i3y.as<C>(), nullptr, s);
 				}
 				return;
 			}
@@ -1011,9 +1035,9 @@ template <class C> struct Rhs<128, C> {
 		if (q.i2) ch.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), pairs, 64, 0.15);
 		if (q.i3) {
 			const int act = (sizeof(C) == 8 && use_full128()) ? active_i3_full128_clusters() : active_i3_clusters128<C>();
-			ch.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), act, 256, 0.15);
+			ch.i3 = best_chunks((long)ncells, std::max(1, i3_count(*q.i3)), act, 256, 0.15);
 		}
-		scale_chunks(ws, q, ch, q.i3 ? q.i3->nterms : 0);
+		scale_chunks(ws, q, ch, q.i3 ? i3_count(*q.i3) : 0);
 		spectra(ws, ncells, W, s);
 		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s);
 		if (parts & RHS_CD) {
@@ -1023,13 +1047,14 @@ template <class C> struct Rhs<128, C> {
 		}
 	}
 
-	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells) {
+	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, int ncells, cudaStream_t s) {
 		AsmParamsT<C> a{};
 		a.What = ws.What.as<C>();
 		a.FS = (parts & RHS_CC) ? ws.fs.as<C>() : nullptr;
 		a.FS4 = (parts & RHS_CD) ? ws.fs4.as<C>() : nullptr;
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
+		if (parts & RHS_CD) sum_slots(ws, a, ncells, (long)ncells * ch.i3, 4 * PP, 4 * NN, pairs_units() ? 2 : 0, s);
 		a.s2 = 1.0 / (double)PP;
 		a.s1 = a.s2 * a.s2;
 		return a;
@@ -1038,7 +1063,7 @@ template <class C> struct Rhs<128, C> {
 	static void operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *cc, double2 *cd, cudaStream_t s) {
 		Chunks ch;
 		prepare(ws, q, ncells, W, parts, ch, s);
-		AsmParamsT<C> a = asm_params(ws, parts, ch, q, ncells);
+		AsmParamsT<C> a = asm_params(ws, parts, ch, ncells, s);
 		a.mode = 0; a.out_cc = cc; a.out_cd = cd;
 		launch_assemble128(a, ncells, s);
 	}
@@ -1046,7 +1071,7 @@ template <class C> struct Rhs<128, C> {
 	static void update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc, double2 *out, cudaStream_t s) {
 		Chunks ch;
 		prepare(ws, q, ncells, wcur, RHS_ALL, ch, s);
-		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, ncells);
+		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, ncells, s);
 		a.mode = 1; a.base = base; a.wcur = wcur; a.B = B; a.dtc = dtc; a.out = out;
 		launch_assemble128(a, ncells, s);
 	}

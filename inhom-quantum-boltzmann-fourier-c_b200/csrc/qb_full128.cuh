@@ -100,8 +100,8 @@ __device__ __forceinline__ void fft128_line(C (&x)[8], int tau, C *S, int line, 
 	else fft1d_accw<64, DIR>(x, tau & 7, ColHalf<C>(S, line, h), wp);
 }
 
-// 128-point transform by decimation in time of a column whose lane tau holds
-// the samples at rows pos128(tau, e) (the output order of fft128_line):
+// 128-point transform by decimation in time of a column (or row) whose lane tau
+// holds the samples at positions pos128(tau, e) (the output order of fft128_line):
 // lanes 0-7 hold the even samples 2m, lanes 8-15 the odd ones, m = (tau & 7) +
 // 8 e, which is the input order of fft1d<64> on each half.  After the two
 // 64-point transforms E and O, the butterfly Z[k] = E[k] + w^k O[k],
@@ -111,10 +111,11 @@ __device__ __forceinline__ void fft128_line(C (&x)[8], int tau, C *S, int line, 
 // fft128_line it needs no reordering in between.
 __device__ __forceinline__ int dpos128(int tau, int i) { return (tau & 7) + 16 * (i >> 1) + 8 * (tau >> 3) + 64 * (i & 1); }
 
-template <int DIR, class C>
-__device__ __forceinline__ void fft128_dit_col(C (&x)[8], int tau, C *S, int col, const C *tw128, const C (&wp)[8]) {
+template <int DIR, bool ROW, class C>
+__device__ __forceinline__ void fft128_dit(C (&x)[8], int tau, C *S, int line, const C *tw128, const C (&wp)[8]) {
 	const int h = tau >> 3, t = tau & 7;
-	fft1d_accw<64, DIR>(x, t, ColHalf<C>(S, col, h), wp);
+	if constexpr (ROW) fft1d_accw<64, DIR>(x, t, RowHalf<C>(S, line, h), wp);
+	else fft1d_accw<64, DIR>(x, t, ColHalf<C>(S, line, h), wp);
 	C y[8];
 #pragma unroll
 	for (int j = 0; j < 4; j++) {
@@ -131,6 +132,17 @@ __device__ __forceinline__ void fft128_dit_col(C (&x)[8], int tau, C *S, int col
 	for (int i = 0; i < 8; i++) x[i] = y[i];
 }
 
+// the rows of IFFT2(Y): x holds 8 values of row `row` in pos128 order; inverse
+// transform, into the shared grid
+template <class C>
+__device__ __forceinline__ void y_row(C (&x)[8], int tau, C *S, int row, const C *tw128, const C (&wp)[8]) {
+	fft128_dit<+1, true>(x, tau, S, row, tw128, wp);
+	const int m = ((row >> 6) & 1) << 3, k0 = (tau & 7) + 8 * (tau >> 3);
+#pragma unroll
+	for (int i = 0; i < 8; i++)                     // positions dpos128(tau, i)
+		S[row * F128::LDP + 64 * (i & 1) + ((k0 + 16 * (i >> 1)) ^ m ^ ((i & 1) << 3))] = x[i];
+}
+
 // tensor-memory accumulators: 2 outputs x 4 row iterations x 8 values per
 // thread; the four warps of a lane quarter split the 512 columns
 struct F128Tmem {
@@ -142,11 +154,14 @@ struct F128Tmem {
 	}
 };
 
-// Ghat: B layout; pscr: [cluster][4][P*P] natural; out: [cell][chunk][4][P*P] B layout.
+// The chains run with i outermost for the pairs of opposite shifts (I3Units), as
+// in k_i3p.  Ghat: B layout; pscr: [cluster][4][P*P] natural; yscr:
+// [cluster][2][P*P]; out: [cell][chunk][4][P*P] B layout; zout:
+// [cell][chunk][rank][4][N*N].
 // kind: null (every cell) or the per-cell form of k_nyquist_kind; this kernel
 // then takes the cells of kind 1 (the real form k_i3_full128r takes kind 0).
 template <class C>
-__global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p, C *pscr, const int *kind) {
+__global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p, C *pscr, C *yscr, const int *kind) {
 	static_assert(sizeof(C) == 8, "the whole-grid form is FP32 only");
 	using F = F128;
 	using R = typename CT<C>::R;
@@ -182,8 +197,16 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 	C *Pall = pscr + cid * 4 * (long)F::P * F::P;
 	const C *Gcell = p.Ghat + cell * p.g_cell;
 	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
+	// this CTA's partial of the Z sums and its Y_i (element order of the threads)
+	const long slot = cell * p.nchunk + chunk;
+	C *zbase = p.zout + (slot * 2 + rank) * 4 * (long)F::N * F::N;
+	C *ybuf = yscr + (cid * 2 + rank) * (long)F::P * F::P + tid;
+	for (int i = tid; i < 4 * F::N * F::N; i += F::NT) zbase[i] = czero<C>();
+	__syncthreads();
 #pragma unroll 1
-	for (int t = t0; t < t1; t++) {
+	for (int un = t0; un < t1; un++) {
+		const int t = p.un.term(un);
+		const bool pr = p.un.pair(un);
 		// spectra of components 2 rank + q (sign -1), natural layout, to L2
 #pragma unroll 1
 		for (int q = 0; q < 2; q++) {
@@ -233,12 +256,16 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 		const R *psi2 = p.psi2T + (long)p.psi2_idx[t] * F::P * F::P;
 		const R sc = (R)p.psi2_scale[t];
 #pragma unroll 1
-		for (int q = 0; q < 2; q++) {
-			const int j = 2 * rank + q;
-			const C *Pj = Pall + (long)j * F::P * F::P;
+		for (int i = 0; i < 4; i++) {
+			const C *Gg = Gcell + (long)i * F::P * F::P;
+			const C *Pa = Pall + (long)i * F::P * F::P;
+			const R coef = (R)(i == 0 ? 1.0 : -1.0);
 #pragma unroll 1
-			for (int cmb = 0; cmb < p.ncombo[j]; cmb++) {
-				const C *Gg = Gcell + (long)p.cgi[j][cmb] * F::P * F::P;
+			for (int q = 0; q < 2; q++) {
+				const int j = 2 * rank + q;
+				const C *Pj = Pall + (long)j * F::P * F::P;
+				const C *Wj = Gcell + (long)j * F::P * F::P;
+				const R eta = (R)(j == 0 ? 1.0 : -1.0);
 				// rows: inverse transform along k of W^_i . P_j
 #pragma unroll 1
 				for (int it = 0; it < 4; it++) {
@@ -269,16 +296,15 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 						x[e].x *= f;
 						x[e].y *= f;
 					}
-					fft128_dit_col<-1>(x, tau, S, col, tw128, wp);
+					fft128_dit<-1, false>(x, tau, S, col, tw128, wp);
 					const int d0 = (tau & 7) + 8 * (tau >> 3);   // rows d0 + 16 (i / 2) + 64 (i % 2)
 #pragma unroll
-					for (int i = 0; i < 8; i++) S[(d0 + 16 * (i >> 1) + 64 * (i & 1)) * F::LDP + cs_.cx[i & 1]] = x[i];
+					for (int m = 0; m < 8; m++) S[(d0 + 16 * (m >> 1) + 64 * (m & 1)) * F::LDP + cs_.cx[m & 1]] = x[m];
 				}
 				__syncthreads();
-				// rows: forward transform along k, times P_a, accumulate
-				const int a = p.ca[j][cmb];
-				const C *Pa = Pall + (long)a * F::P * F::P;
-				const R coef = (R)p.ccoef[j][cmb];
+				// rows: forward transform along k, X_j += eta_i P_i . T_ij; Y_i collects
+				// eta_j W^_j . T_ij (the term of j = 2 rank waits in L2) and its rows are
+				// transformed as they are complete
 #pragma unroll 1
 				for (int it = 0; it < 4; it++) {
 					const int row = it * 32 + sub;
@@ -298,11 +324,48 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 						acc[e].y += coef * v.y;
 					}
 					tmem_st8(TM::addr(tbase, q, it, 0), acc);
+					if (pr) {
+						const C *wj = Wj + F::brow(row);
+						C *y = ybuf + it * 8 * F::NT;
+#pragma unroll
+						for (int e = 0; e < 8; e++) x[e] = cscale(cmul(wj[pos128(tau, e)], x[e]), eta);
+						if (q == 0) {
+#pragma unroll
+							for (int e = 0; e < 8; e++) y[e * F::NT] = x[e];
+						} else {
+#pragma unroll
+							for (int e = 0; e < 8; e++) x[e] = cadd(y[e * F::NT], x[e]);
+							y_row(x, tau, S, row, tw128, wp);
+						}
+					}
 					tmem_wait_st();
 				}
 				// no barrier: the next chain's first row pass writes only the
 				// rows this thread's 16-lane group has just read
 			}
+			if (!pr) continue;
+			// columns of IFFT2(Y_i) inside Extract; Z_i += conj(psi1) . them
+			__syncthreads();
+#pragma unroll 1
+			for (int it = 0; it < 4; it += 3) {                  // columns 0..31, 96..127
+				const int col = it * 32 + sub, ks = F::src(col);
+				const LineSlots cs_ = col_slots(col, tau);
+				C x[8];
+#pragma unroll
+				for (int r = 0; r < 8; r++) x[r] = S[cs_.at_in(r)];
+				fft128_line<+1, false>(x, tau, S, col, tw128, wp);
+				C *z = zbase + (long)i * F::N * F::N + ks;
+				const C *ps = p.psi1 + (long)t * F::N * F::N + ks;
+#pragma unroll
+				for (int e = 0; e < 8; e++) {                    // rows pos128(tau, e): e = 0, 1 (0..31), 6, 7 (96..127)
+					if (e >= 2 && e < 6) continue;
+					const int o = F::src(pos128(tau, e)) * F::N;
+					C w = ps[o];
+					w.y = -w.y;
+					z[o] = cfma(w, x[e], z[o]);
+				}
+			}
+			__syncthreads();                                     // the next chain's rows reuse S
 		}
 		cl.sync();                                          // the partner is done with this term's spectra
 	}
@@ -355,8 +418,14 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 // pscr: [cluster][4][P*P] real, natural order; out as k_i3_full128 (real
 // parts; imaginary parts written as zero).
 struct F128TmemR {
-	static constexpr unsigned PER_THREAD = 2 * 4 * 8;         // 64 (real FP32)
-	static constexpr unsigned NCOLS = 4 * PER_THREAD;         // 256
+	// 2 outputs x 4 row iterations x 8 real accumulators, then 4 x 8 complex values of Y
+	static constexpr unsigned PER_THREAD = 2 * 4 * 8;         // 64
+	static constexpr unsigned ACOLS = 4 * PER_THREAD;         // 256
+	static constexpr unsigned NCOLS = 2 * ACOLS;              // 512
+	__device__ __forceinline__ static unsigned yaddr(unsigned base, int it) {
+		const unsigned w = threadIdx.x >> 5;
+		return base + ((32u * (w & 3u)) << 16) + ACOLS + (w >> 2) * 64u + (unsigned)it * 16u;
+	}
 	__device__ __forceinline__ static unsigned addr(unsigned base, int q, int it) {
 		const unsigned w = threadIdx.x >> 5;
 		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * PER_THREAD + (unsigned)(q * 4 + it) * 8;
@@ -399,8 +468,17 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128r(const I3ParamsT<flo
 	float *Pall = pscr + cid * 4 * PP;
 	const C *Gcell = p.Ghat + cell * p.g_cell;
 	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
+	// packed sums A_c = Z_2c + i Z_2c+1 on the frequencies -N/2 .. N/2 (both ends:
+	// separating the two real-grid parts needs the partner of -N/2)
+	constexpr int H = F::N / 2, ZA = (F::N + 1) * (F::N + 1);
+	const long slot = cell * p.nchunk + chunk;
+	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
+	for (int i = tid; i < 2 * ZA; i += F::NT) za[i] = czero<C>();
+	__syncthreads();
 #pragma unroll 1
-	for (int t = t0; t < t1; t++) {
+	for (int un = t0; un < t1; un++) {
+		const int t = p.un.term(un);
+		const bool pr = p.un.pair(un);
 		// spectra of components 2 rank (real part) and 2 rank + 1 (imaginary part)
 		{
 			const double2 *sa = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank] * F::N * F::N;
@@ -452,13 +530,17 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128r(const I3ParamsT<flo
 		const float *psi2 = p.psi2T + (long)p.psi2_idx[t] * PP;
 		const float sc = (float)p.psi2_scale[t];
 #pragma unroll 1
-		for (int q = 0; q < 2; q++) {
-			const int j = 2 * rank + q;
-			const float *Pj = Pall + (long)j * PP;
+		for (int c = 0; c < 2; c++) {                        // the combos i = 2c (real part) and 2c + 1 (imaginary part)
+			const C *G0 = Gcell + (long)(2 * c) * PP, *G1 = G0 + PP;
+			const float *P0 = Pall + (long)(2 * c) * PP, *P1 = P0 + PP;
+			const float c0 = c == 0 ? 1.f : -1.f;            // eta_2c; eta_2c+1 = -1
 #pragma unroll 1
-			for (int cmb = 0; cmb + 1 < p.ncombo[j]; cmb += 2) {
-				const C *G0 = Gcell + (long)p.cgi[j][cmb] * PP, *G1 = Gcell + (long)p.cgi[j][cmb + 1] * PP;
-				// rows: inverse transform along k of (W^_i0 + i W^_i1) . P_j
+			for (int q = 0; q < 2; q++) {
+				const int j = 2 * rank + q;
+				const float *Pj = Pall + (long)j * PP;
+				const C *Wj = Gcell + (long)j * PP;
+				const float eta = j == 0 ? 1.f : -1.f;
+				// rows: inverse transform along k of (W^_2c + i W^_2c+1) . P_j
 #pragma unroll 1
 				for (int it = 0; it < 4; it++) {
 					const int row = it * 32 + sub;
@@ -493,16 +575,16 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128r(const I3ParamsT<flo
 						x[e].x *= f;
 						x[e].y *= f;
 					}
-					fft128_dit_col<-1>(x, tau, S, col, tw128, wp);
+					fft128_dit<-1, false>(x, tau, S, col, tw128, wp);
 					const int d0 = (tau & 7) + 8 * (tau >> 3);
 #pragma unroll
-					for (int i = 0; i < 8; i++) S[(d0 + 16 * (i >> 1) + 64 * (i & 1)) * F::LDP + cs_.cx[i & 1]] = x[i];
+					for (int m = 0; m < 8; m++) S[(d0 + 16 * (m >> 1) + 64 * (m & 1)) * F::LDP + cs_.cx[m & 1]] = x[m];
 				}
 				__syncthreads();
-				// rows: forward transform along k; the real part belongs to i0,
-				// the imaginary part to i1
-				const float *P0 = Pall + (long)p.ca[j][cmb] * PP, *P1 = Pall + (long)p.ca[j][cmb + 1] * PP;
-				const float c0 = (float)p.ccoef[j][cmb], c1 = (float)p.ccoef[j][cmb + 1];
+				// rows: forward transform along k; the real part is T of i = 2c, the
+				// imaginary part of 2c + 1.  Y_2c + i Y_2c+1 collects eta_j W^_j . T (W^_j
+				// real; the term of j = 2 rank waits in tensor memory) and its rows are
+				// transformed as they are complete
 #pragma unroll 1
 				for (int it = 0; it < 4; it++) {
 					const int row = it * 32 + sub;
@@ -518,16 +600,75 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128r(const I3ParamsT<flo
 #pragma unroll
 					for (int e = 0; e < 8; e++) {
 						const int n = pos128(tau, e);
-						acc[e] += c0 * (p0[n] * x[e].x) + c1 * (p1[n] * x[e].y);
+						acc[e] += c0 * (p0[n] * x[e].x) - p1[n] * x[e].y;
 					}
 					tmem_st8r(TM::addr(tbase, q, it), acc);
+					if (pr) {
+						const C *wj = Wj + F::brow(row);
+#pragma unroll
+						for (int e = 0; e < 8; e++) x[e] = cscale(x[e], eta * wj[pos128(tau, e)].x);
+						if (q == 0) {
+							tmem_st8(TM::yaddr(tbase, it), x);
+						} else {
+							C y[8];
+							tmem_ld8(TM::yaddr(tbase, it), y);
+							tmem_wait_ld();
+#pragma unroll
+							for (int e = 0; e < 8; e++) x[e] = cadd(y[e], x[e]);
+							y_row(x, tau, S, row, tw128, wp);
+						}
+					}
 					tmem_wait_st();
 				}
 				// no barrier: the next chain's first row pass writes only the
 				// rows this thread's 16-lane group has just read
 			}
+			if (!pr) continue;
+			// A_c += conj(psi1) . IFFT2(Y_2c + i Y_2c+1) on the frequencies -N/2 .. N/2
+			__syncthreads();
+			const C *ps = p.psi1 + (long)t * F::N * F::N;
+#pragma unroll 1
+			for (int it = 0; it < 4; it++) {                     // columns 0..31, 32 (one line of a warp), 96..127
+				if (it == 2 || (it == 1 && warp > 0)) continue;
+				const int col = it * 32 + sub;
+				const LineSlots cs_ = col_slots(col, tau);
+				C x[8];
+#pragma unroll
+				for (int r = 0; r < 8; r++) x[r] = S[cs_.at_in(r)];
+				fft128_line<+1, false>(x, tau, S, col, tw128, wp);
+				if (col == H + 1) continue;
+				const int zk = col <= H ? col : col - F::P;
+#pragma unroll
+				for (int e = 0; e < 8; e++) {
+					if (e > 2 && e < 6) continue;                // rows 48 .. 95
+					const int l = pos128(tau, e), zl = e < 3 ? l : l - F::P;
+					if (zl > H || (zl == H && zk == -H) || (zl == -H && zk == H)) continue;
+					// psi1 is tabulated on -N/2 .. N/2 - 1; at the upper end it is conj psi1(-k)
+					const bool up = zl == H || zk == H;
+					const int a = up ? -zl : zl, b = up ? -zk : zk;
+					C w = ps[(a < 0 ? a + F::N : a) * F::N + (b < 0 ? b + F::N : b)];
+					if (!up) w.y = -w.y;
+					C *z = za + c * ZA + (zl + H) * (F::N + 1) + zk + H;
+					*z = cfma(w, x[e], *z);
+				}
+			}
+			__syncthreads();                                     // the next chain's rows reuse S
 		}
 		cl.sync();                                          // the partner is done with this term's spectra
+	}
+	// A(k) = Z_2c(k) + i Z_2c+1(k) with both parts the transforms of real grids
+	{
+		constexpr int NN = F::N * F::N;
+		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
+		for (int i = tid; i < 2 * NN; i += F::NT) {
+			const int c = i / NN, n = i % NN;
+			int l = n / F::N, k = n % F::N;
+			l = l < H ? l : l - F::N;
+			k = k < H ? k : k - F::N;
+			const C u = za[c * ZA + (l + H) * (F::N + 1) + k + H], v = za[c * ZA + (H - l) * (F::N + 1) + H - k];
+			zo[(long)(2 * c) * NN + n] = mk<C>(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
+			zo[(long)(2 * c + 1) * NN + n] = mk<C>(0.5f * (u.y + v.y), -0.5f * (u.x - v.x));
+		}
 	}
 #pragma unroll 1
 	for (int q = 0; q < 2; q++) {

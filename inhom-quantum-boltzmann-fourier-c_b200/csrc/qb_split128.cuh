@@ -734,7 +734,16 @@ __global__ void __launch_bounds__(512, 1) k_assemble128(const AsmParamsT<C> p) {
 		C v[4];
 		inverse_extract(S, peer, cl, h, tw128, tw64, v);
 #pragma unroll
-		for (int u = 0; u < 4; u++) cd[u] = make_double2((double)v[u].x, (double)v[u].y);
+		for (int u = 0; u < 4; u++) {
+			cd[u] = make_double2((double)v[u].x, (double)v[u].y);
+			if (p.Zp != nullptr) {
+				const int idx = u * 512 + (int)threadIdx.x;
+				const double2 z = zsum(p, cell, j, NN, (32 * h + (idx >> 6)) * N + (idx & 63));
+				const double f = (j == 0 ? 2.0 : -2.0) * p.s1;
+				cd[u].x -= f * z.x;
+				cd[u].y -= f * z.y;
+			}
+		}
 	}
 #pragma unroll
 	for (int u = 0; u < 4; u++) {
