@@ -3,6 +3,7 @@
 #include "qb_kernels.cuh"
 #include "qb_split128.cuh"
 #include "qb_full128.cuh"
+#include "qb_quad128.cuh"
 #include "qb_transport.cuh"
 
 #include <algorithm>
@@ -785,6 +786,42 @@ template <int CS, int NPAIR, class C> void launch_i3_128(const I3ParamsT<C> &p, 
 	}
 	launch128(k_i3_128<CS, NPAIR, C>, "i3_cluster", nclusters * 2 * NPAIR, 2 * NPAIR, smem_i3_128<C>(), s, p, pscr, err);
 }
+int active_quad_clusters() {
+	static DeviceInt cached{-1};
+	if (cached < 0) {
+		check_tmem_coresidency();
+		set_smem(k_i3_quad, Quad128::SMEM);
+		int per_sm = 0;
+		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_i3_quad, Quad128::NT, Quad128::SMEM));
+		if (per_sm * Quad128::TCOLS > 512)
+			QB_FAIL("k_i3_quad: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3(4);
+		cfg.blockDim = dim3(Quad128::NT);
+		cfg.dynamicSmemBytes = Quad128::SMEM;
+		cudaLaunchAttribute attr;
+		attr.id = cudaLaunchAttributeClusterDimension;
+		attr.val.clusterDim.x = 4; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+		cfg.attrs = &attr;
+		cfg.numAttrs = 1;
+		int n = 0;
+		if (cudaOccupancyMaxActiveClusters(&n, k_i3_quad, &cfg) != cudaSuccess || n <= 0) {
+			cudaGetLastError();
+			n = std::max(1, num_sms() / 4);
+		}
+		cached = n;
+	}
+	return cached;
+}
+void launch_i3_quad(const I3ParamsT<double2> &p, const double2 *WhQ, double2 *pscr, double2 *yscr, cudaStream_t s) {
+	active_quad_clusters();                    // attribute + occupancy check
+	launch128(k_i3_quad, "i3_cluster", 4L * p.rg.nslots, 4, Quad128::SMEM, s, p, WhQ, pscr, yscr);
+}
+void launch_b_to_quad(const double2 *in, double2 *out, int ngrids, cudaStream_t s) {
+	ProfScope ps("b_to_quad", s);
+	k_b_to_quad<<<dim3(Quad128::PP / 256, (unsigned)ngrids), 256, 0, s>>>(in, out);
+	QB_CUDA(cudaGetLastError());
+}
 constexpr size_t kFull128Smem = sizeof(float2) * ((size_t)F128::GRID + 128 + 64);
 
 int active_i3_full128_clusters() {
@@ -861,8 +898,7 @@ void check_tmem_coresidency() {
 		{ (const void *)k_i3p<64, double2>, i3p_smem<double2>(), Geo<64>::NT, (int)I3Tmem<double2>::ALLOC, "k_i3p<f64>" },
 		{ (const void *)k_i3p<64, float2>, i3p_smem<float2>(), Geo<64>::NT, (int)I3Tmem<float2>::ALLOC, "k_i3p<f32>" },
 		{ (const void *)k_i3pr<64>, i3pr_smem(), Geo<64>::NT, (int)I3TmemR::ALLOC, "k_i3pr" },
-		{ (const void *)k_i3_128<4, kI3Pairs128, double2>, smem_i3_128<double2>(), G128::NT,
-		  (int)I3Tmem128<double2, 4 / kI3Pairs128>::NCOLS, "k_i3_128<f64>" },
+		{ (const void *)k_i3_quad, Quad128::SMEM, Quad128::NT, Quad128::TCOLS, "k_i3_quad" },
 		{ (const void *)k_i3_128<4, kI3Pairs128, float2>, smem_i3_128<float2>(), G128::NT,
 		  (int)I3Tmem128<float2, 4 / kI3Pairs128>::NCOLS, "k_i3_128<f32>" },
 		{ (const void *)k_i3_128<2, 1, double2>, smem_i3_128<double2>(), G128::NT, (int)I3Tmem128<double2, 2>::NCOLS,
@@ -976,24 +1012,32 @@ template <class C> struct Rhs<128, C> {
 		launch_i2_128(p, units, ws.scr128b.as<C>(), s);
 	}
 
-	// the whole-grid FP32 kernels sum the terms of opposite shifts together
-	// (I3Units), one partial of the Z sums per CTA of their clusters
-	static bool pairs_units() { return sizeof(C) == 8 && use_full128(); }
+	// the terms of opposite shifts are summed together (I3Units), except by the
+	// pair-split FP32 kernel; the whole-grid FP32 kernels leave one partial of the
+	// Z sums per CTA of their 2-CTA clusters
+	static constexpr int kZRanks = sizeof(C) == 8 ? 2 : 1;
+	static bool pairs_units() { return sizeof(C) == 16 || use_full128(); }
 	static int i3_count(const DevI3 &t) {
 		I3Units u;
 		if (pairs_units()) u.M = t.pairM;
 		return u.count(t.nterms);
 	}
 
-	static void i3_sums(Workspace &ws, const DevI3 &t, int ncells, const double2 *W, int nchunk, cudaStream_t s) {
-		const long ncl = (long)ncells * nchunk;
-		ws.i3p.ensure(sizeof(C) * ncl * 4 * PP);
-		ws.scr128a.ensure(sizeof(C) * ncl * 4 * PP);
+	static void i3_sums(Workspace &ws, const DevI3 &t, int ncells, const double2 *W, const Chunks &ch, cudaStream_t s) {
+		const int nchunk = ch.i3;
 		I3ParamsT<C> p{};
 		p.nchunk = nchunk; p.nterms = i3_count(t);
+		long ncl = (long)ncells * nchunk, slots = ncl;
+		if (ch.i3_slots > 0) {
+			p.rg = term_ranges(ch.i3_slots, p.nterms, ncells);
+			ncl = p.rg.nslots;
+			slots = ncl * p.rg.maxc;
+		}
+		ws.i3p.ensure(sizeof(C) * slots * 4 * PP);
+		ws.scr128a.ensure(sizeof(C) * ncl * 4 * PP);
 		if (pairs_units()) {
 			p.un.M = t.pairM;
-			ws.i3z.ensure(sizeof(C) * ncl * 2 * 4 * NN);
+			ws.i3z.ensure(sizeof(C) * slots * kZRanks * 4 * NN);
 			p.zout = ws.i3z.as<C>();
 		}
 		p.src = W; p.src_cell = 4 * NN;
@@ -1025,7 +1069,15 @@ template <class C> struct Rhs<128, C> {
 				return;
 			}
 		}
-		launch_i3_128<4, kI3Pairs128>(p, ncl, ws.scr128a.as<C>(), ws.kerr.as<int>(), s);
+		if constexpr (sizeof(C) == 16) {
+			ws.i3y.ensure(sizeof(C) * ncl * 4 * PP);
+			ws.WhatQ.ensure(sizeof(C) * 4 * ncells * PP);
+			for (int c0 = 0; c0 < 4 * ncells; c0 += 32768)
+				launch_b_to_quad(ws.What.as<C>() + c0 * PP, ws.WhatQ.as<C>() + c0 * PP, std::min(32768, 4 * ncells - c0), s);
+			launch_i3_quad(p, ws.WhatQ.as<C>(), ws.scr128a.as<C>(), ws.i3y.as<C>(), s);
+		} else {
+			launch_i3_128<4, kI3Pairs128>(p, ncl, ws.scr128a.as<C>(), ws.kerr.as<int>(), s);
+		}
 	}
 
 	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, Chunks &ch, cudaStream_t s) {
@@ -1034,7 +1086,10 @@ template <class C> struct Rhs<128, C> {
 		if (q.i1) ch.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), pairs, 64, 0.15);
 		if (q.i2) ch.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), pairs, 64, 0.15);
 		if (q.i3) {
-			const int act = (sizeof(C) == 8 && use_full128()) ? active_i3_full128_clusters() : active_i3_clusters128<C>();
+			if constexpr (sizeof(C) == 16) {
+				if (q.i3->nterms > 0) ch.i3_slots = (int)std::min<long>(active_quad_clusters(), (long)ncells * i3_count(*q.i3));
+			}
+			const int act = sizeof(C) == 16 ? 1 : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
 			ch.i3 = best_chunks((long)ncells, std::max(1, i3_count(*q.i3)), act, 256, 0.15);
 		}
 		scale_chunks(ws, q, ch, q.i3 ? i3_count(*q.i3) : 0);
@@ -1043,18 +1098,21 @@ template <class C> struct Rhs<128, C> {
 		if (parts & RHS_CD) {
 			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch.i1, s);
 			i2_sums(ws, *q.i2, ncells, W, ch.i2, s);
-			i3_sums(ws, *q.i3, ncells, W, ch.i3, s);
+			i3_sums(ws, *q.i3, ncells, W, ch, s);
 		}
 	}
 
-	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, int ncells, cudaStream_t s) {
+	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells, cudaStream_t s) {
 		AsmParamsT<C> a{};
 		a.What = ws.What.as<C>();
 		a.FS = (parts & RHS_CC) ? ws.fs.as<C>() : nullptr;
 		a.FS4 = (parts & RHS_CD) ? ws.fs4.as<C>() : nullptr;
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
-		if (parts & RHS_CD) sum_slots(ws, a, ncells, (long)ncells * ch.i3, 4 * PP, 4 * NN, pairs_units() ? 2 : 0, s);
+		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, i3_count(*q.i3), ncells);
+		a.xquad = sizeof(C) == 16;
+		const long slots = ch.i3_slots > 0 ? (long)ch.i3_slots : (long)ncells * ch.i3;
+		if (parts & RHS_CD) sum_slots(ws, a, ncells, slots, 4 * PP, 4 * NN, pairs_units() ? kZRanks : 0, s);
 		a.s2 = 1.0 / (double)PP;
 		a.s1 = a.s2 * a.s2;
 		return a;
@@ -1063,7 +1121,7 @@ template <class C> struct Rhs<128, C> {
 	static void operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *cc, double2 *cd, cudaStream_t s) {
 		Chunks ch;
 		prepare(ws, q, ncells, W, parts, ch, s);
-		AsmParamsT<C> a = asm_params(ws, parts, ch, ncells, s);
+		AsmParamsT<C> a = asm_params(ws, parts, ch, q, ncells, s);
 		a.mode = 0; a.out_cc = cc; a.out_cd = cd;
 		launch_assemble128(a, ncells, s);
 	}
@@ -1071,7 +1129,7 @@ template <class C> struct Rhs<128, C> {
 	static void update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc, double2 *out, cudaStream_t s) {
 		Chunks ch;
 		prepare(ws, q, ncells, wcur, RHS_ALL, ch, s);
-		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, ncells, s);
+		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, ncells, s);
 		a.mode = 1; a.base = base; a.wcur = wcur; a.B = B; a.dtc = dtc; a.out = out;
 		launch_assemble128(a, ncells, s);
 	}

@@ -85,7 +85,7 @@ struct Workspace {
 	int prec = 64;                           // working precision of the collision operator: 64 (FP64) or 32 (FP32 form)
 	int conserve = 0;                        // restore the collision invariants after each velocity-space collision step
 	cudaStream_t stream = nullptr;           // own stream (upstream API calls)
-	DevBuf What, i1cc, i1i4, i2p, i3p, i3s, i3z, i3zsum, i3zs, i3y, fs, fs4, wmid;      // collision scratch
+	DevBuf What, WhatQ, i1cc, i1i4, i2p, i3p, i3s, i3z, i3zsum, i3zs, i3y, fs, fs4, wmid;      // collision scratch
 	DevBuf fa, fb, va, vb;                   // state scratch (Fourier / velocity)
 	DevBuf io_in, io_out, bext, vgrid;       // staging for host-pointer calls
 	DevBuf aux, aux2;

@@ -1408,6 +1408,7 @@ template <class C> struct AsmParamsT {
 	const C *Qp; int nq;              // [cell][4][nq][P*P] I2 partials, or null
 	const C *Xp; int nx;              // [cell][nx][4][P*P] I3 partials, or null
 	TermRanges xrg;                   // xrg.nslots > 0: Xp holds [slot][4][P*P] partials of term ranges
+	bool xquad;                       // P = 128: Xp in quad order (Quad128) instead of the B layout
 	const C *Zp; int nz;              // extracted I3 sums of the opposite shifts, [slot of Xp][nz][4][N*N], or null
 	double s1, s2;
 	int mode;

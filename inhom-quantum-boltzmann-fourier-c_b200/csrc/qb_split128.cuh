@@ -656,6 +656,9 @@ __device__ __forceinline__ void inverse_extract(C *S, const C *peer, cg::cluster
 	cl.sync();
 }
 
+// quad-order offset (qb_quad128.cuh) of the element at row m of half h (natural row 2 m + h) and column k
+__device__ __forceinline__ long quad_from_b(int h, int m, int k) { return (long)(2 * h + (k & 1)) * 4096 + m * 64 + (k >> 1); }
+
 // K6 (128): assembly of Cc and Cd for one (cell, component j), one CTA pair;
 // same arithmetic as k_assemble (upstream collision.c:95-167, 232-253,
 // simulation.c:75-135), spectra in B layout
@@ -715,7 +718,14 @@ __global__ void __launch_bounds__(512, 1) k_assemble128(const AsmParamsT<C> p) {
 			}
 			if (p.Xp != nullptr) {
 				C s = czero<C>();
-				for (int k = 0; k < p.nx; k++) s = cadd(s, p.Xp[((cell * p.nx + k) * 4 + j) * PP + o]);
+				const long xo = p.xquad ? quad_from_b(h, i >> 7, i & 127) : o;
+				if (p.xrg.nslots > 0) {
+					const TermRanges &g = p.xrg;
+					const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
+					for (int k = k0; k <= k1; k++) s = cadd(s, p.Xp[(((long)k * g.maxc + (cell - g.first_cell(k))) * 4 + j) * PP + xo]);
+				} else {
+					for (int k = 0; k < p.nx; k++) s = cadd(s, p.Xp[((cell * p.nx + k) * 4 + j) * PP + xo]);
+				}
 				z.x -= eta2[j] * s1 * s.x; z.y -= eta2[j] * s1 * s.y;
 			}
 			if (p.FS4 != nullptr) {
