@@ -3,6 +3,7 @@
 #include "qb_kernels.cuh"
 #include "qb_split128.cuh"
 #include "qb_full128.cuh"
+#include "qb_wide64.cuh"
 #include "qb_quad128.cuh"
 #include "qb_transport.cuh"
 
@@ -231,11 +232,11 @@ int best_chunks(long units, int nterms, int slots, int max_chunks, double penalt
 	return best;
 }
 
-template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C *out, cudaStream_t s) {
+template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C *out, cudaStream_t s, C *out2 = nullptr) {
 	static DeviceFlag init;
 	if (!init) { set_smem(k_pad_fft<P, C>, smem_grids<P, C>(1)); init = true; }
 	ProfScope ps("pad_fft", s);
-	k_pad_fft<P, C><<<ngrids, Geo<P>::NT, smem_grids<P, C>(1), s>>>(src, out);
+	k_pad_fft<P, C><<<ngrids, Geo<P>::NT, smem_grids<P, C>(1), s>>>(src, out, out2);
 	QB_CUDA(cudaGetLastError());
 }
 
@@ -388,6 +389,51 @@ template <class C> int active_i3p_clusters() {
 		cached = n;
 	}
 	return cached;
+}
+
+int active_i3w_clusters() {
+	static DeviceInt cached{-1};
+	if (cached < 0) {
+		check_tmem_coresidency();
+		auto kern = k_i3w<double2>;
+		const size_t smem = i3w_smem<double2>();
+		set_smem(kern, smem);
+		int per_sm = 0;
+		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, smem));
+		if (per_sm * (int)WideTmem::COLS > 512)
+			QB_FAIL("k_i3w: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3(2);
+		cfg.blockDim = dim3(512);
+		cfg.dynamicSmemBytes = smem;
+		cudaLaunchAttribute attr;
+		attr.id = cudaLaunchAttributeClusterDimension;
+		attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+		cfg.attrs = &attr;
+		cfg.numAttrs = 1;
+		int n = 0;
+		if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+			cudaGetLastError();
+			n = std::max(1, num_sms() / 2);
+		}
+		cached = n;
+	}
+	return cached;
+}
+void launch_i3w(const I3ParamsT<double2> &p, long nclusters, double2 *pscr, cudaStream_t s) {
+	active_i3w_clusters();                     // attribute + occupancy check
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3((unsigned)(nclusters * 2));
+	cfg.blockDim = dim3(512);
+	cfg.dynamicSmemBytes = i3w_smem<double2>();
+	cfg.stream = s;
+	cudaLaunchAttribute attr;
+	attr.id = cudaLaunchAttributeClusterDimension;
+	attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	ProfScope ps("i3_cluster", s);
+	QB_CUDA(cudaLaunchKernelEx(&cfg, k_i3w<double2>, p, pscr));
 }
 
 template <class C> void launch_i3p(const I3ParamsT<C> &p, long nclusters, const int *kind, cudaStream_t s) {
@@ -546,7 +592,12 @@ template <int P, class C> struct Rhs {
 	// spectra of the four components
 	static void spectra(Workspace &ws, int ncells, const double2 *W, cudaStream_t s) {
 		ws.What.ensure(sizeof(C) * 4 * ncells * PP);
-		launch_pad_fft<P>(4 * ncells, W, ws.What.as<C>(), s);
+		C *wide = nullptr;                      // the copy that k_i3w reads
+		if (P == 64 && sizeof(C) == 16) {
+			ws.WhatQ.ensure(sizeof(C) * 4 * ncells * PP);
+			wide = ws.WhatQ.as<C>();
+		}
+		launch_pad_fft<P>(4 * ncells, W, ws.What.as<C>(), s, wide);
 	}
 
 	// S sums for Cc (tasks g = W_1..W_3, F = -4 W^_0 + 2) or I4 (g = W_0..W_3, F = 2 W^_0 - 1)
@@ -631,7 +682,14 @@ template <int P, class C> struct Rhs {
 					return;
 				}
 			}
-			launch_i3p<C>(p, p.rg.nslots > 0 ? (long)p.rg.nslots : (long)ncells * nchunk, nullptr, s);
+			if constexpr (sizeof(C) == 16) {
+				const long ncl = p.rg.nslots > 0 ? (long)p.rg.nslots : (long)ncells * nchunk;
+				ws.i3y.ensure(sizeof(C) * ncl * 8 * PP);
+				p.Ghat = ws.WhatQ.as<C>();
+				launch_i3w(p, ncl, ws.i3y.as<C>(), s);
+			} else {
+				launch_i3p<C>(p, (long)ncells * nchunk, nullptr, s);
+			}
 		} else {
 			if constexpr (P == 32 && sizeof(C) == 8) {
 				if (ws.i3_variant == 1) {
@@ -655,7 +713,7 @@ template <int P, class C> struct Rhs {
 		// of the (cell, term) work, one partial per cell it touches
 		const bool ranges = ws.i3_ranges >= 0 ? ws.i3_ranges == 1 : term_ranges_enabled();
 		if (P == 64 && sizeof(C) == 16 && q.i3 && q.i3->nterms > 0 && ranges)
-			ch.i3_slots = (int)std::min<long>(active_i3p_clusters<C>(), (long)ncells * i3_count(ws, *q.i3));
+			ch.i3_slots = (int)std::min<long>(active_i3w_clusters(), (long)ncells * i3_count(ws, *q.i3));
 		spectra(ws, ncells, W, s);
 		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s);
 		if (parts & RHS_CD) {
@@ -895,7 +953,7 @@ void check_tmem_coresidency() {
 	static DeviceFlag done;
 	if (done) return;
 	std::vector<TmemKernel> ks = {
-		{ (const void *)k_i3p<64, double2>, i3p_smem<double2>(), Geo<64>::NT, (int)I3Tmem<double2>::ALLOC, "k_i3p<f64>" },
+		{ (const void *)k_i3w<double2>, i3w_smem<double2>(), 512, (int)WideTmem::COLS, "k_i3w" },
 		{ (const void *)k_i3p<64, float2>, i3p_smem<float2>(), Geo<64>::NT, (int)I3Tmem<float2>::ALLOC, "k_i3p<f32>" },
 		{ (const void *)k_i3pr<64>, i3pr_smem(), Geo<64>::NT, (int)I3TmemR::ALLOC, "k_i3pr" },
 		{ (const void *)k_i3_quad, Quad128::SMEM, Quad128::NT, Quad128::TCOLS, "k_i3_quad" },
@@ -1186,7 +1244,7 @@ Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) 
 		switch (N) {
 		case 8: act = f32 ? active_i3q<16, float2>() : active_i3q<16, double2>(); break;
 		case 16: act = f32 ? active_i3q<32, float2>() : active_i3q<32, double2>(); break;
-		default: act = f32 ? active_i3p_clusters<float2>() : active_i3p_clusters<double2>(); break;
+		default: act = f32 ? active_i3p_clusters<float2>() : active_i3w_clusters(); break;
 		}
 		// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written
 		// and read back at HBM speed; one term takes a cluster ~36 us there: 0.15

@@ -145,9 +145,10 @@ __device__ __forceinline__ void smem_to_global(C *__restrict__ out, const C *S) 
 }
 
 // ---------------------------------------------------------------------------
-// K1: padded forward spectra  out[b] = FFT2(Pad(src[b]))   (one CTA per grid)
+// K1: padded forward spectra  out[b] = FFT2(Pad(src[b]))   (one CTA per grid);
+// out2 (may be null, P = 64): the same in the thread order of k_i3w
 template <int P, class C>
-__global__ void __launch_bounds__(Geo<P>::NT) k_pad_fft(const double2 *__restrict__ src, C *__restrict__ out) {
+__global__ void __launch_bounds__(Geo<P>::NT) k_pad_fft(const double2 *__restrict__ src, C *__restrict__ out, C *__restrict__ out2) {
 	using G = Geo<P, C>;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	C *S = reinterpret_cast<C *>(smem_raw), *tw = S + G::GRID;
@@ -156,6 +157,8 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_pad_fft(const double2 *__restric
 	const long b = blockIdx.x;
 	fft2_pad<P, -1>(S, tw, src + b * G::N * G::N, MulNone<C>{});
 	smem_to_global<P>(out + b * P * P, S);
+	if (P == 64 && out2 != nullptr)
+		for (int i = threadIdx.x; i < P * P; i += G::NT) out2[b * P * P + i] = S[G::at((i & 255) >> 2, (i & 3) + 4 * (i >> 8))];
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,374 @@
+// qb_wide64.cuh — 64 x 64 transforms with 16 values a thread, and the I3 sums
+// at N = 32 built on them.
+//
+// A group of 256 threads holds a 64 x 64 complex grid, 16 values a thread, and
+// transforms it in three register stages with two exchanges through shared
+// memory instead of the four stages and three exchanges of 8 values a thread.
+// Inverse transform of a(l, k):
+//   A  thread (l, tau), values k = tau + 4 r:             DFT16 over r -> q
+//   B  thread (q, lam), values (l = lam + 16 s, tau):     x w64^(tau q), DFT4 over
+//      tau -> p and over s -> u, x w64^(lam u)
+//   C  thread (q + 16 p, u), values lam:                  DFT16 over lam -> v
+// gives b(u + 4 v, q + 16 p); the forward transform is the mirror image (C, B,
+// A with the same twiddles) and returns to the positions of A.  Every stage
+// writes its results to the slots it read, so an exchange costs one barrier of
+// the group, and a transform that starts at the positions where the last one
+// ended needs none before it.
+//
+// Shared grid: slot(row, col) = 64 row + (col ^ sw(row)), sw = bits (0, 2, 1) of
+// the row; with 16-byte values every access of the three stages is free of
+// bank conflicts without padding (eight lanes of A: two rows x four
+// consecutive columns, of B: eight consecutive rows, of C: eight consecutive
+// columns).
+#pragma once
+#include "qb_kernels.cuh"
+
+namespace qb {
+
+// 16-point DFT in registers: natural order in, frequency f in x[pos16(f)]
+__host__ __device__ constexpr int pos16(int f) { return (f & 3) * 4 + (f >> 2); }
+template <int DIR, class C> __device__ __forceinline__ void dft16(C (&x)[16]) {
+	using R = typename CT<C>::R;
+	constexpr double a = 0.92387953251128675613, b = 0.38268343236508977173;
+#pragma unroll
+	for (int n = 0; n < 4; n++) dft4<DIR>(x[n], x[n + 4], x[n + 8], x[n + 12]);
+	// x[n + 4 k] holds partial frequency k of residue n: times w16^(n k)
+	C w1, w3;
+	w1.x = (R)a; w1.y = (R)(DIR < 0 ? -b : b);
+	w3.x = (R)b; w3.y = (R)(DIR < 0 ? -a : a);
+	x[5] = cmul(x[5], w1);
+	x[6] = mul_w8<DIR>(x[6]);
+	x[7] = cmul(x[7], w3);
+	x[9] = mul_w8<DIR>(x[9]);
+	x[10] = mul_i<DIR>(x[10]);
+	x[11] = mul_w8_3<DIR>(x[11]);
+	x[13] = cmul(x[13], w3);
+	x[14] = mul_w8_3<DIR>(x[14]);
+	C w9; w9.x = -w1.x; w9.y = -w1.y;                        // w16^9 = -w16
+	x[15] = cmul(x[15], w9);
+#pragma unroll
+	for (int k = 0; k < 4; k++) dft4<DIR>(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
+	// frequency k + 4 m is in x[4 k + m]
+}
+
+template <class C> struct Wide64 {
+	static constexpr int GT = 256;           // threads of a group
+	C *U;                                    // the group's grid
+	const C *tw;                             // w64^e, e < 64, forward sign
+	int t, bar;                              // thread of the group, its named barrier
+	__device__ __forceinline__ static int sw(int row) { return ((row & 1) << 2) | ((row >> 1) & 3); }
+	__device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(GT) : "memory"); }
+	// A: this thread's row and first column
+	__device__ __forceinline__ int row_a() const { return t >> 2; }
+	__device__ __forceinline__ int col_a() const { return t & 3; }
+	// C: this thread's column as a frequency / grid index and its first row (rows u + 4 v)
+	__device__ __forceinline__ int col_c() const { const int c = t & 63; return (c >> 2) + 16 * (c & 3); }
+	__device__ __forceinline__ int row_c() const { return t >> 6; }
+
+	// slots of A: index q (columns tau + 4 q)
+	template <class F> __device__ __forceinline__ void slots_a(const F &f) const {
+		const int l = t >> 2, s = sw(l), b0 = l * 64 + ((t & 3) ^ s), b1 = l * 64 + (((t & 3) + 4) ^ s);
+#pragma unroll
+		for (int q = 0; q < 16; q++) f(q, U[((q & 1) ? b1 : b0) + 8 * (q >> 1)]);
+	}
+	// slots of B: index (s or u, tau or p)
+	template <class F> __device__ __forceinline__ void slots_b(const F &f) const {
+		const int q = t >> 4, lam = t & 15, s = sw(lam), b = lam * 64 + 8 * (q >> 1), h = 4 * (q & 1);
+#pragma unroll
+		for (int c = 0; c < 4; c++) {
+			const int a = b + ((c + h) ^ s);
+#pragma unroll
+			for (int r = 0; r < 4; r++) f(r, c, U[a + 16 * 64 * r]);
+		}
+	}
+	// slots of C: index lam
+	template <class F> __device__ __forceinline__ void slots_c(const F &f) const {
+		const int c = t & 63, b = (t >> 6) * 16 * 64;
+#pragma unroll
+		for (int m = 0; m < 16; m++) f(m, U[b + m * 64 + (c ^ sw(m))]);
+	}
+	// B of both directions: times w64^(c q) (inverse) or w64^(r lam) (forward), DFT4s, times the other
+	template <int DIR> __device__ __forceinline__ void stage_b() const {
+		const int q = t >> 4, lam = t & 15;
+		C y[4][4];
+		slots_b([&](int r, int c, const C &v) { y[r][c] = v; });
+		C wq[3], wl[3];
+#pragma unroll
+		for (int m = 0; m < 3; m++) {
+			wq[m] = tw[(m + 1) * q];
+			wl[m] = tw[(m + 1) * lam];
+			if (DIR > 0) { wq[m].y = -wq[m].y; wl[m].y = -wl[m].y; }
+		}
+		if (DIR > 0) {
+#pragma unroll
+			for (int r = 0; r < 4; r++)
+#pragma unroll
+				for (int c = 1; c < 4; c++) y[r][c] = cmul(y[r][c], wq[c - 1]);
+		} else {
+#pragma unroll
+			for (int r = 1; r < 4; r++)
+#pragma unroll
+				for (int c = 0; c < 4; c++) y[r][c] = cmul(y[r][c], wl[r - 1]);
+		}
+#pragma unroll
+		for (int r = 0; r < 4; r++) dft4<DIR>(y[r][0], y[r][1], y[r][2], y[r][3]);
+#pragma unroll
+		for (int c = 0; c < 4; c++) dft4<DIR>(y[0][c], y[1][c], y[2][c], y[3][c]);
+		if (DIR > 0) {
+#pragma unroll
+			for (int r = 1; r < 4; r++)
+#pragma unroll
+				for (int c = 0; c < 4; c++) y[r][c] = cmul(y[r][c], wl[r - 1]);
+		} else {
+#pragma unroll
+			for (int r = 0; r < 4; r++)
+#pragma unroll
+				for (int c = 1; c < 4; c++) y[r][c] = cmul(y[r][c], wq[c - 1]);
+		}
+		slots_b([&](int r, int c, C &v) { v = y[r][c]; });
+	}
+	// x[r] = a(row_a, col_a + 4 r) -> x[pos16(v)] = b(row_c + 4 v, col_c)
+	__device__ __forceinline__ void inverse(C (&x)[16]) const {
+		dft16<+1>(x);
+		slots_a([&](int q, C &v) { v = x[pos16(q)]; });
+		sync();
+		stage_b<+1>();
+		sync();
+		slots_c([&](int m, const C &v) { x[m] = v; });
+		dft16<+1>(x);
+	}
+	// x[v] = b(row_c + 4 v, col_c) -> x[pos16(r)] = a(row_a, col_a + 4 r)
+	__device__ __forceinline__ void forward(C (&x)[16]) const {
+		dft16<-1>(x);
+		slots_c([&](int m, C &v) { v = x[pos16(m)]; });
+		sync();
+		stage_b<-1>();
+		sync();
+		slots_a([&](int q, const C &v) { x[q] = v; });
+		dft16<-1>(x);
+	}
+};
+
+// tensor memory of a thread of k_i3w: 16 accumulators, then 16 values of P_j,
+// value r at word 4 r (FP64); four warps share a lane quarter
+struct WideTmem {
+	static constexpr unsigned COLS = 512;
+	__device__ __forceinline__ static unsigned x(unsigned base) {
+		const unsigned w = threadIdx.x >> 5;
+		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * 128u;
+	}
+	__device__ __forceinline__ static unsigned p(unsigned base) { return x(base) + 64u; }
+};
+template <class C> constexpr size_t i3w_smem() {
+	// two grids, the Y values in transit, psi2 (16 reals a thread of a group), the twiddles
+	return sizeof(C) * (3 * 4096 + 64) + sizeof(typename CT<C>::R) * 4096;
+}
+
+// K4w: the I3 sums of the collision operator at N = 32 on a cluster of 2 CTAs
+// of two groups, group g of CTA r for component j = 2 r + g.  Per unit
+// (I3Units) a group writes P_j to the cluster's scratch in L2 and keeps it in
+// tensor memory; after a cluster barrier it runs the chains of i = 0..3:
+//   X_j += eta_i P_i . T_ij  (tensor memory),  y = eta_j W^_j . T_ij.
+// Y_i of the CTA's two components goes to group i % 2 (through shared memory)
+// which adds conj(psi1) . Extract(IFFT2(Y_i)) to the CTA's partial of Z_i.  The
+// groups meet at that hand-over and at the cluster barrier only.  Ghat (W^) and
+// pscr are in thread order (value r of thread t of A at 256 r + t): a warp's
+// load is four full lines, where the natural order gives eight half lines and
+// twice the cycles of the shared-memory and L1 pipe, which bounds this kernel.
+// Measured (64 cells, J = M = 16, FP64): the Strang step 17.7 ms with k_i3p (8
+// values a thread, FP64 pipe 42%, shared-memory pipe 72%), 16.2 ms with 16
+// values in the natural order, 15.5 ms in thread order.
+// out: [slot][4][PP], zout: [slot][rank][4][N*N], slots of the term ranges (or
+// (cell, chunk)); pscr: [cluster][2][4][PP] (two units in turn: one cluster
+// barrier a unit).
+template <class C>
+__global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
+	using R = typename CT<C>::R;
+	using TM = WideTmem;
+	constexpr int N = 32, NN = N * N, P = 64, PP = P * P, GT = 256;
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	__shared__ unsigned tmem_slot;
+	C *grids = reinterpret_cast<C *>(smem_raw), *Yb = grids + 2 * PP, *tw = Yb + PP;
+	R *psi = reinterpret_cast<R *>(tw + 64);
+	cg::cluster_group cl = cg::this_cluster();
+	const int rank = (int)cl.block_rank();
+	const int cid = (int)(blockIdx.x / 2);
+	const int g = threadIdx.x / GT, t = threadIdx.x % GT, warp = threadIdx.x >> 5;
+	if (warp == 0) tmem_alloc(&tmem_slot, TM::COLS);
+	init_twiddles<64>(tw);
+	tmem_fence_before();
+	__syncthreads();
+	tmem_fence_after();
+	const unsigned tx = TM::x(tmem_slot), tp = TM::p(tmem_slot);
+	const Wide64<C> F{ grids + g * PP, tw, t, g + 1 };
+	const int j = 2 * rank + g;
+	const R etaj = (R)(j == 0 ? 1.0 : -1.0);
+	const int oa = F.row_a() * P + F.col_a();                // element of A (+ 4 r)
+	const int kc = F.col_c(), ks = kc < N / 2 ? kc : (kc >= 3 * N / 2 ? kc - N : -1);
+	const int oz = F.row_c() * N + ks;                       // N-grid element of C: rows u + 4 v (v < 4), u + 4 v - 32 (v >= 12)
+	C *Pall = pscr + (long)cid * 8 * PP + t;
+	Yb += t;
+	int psi_idx = -1, par = 0;
+	long u, u1;
+	if (p.rg.nslots > 0) {
+		u = p.rg.start(cid);
+		u1 = p.rg.start(cid + 1);
+	} else {
+		const int chunk = (int)(cid % p.nchunk);
+		const long cell = cid / p.nchunk;
+		u = cell * p.nterms + (long)chunk * p.nterms / p.nchunk;
+		u1 = cell * p.nterms + (long)(chunk + 1) * p.nterms / p.nchunk;
+	}
+	// one segment per cell of the range (the (cell, chunk) grid has one)
+#pragma unroll 1
+	while (u < u1) {
+		const long cell = u / p.nterms;
+		const int t0 = (int)(u % p.nterms);
+		const int t1 = (int)min((long)p.nterms, t0 + (u1 - u));
+		u += t1 - t0;
+		const long slot = p.rg.nslots > 0 ? (long)cid * p.rg.maxc + (cell - p.rg.first_cell(cid))
+		                                  : cell * p.nchunk + (int)(cid % p.nchunk);
+		const C *Wc = p.Ghat + cell * p.g_cell + t;
+		const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[j] * NN + oz;
+		C *Zo = p.zout + (slot * 2 + rank) * 4 * (long)NN + oz;
+		{
+			const C z[4] = { czero<C>(), czero<C>(), czero<C>(), czero<C>() };
+#pragma unroll
+			for (int h = 0; h < 4; h++) tmem_st4(tx + 16 * h, z);
+			tmem_wait_st();
+			if (ks >= 0) {
+#pragma unroll 1
+				for (int i = g; i < 4; i += 2)
+#pragma unroll
+					for (int v = 0; v < 8; v++) Zo[i * NN + 4 * v * N] = czero<C>();
+			}
+		}
+#pragma unroll 1
+		for (int un = t0; un < t1; un++) {
+			const int term = p.un.term(un);
+			const bool pr = p.un.pair(un);
+			const C *psi1 = p.psi1 + (long)term * NN + oz;
+			C *Pu = Pall + par * 4 * PP;
+			par ^= 1;
+			C x[16];
+			F.sync();                                        // the last chain's rows are read
+			// P_j = FFT2(Pad(psi1 . W_j))
+#pragma unroll
+			for (int v = 0; v < 16; v++) x[v] = czero<C>();
+			if (ks >= 0) {
+#pragma unroll
+				for (int v = 0; v < 8; v++) {
+					const double2 w = src[4 * v * N];
+					x[v < 4 ? v : v + 8] = cmul(psi1[4 * v * N], mk<C>(w.x, w.y));
+				}
+			}
+			F.forward(x);
+#pragma unroll
+			for (int h = 0; h < 4; h++) {
+				C a[4];
+#pragma unroll
+				for (int r = 0; r < 4; r++) {
+					a[r] = x[pos16(4 * h + r)];
+					__stcg(Pu + j * PP + GT * (4 * h + r), a[r]);
+				}
+				tmem_st4(tp + 16 * h, a);
+			}
+			tmem_wait_st();
+			cl.sync();                                       // the unit's P grids are in L2
+			if (p.psi2_idx[term] != psi_idx) {               // a new angle: its psi2 in the order of C
+				psi_idx = p.psi2_idx[term];
+				const R *s = p.psi2T + (long)psi_idx * PP + kc * P + F.row_c();
+#pragma unroll
+				for (int v = 0; v < 8; v++) psi[(8 * g + v) * GT + t] = s[4 * (8 * g + v)];
+				__syncthreads();
+			}
+			const R sc = (R)p.psi2_scale[term];
+#pragma unroll 1
+			for (int i = 0; i < 4; i++) {
+				const C *Wi = Wc + i * PP;
+#pragma unroll
+				for (int r = 0; r < 16; r++) x[r] = Wi[GT * r];
+#pragma unroll
+				for (int h = 0; h < 4; h++) {
+					C a[4];
+					tmem_ld4(tp + 16 * h, a);
+					tmem_wait_ld();
+#pragma unroll
+					for (int r = 0; r < 4; r++) x[4 * h + r] = cmul(x[4 * h + r], a[r]);
+				}
+				F.inverse(x);
+				{
+					C y[16];
+#pragma unroll
+					for (int v = 0; v < 16; v++) y[v] = cscale(x[pos16(v)], psi[v * GT + t]);
+#pragma unroll
+					for (int v = 0; v < 16; v++) x[v] = y[v];
+				}
+				F.forward(x);
+				// X_j += eta_i P_i . T_ij (psi2's scale applied here)
+				const C *Pi = Pu + i * PP;
+				const R ci = i == 0 ? sc : -sc;
+#pragma unroll
+				for (int h = 0; h < 4; h++) {
+					C a[4], w[4];
+#pragma unroll
+					for (int r = 0; r < 4; r++) w[r] = __ldcg(Pi + GT * (4 * h + r));
+					tmem_ld4(tx + 16 * h, a);
+					tmem_wait_ld();
+#pragma unroll
+					for (int r = 0; r < 4; r++) {
+						const C v = cmul(w[r], x[pos16(4 * h + r)]);
+						a[r].x += ci * v.x;
+						a[r].y += ci * v.y;
+					}
+					tmem_st4(tx + 16 * h, a);
+				}
+				if (pr) {
+					// y = eta_j W^_j . T_ij; the group of i % 2 takes the sum of both
+					const C *Wj = Wc + j * PP;
+					const R cj = etaj * sc;
+					const int hand = 3 + (i & 1);
+#pragma unroll
+					for (int r = 0; r < 16; r++) x[pos16(r)] = cscale(cmul(Wj[GT * r], x[pos16(r)]), cj);
+					if ((i & 1) != g) {
+#pragma unroll
+						for (int r = 0; r < 16; r++) Yb[r * GT] = x[pos16(r)];
+						asm volatile("bar.arrive %0, 512;" ::"r"(hand) : "memory");
+					} else {
+						asm volatile("bar.sync %0, 512;" ::"r"(hand) : "memory");
+						C y[16];
+#pragma unroll
+						for (int r = 0; r < 16; r++) y[r] = cadd(Yb[r * GT], x[pos16(r)]);
+						F.inverse(y);
+						F.sync();                                // the next chain writes rows
+						if (ks >= 0) {
+							C *z = Zo + i * NN;
+#pragma unroll
+							for (int v = 0; v < 8; v++) {
+								C w = psi1[4 * v * N];
+								w.y = -w.y;
+								z[4 * v * N] = cfma(w, y[pos16(v < 4 ? v : v + 8)], z[4 * v * N]);
+							}
+						}
+					}
+				}
+				tmem_wait_st();
+			}
+		}
+		C *o = p.out + (slot * 4 + j) * (long)PP + oa;
+#pragma unroll
+		for (int h = 0; h < 4; h++) {
+			C a[4];
+			tmem_ld4(tx + 16 * h, a);
+			tmem_wait_ld();
+#pragma unroll
+			for (int r = 0; r < 4; r++) o[4 * (4 * h + r)] = a[r];
+		}
+	}
+	tmem_fence_before();
+	__syncthreads();
+	tmem_fence_after();
+	if (warp == 0) tmem_dealloc(tmem_slot, TM::COLS);
+}
+
+}  // namespace qb
