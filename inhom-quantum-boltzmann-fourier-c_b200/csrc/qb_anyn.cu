@@ -420,6 +420,14 @@ template <class V, class Ld, class St> __device__ __forceinline__ void batched(i
 }
 template <class C> struct Two { C a, b; };
 
+// Terms of a wave of the I3 sums: unit t0 + tt of I3Units (qb_kernels.cuh; the
+// pairs of opposite shifts of FourierI3 come from the chains of one of them)
+struct WaveUnits {
+	int M;                                // terms an angle, 0: every unit is one term
+	__device__ __forceinline__ int term(int u) const { return M > 0 ? u / ((M + 1) / 2) * M + u % ((M + 1) / 2) : u; }
+	__device__ __forceinline__ bool pair(int u) const { return M > 0 && 2 * (u % ((M + 1) / 2)) != M - 1; }
+};
+
 // rows of Pad(mult . W_comp) for unit u = (cell nt + tt) nsub + sub, forward
 // transform: out[u] (row pass of the spectra, of P_j and of the first
 // transforms of the I1 / I2 terms).  psel: 0 no factor, 1 / 2 real table A / B
@@ -431,6 +439,7 @@ template <class C> struct PadRowsP {
 	int comp[8], psel[8], comp2[8];      // psel 4: psiC . (W_comp + i W_comp2)
 	const R *psiA, *psiB;                 // real N x N tables, one per term
 	const C *psiC;                        // complex N x N tables, one per term
+	WaveUnits un;                         // terms of psiC
 	C *out;
 	// kind != null: the cells of kind 0 (real form) take the first nsub_rf
 	// subs with comp_rf / comp2_rf / psel_rf instead
@@ -450,7 +459,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	const int l0 = (int)(blockIdx.x % bpg) * nl;
 	const int sub = (int)(u % p.nsub);
 	const long ct = u / p.nsub;
-	const int t = p.t0 + (int)(ct % p.nt);
+	const int t = p.un.term(p.t0 + (int)(ct % p.nt));
 	const long cell = ct / p.nt;
 	int ps = p.psel[sub], ca = p.comp[sub], cb = p.comp2[sub];
 	if (p.kind != nullptr && p.kind[cell] == 0) {
@@ -754,6 +763,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 template <class C> struct I3ColsP {
 	using R = typename CT<C>::R;
 	C *Y; const R *psi2T; const int *idx; const double *scale; int N, nl, nt, t0;
+	WaveUnits un;
 	const int *kind;                      // null: every cell complex; kind 0: units c >= 8 idle
 	Plan pl;
 };
@@ -767,7 +777,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads, p
 	const long u = blockIdx.x / bpg;
 	const int k0 = (int)(blockIdx.x % bpg) * nl;
 	const int ct = (int)(u >> 4);                                  // (cell, term) of the wave: below 2^31
-	const int cell = ct / p.nt, t = p.t0 + (ct - cell * p.nt);
+	const int cell = ct / p.nt, t = p.un.term(p.t0 + (ct - cell * p.nt));
 	if (p.kind != nullptr && p.kind[cell] == 0 && (u & 15) >= 8) return;
 	load_tw(T.tw, P, p.pl);
 	// columns k0 + line of the chain grid, element i = row i: the first
@@ -810,7 +820,8 @@ inline int own_for_plan(const Plan &pl, bool fp64) {
 	}
 }
 template <class C> struct I3RowsBP {
-	const C *Y, *Pg; C *X; int N, nl, nt;
+	C *Y; const C *Pg; C *X; int N, nl, nt, t0;
+	WaveUnits un;                         // the rows of a pair's chains are kept in Y for k_any_i3_rows_y
 	const int *kind;                      // null: every cell complex
 	Plan pl;
 };
@@ -841,7 +852,8 @@ template <class C, bool RF, int R1, int R2> __device__ __forceinline__ void i3_r
 		const long ct = cell * p.nt + tt;
 		constexpr int kH = RF ? 2 : 4;
 		for (int h = 0; h < kH; h++) {
-			const C *y = p.Y + (ct * 16 + j3 * kH + h) * PP + (long)l0 * P;
+			C *y = p.Y + (ct * 16 + j3 * kH + h) * PP + (long)l0 * P;
+			const bool keep = p.un.pair(p.t0 + tt);
 			const int pitch = T.pitch;
 			auto ld0 = [y, P](int line, int i) { return y[(long)line * P + i]; };
 			auto st1 = [pitch](int line, int i, const C &v, C *out) { out[tat(line, i, pitch)] = v; };
@@ -855,8 +867,9 @@ template <class C, bool RF, int R1, int R2> __device__ __forceinline__ void i3_r
 					const int i = threadIdx.x + e * kThreads;
 					if (i < ne) {
 						const int li = fdiv(i, mgP), k = i - li * P;
-						const C pa = Pa[i], y = r[T.at(li, k)];
-						acc[e].x += e0 * (pa.x * y.x) - pa.y * y.y;
+						const C pa = Pa[i], v = r[T.at(li, k)];
+						acc[e].x += e0 * (pa.x * v.x) - pa.y * v.y;
+						if (keep) y[i] = v;
 					}
 				}
 			} else {
@@ -867,9 +880,10 @@ template <class C, bool RF, int R1, int R2> __device__ __forceinline__ void i3_r
 					const int i = threadIdx.x + e * kThreads;
 					if (i < ne) {
 						const int li = fdiv(i, mgP), k = i - li * P;
-						const C v = cmul(Pa[i], r[T.at(li, k)]);
+						const C t = r[T.at(li, k)], v = cmul(Pa[i], t);
 						acc[e].x += eta * v.x;
 						acc[e].y += eta * v.y;
+						if (keep) y[i] = t;
 					}
 				}
 			}
@@ -898,6 +912,119 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads, r
 	i3_rows_b<C, false, R1, R2>(p, sm);
 }
 
+// The other term of a pair, rows: Y_i = sum_j eta_j W^_j . T_ij of the rows that
+// k_any_i3_rows_b left in Y (unit (cell nt + tt) 4 + i), inverse transform into
+// V[unit].  Real form: unit i < 2 takes the packed chains, Y_2i + i Y_2i+1 =
+// sum_j eta_j W^_j . T (W^_j real), and i >= 2 is idle.
+template <class C> struct I3RowsYP {
+	const C *What, *Y; C *V; int N, nl, nt, t0;
+	WaveUnits un;
+	const int *kind;
+	Plan pl;
+};
+template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k_any_i3_rows_y(const I3RowsYP<C> p) {
+	using R = typename CT<C>::R;
+	extern __shared__ __align__(16) unsigned char sm[];
+	const int P = 2 * p.N, nl = p.nl;
+	const long PP = (long)P * P;
+	Tile<C> T(sm, P, nl);
+	const unsigned mgP = magic_div((unsigned)P);
+	const int bpg = P / nl;
+	const long u = blockIdx.x / bpg;
+	const int l0 = (int)(blockIdx.x % bpg) * nl;
+	const int i3 = (int)(u & 3);
+	const long ct = u >> 2, cell = ct / p.nt;
+	const bool rf = has_rf<C>() && p.kind != nullptr && p.kind[cell] == 0;
+	if ((rf && i3 >= 2) || !p.un.pair(p.t0 + (int)(ct % p.nt))) return;
+	load_tw(T.tw, P, p.pl);
+	const C *W = p.What + cell * 4 * PP + (long)l0 * P, *y = p.Y + ct * 16 * PP + (long)l0 * P;
+	batched<C>(nl * P, [&](int i) {
+		C s = czero<C>();
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+			const R eta = j == 0 ? (R)1 : (R)-1;
+			const C w = W[j * PP + i], t = rf ? y[(2 * j + i3) * PP + i] : y[(4 * j + i3) * PP + i];
+			if (rf) {
+				s.x += eta * w.x * t.x;
+				s.y += eta * w.x * t.y;
+			} else {
+				const C v = cmul(w, t);
+				s.x += eta * v.x;
+				s.y += eta * v.y;
+			}
+		}
+		return s;
+	}, [&](int i, const C &v) {
+		const int li = fdiv(i, mgP), k = i - li * P;
+		T.b[T.at(li, k)] = v;
+	});
+	__syncthreads();
+	C *o = p.V + u * PP + (long)l0 * P;
+	const int pitch = T.pitch;
+	const C *sb = T.b;
+	auto ld0 = [sb, pitch](int line, int i) { return sb[tat(line, i, pitch)]; };
+	auto st1 = [o, P](int line, int i, const C &v, C *) { o[(long)line * P + i] = v; };
+	fft_fx<R1, R2, +1, false, false>(nl, pitch, p.pl, T.tw, T.a, T.b, ld0, st1);
+}
+
+// The other term of a pair, columns: inverse transform of the columns of V and
+// Z[cell][i](k) += conj(psi1_t(k)) . them on the frequencies -N/2 .. N/2 of both
+// dimensions (Z: (N + 1)^2 values, the upper end only in the real form, which
+// needs it to separate the two packed sums; there i < 2).  One CTA per (cell,
+// i, block of nl columns of those N + 1) adds the wave's terms in order.
+template <class C> struct I3ColsZP {
+	const C *V; C *Z; const C *psi1; int N, nl, nt, t0;
+	WaveUnits un;
+	const int *kind;
+	Plan pl;
+};
+template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k_any_i3_cols_z(const I3ColsZP<C> p) {
+	extern __shared__ __align__(16) unsigned char sm[];
+	const int N = p.N, H = N / 2, P = 2 * N, nl = p.nl, ZS = N + 1;
+	const long PP = (long)P * P;
+	Tile<C> T(sm, P, nl);
+	const int bpg = (ZS + nl - 1) / nl;
+	const long ci = blockIdx.x / bpg;             // cell 4 + i
+	const int z0 = (int)(blockIdx.x % bpg) * nl;     // first column, as frequency + N/2
+	const long cell = ci / 4;
+	const int i3 = (int)(ci % 4);
+	const bool rf = has_rf<C>() && p.kind != nullptr && p.kind[cell] == 0;
+	if (rf && i3 >= 2) return;
+	load_tw(T.tw, P, p.pl);
+	const int nz = min(nl, (rf ? ZS : N) - z0);       // columns of this block
+	if (nz <= 0) return;
+	C *Z = p.Z + ci * (long)ZS * ZS;
+	const int pitch = T.pitch;
+	const unsigned mgnl = magic_div((unsigned)nl);
+	for (int tt = 0; tt < p.nt; tt++) {
+		if (!p.un.pair(p.t0 + tt)) continue;
+		const C *v = p.V + ((cell * p.nt + tt) * 4 + i3) * PP;
+		const C *ps = p.psi1 + (long)p.un.term(p.t0 + tt) * N * N;
+		auto ld0 = [v, P, H, z0, nz](int line, int i) {
+			const int f = z0 + min(line, nz - 1) - H;
+			return v[(long)i * P + (f < 0 ? f + P : f)];
+		};
+		auto st_s = [pitch](int line, int i, const C &x, C *out) { out[tat(line, i, pitch)] = x; };
+		const C *r = fft_fx<R1, R2, +1, true, false>(nl, pitch, p.pl, T.tw, T.a, T.b, ld0, st_s);
+		__syncthreads();
+		const int rows = rf ? ZS : N;
+		for (int e = threadIdx.x; e < rows * nl; e += blockDim.x) {
+			const int zr = fdiv(e, mgnl), line = e - zr * nl;
+			if (line >= nz) continue;
+			const int l = zr - H, k = z0 + line - H;
+			if ((l == H && k == -H) || (l == -H && k == H)) continue;
+			// psi1 is tabulated on -N/2 .. N/2 - 1; at the upper end it is conj psi1(-k)
+			const bool up = l == H || k == H;
+			const int a = up ? -l : l, b = up ? -k : k;
+			C w = ps[(long)(a < 0 ? a + N : a) * N + (b < 0 ? b + N : b)];
+			if (!up) w.y = -w.y;
+			C *z = Z + (long)zr * ZS + z0 + line;
+			*z = cfma(w, r[tat(line, l < 0 ? l + P : l, pitch)], *z);
+		}
+		__syncthreads();
+	}
+}
+
 // The I3 chains with the whole P x P grid in shared memory (P = 48 and 96 in
 // FP32, P = 48 in FP64): one CTA per (cell, j, i) runs the wave's terms in
 // order, X[cell][j][i] += eta_i P_i . FFT2(psi2_t . IFFT2(W^_i . P_j)), each
@@ -908,6 +1035,8 @@ template <class C> struct I3FusedP {
 	using R = typename CT<C>::R;
 	const C *What, *Pg; C *X; const R *psi2T; const int *idx; const double *scale;
 	int N, nt, t0;
+	WaveUnits un;
+	C *Y;                                 // chains of the pairs, as k_any_i3_rows_b leaves them
 	const int *kind;                      // null: every cell complex
 	Plan pl;
 };
@@ -928,10 +1057,12 @@ template <class C, bool RF> __device__ __forceinline__ void i3_fused(const I3Fus
 	const C *G = p.What + (cell * 4 + (RF ? 2 * h : h)) * PP;
 	for (int tt = 0; tt < p.nt; tt++) {
 		const long ct = cell * p.nt + tt;
-		const int t = p.t0 + tt;
+		const int t = p.un.term(p.t0 + tt);
+		const bool keep = p.un.pair(p.t0 + tt);
 		const R sc = (R)p.scale[t];
 		const R *ps = p.psi2T + (long)p.idx[t] * PP;
 		const C *Pj = p.Pg + (ct * 4 + (RF ? j3 / 2 : j3)) * PP;
+		C *yk = p.Y + (ct * 16 + (RF ? 2 * j3 : 4 * j3) + h) * PP;
 		{
 			batched<Two<C>>(PPi, [&](int i) {
 				Two<C> v;
@@ -967,6 +1098,7 @@ template <class C, bool RF> __device__ __forceinline__ void i3_fused(const I3Fus
 				const int l = fdiv(i, mgP), k = i - l * P;
 				C x = v.b;
 				const C y0 = r[T.at(l, k)];
+				if (keep) yk[i] = y0;
 				if (RF) {                                  // eta_2h P_2h Re + eta_2h+1 P_2h+1 Im (eta_2h+1 = -1)
 					x.x += eta * (v.a.x * y0.x) - v.a.y * y0.y;
 				} else {
@@ -997,6 +1129,7 @@ template <class C> __global__ void __launch_bounds__(kThreads) k_any_i3_fused(co
 template <class C> struct AsmP {
 	const C *What, *FS, *FS4, *Q, *X;    // FS [cell][3], FS4 / Q [cell][4], X [cell][4][nxp] (null: part absent)
 	int nxp;                             // partials of X per (cell, j), added in order
+	const C *Zp; const int *kind;        // sums of k_any_i3_cols_z (null: none) and the cells' forms
 	C *Z; int N, nl;
 	double s1, s2;
 	int mode;
@@ -1098,7 +1231,22 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 		if (ls < 0 || ks < 0) continue;
 		const C zc = r[T.at(kk, l)], zd = r[T.at(nl + kk, l)];
 		const double2 cc = make_double2(p.s1 * (double)zc.x, p.s1 * (double)zc.y);
-		const double2 cd = make_double2((double)zd.x, (double)zd.y);
+		double2 cd = make_double2((double)zd.x, (double)zd.y);
+		if (p.Zp != nullptr) {                       // - eta2_j s1 Z_j
+			const int H = N / 2, ZS = N + 1, fl = (ls < H ? ls : ls - N) + H, fk = (ks < H ? ks : ks - N) + H;
+			const double f = (j == 0 ? 2.0 : -2.0) * p.s1;
+			if (has_rf<C>() && p.kind != nullptr && p.kind[cell] == 0) {
+				// A = Z_2c + i Z_2c+1, each the transform of a real grid
+				const C *A = p.Zp + (cell * 4 + (j >> 1)) * (long)ZS * ZS;
+				const C u = A[fl * ZS + fk], v = A[(N - fl) * ZS + N - fk];
+				cd.x -= f * 0.5 * ((j & 1) ? (double)u.y + (double)v.y : (double)u.x + (double)v.x);
+				cd.y -= f * 0.5 * ((j & 1) ? (double)v.x - (double)u.x : (double)u.y - (double)v.y);
+			} else {
+				const C z = p.Zp[cj * (long)ZS * ZS + fl * ZS + fk];
+				cd.x -= f * (double)z.x;
+				cd.y -= f * (double)z.y;
+			}
+		}
 		const long q = (long)ls * N + ks, o = cj * NN + q;
 		if (p.mode == 0) {
 			if (p.out_cc) p.out_cc[o] = cc;
@@ -1437,7 +1585,7 @@ template <class C> struct AnyRhs {
 	// in one complex transform, the others the complex chains, in the same
 	// launches (the kernels read a cell's kind; the real form leaves half of
 	// its units idle)
-	int i3_sums(const DevI3 &t, const double2 *W) {
+	int i3_sums(const DevI3 &t, const double2 *W, AsmP<C> &as) {
 		const int nxp = fused_i3() ? 4 : 1;
 		ws.i3p.ensure(sizeof(C) * ncells * 4 * nxp * PP);
 		QB_CUDA(cudaMemsetAsync(ws.i3p.p, 0, sizeof(C) * ncells * 4 * nxp * PP, s));
@@ -1445,8 +1593,29 @@ template <class C> struct AnyRhs {
 		if constexpr (sizeof(typename CT<C>::R) == 4) {
 			if (real_form_enabled()) kind = i3_form_kinds(ws, ncells, W, s);
 		}
+		if (t.pairM > 0) {
+			ws.i3z.ensure(sizeof(C) * 4 * ncells * (N + 1) * (N + 1));
+			QB_CUDA(cudaMemsetAsync(ws.i3z.p, 0, sizeof(C) * 4 * ncells * (N + 1) * (N + 1), s));
+			as.Zp = ws.i3z.as<C>();
+			as.kind = kind;
+		}
 		i3_waves(t, W, nxp, kind);
 		return nxp;
+	}
+
+	// the terms of the opposite shifts of a wave: rows of Y_i (into V, the P grids'
+	// place), columns into Z
+	void other_terms(const DevI3 &t, const C *What, const C *Y, C *V, C *Z, int nc, int n, int t0, const int *kc) {
+		I3RowsYP<C> y{};
+		y.What = What; y.Y = Y; y.V = V; y.N = N; y.nl = nl1; y.nt = n; y.t0 = t0; y.un.M = t.pairM; y.kind = kc; y.pl = pl;
+		by_plan([&](auto kern) { launch(kern, "any_i3_rows_y", blocks((long)nc * n * 4, nl1), smem(nl1, 1), s, y); },
+		        k_any_i3_rows_y<C, 16, 3>, k_any_i3_rows_y<C, 16, 6>, k_any_i3_rows_y<C, 16, 12>, k_any_i3_rows_y<C, 16, 16>,
+		        k_any_i3_rows_y<C, 0, 0>);
+		I3ColsZP<C> z{};
+		z.V = V; z.Z = Z; z.psi1 = Tabs<C>::i3_psi1(t); z.N = N; z.nl = nl1; z.nt = n; z.t0 = t0; z.un.M = t.pairM; z.kind = kc; z.pl = pl;
+		by_plan([&](auto kern) { launch(kern, "any_i3_cols_z", (long)nc * 4 * ((N + nl1) / nl1), smem(nl1, 1), s, z); },
+		        k_any_i3_cols_z<C, 16, 3>, k_any_i3_cols_z<C, 16, 6>, k_any_i3_cols_z<C, 16, 12>, k_any_i3_cols_z<C, 16, 16>,
+		        k_any_i3_cols_z<C, 0, 0>);
 	}
 
 	// the I3 chains in waves of terms and, where one term of the batch
@@ -1455,13 +1624,15 @@ template <class C> struct AnyRhs {
 	// form) and 16 chains (8 in the real form).  A cell's terms still run in
 	// order, so the sums do not depend on the waves.
 	void i3_waves(const DevI3 &t, const double2 *W, int nxp, const int *kind) {
-		const bool fused = nxp == 4;
-		const int per_term = fused ? 4 : 20;
+		const bool fused = nxp == 4, pairs = t.pairM > 0;
+		const WaveUnits un{ t.pairM };
+		const int nunits = pairs ? t.nterms / t.pairM * ((t.pairM + 1) / 2) : t.nterms;
+		const int per_term = fused && !pairs ? 4 : 20;
 		const int cpw = wave_cells(per_term);
-		const int nt = wave(t.nterms, per_term, cpw);
-		ws.wave1.ensure(sizeof(C) * (size_t)cpw * nt * 4 * PP);                // P_j
-		if (!fused) ws.wave2.ensure(sizeof(C) * (size_t)cpw * nt * 16 * PP);   // chains
-		C *Pg = ws.wave1.as<C>(), *Y = fused ? nullptr : ws.wave2.as<C>();
+		const int nt = wave(nunits, per_term, cpw);
+		ws.wave1.ensure(sizeof(C) * (size_t)cpw * nt * 4 * PP);                // P_j, then the rows of Y_i
+		if (per_term == 20) ws.wave2.ensure(sizeof(C) * (size_t)cpw * nt * 16 * PP);   // chains
+		C *Pg = ws.wave1.as<C>(), *Y = per_term == 20 ? ws.wave2.as<C>() : nullptr;
 		int nl4 = nl1;                                      // one tile, at most kOwn elements a thread
 		const int own = own_for_plan(pl, sizeof(C) == 16);
 		while (nl4 > 1 && (nl4 * P > own * kThreads || P % nl4)) nl4--;
@@ -1471,24 +1642,25 @@ template <class C> struct AnyRhs {
 			const C *What = ws.What.as<C>() + (long)c0 * 4 * PP;
 			C *X = ws.i3p.as<C>() + (long)c0 * 4 * nxp * PP;
 			const int *kc = kind ? kind + c0 : nullptr;
-			for (int t0 = 0; t0 < t.nterms; t0 += nt) {
-				const int n = std::min(nt, t.nterms - t0);
+			for (int t0 = 0; t0 < nunits; t0 += nt) {
+				const int n = std::min(nt, nunits - t0);
 				PadRowsP<C> p = pad_params(Wc, n, t0, 4, Pg);
 				for (int g = 0; g < 4; g++) { p.comp[g] = g; p.comp2[g] = g; p.psel[g] = 3; }
 				p.kind = kc; p.nsub_rf = 2;
 				for (int g = 0; g < 2; g++) { p.comp_rf[g] = 2 * g; p.comp2_rf[g] = 2 * g + 1; p.psel_rf[g] = 4; }
-				p.psiC = Tabs<C>::i3_psi1(t);
+				p.psiC = Tabs<C>::i3_psi1(t); p.un = un;
 				pad_rows(p, nc);
 				plain(Pg, (long)nc * n * 4, -1, true, kc, (long)n * 4, 4, 2, true);
 				if (fused) {
 					I3FusedP<C> f{};
 					f.What = What; f.Pg = Pg; f.X = X;
 					f.psi2T = Tabs<C>::i3_psi2T(t); f.idx = t.idx.as<int>(); f.scale = t.scale.as<double>();
-					f.N = N; f.nt = n; f.t0 = t0; f.kind = kc;
+					f.N = N; f.nt = n; f.t0 = t0; f.kind = kc; f.un = un; f.Y = Y;
 					// FP32 default: radix-8 stages (the radix-16 register DFTs push this
 					// kernel to 173 registers, one CTA an SM); FP64 runs one CTA an SM anyway
 					f.pl = (ws.anyn_plan == 0 && sizeof(C) == 8) ? with_tw(make_plan(P, 1)) : pl;
 					launch(k_any_i3_fused<C>, "any_i3_fused", (long)nc * 16, tile_bytes<C>(P, P), s, f);
+					if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * (N + 1) * (N + 1), nc, n, t0, kc);
 					continue;
 				}
 				I3RowsAP<C> a{};
@@ -1498,15 +1670,16 @@ template <class C> struct AnyRhs {
 				        k_any_i3_rows_a<C, 0, 0>);
 				I3ColsP<C> c{};
 				c.Y = Y; c.psi2T = Tabs<C>::i3_psi2T(t); c.idx = t.idx.as<int>(); c.scale = t.scale.as<double>();
-				c.N = N; c.nl = nl1; c.nt = n; c.t0 = t0; c.kind = kc; c.pl = pl;
+				c.N = N; c.nl = nl1; c.nt = n; c.t0 = t0; c.kind = kc; c.un = un; c.pl = pl;
 				by_plan([&](auto kern) { launch(kern, "any_i3_cols", blocks((long)nc * n * 16, nl1), smem(nl1, 1), s, c); },
 				        k_any_i3_cols<C, 16, 3>, k_any_i3_cols<C, 16, 6>, k_any_i3_cols<C, 16, 12>, k_any_i3_cols<C, 16, 16>,
 				        k_any_i3_cols<C, 0, 0>);
 				I3RowsBP<C> b{};
-				b.Y = Y; b.Pg = Pg; b.X = X; b.N = N; b.nl = nl4; b.nt = n; b.kind = kc; b.pl = pl;
+				b.Y = Y; b.Pg = Pg; b.X = X; b.N = N; b.nl = nl4; b.nt = n; b.t0 = t0; b.kind = kc; b.un = un; b.pl = pl;
 				by_plan([&](auto kern) { launch(kern, "any_i3_rows_b", blocks((long)nc * 4, nl4), smem(nl4, 1), s, b); },
 				        k_any_i3_rows_b<C, 16, 3>, k_any_i3_rows_b<C, 16, 6>, k_any_i3_rows_b<C, 16, 12>,
 				        k_any_i3_rows_b<C, 16, 16>, k_any_i3_rows_b<C, 0, 0>);
+				if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * (N + 1) * (N + 1), nc, n, t0, kc);
 			}
 		}
 	}
@@ -1520,7 +1693,7 @@ template <class C> struct AnyRhs {
 		if (parts & RHS_CD) {
 			if (q.i4) { i1_sums(*q.i4, W, false, ws.i1i4, ws.fs4); a.FS4 = ws.fs4.as<C>(); }
 			if (q.i2) { i2_sums(*q.i2, W); a.Q = ws.i2p.as<C>(); }
-			if (q.i3) { a.nxp = i3_sums(*q.i3, W); a.X = ws.i3p.as<C>(); }
+			if (q.i3) { a.nxp = i3_sums(*q.i3, W, a); a.X = ws.i3p.as<C>(); }
 		}
 		a.N = N;
 		a.s2 = 1.0 / (double)PP;
