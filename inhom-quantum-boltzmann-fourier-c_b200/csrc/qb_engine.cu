@@ -1590,7 +1590,7 @@ void transport_maxwell_lines(int m, int ncells, const double *in, double *out, c
 }
 
 void flux_pair(int m, const double *A_dev, const double *U_dev, double *out_dev, cudaStream_t s) {
-	k_flux_pair<<<1, 32, 0, s>>>(m, 0, A_dev, U_dev, out_dev);
+	k_flux_pair<<<1, 64, 0, s>>>(m, 0, A_dev, U_dev, out_dev);
 	QB_CUDA(cudaGetLastError());
 }
 
@@ -1748,7 +1748,7 @@ void inhom_step_maxwell(Workspace &ws, const QuadSet &q, int ncells, const doubl
 	k_transport_maxwell<<<nb, 256, 0, s>>>(p);
 	QB_CUDA(cudaGetLastError());
 	fourier_collision(ws, q, ncells, Vt, Bext, dt, s);
-	k_maxwell_flux<<<1, 32, 0, s>>>(N, vx_dev, Vt, Vt + (ncells - 1) * cs, bnd);
+	k_maxwell_flux<<<1, 64, 0, s>>>(N, vx_dev, Vt, Vt + (ncells - 1) * cs, bnd);
 	p.in = Vt; p.out = Wnext;
 	k_transport_maxwell<<<nb, 256, 0, s>>>(p);
 	QB_CUDA(cudaGetLastError());

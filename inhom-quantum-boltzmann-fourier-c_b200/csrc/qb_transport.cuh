@@ -102,16 +102,38 @@ __global__ void __launch_bounds__(256) k_transport(const TransportParams p) {
 // (SlopeLimiterStepMaxwell on caller data).
 __device__ __forceinline__ int mx_src(int remapN, int m, int mm) { return (remapN && mm < m / 2) ? mm + remapN : mm; }
 
+// sum of |A| U (absA) or A U over mm in [i0, i1) of grid U (remapped), in upstream
+// order, by one warp: the lanes load and multiply 32 terms, the next 32 ahead,
+// and every lane adds them one after the other, so only the additions are
+// serial (m = 1024: 3 us a sum; loads by the adding thread took 30)
+__device__ __forceinline__ double seq_flux(int m, int remapN, const double *__restrict__ A, const double *__restrict__ U, int i0, int i1, bool absA) {
+	const int lane = threadIdx.x & 31;
+	auto term = [&](int i) {
+		if (i >= i1) return 0.0;
+		const double a = A[i];
+		return mul_(absA ? fabs(a) : a, U[mx_src(remapN, m, i)]);
+	};
+	double s = 0, t = term(i0 + lane);
+	for (int i = i0; i < i1; i += 32) {
+		const double next = term(i + 32 + lane);
+		if (i + 32 <= i1) {
+#pragma unroll
+			for (int k = 0; k < 32; k++) s = add_(s, __shfl_sync(0xffffffffu, t, k));
+		} else {
+			for (int k = 0; k < i1 - i; k++) s = add_(s, __shfl_sync(0xffffffffu, t, k));
+		}
+		t = next;
+	}
+	return s;
+}
+
 // Sequential flux sums in upstream order (CalculateRightwardFlux /
-// CalculateLeftwardFlux, finite_volume.c:186-216), one thread:
+// CalculateLeftwardFlux, finite_volume.c:186-216), two warps:
 //   out[0] = sum_{mm<m/2} A U ;  out[1] = sum_{mm>=m/2} |A| U   of grid U (remapped)
-__global__ void k_flux_pair(int m, int remapN, const double *__restrict__ A, const double *__restrict__ U, double *out) {
-	if (threadIdx.x != 0 || blockIdx.x != 0) return;
-	double r = 0, l = 0;
-	for (int i = 0; i < m / 2; i++) r = add_(r, mul_(A[i], U[mx_src(remapN, m, i)]));
-	for (int i = m / 2; i < m; i++) l = add_(l, mul_(fabs(A[i]), U[mx_src(remapN, m, i)]));
-	out[0] = r;
-	out[1] = l;
+__global__ void __launch_bounds__(64) k_flux_pair(int m, int remapN, const double *__restrict__ A, const double *__restrict__ U, double *out) {
+	const int w = threadIdx.x >> 5;
+	const double s = w == 0 ? seq_flux(m, remapN, A, U, 0, m / 2, false) : seq_flux(m, remapN, A, U, m / 2, m, true);
+	if ((threadIdx.x & 31) == 0) out[w] = s;
 }
 
 // boundary data of InhomStepMaxwell (simulation.c:887-919): normalised Maxwell
@@ -121,14 +143,14 @@ __global__ void k_maxwell_setup(int N, const double *__restrict__ A, const doubl
                                 const double *__restrict__ W0, const double *__restrict__ Wn, double *bnd, double *UL, double *UR) {
 	const int m = N * N;
 	__shared__ double sh[4];
-	if (threadIdx.x == 0) {
-		double r = 0, l = 0, fl = 0, fr = 0;
-		for (int i = 0; i < m / 2; i++) r = add_(r, mul_(A[i], WL[mx_src(N, m, i)]));          // rightward flux of WL trace
-		for (int i = m / 2; i < m; i++) l = add_(l, mul_(fabs(A[i]), WR[mx_src(N, m, i)]));    // leftward flux of WR trace
-		for (int i = m / 2; i < m; i++) fl = add_(fl, mul_(fabs(A[i]), W0[mx_src(N, m, i)]));  // leftward flux at left boundary
-		for (int i = 0; i < m / 2; i++) fr = add_(fr, mul_(A[i], Wn[mx_src(N, m, i)]));        // rightward flux at right boundary
-		sh[0] = __ddiv_rn(1.0, r); sh[1] = __ddiv_rn(1.0, l); sh[2] = fl; sh[3] = fr;
-		bnd[0] = sh[0]; bnd[1] = sh[1]; bnd[2] = fl; bnd[3] = fr;
+	const int w = threadIdx.x >> 5;
+	if (w < 4) {
+		double v;
+		if (w == 0) v = __ddiv_rn(1.0, seq_flux(m, N, A, WL, 0, m / 2, false));       // rightward flux of WL trace
+		else if (w == 1) v = __ddiv_rn(1.0, seq_flux(m, N, A, WR, m / 2, m, true));   // leftward flux of WR trace
+		else if (w == 2) v = seq_flux(m, N, A, W0, m / 2, m, true);                   // leftward flux at left boundary
+		else v = seq_flux(m, N, A, Wn, 0, m / 2, false);                              // rightward flux at right boundary
+		if ((threadIdx.x & 31) == 0) { sh[w] = v; bnd[w] = v; }
 	}
 	__syncthreads();
 	for (int t = threadIdx.x; t < 4 * m; t += blockDim.x) {
@@ -139,14 +161,10 @@ __global__ void k_maxwell_setup(int N, const double *__restrict__ A, const doubl
 }
 
 // outgoing fluxes only (second half step, simulation.c:1059-1066): bnd[2..3]
-__global__ void k_maxwell_flux(int N, const double *__restrict__ A, const double *__restrict__ W0, const double *__restrict__ Wn, double *bnd) {
-	if (threadIdx.x != 0 || blockIdx.x != 0) return;
-	const int m = N * N;
-	double fl = 0, fr = 0;
-	for (int i = m / 2; i < m; i++) fl = add_(fl, mul_(fabs(A[i]), W0[mx_src(N, m, i)]));
-	for (int i = 0; i < m / 2; i++) fr = add_(fr, mul_(A[i], Wn[mx_src(N, m, i)]));
-	bnd[2] = fl;
-	bnd[3] = fr;
+__global__ void __launch_bounds__(64) k_maxwell_flux(int N, const double *__restrict__ A, const double *__restrict__ W0, const double *__restrict__ Wn, double *bnd) {
+	const int m = N * N, w = threadIdx.x >> 5;
+	const double s = w == 0 ? seq_flux(m, N, A, W0, m / 2, m, true) : seq_flux(m, N, A, Wn, 0, m / 2, false);
+	if ((threadIdx.x & 31) == 0) bnd[2 + w] = s;
 }
 
 struct MaxwellParams {
