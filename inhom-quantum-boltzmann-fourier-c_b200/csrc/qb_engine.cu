@@ -145,7 +145,25 @@ Workspace::~Workspace() {
 	if (ev_out) cudaEventDestroy(ev_out);
 	if (ev_t) cudaEventDestroy(ev_t);
 	if (ev_i) cudaEventDestroy(ev_i);
+	if (ev_fork) cudaEventDestroy(ev_fork);
+	if (ev_join) cudaEventDestroy(ev_join);
+	if (side) cudaStreamDestroy(side);
 	if (stream) cudaStreamDestroy(stream);
+}
+
+cudaStream_t Workspace::fork(cudaStream_t s) {
+	if (side == nullptr) {
+		QB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+		QB_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+		QB_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+	}
+	QB_CUDA(cudaEventRecord(ev_fork, s));
+	QB_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
+	return side;
+}
+void Workspace::join(cudaStream_t s) {
+	QB_CUDA(cudaEventRecord(ev_join, side));
+	QB_CUDA(cudaStreamWaitEvent(s, ev_join, 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -488,6 +506,13 @@ template <int P, class C> void launch_fft_full(const FullParamsT<C> &p, long ngr
 	QB_CUDA(cudaGetLastError());
 }
 
+// The sums of small batches leave SMs idle and take longest in their launches:
+// below this many (cell, unit) pieces of I3 work a resident cluster (or CTA),
+// the I1, I2 and I4 sums run beside the I3 sums on a second stream. Above, the I3
+// kernels fill the GPU by themselves and SMs held by another kernel at
+// their start would delay their last cluster.
+constexpr long kForkUnits = 8;
+
 template <class C> void launch_sum_slots(const SumSlotsT<C> &p, int ncells, cudaStream_t s) {
 	ProfScope ps("sum_slots", s);
 	k_sum_slots<C><<<dim3((unsigned)((p.len + 255) / 256), (unsigned)ncells), 256, 0, s>>>(p);
@@ -584,6 +609,15 @@ template <> struct Tab<float2> {
 
 // ---------------------------------------------------------------------------
 // the factored right-hand side for one padded size P and working complex type C
+// resident clusters (N = 32) or CTAs (N = 8, 16) of the I3 sums
+int resident_i3(int N, bool f32) {
+	switch (N) {
+	case 8: return f32 ? active_i3q<16, float2>() : active_i3q<16, double2>();
+	case 16: return f32 ? active_i3q<32, float2>() : active_i3q<32, double2>();
+	default: return f32 ? active_i3p_clusters<float2>() : active_i3w_clusters();
+	}
+}
+
 template <int P, class C> struct Rhs {
 	static constexpr int N = P / 2;
 	static constexpr long NN = (long)N * N, PP = (long)P * P;
@@ -629,7 +663,17 @@ template <int P, class C> struct Rhs {
 		p.psi1 = T::i2_psi1(t); p.psi2 = T::i2_psi2(t);
 		p.out = ws.i2p.as<C>();
 		launch_i2<P>(p, (long)ncells * 4 * nchunk, s);
+		if (sum_i2(nchunk, ncells)) {
+			ws.i2s.ensure(sizeof(C) * ncells * 4 * PP);
+			SumSlotsT<C> r{};
+			r.nx = nchunk; r.per = 1;
+			r.in = ws.i2p.as<C>(); r.out = ws.i2s.as<C>(); r.len = (int)PP;
+			launch_sum_slots(r, 4 * ncells, s);
+		}
 	}
+	// the I2 partials of a cell get their own launch as those of I3 do (the
+	// assembly reads them once for each component)
+	static bool sum_i2(int nchunk, int ncells) { return nchunk >= kSumSlots && 4 * ncells <= 65535; }
 
 	// the terms of opposite shifts are summed together (I3Units), except by the
 	// tensor-core form; each CTA of the clusters of k_i3p and k_i3pr leaves its
@@ -715,12 +759,16 @@ template <int P, class C> struct Rhs {
 		if (P == 64 && sizeof(C) == 16 && q.i3 && q.i3->nterms > 0 && ranges)
 			ch.i3_slots = (int)std::min<long>(active_i3w_clusters(), (long)ncells * i3_count(ws, *q.i3));
 		spectra(ws, ncells, W, s);
-		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s);
+		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
+		const cudaStream_t s2 = small ? ws.fork(s) : s;
+		if (small) i3_sums(ws, *q.i3, ncells, W, ch, s);
+		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s2);
 		if (parts & RHS_CD) {
-			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch.i1, s);
-			i2_sums(ws, *q.i2, ncells, W, ch.i2, s);
-			i3_sums(ws, *q.i3, ncells, W, ch, s);
+			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch.i1, s2);
+			i2_sums(ws, *q.i2, ncells, W, ch.i2, s2);
+			if (!small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		}
+		if (small) ws.join(s);
 	}
 
 	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells, cudaStream_t s) {
@@ -729,6 +777,7 @@ template <int P, class C> struct Rhs {
 		a.FS = (parts & RHS_CC) ? ws.fs.as<C>() : nullptr;
 		a.FS4 = (parts & RHS_CD) ? ws.fs4.as<C>() : nullptr;
 		a.Qp = (parts & RHS_CD) ? ws.i2p.as<C>() : nullptr; a.nq = ch.i2;
+		if ((parts & RHS_CD) && sum_i2(ch.i2, ncells)) { a.Qp = ws.i2s.as<C>(); a.nq = 1; }
 		a.Xp = (parts & RHS_CD) ? ws.i3p.as<C>() : nullptr; a.nx = ch.i3;
 		if (ch.i3_slots > 0 && (parts & RHS_CD)) a.xrg = term_ranges(ch.i3_slots, i3_count(ws, *q.i3), ncells);
 		const long slots = ch.i3_slots > 0 ? (long)ch.i3_slots : (long)ncells * ch.i3;
@@ -1152,12 +1201,17 @@ template <class C> struct Rhs<128, C> {
 		}
 		scale_chunks(ws, q, ch, q.i3 ? i3_count(*q.i3) : 0);
 		spectra(ws, ncells, W, s);
-		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s);
+		const int act = sizeof(C) == 16 ? active_quad_clusters() : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
+		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(*q.i3) < kForkUnits * act;
+		const cudaStream_t s2 = small ? ws.fork(s) : s;
+		if (small) i3_sums(ws, *q.i3, ncells, W, ch, s);
+		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s2);
 		if (parts & RHS_CD) {
-			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch.i1, s);
-			i2_sums(ws, *q.i2, ncells, W, ch.i2, s);
-			i3_sums(ws, *q.i3, ncells, W, ch, s);
+			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch.i1, s2);
+			i2_sums(ws, *q.i2, ncells, W, ch.i2, s2);
+			if (!small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		}
+		if (small) ws.join(s);
 	}
 
 	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells, cudaStream_t s) {
@@ -1238,18 +1292,9 @@ Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) 
 	const int sms = num_sms();
 	if (q.i1) c.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), sms, 64);
 	if (q.i2) c.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), sms, 64);
-	if (q.i3) {
-		int act = 0;
-		const bool f32 = prec == 32;
-		switch (N) {
-		case 8: act = f32 ? active_i3q<16, float2>() : active_i3q<16, double2>(); break;
-		case 16: act = f32 ? active_i3q<32, float2>() : active_i3q<32, double2>(); break;
-		default: act = f32 ? active_i3p_clusters<float2>() : active_i3w_clusters(); break;
-		}
-		// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written
-		// and read back at HBM speed; one term takes a cluster ~36 us there: 0.15
-		c.i3 = best_chunks((long)ncells, std::max(1, i3_units), act, 256, 0.15);
-	}
+	// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written
+	// and read back at HBM speed; one term takes a cluster ~36 us there: 0.15
+	if (q.i3) c.i3 = best_chunks((long)ncells, std::max(1, i3_units), resident_i3(N, prec == 32), 256, 0.15);
 	return c;
 }
 

@@ -85,7 +85,7 @@ struct Workspace {
 	int prec = 64;                           // working precision of the collision operator: 64 (FP64) or 32 (FP32 form)
 	int conserve = 0;                        // restore the collision invariants after each velocity-space collision step
 	cudaStream_t stream = nullptr;           // own stream (upstream API calls)
-	DevBuf What, WhatQ, i1cc, i1i4, i2p, i3p, i3s, i3z, i3zsum, i3zs, i3y, fs, fs4, wmid;      // collision scratch
+	DevBuf What, WhatQ, i1cc, i1i4, i2p, i2s, i3p, i3s, i3z, i3zsum, i3zs, i3y, fs, fs4, wmid;      // collision scratch
 	DevBuf fa, fb, va, vb;                   // state scratch (Fourier / velocity)
 	DevBuf io_in, io_out, bext, vgrid;       // staging for host-pointer calls
 	DevBuf aux, aux2;
@@ -126,6 +126,12 @@ struct Workspace {
 	// which collide on the caller's stream while the interior collides on `stream`
 	std::unique_ptr<Workspace> edge;
 	cudaEvent_t ev_t = nullptr, ev_i = nullptr;
+	// second stream of one evaluation: the I1, I2 and I4 sums of a small batch
+	// beside its I3 sums, between fork (after the caller's work so far) and join
+	cudaStream_t side = nullptr;
+	cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+	cudaStream_t fork(cudaStream_t s);
+	void join(cudaStream_t s);
 	explicit Workspace(int N);
 	~Workspace();
 };
