@@ -114,7 +114,42 @@ void DevBuf::ensure(size_t n) {
 	bytes = n;
 }
 
+void DevBufSet::reserve() {
+	bool grow = false;
+	for (auto &w : want) grow = grow || w.first->bytes < w.second;
+	if (grow) {
+		// the buffers of earlier reservations move along
+		for (DevBuf *m : members)
+			if (m->view && std::none_of(want.begin(), want.end(), [m](const auto &w) { return w.first == m; })) want.emplace_back(m, m->bytes);
+		members.clear();
+		size_t total = 0;
+		for (auto &w : want) {
+			w.second = (std::max(w.first->bytes, w.second) + 255) / 256 * 256;
+			w.first->release();
+			total += w.second;
+		}
+		whole.release();
+		whole.ensure(total);
+		char *p = static_cast<char *>(whole.p);
+		for (auto &w : want) {
+			w.first->p = p;
+			w.first->bytes = w.second;
+			w.first->device = whole.device;
+			w.first->view = true;
+			members.push_back(w.first);
+			p += w.second;
+		}
+	}
+	want.clear();
+}
+
 void DevBuf::release() {
+	if (view) {
+		p = nullptr;
+		bytes = 0;
+		view = false;
+		return;
+	}
 	if (p != nullptr) {
 		g_buffer_generation.fetch_add(1, std::memory_order_acq_rel);
 		int cur = -1;
@@ -745,6 +780,38 @@ template <int P, class C> struct Rhs {
 		}
 	}
 
+	// the scratch of one evaluation in one allocation (each user's ensure finds it there)
+	static void reserve(Workspace &ws, const QuadSet &q, int ncells, const Chunks &ch, int parts) {
+		DevBufSet &b = ws.scratch;
+		const size_t g = sizeof(C) * (size_t)ncells * PP;
+		b.add(ws.What, 4 * g);
+		if (P == 64 && sizeof(C) == 16) b.add(ws.WhatQ, 4 * g);
+		if (parts & RHS_CC) {
+			b.add(ws.i1cc, 3 * ch.i1 * g);
+			b.add(ws.fs, 3 * g);
+		}
+		if (parts & RHS_CD) {
+			b.add(ws.i1i4, 4 * ch.i1 * g);
+			b.add(ws.fs4, 4 * g);
+			b.add(ws.i2p, 4 * ch.i2 * g);
+			if (sum_i2(ch.i2, ncells)) b.add(ws.i2s, 4 * g);
+			size_t slots = (size_t)ncells * ch.i3, used = slots;
+			if (ch.i3_slots > 0) {
+				const TermRanges r = term_ranges(ch.i3_slots, i3_count(ws, *q.i3), ncells);
+				slots = (size_t)r.nslots * r.maxc;
+				used = r.nslots;
+			}
+			b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
+			if (pairs_units(ws)) b.add(ws.i3z, sizeof(C) * slots * kZRanks * 4 * NN);
+			if (P == 64 && sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 8 * PP);
+			if (used >= (size_t)kSumSlots * ncells) {
+				b.add(ws.i3s, 4 * g);
+				if (pairs_units(ws)) b.add(ws.i3zsum, g);
+			}
+		}
+		b.reserve();
+	}
+
 	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, Chunks &ch, cudaStream_t s) {
 		T::prepare(q, s);
 		ch = pick_chunks(N, ncells, q, (int)(8 * sizeof(typename CT<C>::R)), q.i3 ? i3_count(ws, *q.i3) : 0);
@@ -758,6 +825,7 @@ template <int P, class C> struct Rhs {
 		const bool ranges = ws.i3_ranges >= 0 ? ws.i3_ranges == 1 : term_ranges_enabled();
 		if (P == 64 && sizeof(C) == 16 && q.i3 && q.i3->nterms > 0 && ranges)
 			ch.i3_slots = (int)std::min<long>(active_i3w_clusters(), (long)ncells * i3_count(ws, *q.i3));
+		reserve(ws, q, ncells, ch, parts);
 		spectra(ws, ncells, W, s);
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
 		const cudaStream_t s2 = small ? ws.fork(s) : s;
@@ -1200,6 +1268,38 @@ template <class C> struct Rhs<128, C> {
 			ch.i3 = best_chunks((long)ncells, std::max(1, i3_count(*q.i3)), act, 256, 0.15);
 		}
 		scale_chunks(ws, q, ch, q.i3 ? i3_count(*q.i3) : 0);
+		{
+			DevBufSet &b = ws.scratch;
+			const size_t g = sizeof(C) * (size_t)ncells * PP;
+			b.add(ws.What, 4 * g);
+			if (sizeof(C) == 16) b.add(ws.WhatQ, 4 * g);
+			if (parts & RHS_CC) {
+				b.add(ws.i1cc, 3 * ch.i1 * g);
+				b.add(ws.fs, 3 * g);
+			}
+			if (parts & RHS_CD) {
+				b.add(ws.i1i4, 4 * ch.i1 * g);
+				b.add(ws.fs4, 4 * g);
+				b.add(ws.i2p, 4 * ch.i2 * g);
+				b.add(ws.scr128b, 4 * ch.i2 * g);
+				size_t slots = (size_t)ncells * ch.i3, used = slots;
+				if (ch.i3_slots > 0) {
+					const TermRanges r = term_ranges(ch.i3_slots, i3_count(*q.i3), ncells);
+					slots = (size_t)r.nslots * r.maxc;
+					used = r.nslots;
+				}
+				b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
+				b.add(ws.scr128a, sizeof(C) * used * 4 * PP);
+				if (pairs_units()) b.add(ws.i3z, sizeof(C) * slots * kZRanks * 4 * NN);
+				if (sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 4 * PP);
+				else if (use_full128()) b.add(ws.i3y, sizeof(C) * used * 2 * PP);
+				if (used >= (size_t)kSumSlots * ncells) {
+					b.add(ws.i3s, 4 * g);
+					if (pairs_units()) b.add(ws.i3zsum, g);
+				}
+			}
+			b.reserve();
+		}
 		spectra(ws, ncells, W, s);
 		const int act = sizeof(C) == 16 ? active_quad_clusters() : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(*q.i3) < kForkUnits * act;

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace qb {
@@ -32,18 +33,30 @@ struct DevBuf {
 	void *p = nullptr;
 	size_t bytes = 0;
 	int device = -1;
+	bool view = false;                       // part of another buffer (DevBufSet): not freed here
 	DevBuf() = default;
 	DevBuf(const DevBuf &) = delete;
 	DevBuf &operator=(const DevBuf &) = delete;
-	DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), device(o.device) { o.p = nullptr; o.bytes = 0; }
+	DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), device(o.device), view(o.view) { o.p = nullptr; o.bytes = 0; }
 	DevBuf &operator=(DevBuf &&o) noexcept {
-		if (this != &o) { release(); p = o.p; bytes = o.bytes; device = o.device; o.p = nullptr; o.bytes = 0; }
+		if (this != &o) { release(); p = o.p; bytes = o.bytes; device = o.device; view = o.view; o.p = nullptr; o.bytes = 0; }
 		return *this;
 	}
 	void ensure(size_t n);        // grow (contents discarded)
 	void release();
 	~DevBuf() { release(); }
 	template <class T> T *as() const { return static_cast<T *>(p); }
+};
+
+// Buffers that are sized together, in one allocation: a fresh workspace pays for
+// one cudaMalloc instead of one a buffer (0.1-0.3 ms each). Growth discards
+// the contents of all of them.
+struct DevBufSet {
+	DevBuf whole;
+	std::vector<std::pair<DevBuf *, size_t>> want;
+	std::vector<DevBuf *> members;           // every buffer that may lie in `whole`
+	void add(DevBuf &b, size_t n) { want.emplace_back(&b, n); }
+	void reserve();               // makes every added buffer as large as asked and clears the list
 };
 
 // ---- quadrature tables on the device -----------------------------------------
@@ -85,6 +98,7 @@ struct Workspace {
 	int prec = 64;                           // working precision of the collision operator: 64 (FP64) or 32 (FP32 form)
 	int conserve = 0;                        // restore the collision invariants after each velocity-space collision step
 	cudaStream_t stream = nullptr;           // own stream (upstream API calls)
+	DevBufSet scratch;                       // one allocation for the buffers of the next line (but wmid)
 	DevBuf What, WhatQ, i1cc, i1i4, i2p, i2s, i3p, i3s, i3z, i3zsum, i3zs, i3y, fs, fs4, wmid;      // collision scratch
 	DevBuf fa, fb, va, vb;                   // state scratch (Fourier / velocity)
 	DevBuf io_in, io_out, bext, vgrid;       // staging for host-pointer calls
