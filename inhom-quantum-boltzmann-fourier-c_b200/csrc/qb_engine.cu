@@ -285,11 +285,11 @@ int best_chunks(long units, int nterms, int slots, int max_chunks, double penalt
 	return best;
 }
 
-template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C *out, cudaStream_t s, C *out2 = nullptr) {
+template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C *out, cudaStream_t s, C *out2 = nullptr, float *outr = nullptr) {
 	static DeviceFlag init;
 	if (!init) { set_smem(k_pad_fft<P, C>, smem_grids<P, C>(1)); init = true; }
 	ProfScope ps("pad_fft", s);
-	k_pad_fft<P, C><<<ngrids, Geo<P>::NT, smem_grids<P, C>(1), s>>>(src, out, out2);
+	k_pad_fft<P, C><<<ngrids, Geo<P>::NT, smem_grids<P, C>(1), s>>>(src, out, out2, outr);
 	QB_CUDA(cudaGetLastError());
 }
 
@@ -334,13 +334,13 @@ template <int P, int CS, class C> void launch_i3(const I3ParamsT<C> &p, long ncl
 	QB_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
 }
 
-// I3 kernels of the FP32 form at N = 32 (k_i3p) and N = 64 (k_i3_full128:
+// I3 kernels of the FP32 form at N = 32 (k_i3w) and N = 64 (k_i3_full128:
 // 2-CTA clusters, a whole grid per CTA, all 512 tensor-memory columns per CTA,
 // so exactly one CTA per SM, checked).  By default the cells whose Nyquist
-// content is at most kRealFormBound take the real forms (k_i3pr,
+// content is at most kRealFormBound take the real forms (k_i3wr,
 // k_i3_full128r) and the others the complex kernels.  QB_I3_KERNEL selects one
 // kernel for every cell instead (for comparisons): "complex" the complex
-// kernels, "pair" the complex k_i3p and the pair-split k_i3_128.
+// kernels, "pair" the complex k_i3w and the pair-split k_i3_128.
 inline const char *i3_kernel_env() {
 	static const char *e = getenv("QB_I3_KERNEL");
 	return e ? e : "";
@@ -388,97 +388,55 @@ inline void scale_chunks(const Workspace &ws, const QuadSet &q, Chunks &ch, int 
 }
 
 constexpr double kRealFormBound = 1e-6;
-// The real forms pack the combos of an output in pairs.  Both callers of the
-// I3 sums (the Cd assembly and the single-integral path) set 4 combos per
-// output, so this holds today; it guards the real-form launch against a
-// future caller with an odd count, which then takes the complex kernel.
-template <class C> bool even_combos(const I3ParamsT<C> &p) {
-	for (int r = 0; r < 4; r++)
-		if (p.ncombo[r] & 1) return false;
-	return true;
-}
-
 void launch_nyquist_kind(int N, int ncells, const double2 *W, double bound, int *kind, unsigned long long *stats, cudaStream_t s) {
 	ProfScope ps("nyquist_kind", s);
 	k_nyquist_kind<<<ncells, kNyqThreads, 0, s>>>(N, W, bound, kind, stats);
 	QB_CUDA(cudaGetLastError());
 }
 
-// k_i3p (P = 64): 2-CTA clusters, TMEM accumulators.  The allocation of
-// I3Tmem<C>::NCOLS columns never waits as long as no more CTAs share an SM
-// than its 512 columns hold; the shared-memory (FP64) or register (FP32)
-// footprint keeps it at one CTA per SM, checked here before the first launch.
-// three grids and the twiddles; in FP32 two more grids receive the partner's P grids
-template <class C> size_t i3p_smem() {
-	return sizeof(C) * ((size_t)(sizeof(C) == 8 ? 5 : 3) * Geo<64, C>::GRID + 64);
-}
-// the real form receives the partner's packed P grid in its second grid slot
-inline size_t i3pr_smem() { return sizeof(float2) * ((size_t)3 * Geo<64, float2>::GRID + 64); }
-
-template <class C> int active_i3p_clusters() {
-	static DeviceInt cached{-1};
-	if (cached < 0) {
-		check_tmem_coresidency();
-		auto kern = k_i3p<64, C>;
-		set_smem(kern, i3p_smem<C>());
-		int per_sm = 0;
-		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Geo<64>::NT, i3p_smem<C>()));
-		if (per_sm * (int)I3Tmem<C>::ALLOC > 512)
-			QB_FAIL("k_i3p: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
-		cudaLaunchConfig_t cfg = {};
-		cfg.gridDim = dim3(2);
-		cfg.blockDim = dim3(Geo<64>::NT);
-		cfg.dynamicSmemBytes = i3p_smem<C>();
-		cudaLaunchAttribute attr;
-		attr.id = cudaLaunchAttributeClusterDimension;
-		attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-		cfg.attrs = &attr;
-		cfg.numAttrs = 1;
-		int n = 0;
-		if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-			cudaGetLastError();
-			n = std::max(1, num_sms() / 2);
-		}
-		cached = n;
+// k_i3w and k_i3wr (P = 64): 2-CTA clusters, accumulators in tensor memory. Their
+// allocations never wait as long as no more CTAs share an SM than its 512
+// columns hold (one CTA an SM in FP64, two in FP32), checked here before the
+// first launch. Clusters resident on the GPU (occupancy query).
+template <class K> int i3w_clusters(K kern, size_t smem, int cols, const char *name) {
+	check_tmem_coresidency();
+	set_smem(kern, smem);
+	int per_sm = 0;
+	QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, smem));
+	if (per_sm * cols > 512)
+		QB_FAIL(std::string(name) + ": " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(2);
+	cfg.blockDim = dim3(512);
+	cfg.dynamicSmemBytes = smem;
+	cudaLaunchAttribute attr;
+	attr.id = cudaLaunchAttributeClusterDimension;
+	attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	int n = 0;
+	if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+		cudaGetLastError();
+		n = std::max(1, num_sms() / 2);
 	}
+	return n;
+}
+template <class C> int active_i3w_clusters() {
+	static DeviceInt cached{-1};
+	if (cached < 0) cached = i3w_clusters(k_i3w<C>, i3w_smem<C>(), (int)WideTmem<sizeof(C) / 4>::COLS, "k_i3w");
 	return cached;
 }
-
-int active_i3w_clusters() {
+int active_i3wr_clusters() {
 	static DeviceInt cached{-1};
-	if (cached < 0) {
-		check_tmem_coresidency();
-		auto kern = k_i3w<double2>;
-		const size_t smem = i3w_smem<double2>();
-		set_smem(kern, smem);
-		int per_sm = 0;
-		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, smem));
-		if (per_sm * (int)WideTmem::COLS > 512)
-			QB_FAIL("k_i3w: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
-		cudaLaunchConfig_t cfg = {};
-		cfg.gridDim = dim3(2);
-		cfg.blockDim = dim3(512);
-		cfg.dynamicSmemBytes = smem;
-		cudaLaunchAttribute attr;
-		attr.id = cudaLaunchAttributeClusterDimension;
-		attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-		cfg.attrs = &attr;
-		cfg.numAttrs = 1;
-		int n = 0;
-		if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-			cudaGetLastError();
-			n = std::max(1, num_sms() / 2);
-		}
-		cached = n;
-	}
+	if (cached < 0) cached = i3w_clusters(k_i3wr, i3w_smem<float2>(), (int)WideTmem<1>::COLS, "k_i3wr");
 	return cached;
 }
-void launch_i3w(const I3ParamsT<double2> &p, long nclusters, double2 *pscr, cudaStream_t s) {
-	active_i3w_clusters();                     // attribute + occupancy check
+template <class... KA, class... A>
+void launch_pairs(void (*kern)(KA...), long nclusters, size_t smem, cudaStream_t s, A... args) {
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3((unsigned)(nclusters * 2));
 	cfg.blockDim = dim3(512);
-	cfg.dynamicSmemBytes = i3w_smem<double2>();
+	cfg.dynamicSmemBytes = smem;
 	cfg.stream = s;
 	cudaLaunchAttribute attr;
 	attr.id = cudaLaunchAttributeClusterDimension;
@@ -486,51 +444,15 @@ void launch_i3w(const I3ParamsT<double2> &p, long nclusters, double2 *pscr, cuda
 	cfg.attrs = &attr;
 	cfg.numAttrs = 1;
 	ProfScope ps("i3_cluster", s);
-	QB_CUDA(cudaLaunchKernelEx(&cfg, k_i3w<double2>, p, pscr));
+	QB_CUDA(cudaLaunchKernelEx(&cfg, kern, KA(args)...));
 }
-
-template <class C> void launch_i3p(const I3ParamsT<C> &p, long nclusters, const int *kind, cudaStream_t s) {
-	active_i3p_clusters<C>();                  // attribute + occupancy check
-	auto kern = k_i3p<64, C>;
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned)(nclusters * 2));
-	cfg.blockDim = dim3(Geo<64>::NT);
-	cfg.dynamicSmemBytes = i3p_smem<C>();
-	cfg.stream = s;
-	cudaLaunchAttribute attr;
-	attr.id = cudaLaunchAttributeClusterDimension;
-	attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-	cfg.attrs = &attr;
-	cfg.numAttrs = 1;
-	ProfScope ps("i3_cluster", s);
-	QB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, kind));
+template <class C> void launch_i3w(const I3ParamsT<C> &p, long nclusters, C *pscr, const int *kind, cudaStream_t s) {
+	active_i3w_clusters<C>();                  // attribute + occupancy check
+	launch_pairs(k_i3w<C>, nclusters, i3w_smem<C>(), s, p, pscr, kind);
 }
-
-// the real form at P = 64 (FP32): same shared memory as k_i3p, 128 tensor-memory columns
-void launch_i3pr(const I3ParamsT<float2> &p, long nclusters, const int *kind, cudaStream_t s) {
-	static DeviceFlag init;
-	auto kern = k_i3pr<64>;
-	if (!init) {
-		check_tmem_coresidency();
-		set_smem(kern, i3pr_smem());
-		int per_sm = 0;
-		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Geo<64>::NT, i3pr_smem()));
-		if (per_sm * (int)I3TmemR::ALLOC > 512)
-			QB_FAIL("k_i3pr: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
-		init = true;
-	}
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned)(nclusters * 2));
-	cfg.blockDim = dim3(Geo<64>::NT);
-	cfg.dynamicSmemBytes = i3pr_smem();
-	cfg.stream = s;
-	cudaLaunchAttribute attr;
-	attr.id = cudaLaunchAttributeClusterDimension;
-	attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-	cfg.attrs = &attr;
-	cfg.numAttrs = 1;
-	ProfScope ps("i3_cluster", s);
-	QB_CUDA(cudaLaunchKernelEx(&cfg, kern, p, kind));
+void launch_i3wr(const I3ParamsT<float2> &p, long nclusters, const float *WhR, float *pscr, const int *kind, cudaStream_t s) {
+	active_i3wr_clusters();                    // attribute + occupancy check
+	launch_pairs(k_i3wr, nclusters, i3w_smem<float2>(), s, p, WhR, pscr, kind);
 }
 
 template <int P, class C> void launch_fft_full(const FullParamsT<C> &p, long ngrids, cudaStream_t s) {
@@ -649,7 +571,7 @@ int resident_i3(int N, bool f32) {
 	switch (N) {
 	case 8: return f32 ? active_i3q<16, float2>() : active_i3q<16, double2>();
 	case 16: return f32 ? active_i3q<32, float2>() : active_i3q<32, double2>();
-	default: return f32 ? active_i3p_clusters<float2>() : active_i3w_clusters();
+	default: return f32 ? active_i3w_clusters<float2>() : active_i3w_clusters<double2>();
 	}
 }
 
@@ -658,15 +580,20 @@ template <int P, class C> struct Rhs {
 	static constexpr long NN = (long)N * N, PP = (long)P * P;
 	using T = Tab<C>;
 
+	// the spectra in thread order, and in FP32 their real parts
+	static size_t wide_bytes(int ncells) { return (sizeof(C) + (sizeof(C) == 8 ? sizeof(float) : 0)) * 4 * ncells * PP; }
+
 	// spectra of the four components
 	static void spectra(Workspace &ws, int ncells, const double2 *W, cudaStream_t s) {
 		ws.What.ensure(sizeof(C) * 4 * ncells * PP);
-		C *wide = nullptr;                      // the copy that k_i3w reads
-		if (P == 64 && sizeof(C) == 16) {
-			ws.WhatQ.ensure(sizeof(C) * 4 * ncells * PP);
+		C *wide = nullptr;                      // the copies that k_i3w and k_i3wr read
+		float *real = nullptr;
+		if (P == 64) {
+			ws.WhatQ.ensure(wide_bytes(ncells));
 			wide = ws.WhatQ.as<C>();
+			if (sizeof(C) == 8) real = reinterpret_cast<float *>(wide + 4 * ncells * PP);
 		}
-		launch_pad_fft<P>(4 * ncells, W, ws.What.as<C>(), s, wide);
+		launch_pad_fft<P>(4 * ncells, W, ws.What.as<C>(), s, wide, real);
 	}
 
 	// S sums for Cc (tasks g = W_1..W_3, F = -4 W^_0 + 2) or I4 (g = W_0..W_3, F = 2 W^_0 - 1)
@@ -711,7 +638,7 @@ template <int P, class C> struct Rhs {
 	static bool sum_i2(int nchunk, int ncells) { return nchunk >= kSumSlots && 4 * ncells <= 65535; }
 
 	// the terms of opposite shifts are summed together (I3Units), except by the
-	// tensor-core form; each CTA of the clusters of k_i3p and k_i3pr leaves its
+	// tensor-core form; each CTA of the clusters of k_i3w and k_i3wr leaves its
 	// own partial of the Z sums
 	static constexpr int kZRanks = P == 64 ? 2 : 1;
 	static bool pairs_units(const Workspace &ws) { return !(P == 32 && sizeof(C) == 8 && ws.i3_variant == 1); }
@@ -749,26 +676,21 @@ template <int P, class C> struct Rhs {
 		p.out = ws.i3p.as<C>();
 		p.err = ws.kerr.as<int>();
 		if constexpr (P == 64) {
+			const long ncl = p.rg.nslots > 0 ? (long)p.rg.nslots : (long)ncells * nchunk;
+			ws.i3y.ensure(sizeof(C) * ncl * 8 * PP);
+			p.Ghat = ws.WhatQ.as<C>();
+			const int *kind = nullptr;
 			if constexpr (sizeof(C) == 8) {
-				if (use_real_form() && even_combos(p)) {
+				if (use_real_form()) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
 					ws.i3zs.ensure(sizeof(C) * slots * kZRanks * 2 * (N + 1) * (N + 1));
 					p.zscr = ws.i3zs.as<C>();
-					int *kind = ws.i3kind.as<int>();
-					launch_nyquist_kind(P / 2, ncells, W, kRealFormBound, kind, ws.i3stats.as<unsigned long long>(), s);
-					launch_i3pr(p, (long)ncells * nchunk, kind, s);
-					launch_i3p<C>(p, (long)ncells * nchunk, kind, s);       // cells above the bound
-					return;
+					launch_nyquist_kind(P / 2, ncells, W, kRealFormBound, ws.i3kind.as<int>(), ws.i3stats.as<unsigned long long>(), s);
+					kind = ws.i3kind.as<int>();
+					launch_i3wr(p, ncl, reinterpret_cast<const float *>(ws.WhatQ.as<C>() + 4 * ncells * PP), ws.i3y.as<float>(), kind, s);
 				}
 			}
-			if constexpr (sizeof(C) == 16) {
-				const long ncl = p.rg.nslots > 0 ? (long)p.rg.nslots : (long)ncells * nchunk;
-				ws.i3y.ensure(sizeof(C) * ncl * 8 * PP);
-				p.Ghat = ws.WhatQ.as<C>();
-				launch_i3w(p, ncl, ws.i3y.as<C>(), s);
-			} else {
-				launch_i3p<C>(p, (long)ncells * nchunk, nullptr, s);
-			}
+			launch_i3w<C>(p, ncl, ws.i3y.as<C>(), kind, s);      // FP32: the cells above the bound
 		} else {
 			if constexpr (P == 32 && sizeof(C) == 8) {
 				if (ws.i3_variant == 1) {
@@ -785,7 +707,7 @@ template <int P, class C> struct Rhs {
 		DevBufSet &b = ws.scratch;
 		const size_t g = sizeof(C) * (size_t)ncells * PP;
 		b.add(ws.What, 4 * g);
-		if (P == 64 && sizeof(C) == 16) b.add(ws.WhatQ, 4 * g);
+		if (P == 64) b.add(ws.WhatQ, wide_bytes(ncells));
 		if (parts & RHS_CC) {
 			b.add(ws.i1cc, 3 * ch.i1 * g);
 			b.add(ws.fs, 3 * g);
@@ -803,7 +725,8 @@ template <int P, class C> struct Rhs {
 			}
 			b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
 			if (pairs_units(ws)) b.add(ws.i3z, sizeof(C) * slots * kZRanks * 4 * NN);
-			if (P == 64 && sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 8 * PP);
+			if (P == 64) b.add(ws.i3y, sizeof(C) * used * 8 * PP);
+			if (P == 64 && sizeof(C) == 8 && use_real_form()) b.add(ws.i3zs, sizeof(C) * slots * kZRanks * 2 * (N + 1) * (N + 1));
 			if (used >= (size_t)kSumSlots * ncells) {
 				b.add(ws.i3s, 4 * g);
 				if (pairs_units(ws)) b.add(ws.i3zsum, g);
@@ -820,11 +743,11 @@ template <int P, class C> struct Rhs {
 			ch.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), num_sms(), 256, 0.15);      // one CTA per SM
 		}
 		scale_chunks(ws, q, ch, q.i3 ? i3_count(ws, *q.i3) : 0);
-		// FP64 at N = 32: every resident cluster of k_i3p takes one contiguous range
+		// FP64 at N = 32: every resident cluster of k_i3w takes one contiguous range
 		// of the (cell, term) work, one partial per cell it touches
 		const bool ranges = ws.i3_ranges >= 0 ? ws.i3_ranges == 1 : term_ranges_enabled();
 		if (P == 64 && sizeof(C) == 16 && q.i3 && q.i3->nterms > 0 && ranges)
-			ch.i3_slots = (int)std::min<long>(active_i3w_clusters(), (long)ncells * i3_count(ws, *q.i3));
+			ch.i3_slots = (int)std::min<long>(active_i3w_clusters<C>(), (long)ncells * i3_count(ws, *q.i3));
 		reserve(ws, q, ncells, ch, parts);
 		spectra(ws, ncells, W, s);
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
@@ -1070,9 +993,9 @@ void check_tmem_coresidency() {
 	static DeviceFlag done;
 	if (done) return;
 	std::vector<TmemKernel> ks = {
-		{ (const void *)k_i3w<double2>, i3w_smem<double2>(), 512, (int)WideTmem::COLS, "k_i3w" },
-		{ (const void *)k_i3p<64, float2>, i3p_smem<float2>(), Geo<64>::NT, (int)I3Tmem<float2>::ALLOC, "k_i3p<f32>" },
-		{ (const void *)k_i3pr<64>, i3pr_smem(), Geo<64>::NT, (int)I3TmemR::ALLOC, "k_i3pr" },
+		{ (const void *)k_i3w<double2>, i3w_smem<double2>(), 512, (int)WideTmem<4>::COLS, "k_i3w<f64>" },
+		{ (const void *)k_i3w<float2>, i3w_smem<float2>(), 512, (int)WideTmem<2>::COLS, "k_i3w<f32>" },
+		{ (const void *)k_i3wr, i3w_smem<float2>(), 512, (int)WideTmem<1>::COLS, "k_i3wr" },
 		{ (const void *)k_i3_quad, Quad128::SMEM, Quad128::NT, Quad128::TCOLS, "k_i3_quad" },
 		{ (const void *)k_i3_128<4, kI3Pairs128, float2>, smem_i3_128<float2>(), G128::NT,
 		  (int)I3Tmem128<float2, 4 / kI3Pairs128>::NCOLS, "k_i3_128<f32>" },
@@ -1230,7 +1153,7 @@ template <class C> struct Rhs<128, C> {
 		if constexpr (sizeof(C) == 8) {
 			if (use_full128()) {
 				ws.i3y.ensure(sizeof(C) * ncl * 2 * PP);
-				if (use_real_form() && even_combos(p)) {
+				if (use_real_form() ) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
 					ws.i3zs.ensure(sizeof(C) * ncl * 2 * 2 * (N + 1) * (N + 1));
 					p.zscr = ws.i3zs.as<C>();

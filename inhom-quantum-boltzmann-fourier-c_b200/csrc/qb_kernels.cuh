@@ -146,9 +146,10 @@ __device__ __forceinline__ void smem_to_global(C *__restrict__ out, const C *S) 
 
 // ---------------------------------------------------------------------------
 // K1: padded forward spectra  out[b] = FFT2(Pad(src[b]))   (one CTA per grid);
-// out2 (may be null, P = 64): the same in the thread order of k_i3w
+// out2 (may be null, P = 64): the same in the thread order of k_i3w; outr (may be
+// null): its real parts in that order
 template <int P, class C>
-__global__ void __launch_bounds__(Geo<P>::NT) k_pad_fft(const double2 *__restrict__ src, C *__restrict__ out, C *__restrict__ out2) {
+__global__ void __launch_bounds__(Geo<P>::NT) k_pad_fft(const double2 *__restrict__ src, C *__restrict__ out, C *__restrict__ out2, float *__restrict__ outr) {
 	using G = Geo<P, C>;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	C *S = reinterpret_cast<C *>(smem_raw), *tw = S + G::GRID;
@@ -158,7 +159,11 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_pad_fft(const double2 *__restric
 	fft2_pad<P, -1>(S, tw, src + b * G::N * G::N, MulNone<C>{});
 	smem_to_global<P>(out + b * P * P, S);
 	if (P == 64 && out2 != nullptr)
-		for (int i = threadIdx.x; i < P * P; i += G::NT) out2[b * P * P + i] = S[G::at((i & 255) >> 2, (i & 3) + 4 * (i >> 8))];
+		for (int i = threadIdx.x; i < P * P; i += G::NT) {
+			const C v = S[G::at((i & 255) >> 2, (i & 3) + 4 * (i >> 8))];
+			out2[b * P * P + i] = v;
+			if (outr != nullptr) outr[b * P * P + i] = (float)v.x;
+		}
 }
 
 // ---------------------------------------------------------------------------
@@ -729,587 +734,6 @@ __device__ __forceinline__ void tmem_st8r(unsigned taddr, const float (&v)[8]) {
 	for (int e = 0; e < 8; e++) r[e] = __float_as_uint(v[e]);
 	asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
 	             :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-
-// length-L transform with the lane's twiddle powers w_L^(tau q), q = 1..4
-// (forward sign), read from tensor memory at taddr (4 complex FP64 values);
-// w^5..w^7 = w^4 w^1..w^3.  The load is issued before the first radix-8
-// stage and waited for after it.
-template <int L, int DIR, class Acc>
-__device__ __forceinline__ void fft1d_acct(double2 (&x)[8], int tau, const Acc &sc, unsigned taddr) {
-	double2 w[4];
-	tmem_ld4(taddr, w);
-	dft8<DIR>(x);
-	tmem_wait_ld();
-	if (DIR > 0) {
-#pragma unroll
-		for (int q = 0; q < 4; q++) w[q].y = -w[q].y;
-	}
-#pragma unroll
-	for (int q = 1; q <= 4; q++) x[q] = cmul(x[q], w[q - 1]);
-#pragma unroll
-	for (int q = 5; q < 8; q++) x[q] = cmul(x[q], cmul(w[3], w[q - 5]));
-	fft1d_tail<L, DIR>(x, tau, sc);
-}
-
-// the lane's twiddle powers computed once per kernel: FP32 in registers (wp,
-// fft1d_accw), FP64 in tensor memory (registers are exhausted there; the
-// loads replace the six complex multiplies of the power recurrence and add
-// no shared-memory traffic)
-template <int L, int DIR, class C, class Acc>
-__device__ __forceinline__ void fft1d_lane(C (&x)[8], int tau, const Acc &sc, const C (&wp)[8], unsigned twaddr) {
-	if constexpr (sizeof(C) == 8) fft1d_accw<L, DIR>(x, tau, sc, wp);
-	else fft1d_acct<L, DIR>(x, tau, sc, twaddr);
-}
-
-// TMEM accumulators of k_i3p: 2 outputs x 8 values per thread
-template <class C> struct I3Tmem {
-	static constexpr unsigned WPC = sizeof(C) / 4;            // 32-bit columns per complex value
-	static constexpr unsigned PER_THREAD = 2 * 8 * WPC;       // columns of one thread's slice
-	static constexpr unsigned NCOLS = 4 * PER_THREAD;         // 4 warps share a lane quarter: 256 (FP64), 128 (FP32)
-	// after the accumulators each thread keeps its 8 psi2 values of the current
-	// term, 8 values of the current Y_i and (FP64) its twiddle powers w^1..w^4;
-	// columns a slot: 16 / 32 / 16 (FP64), 8 / 16 (FP32)
-	static constexpr unsigned ALLOC = sizeof(C) == 16 ? 512 : 256;
-	// column address of value e of output q of this thread
-	__device__ __forceinline__ static unsigned addr(unsigned base, int q, int e) {
-		const unsigned w = threadIdx.x >> 5;
-		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * PER_THREAD + (unsigned)(q * 8 + e) * WPC;
-	}
-	static constexpr unsigned PSI = 8 * WPC / 2, YI = 8 * WPC;   // columns a slot
-	__device__ __forceinline__ static unsigned lanes() { return (32u * ((threadIdx.x >> 5) & 3u)) << 16; }
-	__device__ __forceinline__ static unsigned slot() { return threadIdx.x >> 7; }
-	__device__ __forceinline__ static unsigned psiaddr(unsigned base) { return base + lanes() + NCOLS + slot() * PSI; }
-	__device__ __forceinline__ static unsigned yaddr(unsigned base) { return base + lanes() + NCOLS + 4 * PSI + slot() * YI; }
-	__device__ __forceinline__ static unsigned twaddr(unsigned base) { return base + lanes() + NCOLS + 4 * (PSI + YI) + slot() * 16u; }
-};
-
-// FP32 at P = 64: each CTA of the pair pushes its P grids of the term into the
-// partner's shared memory by bulk copies (cp.async.bulk between the pair's
-// shared memories, completing on the partner's mbarrier), so that every P_a
-// of the chains is read from local shared memory.  push_issue sends `bytes`
-// of the own grids at `own` to `peer_copy` in the partner, after the CTA
-// barrier that follows the grid's transform (the partner has finished reading
-// its copy of the previous term: a cluster barrier ends every term).
-// push_wait waits for the partner's copies before the chains (bounded: a wait
-// that runs out sets the error word).  push_release keeps the copies' sources
-// until they have been read, before the next term overwrites them.
-__device__ __forceinline__ uint32_t smem_u32a(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// `expect` > 0: this CTA's arrival on its own mbarrier for the term, expecting
-// that many bytes from the partner (the first of the term's copies)
-__device__ __forceinline__ void push_issue(const void *own, void *peer_copy, uint32_t bytes, uint64_t *mbar, int prank,
-                                           uint32_t expect) {
-	if (threadIdx.x == 0) {
-		const uint32_t mb = smem_u32a(mbar);
-		uint32_t dst, mbr;
-		asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32a(peer_copy)), "r"(prank));
-		asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(mbr) : "r"(mb), "r"(prank));
-		if (expect > 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(expect) : "memory");
-		asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-		             "r"(smem_u32a(own)), "r"(bytes), "r"(mbr) : "memory");
-		asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-	}
-}
-__device__ __forceinline__ void push_wait(uint64_t *mbar, unsigned &phase, int *err) {
-	const uint32_t mb = smem_u32a(mbar);
-	bool ok = false;
-	for (unsigned i = 0; i < (1u << 24) && !ok; i++) {
-		uint32_t done = 0;
-		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-		             : "=r"(done) : "r"(mb), "r"(phase) : "memory");
-		ok = done != 0;
-	}
-	if (!ok && err != nullptr && (threadIdx.x & 31) == 0) atomicExch(err, 1);
-	phase ^= 1u;
-}
-__device__ __forceinline__ void push_release() {
-	if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-__device__ __forceinline__ void push_init(uint64_t *mbar) {
-	if (threadIdx.x == 0) {
-		asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32a(mbar)) : "memory");
-		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-	}
-}
-__device__ __forceinline__ void fence_async_smem_a() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// ---------------------------------------------------------------------------
-// K4p: the I3 sums of the collision operator on a cluster of 2 CTAs, CTA r
-// holding components 2r and 2r + 1: per term it computes both spectra
-// P_{t,c} = FFT2(Pad(psi1_t . W_c)) into its shared memory and, after a
-// cluster barrier, the 8 (pair, combo) chains of its two outputs
-//   X_j += eta_i P_i . T_ij,  T_ij = FFT2(psi2_t . IFFT2(W^_i . P_j)),  j in {2r, 2r + 1}
-// with P_i of the partner's components read through distributed shared
-// memory.  The chains run with i outermost: for a pair of opposite shifts
-// (I3Units) the CTA adds its two terms of Y_i = sum_j eta_j W^_j . T_ij, takes
-// IFFT2(Y_i) (every row, the columns that Extract keeps) and adds conj(psi1) .
-// Extract of it to its partial of Z_i; the two CTAs' partials are summed by
-// the assembly, which costs 4 extra transforms of 12 passes against 32 for the
-// chains but no exchange between the CTAs.  The two 8-value accumulators of every thread live in TMEM, which
-// frees their registers and lets 2-CTA clusters use all 148 SMs (4-CTA
-// clusters of k_i3 fit 33 of 37 four-SM slots).  The rest of the TMEM
-// allocation caches values each thread reuses at its own positions: its psi2
-// values of the current term (one L2 read for the term's 8 chains), its P_j
-// values of the current output (one shared-memory read for the output's 4
-// chains) and, in FP64, its twiddle powers (FP32 keeps them in registers).
-// Output as k_i3 with CS = 4.
-//
-// kind: null (every cell) or the per-cell form of k_nyquist_kind; this kernel
-// then takes the cells of kind 1 (the real form k_i3pr takes kind 0).
-template <int P, class C>
-__global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3p(const I3ParamsT<C> p, const int *kind) {
-	using G = Geo<P, C>;
-	using Lp = Len<P>;
-	using R = typename CT<C>::R;
-	using TM = I3Tmem<C>;
-	constexpr bool kPush = sizeof(C) == 8;                   // FP32: the partner's P grids copied in (Pr)
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__shared__ unsigned tmem_slot;
-	__shared__ __align__(8) uint64_t pmbar;
-	unsigned pphase = 0;
-	C *Pq = reinterpret_cast<C *>(smem_raw);                 // P of components 2r, 2r + 1 (2 grids)
-	C *Ug = Pq + 2 * G::GRID, *tw = Pq + 3 * G::GRID;
-	C *Pr = tw + P;                                          // FP32: the partner's 2 P grids
-	cg::cluster_group cluster = cg::this_cluster();
-	const int rank = (int)cluster.block_rank();
-	const long cid = blockIdx.x / 2;
-	// work of this cluster: terms [u, u1) of the flattened (cell, term) order
-	long u, u1;
-	if (p.rg.nslots > 0) {
-		u = p.rg.start((int)cid);
-		u1 = p.rg.start((int)cid + 1);
-	} else {
-		const int chunk = (int)(cid % p.nchunk);
-		const long cell = cid / p.nchunk;
-		if (kind != nullptr && kind[cell] != 1) return;     // both CTAs of the cluster leave before any barrier
-		u = cell * p.nterms + (long)chunk * p.nterms / p.nchunk;
-		u1 = cell * p.nterms + (long)(chunk + 1) * p.nterms / p.nchunk;
-	}
-	const int warp = threadIdx.x >> 5;
-	if (warp == 0) tmem_alloc(&tmem_slot, TM::ALLOC);
-	init_twiddles<P>(tw);
-	tmem_fence_before();
-	__syncthreads();
-	tmem_fence_after();
-	const unsigned tbase = tmem_slot;
-	const int line = threadIdx.x / G::T, tau = threadIdx.x % G::T;
-	C wp[8];
-	const unsigned twaddr = TM::twaddr(tbase);
-	if constexpr (sizeof(C) == 8) {
-#pragma unroll
-		for (int q = 0; q < 8; q++) wp[q] = tw[(tau * q) & (P - 1)];
-	} else {
-		double2 a[4];
-#pragma unroll
-		for (int q = 0; q < 4; q++) a[q] = tw[(tau * (q + 1)) & (P - 1)];
-		tmem_st4(twaddr, a);
-	}
-	C *Ppeer = cluster.map_shared_rank(Pq, rank ^ 1);
-	if constexpr (kPush) {
-		push_init(&pmbar);
-		cluster.sync();                                      // the partner's mbarrier is initialised
-	}
-	// one segment per cell of the range (the (cell, chunk) grid has one)
-#pragma unroll 1
-	while (u < u1) {
-	const long cell = u / p.nterms;
-	const int t0 = (int)(u % p.nterms);
-	const int t1 = (int)min((long)p.nterms, t0 + (u1 - u));
-	u += t1 - t0;
-#pragma unroll
-	for (int q = 0; q < 2; q++)
-#pragma unroll
-		for (int e = 0; e < 8; e++) tmem_st(TM::addr(tbase, q, e), czero<C>());
-	tmem_wait_st();
-	const C *Gcell = p.Ghat + cell * p.g_cell;
-	// partial sums of this segment: slot (cluster, cell) of the ranges, or (cell, chunk)
-	const long slot = p.rg.nslots > 0 ? cid * p.rg.maxc + (cell - p.rg.first_cell((int)cid))
-	                                  : cell * p.nchunk + (int)(cid % p.nchunk);
-	// the extracted points of column `line` this thread owns: rows tau + 8 e, e = 0, 1, 6, 7
-	const bool zcol = G::src(line) >= 0;
-	const int zofs = tau * G::N + G::src(line);
-	C *zbase = p.zout + (slot * 2 + rank) * 4 * (long)G::N * G::N + zofs;
-	if (zcol) {
-#pragma unroll 1
-		for (int i = 0; i < 4; i++)
-#pragma unroll
-			for (int e = 0; e < 4; e++) zbase[(i * G::N + 8 * e) * G::N] = czero<C>();
-	}
-	for (int un = t0; un < t1; un++) {
-		const int t = p.un.term(un);
-		const bool pr = p.un.pair(un);
-#pragma unroll 1
-		for (int q = 0; q < 2; q++) {
-			const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank + q] * G::N * G::N;
-			fft2_pad<P, -1>(Pq + q * G::GRID, tw, src, MulCplx<C>{p.psi1 + (long)t * G::N * G::N});
-			if constexpr (kPush) {
-				// FP32: each grid goes to the partner as soon as it is complete, the
-				// first copy overlapping the second transform
-				fence_async_smem_a();
-				__syncthreads();
-				push_issue(Pq + q * G::GRID, Pr + q * G::GRID, (uint32_t)(G::GRID * sizeof(C)), &pmbar, rank ^ 1,
-				           q == 0 ? (uint32_t)(2 * G::GRID * sizeof(C)) : 0u);
-			}
-		}
-		if constexpr (!kPush) cluster.sync();
-		const R *psi2 = p.psi2T + (long)p.psi2_idx[t] * P * P;
-		const R sc = (R)p.psi2_scale[t];
-		{
-			// this thread's psi2 values of the term (column line, rows out_pos(tau, e)), read
-			// once from L2 for the term's 8 chains; the previous term's reads of the slot
-			// have completed (tcgen05.wait::ld in every chain)
-			R f[8];
-#pragma unroll
-			for (int e = 0; e < 8; e++) f[e] = sc * psi2[line * P + Lp::out_pos(tau, e)];
-			tmem_st8r(TM::psiaddr(tbase), f);
-			tmem_wait_st();
-		}
-		if constexpr (kPush) push_wait(&pmbar, pphase, p.err);
-#pragma unroll 1
-		for (int i = 0; i < 4; i++) {
-			const C *Gg = Gcell + (long)i * P * P;
-			const C *Pa = ((i >> 1) == rank ? Pq : (kPush ? Pr : Ppeer)) + (i & 1) * G::GRID;
-			const R coef = (R)(i == 0 ? 1.0 : -1.0);
-			C x[8];
-#pragma unroll 1
-			for (int q = 0; q < 2; q++) {
-				const C *Pj = Pq + q * G::GRID;
-				// rows: IFFT of W^_i . P_j
-				{
-					C g[8];
-#pragma unroll
-					for (int r = 0; r < 8; r++) g[r] = Gg[line * P + tau + G::T * r];
-#pragma unroll
-					for (int r = 0; r < 8; r++) x[r] = cmul(g[r], Pj[G::at(line, tau + G::T * r)]);
-				}
-				fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, twaddr);
-#pragma unroll
-				for (int e = 0; e < 8; e++) Ug[G::at(line, Lp::out_pos(tau, e))] = x[e];
-				__syncthreads();
-				// columns: IFFT, multiply by psi2_t, FFT
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(tau + G::T * r, line)];
-				fft1d_lane<P, +1>(x, tau, G::col(Ug, line), wp, twaddr);
-				{
-					R f[8];
-					tmem_ld8r(TM::psiaddr(tbase), f);
-					tmem_wait_ld();
-#pragma unroll
-					for (int e = 0; e < 8; e++) { x[e].x *= f[e]; x[e].y *= f[e]; }
-				}
-				out_to_in_acc<P>(x, tau, G::col(Ug, line));
-				fft1d_lane<P, -1>(x, tau, G::col(Ug, line), wp, twaddr);
-#pragma unroll
-				for (int e = 0; e < 8; e++) Ug[G::at(Lp::out_pos(tau, e), line)] = x[e];
-				__syncthreads();
-				// rows: FFT; X_j += eta_i P_i . T_ij in TMEM (P_i own or the partner's)
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(line, tau + G::T * r)];
-				fft1d_lane<P, -1>(x, tau, G::row(Ug, line), wp, twaddr);
-				{
-					C acc[8];
-					if constexpr (sizeof(C) == 16) tmem_ld8(TM::addr(tbase, q, 0), acc);   // one load (FP64); FP32 per value measured faster
-					else {
-#pragma unroll
-						for (int e = 0; e < 8; e++) tmem_ld(TM::addr(tbase, q, e), acc[e]);
-					}
-					tmem_wait_ld();
-#pragma unroll
-					for (int e = 0; e < 8; e++) {
-						const C v = cmul(Pa[G::at(line, Lp::out_pos(tau, e))], x[e]);
-						acc[e].x += coef * v.x;
-						acc[e].y += coef * v.y;
-					}
-					if constexpr (sizeof(C) == 16) tmem_st8(TM::addr(tbase, q, 0), acc);
-					else {
-#pragma unroll
-						for (int e = 0; e < 8; e++) tmem_st(TM::addr(tbase, q, e), acc[e]);
-					}
-				}
-				// Y_i: the term of j = 2r waits in TMEM for that of j = 2r + 1
-				if (pr) {
-					const C *Wj = Gcell + (long)(2 * rank + q) * P * P + line * P + tau;
-					const R eta = (R)(2 * rank + q == 0 ? 1.0 : -1.0);
-#pragma unroll
-					for (int e = 0; e < 8; e++) x[e] = cscale(cmul(Wj[G::T * e], x[e]), eta);
-					if (q == 0) {
-						tmem_st8(TM::yaddr(tbase), x);
-					} else {
-						C y[8];
-						tmem_ld8(TM::yaddr(tbase), y);
-						tmem_wait_ld();
-#pragma unroll
-						for (int e = 0; e < 8; e++) x[e] = cadd(y[e], x[e]);
-					}
-				}
-				tmem_wait_st();
-				// no barrier here: the row passes that end this chain and begin the
-				// next touch only the rows of their own 8-lane group, and the next
-				// column pass waits behind the next chain's first barrier
-			}
-			if (!pr) continue;
-			// Z_i += conj(psi1) . Extract(IFFT2(Y_i))
-			fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, twaddr);
-#pragma unroll
-			for (int e = 0; e < 8; e++) Ug[G::at(line, Lp::out_pos(tau, e))] = x[e];
-			__syncthreads();
-			if (zcol) {                                      // whole warps: lines 0 .. 15 and 48 .. 63
-				C z[4], w[4];
-				C *zi = zbase + (long)i * G::N * G::N;
-				const C *ps = p.psi1 + (long)t * G::N * G::N + zofs;
-#pragma unroll
-				for (int e = 0; e < 4; e++) { z[e] = zi[8 * e * G::N]; w[e] = ps[8 * e * G::N]; }
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(tau + G::T * r, line)];
-				fft1d_lane<P, +1>(x, tau, G::col(Ug, line), wp, twaddr);
-#pragma unroll
-				for (int e = 0; e < 4; e++) {
-					w[e].y = -w[e].y;
-					zi[8 * e * G::N] = cadd(z[e], cmul(w[e], x[e < 2 ? e : e + 4]));
-				}
-			}
-			__syncthreads();                                 // the next chain's rows reuse Ug
-		}
-		if constexpr (kPush) push_release();              // the own P grids are read by the copy before they change
-		cluster.sync();
-	}
-#pragma unroll 1
-	for (int q = 0; q < 2; q++) {
-		C acc[8];
-		tmem_ld8(TM::addr(tbase, q, 0), acc);
-		tmem_wait_ld();
-		C *o = p.out + (slot * 4 + 2 * rank + q) * (long)P * P + line * P;
-#pragma unroll
-		for (int e = 0; e < 8; e++) o[Lp::out_pos(tau, e)] = acc[e];
-	}
-	}
-	tmem_fence_before();
-	__syncthreads();
-	tmem_fence_after();
-	if (warp == 0) tmem_dealloc(tbase, TM::ALLOC);
-}
-
-// k_i3p in real arithmetic (FP32 form, cells without Nyquist content): the
-// identity of k_i3_full128r at P = 64.  One transform of psi1_t . (W_2r +
-// i W_2r+1) gives the real spectra P_2r (real part) and P_2r+1 (imaginary
-// part) in one shared grid; the chains of combos (i0, i1) of an output share
-// one complex transform of P_j . (W^_i0 + i W^_i1), and the real accumulators
-// take eta_i0 P_i0 . Re + eta_i1 P_i1 . Im; Y_i0 + i Y_i1 is packed the same way.
-// Same shared-memory layout as k_i3p (the second P grid unused); tensor memory:
-// 2 x 8 real accumulators, 8 psi2 values and 8 complex values of Y per thread.
-struct I3TmemR {
-	static constexpr unsigned PER_THREAD = 16, NCOLS = 64, PSI = 8, YI = 16, ALLOC = 256;
-	__device__ __forceinline__ static unsigned lanes() { return (32u * ((threadIdx.x >> 5) & 3u)) << 16; }
-	__device__ __forceinline__ static unsigned slot() { return threadIdx.x >> 7; }
-	__device__ __forceinline__ static unsigned addr(unsigned base, int q) { return base + lanes() + (threadIdx.x >> 7) * PER_THREAD + (unsigned)q * 8; }
-	__device__ __forceinline__ static unsigned psiaddr(unsigned base) { return base + lanes() + NCOLS + slot() * PSI; }
-	__device__ __forceinline__ static unsigned yaddr(unsigned base) { return base + lanes() + NCOLS + 4 * PSI + slot() * YI; }
-};
-
-template <int P>
-__global__ void __launch_bounds__(Geo<P>::NT, 1) k_i3pr(const I3ParamsT<float2> p, const int *kind) {
-	using C = float2;
-	using G = Geo<P, C>;
-	using Lp = Len<P>;
-	using TM = I3TmemR;
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__shared__ unsigned tmem_slot;
-	C *Pq = reinterpret_cast<C *>(smem_raw);                 // P_2r + i P_2r+1
-	C *Ug = Pq + 2 * G::GRID, *tw = Pq + 3 * G::GRID;
-	C *Pr = Pq + G::GRID;                                    // the partner's packed P grid, copied in
-	__shared__ __align__(8) uint64_t pmbar;
-	unsigned pphase = 0;
-	cg::cluster_group cluster = cg::this_cluster();
-	const int rank = (int)cluster.block_rank();
-	const long cid = blockIdx.x / 2;
-	const int chunk = (int)(cid % p.nchunk);
-	const long cell = cid / p.nchunk;
-	if (kind[cell] != 0) return;                          // both CTAs of the cluster leave before any barrier
-	const int warp = threadIdx.x >> 5;
-	if (warp == 0) tmem_alloc(&tmem_slot, TM::ALLOC);
-	init_twiddles<P>(tw);
-	tmem_fence_before();
-	__syncthreads();
-	tmem_fence_after();
-	const unsigned tbase = tmem_slot;
-	const int line = threadIdx.x / G::T, tau = threadIdx.x % G::T;
-	C wp[8];
-#pragma unroll
-	for (int q = 0; q < 8; q++) wp[q] = tw[(tau * q) & (P - 1)];
-	{
-		const float z[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
-		tmem_st8r(TM::addr(tbase, 0), z);
-		tmem_st8r(TM::addr(tbase, 1), z);
-		tmem_wait_st();
-	}
-	const C *Gcell = p.Ghat + cell * p.g_cell;
-	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
-	// packed sums A_c = Z_2c + i Z_2c+1 on the frequencies -N/2 .. N/2 (both ends:
-	// separating the two real-grid parts needs the partner of -N/2)
-	constexpr int H = G::N / 2, ZA = (G::N + 1) * (G::N + 1);
-	const long slot = cell * p.nchunk + chunk;
-	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
-	for (int i = threadIdx.x; i < 2 * ZA; i += G::NT) za[i] = czero<C>();
-	const int zk = line <= H ? line : line - P;              // this thread's column as a frequency
-	const bool zcol = line <= H || line >= P - H;
-	push_init(&pmbar);
-	cluster.sync();                                          // the partner's mbarrier is initialised
-	for (int un = t0; un < t1; un++) {
-		const int t = p.un.term(un);
-		const bool pr = p.un.pair(un);
-		{
-			const double2 *sa = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank] * G::N * G::N;
-			const double2 *sb = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank + 1] * G::N * G::N;
-			fft2_pad<P, -1>(Pq, tw, sa, MulCplxPair<C>{p.psi1 + (long)t * G::N * G::N, sb});
-		}
-		fence_async_smem_a();
-		__syncthreads();                                     // no distributed-shared-memory reads: a CTA barrier
-		push_issue(Pq, Pr, (uint32_t)(G::GRID * sizeof(C)), &pmbar, rank ^ 1, (uint32_t)(G::GRID * sizeof(C)));
-		const float *psi2 = p.psi2T + (long)p.psi2_idx[t] * P * P;
-		const float sc = (float)p.psi2_scale[t];
-		{
-			float f[8];
-#pragma unroll
-			for (int e = 0; e < 8; e++) f[e] = sc * psi2[line * P + Lp::out_pos(tau, e)];
-			tmem_st8r(TM::psiaddr(tbase), f);
-			tmem_wait_st();
-		}
-		push_wait(&pmbar, pphase, p.err);
-#pragma unroll 1
-		for (int c = 0; c < 2; c++) {                        // the combos i = 2c (real part) and 2c + 1 (imaginary part)
-			const C *G0 = Gcell + (long)(2 * c) * P * P, *G1 = G0 + (long)P * P;
-			const C *Pa = (c == rank ? Pq : Pr);             // P_2c + i P_2c+1
-			const float c0 = c == 0 ? 1.f : -1.f;            // eta_2c; eta_2c+1 = -1
-			C x[8];
-#pragma unroll 1
-			for (int q = 0; q < 2; q++) {
-				// rows: IFFT of P_j . (W^_2c + i W^_2c+1)
-				{
-					float g0[8], g1[8];
-#pragma unroll
-					for (int r = 0; r < 8; r++) {
-						g0[r] = G0[line * P + tau + G::T * r].x;
-						g1[r] = G1[line * P + tau + G::T * r].x;
-					}
-#pragma unroll
-					for (int r = 0; r < 8; r++) {
-						const C pv = Pq[G::at(line, tau + G::T * r)];
-						const float pj = q ? pv.y : pv.x;
-						x[r] = mk<C>(pj * g0[r], pj * g1[r]);
-					}
-				}
-				fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, 0u);
-#pragma unroll
-				for (int e = 0; e < 8; e++) Ug[G::at(line, Lp::out_pos(tau, e))] = x[e];
-				__syncthreads();
-				// columns: IFFT, multiply by psi2_t, FFT
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(tau + G::T * r, line)];
-				fft1d_lane<P, +1>(x, tau, G::col(Ug, line), wp, 0u);
-				{
-					float f[8];
-					tmem_ld8r(TM::psiaddr(tbase), f);
-					tmem_wait_ld();
-#pragma unroll
-					for (int e = 0; e < 8; e++) { x[e].x *= f[e]; x[e].y *= f[e]; }
-				}
-				out_to_in_acc<P>(x, tau, G::col(Ug, line));
-				fft1d_lane<P, -1>(x, tau, G::col(Ug, line), wp, 0u);
-#pragma unroll
-				for (int e = 0; e < 8; e++) Ug[G::at(Lp::out_pos(tau, e), line)] = x[e];
-				__syncthreads();
-				// rows: FFT; the real part is T of i = 2c, the imaginary part of 2c + 1
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(line, tau + G::T * r)];
-				fft1d_lane<P, -1>(x, tau, G::row(Ug, line), wp, 0u);
-				{
-					float acc[8];
-					tmem_ld8r(TM::addr(tbase, q), acc);
-					tmem_wait_ld();
-#pragma unroll
-					for (int e = 0; e < 8; e++) {
-						const C pv = Pa[G::at(line, Lp::out_pos(tau, e))];
-						acc[e] += c0 * (pv.x * x[e].x) - pv.y * x[e].y;
-					}
-					tmem_st8r(TM::addr(tbase, q), acc);
-				}
-				// Y_2c + i Y_2c+1 += eta_j W^_j . T (W^_j real)
-				if (pr) {
-					const C *Wj = Gcell + (long)(2 * rank + q) * P * P + line * P + tau;
-					const float eta = 2 * rank + q == 0 ? 1.f : -1.f;
-#pragma unroll
-					for (int e = 0; e < 8; e++) x[e] = cscale(x[e], eta * Wj[G::T * e].x);
-					if (q == 0) {
-						tmem_st8(TM::yaddr(tbase), x);
-					} else {
-						C y[8];
-						tmem_ld8(TM::yaddr(tbase), y);
-						tmem_wait_ld();
-#pragma unroll
-						for (int e = 0; e < 8; e++) x[e] = cadd(y[e], x[e]);
-					}
-				}
-				tmem_wait_st();
-				// no barrier here, as in k_i3p
-			}
-			if (!pr) continue;
-			// A_c += conj(psi1) . IFFT2(Y_2c + i Y_2c+1) on the frequencies -N/2 .. N/2
-			fft1d_lane<P, +1>(x, tau, G::row(Ug, line), wp, 0u);
-#pragma unroll
-			for (int e = 0; e < 8; e++) Ug[G::at(line, Lp::out_pos(tau, e))] = x[e];
-			__syncthreads();
-			if (line < H + 32 / G::T || line >= P - H) {     // whole warps; line H is the only one of its warp with zcol
-				const C *ps = p.psi1 + (long)t * G::N * G::N;
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = Ug[G::at(tau + G::T * r, line)];
-				fft1d_lane<P, +1>(x, tau, G::col(Ug, line), wp, 0u);
-				if (zcol) {
-#pragma unroll
-					for (int e = 0; e < 8; e++) {
-						if (e > 2 && e < 6) continue;            // rows 24 .. 47
-						const int l = tau + G::T * e, zl = e < 3 ? l : l - P;
-						if (zl > H || (zl == H && zk == -H) || (zl == -H && zk == H)) continue;
-						// psi1 is tabulated on -N/2 .. N/2 - 1; at the upper end it is conj psi1(-k)
-						const bool up = zl == H || zk == H;
-						const int a = up ? -zl : zl, b = up ? -zk : zk;
-						C w = ps[(a < 0 ? a + G::N : a) * G::N + (b < 0 ? b + G::N : b)];
-						if (!up) w.y = -w.y;
-						C *z = za + c * ZA + (zl + H) * (G::N + 1) + zk + H;
-						*z = cadd(*z, cmul(w, x[e]));
-					}
-				}
-			}
-			__syncthreads();                                 // the next chain's rows reuse Ug
-		}
-		push_release();                                      // the own P grid is read by the copy before it changes
-		cluster.sync();
-	}
-	// A(k) = Z_2c(k) + i Z_2c+1(k) with both parts the transforms of real grids
-	{
-		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)G::N * G::N;
-		for (int i = threadIdx.x; i < 2 * G::N * G::N; i += G::NT) {
-			const int c = i / (G::N * G::N), n = i % (G::N * G::N);
-			int l = n / G::N, k = n % G::N;
-			l = l < H ? l : l - G::N;
-			k = k < H ? k : k - G::N;
-			const C u = za[c * ZA + (l + H) * (G::N + 1) + k + H], v = za[c * ZA + (H - l) * (G::N + 1) + H - k];
-			zo[(long)(2 * c) * G::N * G::N + n] = mk<C>(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
-			zo[(long)(2 * c + 1) * G::N * G::N + n] = mk<C>(0.5f * (u.y + v.y), -0.5f * (u.x - v.x));
-		}
-	}
-#pragma unroll 1
-	for (int q = 0; q < 2; q++) {
-		float acc[8];
-		tmem_ld8r(TM::addr(tbase, q), acc);
-		tmem_wait_ld();
-		C *o = p.out + ((cell * p.nchunk + chunk) * 4 + 2 * rank + q) * (long)P * P + line * P;
-#pragma unroll
-		for (int e = 0; e < 8; e++) o[Lp::out_pos(tau, e)] = mk<C>(acc[e], 0.0);
-	}
-	tmem_fence_before();
-	__syncthreads();
-	tmem_fence_after();
-	if (warp == 0) tmem_dealloc(tbase, TM::ALLOC);
 }
 
 // ---------------------------------------------------------------------------

@@ -103,7 +103,7 @@ void run(const qb::DevI3 &t, const double2 *f, const double2 *g, const double2 *
 
 	const size_t sm1 = sizeof(double2) * (G::GRID + P), sm2 = sizeof(double2) * (2 * G::GRID + P);
 	QB_CUDA(cudaFuncSetAttribute(qb::k_pad_fft<P, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-	qb::k_pad_fft<P, double2><<<1, G::NT, sm1, s>>>(src + 2 * NN, ghat, nullptr);
+	qb::k_pad_fft<P, double2><<<1, G::NT, sm1, s>>>(src + 2 * NN, ghat, nullptr, nullptr);
 	QB_CUDA(cudaGetLastError());
 
 	qb::I3Params p{};

@@ -15,11 +15,11 @@
 // the group, and a transform that starts at the positions where the last one
 // ended needs none before it.
 //
-// Shared grid: slot(row, col) = 64 row + (col ^ sw(row)), sw = bits (0, 2, 1) of
-// the row; with 16-byte values every access of the three stages is free of
-// bank conflicts without padding (eight lanes of A: two rows x four
-// consecutive columns, of B: eight consecutive rows, of C: eight consecutive
-// columns).
+// Shared grid: slot(row, col) = 64 row + (col ^ sw(row)).  Eight lanes of 16-byte
+// values (16 of 8 bytes) share a pass over the banks: of A two (four) rows x
+// four consecutive columns, of B eight (16) consecutive rows, of C eight (16)
+// consecutive columns.  With sw = bits (0, 2, 1) of the row (bits (1, 0, 3, 2) in
+// FP32) each is free of bank conflicts without padding.
 #pragma once
 #include "qb_kernels.cuh"
 
@@ -56,7 +56,8 @@ template <class C> struct Wide64 {
 	C *U;                                    // the group's grid
 	const C *tw;                             // w64^e, e < 64, forward sign
 	int t, bar;                              // thread of the group, its named barrier
-	__device__ __forceinline__ static int sw(int row) { return ((row & 1) << 2) | ((row >> 1) & 3); }
+	static constexpr int HB = sizeof(C) == 16 ? 1 : 2, HM = (1 << HB) - 1;      // bits of q in the swizzled part of a column
+	__device__ __forceinline__ static int sw(int row) { return ((row & HM) << 2) | ((row >> HB) & 3); }
 	__device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(GT) : "memory"); }
 	// A: this thread's row and first column
 	__device__ __forceinline__ int row_a() const { return t >> 2; }
@@ -67,13 +68,13 @@ template <class C> struct Wide64 {
 
 	// slots of A: index q (columns tau + 4 q)
 	template <class F> __device__ __forceinline__ void slots_a(const F &f) const {
-		const int l = t >> 2, s = sw(l), b0 = l * 64 + ((t & 3) ^ s), b1 = l * 64 + (((t & 3) + 4) ^ s);
+		const int l = t >> 2, s = sw(l), b = l * 64;
 #pragma unroll
-		for (int q = 0; q < 16; q++) f(q, U[((q & 1) ? b1 : b0) + 8 * (q >> 1)]);
+		for (int q = 0; q < 16; q++) f(q, U[b + (((t & 3) + 4 * (q & HM)) ^ s) + (4 << HB) * (q >> HB)]);
 	}
 	// slots of B: index (s or u, tau or p)
 	template <class F> __device__ __forceinline__ void slots_b(const F &f) const {
-		const int q = t >> 4, lam = t & 15, s = sw(lam), b = lam * 64 + 8 * (q >> 1), h = 4 * (q & 1);
+		const int q = t >> 4, lam = t & 15, s = sw(lam), b = lam * 64 + (4 << HB) * (q >> HB), h = 4 * (q & HM);
 #pragma unroll
 		for (int c = 0; c < 4; c++) {
 			const int a = b + ((c + h) ^ s);
@@ -149,16 +150,31 @@ template <class C> struct Wide64 {
 	}
 };
 
-// tensor memory of a thread of k_i3w: 16 accumulators, then 16 values of P_j,
-// value r at word 4 r (FP64); four warps share a lane quarter
-struct WideTmem {
-	static constexpr unsigned COLS = 512;
+// tensor memory of a thread of k_i3w: 16 accumulators of W words, then 16 values
+// of P_j; four warps share a lane quarter.  W = 4 (FP64), 2 (FP32), 1 (FP32, real)
+template <int W> struct WideTmem {
+	static constexpr unsigned COLS = 128 * W, H = 16 * W;
 	__device__ __forceinline__ static unsigned x(unsigned base) {
 		const unsigned w = threadIdx.x >> 5;
-		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * 128u;
+		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * 2u * H;
 	}
-	__device__ __forceinline__ static unsigned p(unsigned base) { return x(base) + 64u; }
+	__device__ __forceinline__ static unsigned p(unsigned base) { return x(base) + H; }
 };
+// four FP32 complex values, or four reals
+__device__ __forceinline__ void tmem_ld4(unsigned taddr, float2 (&v)[4]) {
+	unsigned r[8];
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+#pragma unroll
+	for (int e = 0; e < 4; e++) { v[e].x = __uint_as_float(r[2 * e]); v[e].y = __uint_as_float(r[2 * e + 1]); }
+}
+__device__ __forceinline__ void tmem_st4(unsigned taddr, const float2 (&v)[4]) {
+	unsigned r[8];
+#pragma unroll
+	for (int e = 0; e < 4; e++) { r[2 * e] = __float_as_uint(v[e].x); r[2 * e + 1] = __float_as_uint(v[e].y); }
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+	             :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 template <class C> constexpr size_t i3w_smem() {
 	// two grids, the Y values in transit, psi2 (16 reals a thread of a group), the twiddles
 	return sizeof(C) * (3 * 4096 + 64) + sizeof(typename CT<C>::R) * 4096;
@@ -181,11 +197,14 @@ template <class C> constexpr size_t i3w_smem() {
 // out: [slot][4][PP], zout: [slot][rank][4][N*N], slots of the term ranges (or
 // (cell, chunk)); pscr: [cluster][2][4][PP] (two units in turn: one cluster
 // barrier a unit).
+// kind: null (every cell) or the per-cell form of k_nyquist_kind; this kernel
+// then takes the cells of kind 1 (the real form k_i3wr takes kind 0).
 template <class C>
-__global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
+__global__ void __launch_bounds__(512, Occ<C>::CTAS) k_i3w(const I3ParamsT<C> p, C *pscr, const int *kind) {
 	using R = typename CT<C>::R;
-	using TM = WideTmem;
-	constexpr int N = 32, NN = N * N, P = 64, PP = P * P, GT = 256;
+	using TM = WideTmem<sizeof(C) / 4>;
+	constexpr int N = 32, NN = N * N, P = 64, PP = P * P, GT = 256, H4 = TM::H / 4;
+	if (kind != nullptr && kind[blockIdx.x / 2 / p.nchunk] != 1) return;     // both CTAs of the cluster leave before any barrier
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ unsigned tmem_slot;
 	C *grids = reinterpret_cast<C *>(smem_raw), *Yb = grids + 2 * PP, *tw = Yb + PP;
@@ -234,7 +253,7 @@ __global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
 		{
 			const C z[4] = { czero<C>(), czero<C>(), czero<C>(), czero<C>() };
 #pragma unroll
-			for (int h = 0; h < 4; h++) tmem_st4(tx + 16 * h, z);
+			for (int h = 0; h < 4; h++) tmem_st4(tx + H4 * h, z);
 			tmem_wait_st();
 			if (ks >= 0) {
 #pragma unroll 1
@@ -271,7 +290,7 @@ __global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
 					a[r] = x[pos16(4 * h + r)];
 					__stcg(Pu + j * PP + GT * (4 * h + r), a[r]);
 				}
-				tmem_st4(tp + 16 * h, a);
+				tmem_st4(tp + H4 * h, a);
 			}
 			tmem_wait_st();
 			cl.sync();                                       // the unit's P grids are in L2
@@ -291,7 +310,7 @@ __global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
 #pragma unroll
 				for (int h = 0; h < 4; h++) {
 					C a[4];
-					tmem_ld4(tp + 16 * h, a);
+					tmem_ld4(tp + H4 * h, a);
 					tmem_wait_ld();
 #pragma unroll
 					for (int r = 0; r < 4; r++) x[4 * h + r] = cmul(x[4 * h + r], a[r]);
@@ -313,7 +332,7 @@ __global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
 					C a[4], w[4];
 #pragma unroll
 					for (int r = 0; r < 4; r++) w[r] = __ldcg(Pi + GT * (4 * h + r));
-					tmem_ld4(tx + 16 * h, a);
+					tmem_ld4(tx + H4 * h, a);
 					tmem_wait_ld();
 #pragma unroll
 					for (int r = 0; r < 4; r++) {
@@ -321,7 +340,7 @@ __global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
 						a[r].x += ci * v.x;
 						a[r].y += ci * v.y;
 					}
-					tmem_st4(tx + 16 * h, a);
+					tmem_st4(tx + H4 * h, a);
 				}
 				if (pr) {
 					// y = eta_j W^_j . T_ij; the group of i % 2 takes the sum of both
@@ -359,11 +378,206 @@ __global__ void __launch_bounds__(512, 1) k_i3w(const I3ParamsT<C> p, C *pscr) {
 #pragma unroll
 		for (int h = 0; h < 4; h++) {
 			C a[4];
-			tmem_ld4(tx + 16 * h, a);
+			tmem_ld4(tx + H4 * h, a);
 			tmem_wait_ld();
 #pragma unroll
 			for (int r = 0; r < 4; r++) o[4 * (4 * h + r)] = a[r];
 		}
+	}
+	tmem_fence_before();
+	__syncthreads();
+	tmem_fence_after();
+	if (warp == 0) tmem_dealloc(tmem_slot, TM::COLS);
+}
+
+// ---------------------------------------------------------------------------
+// k_i3w in real arithmetic (FP32 form, cells without Nyquist content): W^ and P
+// are real and a chain maps real grids to real grids (qb_full128.cuh), so the
+// chains of i = 2c and 2c + 1 share one complex transform of P_j . (W^_2c + i
+// W^_2c+1), X_j (real) takes eta_2c P_2c . Re + eta_2c+1 P_2c+1 . Im, and Y_2c +
+// i Y_2c+1 is packed the same way: two chains a unit and group.  A_c = Z_2c + i
+// Z_2c+1 is summed on the frequencies -N/2 .. N/2 of both dimensions (the
+// partner of -N/2 separates the two) in zscr and separated at the end.  WhR: the
+// real parts of W^ in thread order; pscr: [cluster][2][4][PP] reals.
+__global__ void __launch_bounds__(512, 2) k_i3wr(const I3ParamsT<float2> p, const float *__restrict__ WhR, float *pscr, const int *kind) {
+	using C = float2;
+	using TM = WideTmem<1>;
+	constexpr int N = 32, NN = N * N, P = 64, PP = P * P, GT = 256, H = N / 2, ZA = (N + 1) * (N + 1);
+	const int cid = (int)(blockIdx.x / 2), chunk = cid % p.nchunk;
+	const long cell = cid / p.nchunk;
+	if (kind[cell] != 0) return;                             // both CTAs of the cluster leave before any barrier
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	__shared__ unsigned tmem_slot;
+	C *grids = reinterpret_cast<C *>(smem_raw), *Yb = grids + 2 * PP, *tw = Yb + PP;
+	float *psi = reinterpret_cast<float *>(tw + 64);
+	cg::cluster_group cl = cg::this_cluster();
+	const int rank = (int)cl.block_rank();
+	const int g = threadIdx.x / GT, t = threadIdx.x % GT, warp = threadIdx.x >> 5;
+	if (warp == 0) tmem_alloc(&tmem_slot, TM::COLS);
+	init_twiddles<64>(tw);
+	const long slot = cell * p.nchunk + chunk;
+	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
+	for (int i = threadIdx.x; i < 2 * ZA; i += 512) za[i] = czero<C>();
+	tmem_fence_before();
+	__syncthreads();
+	tmem_fence_after();
+	const unsigned tx = TM::x(tmem_slot), tp = TM::p(tmem_slot);
+	const Wide64<C> F{ grids + g * PP, tw, t, g + 1 };
+	const int j = 2 * rank + g;
+	const float etaj = j == 0 ? 1.f : -1.f;
+	const int oa = F.row_a() * P + F.col_a();
+	const int kc = F.col_c(), ks = kc < N / 2 ? kc : (kc >= 3 * N / 2 ? kc - N : -1);
+	const int zk = kc <= H ? kc : kc - P;                    // this thread's column of C as a frequency
+	const int oz = F.row_c() * N + ks;
+	float *Pall = pscr + (long)cid * 8 * PP + t;
+	Yb += t;
+	const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[j] * NN + oz;
+	const float *Wc = WhR + cell * 4 * PP + t;
+	{
+		const float z[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+		tmem_st8r(tx, z);
+		tmem_st8r(tx + 8, z);
+		tmem_wait_st();
+	}
+	const int u0 = (int)((long)chunk * p.nterms / p.nchunk), u1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
+	int psi_idx = -1, par = 0;
+#pragma unroll 1
+	for (int un = u0; un < u1; un++) {
+		const int term = p.un.term(un);
+		const bool pr = p.un.pair(un);
+		float *Pu = Pall + par * 4 * PP;
+		par ^= 1;
+		C x[16];
+		F.sync();                                            // the last chain's rows are read
+		{
+			// P_j = FFT2(Pad(psi1 . W_j)), real
+			const C *psi1 = p.psi1 + (long)term * NN + oz;
+#pragma unroll
+			for (int v = 0; v < 16; v++) x[v] = czero<C>();
+			if (ks >= 0) {
+#pragma unroll
+				for (int v = 0; v < 8; v++) {
+					const double2 w = src[4 * v * N];
+					x[v < 4 ? v : v + 8] = cmul(psi1[4 * v * N], mk<C>(w.x, w.y));
+				}
+			}
+		}
+		F.forward(x);
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			float a[8];
+#pragma unroll
+			for (int r = 0; r < 8; r++) {
+				a[r] = x[pos16(8 * h + r)].x;
+				__stcg(Pu + j * PP + GT * (8 * h + r), a[r]);
+			}
+			tmem_st8r(tp + 8 * h, a);
+		}
+		tmem_wait_st();
+		cl.sync();                                           // the unit's P grids are in L2
+		if (p.psi2_idx[term] != psi_idx) {                   // a new angle: its psi2 in the order of C
+			psi_idx = p.psi2_idx[term];
+			const float *s = p.psi2T + (long)psi_idx * PP + kc * P + F.row_c();
+#pragma unroll
+			for (int v = 0; v < 8; v++) psi[(8 * g + v) * GT + t] = s[4 * (8 * g + v)];
+			__syncthreads();
+		}
+		const float sc = (float)p.psi2_scale[term];
+#pragma unroll 1
+		for (int c = 0; c < 2; c++) {
+			const float *W0 = Wc + 2 * c * PP;
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				float a[8];
+				tmem_ld8r(tp + 8 * h, a);
+#pragma unroll
+				for (int r = 0; r < 8; r++) x[8 * h + r] = mk<C>(W0[GT * (8 * h + r)], W0[PP + GT * (8 * h + r)]);
+				tmem_wait_ld();
+#pragma unroll
+				for (int r = 0; r < 8; r++) x[8 * h + r] = cscale(x[8 * h + r], a[r]);
+			}
+			F.inverse(x);
+			{
+				C y[16];
+#pragma unroll
+				for (int v = 0; v < 16; v++) y[v] = cscale(x[pos16(v)], psi[v * GT + t]);
+#pragma unroll
+				for (int v = 0; v < 16; v++) x[v] = y[v];
+			}
+			F.forward(x);
+			const float *P0 = Pu + 2 * c * PP;
+			const float c0 = c == 0 ? sc : -sc;                  // eta_2c; eta_2c+1 = -1
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				float a[8];
+				tmem_ld8r(tx + 8 * h, a);
+				tmem_wait_ld();
+#pragma unroll
+				for (int r = 0; r < 8; r++) {
+					const C v = x[pos16(8 * h + r)];
+					a[r] += c0 * (__ldcg(P0 + GT * (8 * h + r)) * v.x) - sc * (__ldcg(P0 + PP + GT * (8 * h + r)) * v.y);
+				}
+				tmem_st8r(tx + 8 * h, a);
+			}
+			if (pr) {
+				const float *Wj = Wc + j * PP;
+				const float cj = etaj * sc;
+				const int hand = 3 + c;
+#pragma unroll
+				for (int r = 0; r < 16; r++) x[pos16(r)] = cscale(x[pos16(r)], cj * Wj[GT * r]);
+				if (c != g) {
+#pragma unroll
+					for (int r = 0; r < 16; r++) Yb[r * GT] = x[pos16(r)];
+					asm volatile("bar.arrive %0, 512;" ::"r"(hand) : "memory");
+				} else {
+					asm volatile("bar.sync %0, 512;" ::"r"(hand) : "memory");
+					C y[16];
+#pragma unroll
+					for (int r = 0; r < 16; r++) y[r] = cadd(Yb[r * GT], x[pos16(r)]);
+					F.inverse(y);
+					F.sync();                                // the next chain writes rows
+					if (kc <= H || kc >= P - H) {
+						const C *ps = p.psi1 + (long)term * NN;
+#pragma unroll
+						for (int v = 0; v < 16; v++) {
+							if (v > 4 && v < 12) continue;       // rows 20 .. 47
+							const int l = F.row_c() + 4 * v, zl = v < 5 ? l : l - P;
+							if (zl > H || (zl == H && zk == -H) || (zl == -H && zk == H)) continue;
+							// psi1 is tabulated on -N/2 .. N/2 - 1; at the upper end it is conj psi1(-k)
+							const bool up = zl == H || zk == H;
+							const int a = up ? -zl : zl, b = up ? -zk : zk;
+							C w = ps[(a < 0 ? a + N : a) * N + (b < 0 ? b + N : b)];
+							if (!up) w.y = -w.y;
+							C *z = za + c * ZA + (zl + H) * (N + 1) + zk + H;
+							*z = cfma(w, y[pos16(v)], *z);
+						}
+					}
+				}
+			}
+			tmem_wait_st();
+		}
+	}
+	__syncthreads();                                         // za is complete
+	{
+		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
+		for (int i = threadIdx.x; i < 2 * NN; i += 512) {
+			const int c = i / NN, n = i % NN;
+			int l = n / N, k = n % N;
+			l = l < H ? l : l - N;
+			k = k < H ? k : k - N;
+			const C a = za[c * ZA + (l + H) * (N + 1) + k + H], b = za[c * ZA + (H - l) * (N + 1) + H - k];
+			zo[(long)(2 * c) * NN + n] = mk<C>(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
+			zo[(long)(2 * c + 1) * NN + n] = mk<C>(0.5f * (a.y + b.y), -0.5f * (a.x - b.x));
+		}
+	}
+	C *o = p.out + (slot * 4 + j) * (long)PP + oa;
+#pragma unroll
+	for (int h = 0; h < 2; h++) {
+		float a[8];
+		tmem_ld8r(tx + 8 * h, a);
+		tmem_wait_ld();
+#pragma unroll
+		for (int r = 0; r < 8; r++) o[4 * (8 * h + r)] = mk<C>(a[r], 0.0);
 	}
 	tmem_fence_before();
 	__syncthreads();
