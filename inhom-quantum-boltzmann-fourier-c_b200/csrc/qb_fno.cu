@@ -88,201 +88,372 @@ __global__ void k_fno_in(int B, int P, const double *__restrict__ W, InScale sc,
 	}
 }
 
-// out[b][o][p] = sum_i M[o][i] in[b][i][p] + bias[o] (+ add[b][o][p]); act: store gelu in hout and u in uout
-__global__ void k_fno_pointwise(int B, int P, int cin, int cout, const float *__restrict__ in, const float *__restrict__ M,
-                                const float *__restrict__ bias, const float *__restrict__ add, float *__restrict__ uout,
-                                float *__restrict__ hout, int act) {
-	__shared__ float Ms[kFnoMaxWidth * kFnoMaxWidth + kFnoMaxWidth];
-	for (int i = threadIdx.x; i < cin * cout; i += blockDim.x) Ms[i] = M[i];
-	for (int i = threadIdx.x; i < cout; i += blockDim.x) Ms[cin * cout + i] = bias ? bias[i] : 0.0f;
+// out[b][o][p] = sum_i M[o][i] in[b][i][p] + bias[o] (+ add[b][o][p]); act: store
+// gelu in hout and u in uout.  trans: M^T (the backward of a pointwise map, M[i][o]).
+// A thread keeps the CI (>= cin) inputs of a point in registers and takes every
+// gridDim.y-th block of four outputs, the matrix rows as broadcast float4 reads.
+// Bound by latency and L2: 64 cells, 32 x 32 channels at N = 32: 27 -> 18 us (the
+// inputs were in local memory, their count known at run time only).
+template <int CI>
+__global__ void __launch_bounds__(256) k_fno_pointwise(int B, int P, int cin, int cout, int trans, const float *__restrict__ in,
+                                                       const float *__restrict__ M, const float *__restrict__ bias,
+                                                       const float *__restrict__ add, float *__restrict__ uout, float *__restrict__ hout, int act) {
+	__shared__ __align__(16) float Ms[kFnoMaxWidth][CI];
+	__shared__ float bs[kFnoMaxWidth];
+	for (int i = threadIdx.x; i < cout * CI; i += blockDim.x) {
+		const int o = i / CI, c = i % CI;
+		Ms[o][c] = c < cin ? (trans ? M[c * cout + o] : M[o * cin + c]) : 0.0f;
+	}
+	for (int i = threadIdx.x; i < cout; i += blockDim.x) bs[i] = bias ? bias[i] : 0.0f;
 	__syncthreads();
 	const long n = (long)B * P;
 	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
 		const long b = t / P, p = t % P;
-		float v[kFnoMaxWidth];
-		for (int i = 0; i < cin; i++) v[i] = in[(b * cin + i) * P + p];
-		for (int o = 0; o < cout; o++) {
-			float s = Ms[cin * cout + o];
-			for (int i = 0; i < cin; i++) s = fmaf(Ms[o * cin + i], v[i], s);
-			const long oi = (b * cout + o) * P + p;
-			if (add) s += add[oi];
-			if (uout) uout[oi] = s;
-			hout[oi] = act ? gelu_f(s) : s;
+		const float *x = in + b * cin * P + p;
+		float v[CI];
+#pragma unroll
+		for (int i = 0; i < CI; i++) v[i] = i < cin ? x[(long)i * P] : 0.0f;
+		for (int o0 = 4 * blockIdx.y; o0 < cout; o0 += 4 * gridDim.y) {
+			const int no = min(4, cout - o0);
+			float s[4];
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				if (q >= no) continue;
+				s[q] = bs[o0 + q];
+				if (add) s[q] += add[(b * cout + o0 + q) * P + p];
+			}
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				if (q >= no) continue;
+				const float4 *m = reinterpret_cast<const float4 *>(Ms[o0 + q]);
+				float r = 0.0f;
+#pragma unroll
+				for (int i = 0; i < CI / 4; i++) {
+					const float4 w = m[i];
+					r = fmaf(w.x, v[4 * i], r);
+					r = fmaf(w.y, v[4 * i + 1], r);
+					r = fmaf(w.z, v[4 * i + 2], r);
+					r = fmaf(w.w, v[4 * i + 3], r);
+				}
+				const float u = s[q] + r;
+				const long oi = (b * cout + o0 + q) * P + p;
+				if (uout) uout[oi] = u;
+				hout[oi] = act ? gelu_f(u) : u;
+			}
 		}
 	}
 }
 
-// out[b][i][p] = sum_o M[o][i] in[b][o][p]  (transpose product: backward of a pointwise map)
-__global__ void k_fno_pointwise_t(int B, int P, int cin, int cout, const float *__restrict__ in, const float *__restrict__ M,
-                                  float *__restrict__ out) {
-	__shared__ float Ms[kFnoMaxWidth * kFnoMaxWidth];
-	for (int i = threadIdx.x; i < cin * cout; i += blockDim.x) Ms[i] = M[i];
-	__syncthreads();
-	const long n = (long)B * P;
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-		const long b = t / P, p = t % P;
-		float v[kFnoMaxWidth];
-		for (int o = 0; o < cout; o++) v[o] = in[(b * cout + o) * P + p];
-		for (int i = 0; i < cin; i++) {
-			float s = 0.0f;
-			for (int o = 0; o < cout; o++) s = fmaf(Ms[o * cin + i], v[o], s);
-			out[(b * cin + i) * P + p] = s;
-		}
-	}
-}
-
-// truncated forward DFT of every (b, c) field: H[b][c][k] = scale * sum_p f(p) e^{-i theta(k,p)}
-__global__ void k_fno_dft(int N, int m, const float *__restrict__ f, float2 *__restrict__ H, float scale) {
+// the twiddle of the truncated transforms: tw[j] = e^{2 pi i j / N}, j < N, built once per network
+// truncated forward DFT of every (b, c) field: H[b][c][k] = scale * sum_p f(p) e^{-i theta(k,p)}.
+// Rows: a thread has one l and every (blockDim / N)-th ky, with the twiddle
+// index advanced instead of reduced; columns: a thread gives kx and -kx from the same
+// four sums.  64 cells x 32 channels at N = 32, 12 modes: 59 -> 16 us.
+__global__ void __launch_bounds__(256) k_fno_dft(int N, int m, const float *__restrict__ f, const float2 *__restrict__ twg, float2 *__restrict__ H,
+                                                 float scale) {
 	extern __shared__ float sm[];
-	const int P = N * N, K = (2 * m - 1) * m;
-	float *fs = sm;                                   // P
-	float2 *T = reinterpret_cast<float2 *>(fs + P);  // N x m
-	float2 *tw = T + N * m;                          // N: e^{-2 pi i j / N}
+	const int P = N * N, K = (2 * m - 1) * m, pitch = N + 1;
+	float2 *T = reinterpret_cast<float2 *>(sm);      // N x m
+	float2 *tw = T + N * m;                          // N
+	float *fs = reinterpret_cast<float *>(tw + N);   // N x (N + 1)
 	const long bc = blockIdx.x;
-	for (int i = threadIdx.x; i < P; i += blockDim.x) fs[i] = f[bc * P + i];
-	for (int j = threadIdx.x; j < N; j += blockDim.x) {
-		double s, c;
-		sincospi(-2.0 * j / N, &s, &c);
-		tw[j] = make_float2((float)c, (float)s);
-	}
+	for (int i = threadIdx.x; i < P; i += blockDim.x) fs[(i / N) * pitch + i % N] = f[bc * P + i];
+	for (int j = threadIdx.x; j < N; j += blockDim.x) tw[j] = twg[j];
 	__syncthreads();
-	for (int t = threadIdx.x; t < N * m; t += blockDim.x) {
-		const int l = t / m, ky = t % m;
-		float re = 0.0f, im = 0.0f;
-		for (int kv = 0; kv < N; kv++) {
-			const float2 w = tw[(ky * kv) % N];
-			const float v = fs[l * N + kv];
-			re = fmaf(v, w.x, re);
-			im = fmaf(v, w.y, im);
+	const int ng = blockDim.x / N;                   // N <= 64
+	if ((int)threadIdx.x < ng * N) {
+		const int l = threadIdx.x % N;
+		const float *row = fs + l * pitch;
+		for (int ky = threadIdx.x / N; ky < m; ky += 2 * ng) {
+			const int k2 = min(ky + ng, m - 1);
+			float re = 0.0f, im = 0.0f, re2 = 0.0f, im2 = 0.0f;
+			int j = 0, j2 = 0;
+#pragma unroll 8
+			for (int kv = 0; kv < N; kv++) {
+				const float2 w = tw[j], w2 = tw[j2];
+				const float v = row[kv];
+				re = fmaf(v, w.x, re);
+				im = fmaf(v, -w.y, im);
+				re2 = fmaf(v, w2.x, re2);
+				im2 = fmaf(v, -w2.y, im2);
+				j += ky;
+				if (j >= N) j -= N;
+				j2 += k2;
+				if (j2 >= N) j2 -= N;
+			}
+			T[l * m + ky] = make_float2(re, im);
+			if (ky + ng < m) T[l * m + k2] = make_float2(re2, im2);
 		}
-		T[t] = make_float2(re, im);
 	}
 	__syncthreads();
-	for (int t = threadIdx.x; t < K; t += blockDim.x) {
-		const int kxi = t / m, ky = t % m, kx = kxi - (m - 1);
-		float re = 0.0f, im = 0.0f;
+	for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
+		const int kx = t / m, ky = t % m;
+		float ac = 0.0f, as = 0.0f, bcs = 0.0f, bs = 0.0f;
+		int j = 0;
+#pragma unroll 8
 		for (int l = 0; l < N; l++) {
-			const float2 w = tw[(((kx * l) % N) + N) % N];
-			const float2 a = T[l * m + ky];
-			re += a.x * w.x - a.y * w.y;
-			im += a.x * w.y + a.y * w.x;
+			const float2 w = tw[j], a = T[l * m + ky];
+			ac = fmaf(a.x, w.x, ac);
+			as = fmaf(a.x, w.y, as);
+			bcs = fmaf(a.y, w.x, bcs);
+			bs = fmaf(a.y, w.y, bs);
+			j += kx;
+			if (j >= N) j -= N;
 		}
-		H[bc * K + t] = make_float2(scale * re, scale * im);
+		float2 *h = H + bc * K;
+		h[(m - 1 + kx) * m + ky] = make_float2(scale * (ac + bs), scale * (bcs - as));
+		if (kx > 0) h[(m - 1 - kx) * m + ky] = make_float2(scale * (ac - bs), scale * (bcs + as));
 	}
 }
 
-// truncated inverse: out[b][c][p] (=, or +=) scale * Re sum_k O[b][c][k] e^{+i theta(k,p)}
-__global__ void k_fno_idft(int N, int m, const float2 *__restrict__ O, float *__restrict__ out, float scale, int accumulate) {
+// truncated inverse: out[b][c][p] (=, or +=) scale * Re sum_k O[b][c][k] e^{+i theta(k,p)}, times
+// dgelu(u[b][c][p]) when u is given (the step to the layer below in the backward
+// pass).  The frequencies kx and -kx are summed as O(kx) +- O(-kx); a thread of the
+// second stage has one kv and every (blockDim / N)-th row.  60 -> 24 us (as k_fno_dft).
+__global__ void __launch_bounds__(256) k_fno_idft(int N, int m, const float2 *__restrict__ O, const float2 *__restrict__ twg, float *__restrict__ out,
+                                                  float scale, int accumulate, const float *__restrict__ u) {
 	extern __shared__ float sm[];
 	const int P = N * N, K = (2 * m - 1) * m;
-	float2 *Os = reinterpret_cast<float2 *>(sm);     // K
-	float2 *U = Os + K;                              // N x m
-	float2 *tw = U + N * m;                          // N: e^{+2 pi i j / N}
+	float2 *S = reinterpret_cast<float2 *>(sm);      // m x m: O(kx) + O(-kx) (kx = 0: O(0))
+	float2 *D = S + m * m;                           // m x m: O(kx) - O(-kx)
+	float2 *U = D + m * m;                           // N x m
+	float2 *tw = U + N * m;                          // N
 	const long bc = blockIdx.x;
-	for (int i = threadIdx.x; i < K; i += blockDim.x) Os[i] = O[bc * K + i];
-	for (int j = threadIdx.x; j < N; j += blockDim.x) {
-		double s, c;
-		sincospi(2.0 * j / N, &s, &c);
-		tw[j] = make_float2((float)c, (float)s);
+	for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
+		const int kx = t / m, ky = t % m;
+		const float2 a = O[bc * K + (m - 1 + kx) * m + ky], b = O[bc * K + (m - 1 - kx) * m + ky];
+		S[t] = kx == 0 ? a : make_float2(a.x + b.x, a.y + b.y);
+		D[t] = make_float2(a.x - b.x, a.y - b.y);
 	}
+	for (int j = threadIdx.x; j < N; j += blockDim.x) tw[j] = twg[j];
 	__syncthreads();
 	for (int t = threadIdx.x; t < N * m; t += blockDim.x) {
 		const int l = t / m, ky = t % m;
-		float re = 0.0f, im = 0.0f;
-		for (int kxi = 0; kxi < 2 * m - 1; kxi++) {
-			const int kx = kxi - (m - 1);
-			const float2 w = tw[(((kx * l) % N) + N) % N];
-			const float2 a = Os[kxi * m + ky];
-			re += a.x * w.x - a.y * w.y;
-			im += a.x * w.y + a.y * w.x;
+		float re = S[ky].x, im = S[ky].y;
+		int j = l;
+#pragma unroll 4
+		for (int kx = 1; kx < m; kx++) {
+			const float2 w = tw[j], a = S[kx * m + ky], b = D[kx * m + ky];
+			re = fmaf(a.x, w.x, fmaf(-b.y, w.y, re));
+			im = fmaf(a.y, w.x, fmaf(b.x, w.y, im));
+			j += l;
+			if (j >= N) j -= N;
 		}
 		U[t] = make_float2(re, im);
 	}
 	__syncthreads();
-	for (int t = threadIdx.x; t < P; t += blockDim.x) {
-		const int l = t / N, kv = t % N;
-		float s = 0.0f;
+	const int ng = blockDim.x / N;
+	if ((int)threadIdx.x >= ng * N) return;
+	const int kv = threadIdx.x % N;
+	for (int l0 = threadIdx.x / N; l0 < N; l0 += 4 * ng) {
+		float s[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+		int j = 0;
+#pragma unroll 4
 		for (int ky = 0; ky < m; ky++) {
-			const float2 w = tw[(ky * kv) % N];
-			const float2 a = U[l * m + ky];
-			s += a.x * w.x - a.y * w.y;
+			const float2 w = tw[j];
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				const int l = min(l0 + q * ng, N - 1);
+				const float2 a = U[l * m + ky];
+				s[q] = fmaf(a.x, w.x, fmaf(-a.y, w.y, s[q]));
+			}
+			j += kv;
+			if (j >= N) j -= N;
 		}
-		if (accumulate) out[bc * P + t] += scale * s;
-		else out[bc * P + t] = scale * s;
+#pragma unroll
+		for (int q = 0; q < 4; q++) {
+			const int l = l0 + q * ng;
+			if (l >= N) continue;
+			const long i = bc * P + l * N + kv;
+			float v = scale * s[q];
+			if (accumulate) v += out[i];
+			if (u) v *= dgelu_f(u[i]);
+			out[i] = v;
+		}
 	}
 }
 
 // mode mixing: fwd (conj = 0): out[b][o][k] = sum_i R[i][o][k] in[b][i][k]
 //              bwd (conj = 1): out[b][i][k] = sum_o conj(R[i][o][k]) in[b][o][k]
-__global__ void k_fno_mix(int B, int w, int K, const float2 *__restrict__ in, const float *__restrict__ Rr, const float *__restrict__ Ri,
-                          float2 *__restrict__ out, int conj) {
-	const long n = (long)B * w * K;
+// A thread has one k, four output channels and four cells, so the weights and
+// the inputs are each read a quarter as often (from L2): 64 cells, 32 channels, 276
+// modes: 38 -> 17 us.
+__global__ void __launch_bounds__(128) k_fno_mix(int B, int w, int K, const float2 *__restrict__ in, const float *__restrict__ Rr,
+                                                 const float *__restrict__ Ri, float2 *__restrict__ out, int conj) {
+	const int nc = (w + 3) / 4, nb = (B + 3) / 4;
+	const long n = (long)K * nc * nb;
 	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-		const int k = (int)(t % K);
-		const int c = (int)((t / K) % w);
-		const long b = t / ((long)K * w);
-		float re = 0.0f, im = 0.0f;
+		const int k = (int)(t % K), c0 = 4 * (int)(t / K % nc), b0 = 4 * (int)(t / ((long)K * nc));
+		float re[4][4], im[4][4];
+#pragma unroll
+		for (int c = 0; c < 4; c++)
+#pragma unroll
+			for (int b = 0; b < 4; b++) re[c][b] = im[c][b] = 0.0f;
+#pragma unroll 4
 		for (int j = 0; j < w; j++) {
-			const long ri = conj ? ((long)c * w + j) * K + k : ((long)j * w + c) * K + k;
-			const float rr = Rr[ri], rim = conj ? -Ri[ri] : Ri[ri];
-			const float2 v = in[((long)b * w + j) * K + k];
-			re += rr * v.x - rim * v.y;
-			im += rr * v.y + rim * v.x;
+			float rr[4], ri[4];
+			float2 v[4];
+#pragma unroll
+			for (int c = 0; c < 4; c++) {
+				const int cc = min(c0 + c, w - 1);
+				const long i = conj ? ((long)cc * w + j) * K + k : ((long)j * w + cc) * K + k;
+				rr[c] = Rr[i];
+				ri[c] = conj ? -Ri[i] : Ri[i];
+			}
+#pragma unroll
+			for (int b = 0; b < 4; b++) v[b] = in[((long)min(b0 + b, B - 1) * w + j) * K + k];
+#pragma unroll
+			for (int c = 0; c < 4; c++)
+#pragma unroll
+				for (int b = 0; b < 4; b++) {
+					re[c][b] = fmaf(rr[c], v[b].x, fmaf(-ri[c], v[b].y, re[c][b]));
+					im[c][b] = fmaf(rr[c], v[b].y, fmaf(ri[c], v[b].x, im[c][b]));
+				}
 		}
-		out[t] = make_float2(re, im);
+#pragma unroll
+		for (int c = 0; c < 4; c++)
+#pragma unroll
+			for (int b = 0; b < 4; b++)
+				if (c0 + c < w && b0 + b < B) out[((long)(b0 + b) * w + c0 + c) * K + k] = make_float2(re[c][b], im[c][b]);
 	}
 }
 
-// weight gradient of the mode mixing: dR[i][o][k] = sum_b GO[b][o][k] conj(H[b][i][k])
-__global__ void k_fno_rgrad(int B, int w, int K, const float2 *__restrict__ GO, const float2 *__restrict__ H, float *__restrict__ gRr,
-                            float *__restrict__ gRi) {
-	const long n = (long)w * w * K;
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-		const int k = (int)(t % K);
-		const int o = (int)((t / K) % w);
-		const int i = (int)(t / ((long)K * w));
-		float re = 0.0f, im = 0.0f;
-		for (int b = 0; b < B; b++) {
-			const float2 g = GO[((long)b * w + o) * K + k], h = H[((long)b * w + i) * K + k];
-			re += g.x * h.x + g.y * h.y;
-			im += g.y * h.x - g.x * h.y;
-		}
-		gRr[t] = re;
-		gRi[t] = im;
+// weight gradient of the mode mixing: dR[i][o][k] = sum_b GO[b][o][k] conj(H[b][i][k]).
+// A block has 32 modes and one 4 x 4 block of (i, o); its four warps take a quarter
+// of the cells each and add up in that order.  58 -> 28 us (as k_fno_mix)
+__global__ void __launch_bounds__(128) k_fno_rgrad(int B, int w, int K, const float2 *__restrict__ GO, const float2 *__restrict__ H,
+                                                   float *__restrict__ gRr, float *__restrict__ gRi) {
+	__shared__ float2 sh[3][16][32];
+	const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, nt = (w + 3) / 4;
+	const int k = blockIdx.x * 32 + lane, kk = min(k, K - 1), i0 = 4 * (blockIdx.y / nt), o0 = 4 * (blockIdx.y % nt);
+	float2 acc[4][4];
+#pragma unroll
+	for (int i = 0; i < 4; i++)
+#pragma unroll
+		for (int o = 0; o < 4; o++) acc[i][o] = make_float2(0.0f, 0.0f);
+	const int b0 = (int)((long)seg * B / 4), b1 = (int)((long)(seg + 1) * B / 4);
+#pragma unroll 4
+	for (int b = b0; b < b1; b++) {
+		float2 g[4], h[4];
+#pragma unroll
+		for (int o = 0; o < 4; o++) g[o] = GO[((long)b * w + min(o0 + o, w - 1)) * K + kk];
+#pragma unroll
+		for (int i = 0; i < 4; i++) h[i] = H[((long)b * w + min(i0 + i, w - 1)) * K + kk];
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+#pragma unroll
+			for (int o = 0; o < 4; o++) {
+				acc[i][o].x = fmaf(g[o].x, h[i].x, fmaf(g[o].y, h[i].y, acc[i][o].x));
+				acc[i][o].y = fmaf(g[o].y, h[i].x, fmaf(-g[o].x, h[i].y, acc[i][o].y));
+			}
 	}
-}
-
-// partial[chunk][cx][cy] = sum over the chunk's (b, p) of X[b][cx][p] * Y[b][cy][p]
-// (Y == nullptr: Y = 1, cy = 1).  Chunks of 64 points; fixed order.
-constexpr int kChunk = 64;
-__global__ void k_fno_outer(int B, int P, int cx, int cy, const float *__restrict__ X, const float *__restrict__ Y, float *__restrict__ partial) {
-	__shared__ float xs[kFnoMaxWidth][kChunk + 1];
-	__shared__ float ys[kFnoMaxWidth][kChunk + 1];
-	const long n = (long)B * P;
-	const long t0 = (long)blockIdx.x * kChunk;
-	for (int i = threadIdx.x; i < kChunk; i += blockDim.x) {
-		const long t = t0 + i;
-		const bool ok = t < n;
-		const long b = ok ? t / P : 0, p = ok ? t % P : 0;
-		for (int c = 0; c < cx; c++) xs[c][i] = ok ? X[(b * cx + c) * P + p] : 0.0f;
-		for (int c = 0; c < cy; c++) ys[c][i] = ok ? (Y ? Y[(b * cy + c) * P + p] : 1.0f) : 0.0f;
+	if (seg > 0) {
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+#pragma unroll
+			for (int o = 0; o < 4; o++) sh[seg - 1][4 * i + o][lane] = acc[i][o];
 	}
 	__syncthreads();
-	for (int o = threadIdx.x; o < cx * cy; o += blockDim.x) {
-		const int a = o / cy, c = o % cy;
-		float s = 0.0f;
-		for (int i = 0; i < kChunk; i++) s = fmaf(xs[a][i], ys[c][i], s);
-		partial[(long)blockIdx.x * cx * cy + o] = s;
-	}
+	if (seg > 0 || k >= K) return;
+#pragma unroll
+	for (int i = 0; i < 4; i++)
+#pragma unroll
+		for (int o = 0; o < 4; o++) {
+			if (i0 + i >= w || o0 + o >= w) continue;
+			float2 v = acc[i][o];
+#pragma unroll
+			for (int q = 0; q < 3; q++) { v.x += sh[q][4 * i + o][lane].x; v.y += sh[q][4 * i + o][lane].y; }
+			const long q = ((long)(i0 + i) * w + o0 + o) * K + k;
+			gRr[q] = v.x;
+			gRi[q] = v.y;
+		}
 }
 
-// out[j] = sum_c partial[c][j] in chunk order
-__global__ void k_fno_reduce(int nchunk, int count, const float *__restrict__ partial, float *__restrict__ out) {
-	const int j = blockIdx.x * blockDim.x + threadIdx.x;
-	if (j >= count) return;
+// partial[chunk][cx][cy + 1] = sum over the chunk's (b, p) of X[b][a][p] * Y[b][c][p], and
+// of X alone at c = cy.  Chunks of kChunk points, staged 64 at a time; a thread of
+// the 16 x 16 block has the outputs (ty + 16 i, tx + 16 j).  Fixed order.  32 x 32 channels,
+// 65 536 points: 44 us in two launches (the second for the sums of X) -> 26 us.
+constexpr int kChunk = 128;
+__global__ void __launch_bounds__(256) k_fno_outer(int B, int P, int cx, int cy, const float *__restrict__ X, const float *__restrict__ Y,
+                                                   float *__restrict__ partial) {
+	constexpr int T = 64, PT = T + 4;                    // points a stage, pitch (rows of 17 x 16 bytes)
+	__shared__ __align__(16) float xs[kFnoMaxWidth][PT];
+	__shared__ __align__(16) float ys[kFnoMaxWidth + 1][PT];
+	const long n = (long)B * P;
+	const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, ncy = cy + 1;
+	float acc[4][5];
+#pragma unroll
+	for (int i = 0; i < 4; i++)
+#pragma unroll
+		for (int j = 0; j < 5; j++) acc[i][j] = 0.0f;
+	if (threadIdx.x < T) ys[cy][threadIdx.x] = 1.0f;
+	for (int s = 0; s < kChunk; s += T) {
+		// four consecutive points are in one cell (P is a multiple of 4)
+		const int q4 = 4 * (threadIdx.x & 15);
+		const long t = (long)blockIdx.x * kChunk + s + q4;
+		const bool ok = t < n;
+		const long b = ok ? t / P : 0, p = ok ? t % P : 0;
+		float4 v[8];
+#pragma unroll
+		for (int e = 0; e < 8; e++) {
+			const int c = (threadIdx.x >> 4) + 16 * (e & 3), cn = e < 4 ? cx : cy;
+			v[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			if (ok && c < cn) v[e] = *reinterpret_cast<const float4 *>((e < 4 ? X : Y) + (b * cn + c) * P + p);
+		}
+		__syncthreads();
+#pragma unroll
+		for (int e = 0; e < 8; e++) {
+			const int c = (threadIdx.x >> 4) + 16 * (e & 3);
+			if (c < (e < 4 ? cx : cy)) *reinterpret_cast<float4 *>(e < 4 ? &xs[c][q4] : &ys[c][q4]) = v[e];
+		}
+		__syncthreads();
+#pragma unroll 2
+		for (int q = 0; q < T; q += 4) {
+			float4 x[4], y[5];
+#pragma unroll
+			for (int i = 0; i < 4; i++)
+				if (16 * i < cx) x[i] = *reinterpret_cast<const float4 *>(&xs[min(ty + 16 * i, cx - 1)][q]);
+#pragma unroll
+			for (int j = 0; j < 5; j++)
+				if (16 * j < ncy) y[j] = *reinterpret_cast<const float4 *>(&ys[min(tx + 16 * j, cy)][q]);
+#pragma unroll
+			for (int i = 0; i < 4; i++)
+#pragma unroll
+				for (int j = 0; j < 5; j++)
+					if (16 * i < cx && 16 * j < ncy)
+						acc[i][j] = fmaf(x[i].w, y[j].w, fmaf(x[i].z, y[j].z, fmaf(x[i].y, y[j].y, fmaf(x[i].x, y[j].x, acc[i][j]))));
+		}
+	}
+	float *o = partial + (long)blockIdx.x * cx * ncy;
+#pragma unroll
+	for (int i = 0; i < 4; i++)
+#pragma unroll
+		for (int j = 0; j < 5; j++)
+			if (ty + 16 * i < cx && tx + 16 * j < ncy) o[(ty + 16 * i) * ncy + tx + 16 * j] = acc[i][j];
+}
+
+// dM[a][c] = sum over the chunks of partial[.][a][c], db[a] = of partial[.][a][cy], in a
+// fixed order: eight segments of chunks for 32 outputs a block, then the segments.
+// One thread an output, 1024 chunks: 36 us; 512 chunks in segments: 9 us
+__global__ void __launch_bounds__(256) k_fno_reduce(int nchunk, int cx, int cy, const float *__restrict__ partial, float *__restrict__ dM,
+                                                    float *__restrict__ db) {
+	__shared__ float sh[8][33];
+	const int count = cx * (cy + 1), lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+	const int j = blockIdx.x * 32 + lane;
+	const int c0 = (int)((long)seg * nchunk / 8), c1 = (int)((long)(seg + 1) * nchunk / 8);
 	float s = 0.0f;
-	for (int c = 0; c < nchunk; c++) s += partial[(long)c * count + j];
-	out[j] = s;
+	if (j < count) {
+#pragma unroll 8
+		for (int c = c0; c < c1; c++) s += partial[(long)c * count + j];
+	}
+	sh[seg][lane] = s;
+	__syncthreads();
+	if (seg == 0 && j < count) {
+		for (int q = 1; q < 8; q++) s += sh[q][lane];
+		const int a = j / (cy + 1), c = j % (cy + 1);
+		if (c < cy) dM[a * cy + c] = s;
+		else db[a] = s;
+	}
 }
 
 // dy = 2 (y - t / scale) / n, partial[block] = sum of squares (fixed tree)
@@ -708,7 +879,7 @@ struct qb_fno {
 	qb::DevBuf GO, GH;
 	int use_tc = 0;                               // pointwise maps and truncated DFTs on the tensor cores (BF16, FP32 accumulation)
 	qb::DevBuf kerr;                              // error word of the bounded MMA waits
-	qb::DevBuf twm, tscr, uscr;                   // tensor-core DFTs: the 4 twiddle matrices, stage scratch
+	qb::DevBuf twn, twm, tscr, uscr;                   // tensor-core DFTs: the 4 twiddle matrices, stage scratch
 	const float *Bm1 = nullptr, *Bm2 = nullptr, *BmA = nullptr, *BmB = nullptr;
 
 	// the twiddle matrices of the two-stage DFT and inverse (FP32 [Nn][K], from FP64)
@@ -754,10 +925,22 @@ struct qb_fno {
 		launch(name, k_fno_tc<Ld, Ep, Bb>, grid, fnotc::kThreads, (size_t)fnotc::kSmem, s, ld, ep, bm, K, Nn, kerr.as<int>());
 	}
 
+	// the N-th roots of unity of the FP32 transforms (from FP64)
+	const float2 *roots(cudaStream_t s) {
+		if (twn.p == nullptr) {
+			std::vector<float2> h(N);
+			for (int j = 0; j < N; j++) h[j] = make_float2((float)std::cos(2.0 * M_PI * j / N), (float)std::sin(2.0 * M_PI * j / N));
+			twn.ensure(sizeof(float2) * N);
+			QB_CUDA(cudaMemcpyAsync(twn.p, h.data(), sizeof(float2) * N, cudaMemcpyHostToDevice, s));
+			QB_CUDA(cudaStreamSynchronize(s));
+		}
+		return twn.as<float2>();
+	}
+
 	// H[fld] = scale DFT(f[fld]) for the B w fields
 	void dft(int B, const float *f, float2 *Hout, float scale, cudaStream_t s) {
 		if (!use_tc) {
-			launch("fno_dft", k_fno_dft, (unsigned)(B * w), 256, dft_smem(), s, N, m, f, Hout, scale);
+			launch("fno_dft", k_fno_dft, (unsigned)(B * w), 256, dft_smem(), s, N, m, f, roots(s), Hout, scale);
 			return;
 		}
 		ensure_err(s);
@@ -767,10 +950,10 @@ struct qb_fno {
 		row_gemm("fno_dft_tc", LdDft2{ tscr.as<float>(), N }, EpDft2{ Hout, m, scale }, BMat{ Bm2, 2 * N, nf * m }, (nf * m + 127) / 128,
 		         2 * N, 2 * (2 * m - 1), s);
 	}
-	// out[fld] (=, +=) scale Re IDFT(O[fld])
-	void idft(int B, const float2 *O, float *out, float scale, int accumulate, cudaStream_t s) {
+	// out[fld] (=, +=) scale Re IDFT(O[fld]), then times dgelu(u) when u is given
+	void idft(int B, const float2 *O, float *out, float scale, int accumulate, const float *u, cudaStream_t s) {
 		if (!use_tc) {
-			launch("fno_idft", k_fno_idft, (unsigned)(B * w), 256, idft_smem(), s, N, m, O, out, scale, accumulate);
+			launch("fno_idft", k_fno_idft, (unsigned)(B * w), 256, idft_smem(), s, N, m, O, roots(s), out, scale, accumulate, u);
 			return;
 		}
 		ensure_err(s);
@@ -780,13 +963,15 @@ struct qb_fno {
 		         2 * (2 * m - 1), 2 * N, s);
 		row_gemm("fno_idft_tc", LdIdftB{ uscr.as<float>(), m }, EpIdftB{ out, N, scale, accumulate }, BMat{ BmB, 2 * m, nf * N },
 		         (nf * N + 127) / 128, 2 * m, N, s);
+		const long nw = (long)B * w * P;
+		if (u != nullptr) launch("fno_gelu_bwd", k_fno_gelu_bwd, grid_for(nw), 256, 0, s, nw, u, out);
 	}
 	// mode mixing: out[b][c][k] = sum over the other channel of R (or conj R, backward) times in.
 	// On the tensor cores a mode's B matrix is rebuilt per 128-cell tile, which
 	// pays only when the batch fills the tiles (at 64 cells the FP32 kernel is faster)
 	void mix(int B, const float2 *in, const float *Rr, const float *Ri, float2 *out, int conj, cudaStream_t s) {
 		if (!use_tc || B < 128) {
-			launch("fno_mix", k_fno_mix, grid_for((long)B * w * K), 256, 0, s, B, w, K, in, Rr, Ri, out, conj);
+			launch("fno_mix", k_fno_mix, grid_for(2L * K * ((w + 3) / 4) * ((B + 3) / 4)), 128, 0, s, B, w, K, in, Rr, Ri, out, conj);
 			return;
 		}
 		ensure_err(s);
@@ -806,12 +991,28 @@ struct qb_fno {
 	void pointwise(int B, int cin, int cout, const float *in, const float *M, const float *bias, const float *add, float *uout,
 	               float *hout, int act, cudaStream_t s) {
 		if (use_tc) pointwise_mma(B, cin, cout, 0, in, M, bias, add, uout, hout, act, s);
-		else launch("fno_pointwise", k_fno_pointwise, grid_for((long)B * P), 256, 0, s, B, P, cin, cout, in, M, bias, add, uout, hout, act);
+		else pointwise_f32(B, cin, cout, 0, in, M, bias, add, uout, hout, act, s);
+	}
+	// grid: a thread a point; two (four) blocks share the outputs of a point while the
+	// points alone do not fill the GPU twice
+	void pointwise_f32(int B, int cin, int cout, int trans, const float *in, const float *M, const float *bias, const float *add, float *uout,
+	                   float *hout, int act, cudaStream_t s) {
+		auto go = [&](auto kern) {
+			const unsigned gx = grid_for((long)B * P);
+			const dim3 g(gx, gx < 1200 ? std::max(1, std::min(4, cout / 4)) : 1);
+			qb::ProfScope ps("fno_pointwise", s);
+			kern<<<g, 256, 0, s>>>(B, P, cin, cout, trans, in, M, bias, add, uout, hout, act);
+			QB_CUDA(cudaGetLastError());
+		};
+		if (cin <= 4) go(k_fno_pointwise<4>);
+		else if (cin <= 16) go(k_fno_pointwise<16>);
+		else if (cin <= 32) go(k_fno_pointwise<32>);
+		else go(k_fno_pointwise<64>);
 	}
 	// out = M^T in (the backward of a pointwise map)
 	void pointwise_t(int B, int cin, int cout, const float *in, const float *M, float *out, cudaStream_t s) {
 		if (use_tc) pointwise_mma(B, cin, cout, 1, in, M, nullptr, nullptr, nullptr, out, 0, s);
-		else launch("fno_pointwise_t", k_fno_pointwise_t, grid_for((long)B * P), 256, 0, s, B, P, cin, cout, in, M, out);
+		else pointwise_f32(B, cout, cin, 1, in, M, nullptr, nullptr, nullptr, out, 0, s);
 	}
 	void pointwise_mma(int B, int cin, int cout, int trans, const float *in, const float *M, const float *bias, const float *add,
 	                   float *uout, float *hout, int act, cudaStream_t s) {
@@ -849,13 +1050,13 @@ struct qb_fno {
 		tscr.ensure(sizeof(float) * (long)B * w * m * 2 * N);
 		uscr.ensure(sizeof(float) * (long)B * w * N * 2 * m);
 		const long nchunk = ((long)B * P + kChunk - 1) / kChunk;
-		partial.ensure(sizeof(float) * nchunk * kFnoMaxWidth * kFnoMaxWidth);
+		partial.ensure(sizeof(float) * nchunk * kFnoMaxWidth * (kFnoMaxWidth + 1));
 		lossp.ensure(sizeof(double) * 4096);
 		cap = B;
 	}
 
-	size_t dft_smem() const { return sizeof(float) * P + sizeof(float2) * ((long)N * m + N); }
-	size_t idft_smem() const { return sizeof(float2) * ((long)K + (long)N * m + N); }
+	size_t dft_smem() const { return sizeof(float) * (long)N * (N + 1) + sizeof(float2) * ((long)N * m + N); }
+	size_t idft_smem() const { return sizeof(float2) * (2L * m * m + (long)N * m + N); }
 
 	void forward(int B, const double *W, cudaStream_t s) {
 		reserve(B);
@@ -864,7 +1065,7 @@ struct qb_fno {
 		for (int l = 0; l < L; l++) {
 			dft(B, h[l].as<float>(), H[l].as<float2>(), 1.0f, s);
 			mix(B, H[l].as<float2>(), P_(off.Rr[l]), P_(off.Ri[l]), GO.as<float2>(), 0, s);
-			idft(B, GO.as<float2>(), tmp.as<float>(), 1.0f / (float)P, 0, s);
+			idft(B, GO.as<float2>(), tmp.as<float>(), 1.0f / (float)P, 0, nullptr, s);
 			pointwise(B, w, w, h[l].as<float>(), P_(off.W[l]), P_(off.b[l]), tmp.as<float>(), u[l].as<float>(), h[l + 1].as<float>(),
 			          l < L - 1 ? 1 : 0, s);
 		}
@@ -877,27 +1078,29 @@ struct qb_fno {
 		const long n = (long)B * P;
 		const int nchunk = (int)((n + kChunk - 1) / kChunk);
 		launch("fno_outer", k_fno_outer, nchunk, 256, 0, s, B, P, cout, cin, dout, in, partial.as<float>());
-		launch("fno_reduce", k_fno_reduce, (cout * cin + 255) / 256, 256, 0, s, nchunk, cout * cin, partial.as<float>(), G_(offM));
-		launch("fno_outer", k_fno_outer, nchunk, 256, 0, s, B, P, cout, 1, dout, nullptr, partial.as<float>());
-		launch("fno_reduce", k_fno_reduce, (cout + 255) / 256, 256, 0, s, nchunk, cout, partial.as<float>(), G_(offb));
+		launch("fno_reduce", k_fno_reduce, (cout * (cin + 1) + 31) / 32, 256, 0, s, nchunk, cout, cin, partial.as<float>(), G_(offM), G_(offb));
 	}
 
 	double loss_backward(int B, const double *target, cudaStream_t s) {
-		const long n4 = (long)B * 4 * P, nw = (long)B * w * P;
+		const long n4 = (long)B * 4 * P;
 		const int lb = 512;
 		launch("fno_loss", k_fno_loss, lb, 256, 0, s, B, P, y.as<float>(), target, scale[0], scale[1], scale[2], scale[3], dy.as<float>(), lossp.as<double>());
 		// projection
 		pw_grads(B, w, 4, h[L].as<float>(), dy.as<float>(), off.Q, off.q, s);
 		pointwise_t(B, w, 4, dy.as<float>(), P_(off.Q), dh.as<float>(), s);
 		for (int l = L - 1; l >= 0; l--) {
-			if (l < L - 1) launch("fno_gelu_bwd", k_fno_gelu_bwd, grid_for(nw), 256, 0, s, nw, u[l].as<float>(), dh.as<float>());
-			// dh now holds du
+			// dh holds du of layer l (the layers below the last have had their dgelu factor)
 			pw_grads(B, w, w, h[l].as<float>(), dh.as<float>(), off.W[l], off.b[l], s);
 			dft(B, dh.as<float>(), GO.as<float2>(), 1.0f / (float)P, s);
-			launch("fno_rgrad", k_fno_rgrad, grid_for((long)w * w * K), 256, 0, s, B, w, K, GO.as<float2>(), H[l].as<float2>(), G_(off.Rr[l]), G_(off.Ri[l]));
+			{
+				const unsigned nt = (unsigned)((w + 3) / 4);
+				qb::ProfScope ps("fno_rgrad", s);
+				k_fno_rgrad<<<dim3((unsigned)((K + 31) / 32), nt * nt), 128, 0, s>>>(B, w, K, GO.as<float2>(), H[l].as<float2>(), G_(off.Rr[l]), G_(off.Ri[l]));
+				QB_CUDA(cudaGetLastError());
+			}
 			mix(B, GO.as<float2>(), P_(off.Rr[l]), P_(off.Ri[l]), GH.as<float2>(), 1, s);
 			pointwise_t(B, w, w, dh.as<float>(), P_(off.W[l]), tmp.as<float>(), s);
-			idft(B, GH.as<float2>(), tmp.as<float>(), 1.0f, 1, s);
+			idft(B, GH.as<float2>(), tmp.as<float>(), 1.0f, 1, l > 0 ? u[l - 1].as<float>() : nullptr, s);
 			std::swap(dh, tmp);
 		}
 		// lift
