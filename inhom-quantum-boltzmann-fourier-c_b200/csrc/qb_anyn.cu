@@ -821,6 +821,7 @@ inline int own_for_plan(const Plan &pl, bool fp64) {
 }
 template <class C> struct I3RowsBP {
 	C *Y; const C *Pg; C *X; int N, nl, nt, t0;
+	int ns;                               // X[cell][4][ns]: unit t0 + tt goes to the partial (t0 + tt) % ns, each with CTAs of its own
 	WaveUnits un;                         // the rows of a pair's chains are kept in Y for k_any_i3_rows_y
 	const int *kind;                      // null: every cell complex
 	Plan pl;
@@ -835,12 +836,15 @@ template <class C, bool RF, int R1, int R2> __device__ __forceinline__ void i3_r
 	Tile<C> T(sm, P, nl);
 	const unsigned mgP = magic_div((unsigned)P), mgnl = magic_div((unsigned)nl);
 	const int bpg = P / nl;
-	const long cj = blockIdx.x / bpg;             // cell 4 + j
+	const long cjs = blockIdx.x / bpg;            // (cell 4 + j) ns + partial
+	const int part = (int)(cjs % p.ns), first = (part - p.t0 % p.ns + p.ns) % p.ns;
+	if (first >= p.nt) return;
+	const long cj = cjs / p.ns;
 	const int l0 = (int)(blockIdx.x % bpg) * nl;
 	const long cell = cj / 4;
 	const int j3 = (int)(cj % 4);
 	load_tw(T.tw, P, p.pl);
-	C *X = p.X + cj * PP + (long)l0 * P;
+	C *X = p.X + cjs * PP + (long)l0 * P;
 	constexpr int kOwn = own_for<C, R1, R2>();
 	C acc[kOwn];
 #pragma unroll
@@ -848,7 +852,7 @@ template <class C, bool RF, int R1, int R2> __device__ __forceinline__ void i3_r
 		const int i = threadIdx.x + e * kThreads;
 		acc[e] = i < ne ? X[i] : czero<C>();       // rows l0.. of X are contiguous: element i at X[i]
 	}
-	for (int tt = 0; tt < p.nt; tt++) {
+	for (int tt = first; tt < p.nt; tt += p.ns) {
 		const long ct = cell * p.nt + tt;
 		constexpr int kH = RF ? 2 : 4;
 		for (int h = 0; h < kH; h++) {
@@ -902,7 +906,7 @@ template <class C, bool RF, int R1, int R2> __device__ __forceinline__ void i3_r
 template <class C, int R1, int R2> constexpr int rows_b_ctas() { return sizeof(C) == 8 && own_for<C, R1, R2>() <= 12 ? 3 : 2; }
 template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads, rows_b_ctas<C, R1, R2>()) k_any_i3_rows_b(const I3RowsBP<C> p) {
 	extern __shared__ __align__(16) unsigned char sm[];
-	const long cell = blockIdx.x / (4L * (2 * p.N / p.nl));         // blocks (cell 4 + j) bpg + row block
+	const long cell = blockIdx.x / (4L * p.ns * (2 * p.N / p.nl));  // blocks ((cell 4 + j) ns + partial) bpg + row block
 	if constexpr (has_rf<C>()) {
 		if (p.kind != nullptr && p.kind[cell] == 0) {
 			i3_rows_b<C, true, R1, R2>(p, sm);
@@ -974,6 +978,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 // i, block of nl columns of those N + 1) adds the wave's terms in order.
 template <class C> struct I3ColsZP {
 	const C *V; C *Z; const C *psi1; int N, nl, nt, t0;
+	int ns;                               // Z[cell][4][ns], partials as in k_any_i3_rows_b
 	WaveUnits un;
 	const int *kind;
 	Plan pl;
@@ -984,7 +989,10 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	const long PP = (long)P * P;
 	Tile<C> T(sm, P, nl);
 	const int bpg = (ZS + nl - 1) / nl;
-	const long ci = blockIdx.x / bpg;             // cell 4 + i
+	const long cis = blockIdx.x / bpg;            // (cell 4 + i) ns + partial
+	const int part = (int)(cis % p.ns), first = (part - p.t0 % p.ns + p.ns) % p.ns;
+	if (first >= p.nt) return;
+	const long ci = cis / p.ns;
 	const int z0 = (int)(blockIdx.x % bpg) * nl;     // first column, as frequency + N/2
 	const long cell = ci / 4;
 	const int i3 = (int)(ci % 4);
@@ -993,10 +1001,10 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	load_tw(T.tw, P, p.pl);
 	const int nz = min(nl, (rf ? ZS : N) - z0);       // columns of this block
 	if (nz <= 0) return;
-	C *Z = p.Z + ci * (long)ZS * ZS;
+	C *Z = p.Z + cis * (long)ZS * ZS;
 	const int pitch = T.pitch;
 	const unsigned mgnl = magic_div((unsigned)nl);
-	for (int tt = 0; tt < p.nt; tt++) {
+	for (int tt = first; tt < p.nt; tt += p.ns) {
 		if (!p.un.pair(p.t0 + tt)) continue;
 		const C *v = p.V + ((cell * p.nt + tt) * 4 + i3) * PP;
 		const C *ps = p.psi1 + (long)p.un.term(p.t0 + tt) * N * N;
@@ -1129,7 +1137,7 @@ template <class C> __global__ void __launch_bounds__(kThreads) k_any_i3_fused(co
 template <class C> struct AsmP {
 	const C *What, *FS, *FS4, *Q, *X;    // FS [cell][3], FS4 / Q [cell][4], X [cell][4][nxp] (null: part absent)
 	int nxp;                             // partials of X per (cell, j), added in order
-	const C *Zp; const int *kind;        // sums of k_any_i3_cols_z (null: none) and the cells' forms
+	const C *Zp; int nzp; const int *kind;   // sums of k_any_i3_cols_z, nzp partials a grid (null: none), and the cells' forms
 	C *Z; int N, nl;
 	double s1, s2;
 	int mode;
@@ -1237,14 +1245,18 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 			const double f = (j == 0 ? 2.0 : -2.0) * p.s1;
 			if (has_rf<C>() && p.kind != nullptr && p.kind[cell] == 0) {
 				// A = Z_2c + i Z_2c+1, each the transform of a real grid
-				const C *A = p.Zp + (cell * 4 + (j >> 1)) * (long)ZS * ZS;
-				const C u = A[fl * ZS + fk], v = A[(N - fl) * ZS + N - fk];
-				cd.x -= f * 0.5 * ((j & 1) ? (double)u.y + (double)v.y : (double)u.x + (double)v.x);
-				cd.y -= f * 0.5 * ((j & 1) ? (double)v.x - (double)u.x : (double)u.y - (double)v.y);
+				for (int k = 0; k < p.nzp; k++) {
+					const C *A = p.Zp + ((cell * 4 + (j >> 1)) * p.nzp + k) * (long)ZS * ZS;
+					const C u = A[fl * ZS + fk], v = A[(N - fl) * ZS + N - fk];
+					cd.x -= f * 0.5 * ((j & 1) ? (double)u.y + (double)v.y : (double)u.x + (double)v.x);
+					cd.y -= f * 0.5 * ((j & 1) ? (double)v.x - (double)u.x : (double)u.y - (double)v.y);
+				}
 			} else {
-				const C z = p.Zp[cj * (long)ZS * ZS + fl * ZS + fk];
-				cd.x -= f * (double)z.x;
-				cd.y -= f * (double)z.y;
+				for (int k = 0; k < p.nzp; k++) {
+					const C z = p.Zp[(cj * p.nzp + k) * (long)ZS * ZS + fl * ZS + fk];
+					cd.x -= f * (double)z.x;
+					cd.y -= f * (double)z.y;
+				}
 			}
 		}
 		const long q = (long)ls * N + ks, o = cj * NN + q;
@@ -1580,13 +1592,23 @@ template <class C> struct AnyRhs {
 		return on == 1 && tile_bytes<C>(P, P) <= kMaxSmem;
 	}
 
+	// partial sums of X and Z a (cell, component): the last row pass and the Z
+	// columns run one CTA a (cell, component, line block, partial), and with one CTA
+	// for all terms of a wave a few cells left most SMs idle (12 cells at N = 48:
+	// 144 CTAs of three terms each, 40 us a launch; in four partials the step of 12 cells 12.5 -> 11.8 ms).  Three CTAs an SM; the
+	// count depends on the batch alone, so waves and slices do not change the sums
+	int partials() const {
+		const long ctas = (long)ncells * 4 * (P / nl1);
+		return (int)std::max(1L, std::min(8L, (3 * 148 + ctas - 1) / ctas));
+	}
+
 	// returns the partials of X per (cell, j).  FP32: the cells of kind 0 (no
 	// Nyquist content, Hermitian state) take the real form, two chains packed
 	// in one complex transform, the others the complex chains, in the same
 	// launches (the kernels read a cell's kind; the real form leaves half of
 	// its units idle)
 	int i3_sums(const DevI3 &t, const double2 *W, AsmP<C> &as) {
-		const int nxp = fused_i3() ? 4 : 1;
+		const int nxp = fused_i3() ? 4 : partials();
 		ws.i3p.ensure(sizeof(C) * ncells * 4 * nxp * PP);
 		QB_CUDA(cudaMemsetAsync(ws.i3p.p, 0, sizeof(C) * ncells * 4 * nxp * PP, s));
 		const int *kind = nullptr;
@@ -1594,8 +1616,9 @@ template <class C> struct AnyRhs {
 			if (real_form_enabled()) kind = i3_form_kinds(ws, ncells, W, s);
 		}
 		if (t.pairM > 0) {
-			ws.i3z.ensure(sizeof(C) * 4 * ncells * (N + 1) * (N + 1));
-			QB_CUDA(cudaMemsetAsync(ws.i3z.p, 0, sizeof(C) * 4 * ncells * (N + 1) * (N + 1), s));
+			as.nzp = partials();
+			ws.i3z.ensure(sizeof(C) * 4 * as.nzp * ncells * (N + 1) * (N + 1));
+			QB_CUDA(cudaMemsetAsync(ws.i3z.p, 0, sizeof(C) * 4 * as.nzp * ncells * (N + 1) * (N + 1), s));
 			as.Zp = ws.i3z.as<C>();
 			as.kind = kind;
 		}
@@ -1612,8 +1635,8 @@ template <class C> struct AnyRhs {
 		        k_any_i3_rows_y<C, 16, 3>, k_any_i3_rows_y<C, 16, 6>, k_any_i3_rows_y<C, 16, 12>, k_any_i3_rows_y<C, 16, 16>,
 		        k_any_i3_rows_y<C, 0, 0>);
 		I3ColsZP<C> z{};
-		z.V = V; z.Z = Z; z.psi1 = Tabs<C>::i3_psi1(t); z.N = N; z.nl = nl1; z.nt = n; z.t0 = t0; z.un.M = t.pairM; z.kind = kc; z.pl = pl;
-		by_plan([&](auto kern) { launch(kern, "any_i3_cols_z", (long)nc * 4 * ((N + nl1) / nl1), smem(nl1, 1), s, z); },
+		z.V = V; z.Z = Z; z.psi1 = Tabs<C>::i3_psi1(t); z.ns = partials(); z.N = N; z.nl = nl1; z.nt = n; z.t0 = t0; z.un.M = t.pairM; z.kind = kc; z.pl = pl;
+		by_plan([&](auto kern) { launch(kern, "any_i3_cols_z", (long)nc * 4 * z.ns * ((N + nl1) / nl1), smem(nl1, 1), s, z); },
 		        k_any_i3_cols_z<C, 16, 3>, k_any_i3_cols_z<C, 16, 6>, k_any_i3_cols_z<C, 16, 12>, k_any_i3_cols_z<C, 16, 16>,
 		        k_any_i3_cols_z<C, 0, 0>);
 	}
@@ -1624,7 +1647,7 @@ template <class C> struct AnyRhs {
 	// form) and 16 chains (8 in the real form).  A cell's terms still run in
 	// order, so the sums do not depend on the waves.
 	void i3_waves(const DevI3 &t, const double2 *W, int nxp, const int *kind) {
-		const bool fused = nxp == 4, pairs = t.pairM > 0;
+		const bool fused = fused_i3(), pairs = t.pairM > 0;
 		const WaveUnits un{ t.pairM };
 		const int nunits = pairs ? t.nterms / t.pairM * ((t.pairM + 1) / 2) : t.nterms;
 		const int per_term = fused && !pairs ? 4 : 20;
@@ -1660,7 +1683,7 @@ template <class C> struct AnyRhs {
 					// kernel to 173 registers, one CTA an SM); FP64 runs one CTA an SM anyway
 					f.pl = (ws.anyn_plan == 0 && sizeof(C) == 8) ? with_tw(make_plan(P, 1)) : pl;
 					launch(k_any_i3_fused<C>, "any_i3_fused", (long)nc * 16, tile_bytes<C>(P, P), s, f);
-					if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * (N + 1) * (N + 1), nc, n, t0, kc);
+					if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * partials() * (N + 1) * (N + 1), nc, n, t0, kc);
 					continue;
 				}
 				I3RowsAP<C> a{};
@@ -1675,11 +1698,11 @@ template <class C> struct AnyRhs {
 				        k_any_i3_cols<C, 16, 3>, k_any_i3_cols<C, 16, 6>, k_any_i3_cols<C, 16, 12>, k_any_i3_cols<C, 16, 16>,
 				        k_any_i3_cols<C, 0, 0>);
 				I3RowsBP<C> b{};
-				b.Y = Y; b.Pg = Pg; b.X = X; b.N = N; b.nl = nl4; b.nt = n; b.t0 = t0; b.kind = kc; b.un = un; b.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i3_rows_b", blocks((long)nc * 4, nl4), smem(nl4, 1), s, b); },
+				b.Y = Y; b.Pg = Pg; b.X = X; b.ns = nxp; b.N = N; b.nl = nl4; b.nt = n; b.t0 = t0; b.kind = kc; b.un = un; b.pl = pl;
+				by_plan([&](auto kern) { launch(kern, "any_i3_rows_b", blocks((long)nc * 4 * nxp, nl4), smem(nl4, 1), s, b); },
 				        k_any_i3_rows_b<C, 16, 3>, k_any_i3_rows_b<C, 16, 6>, k_any_i3_rows_b<C, 16, 12>,
 				        k_any_i3_rows_b<C, 16, 16>, k_any_i3_rows_b<C, 0, 0>);
-				if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * (N + 1) * (N + 1), nc, n, t0, kc);
+				if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * partials() * (N + 1) * (N + 1), nc, n, t0, kc);
 			}
 		}
 	}
