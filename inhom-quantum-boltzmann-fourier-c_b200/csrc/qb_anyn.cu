@@ -27,12 +27,13 @@
 // launch (the CTA holding its line), which adds the wave's terms in order, and
 // the waves follow one another on the stream, so the result is deterministic.
 #include "qb_engine.h"
-#include "qb_fft.cuh"
+#include "qb_grid16.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <set>
 #include <tuple>
@@ -55,99 +56,6 @@ struct Plan {
 
 __device__ __forceinline__ int src_idx(int p, int N) {         // padded index -> N-grid index, or -1 (zero band)
 	return p < N / 2 ? p : (p >= 3 * N / 2 ? p - N : -1);
-}
-
-template <int DIR, class C> __device__ __forceinline__ void dft3(C &x0, C &x1, C &x2) {
-	using R = typename CT<C>::R;
-	const C t1 = cadd(x1, x2);
-	const C m = csub(x0, cscale(t1, (R)0.5));
-	const C d = mul_i<DIR>(cscale(csub(x1, x2), (R)0.86602540378443864676));   // sin(2 pi / 3)
-	x0 = cadd(x0, t1);
-	x1 = cadd(m, d);
-	x2 = csub(m, d);
-}
-
-// cos and sin of 2 pi m / R for R = 6, 12, 16 (the twiddles of the composite
-// register DFTs; folded to constants when m is known at compile time)
-__host__ __device__ constexpr double cos_r(int R, int m) {
-	constexpr double h = 0.5, c3 = 0.86602540378443864676, c8 = 0.70710678118654752440;
-	constexpr double a = 0.92387953251128675613, b = 0.38268343236508977173;
-	if (R == 16) {
-		const double t[16] = { 1, a, c8, b, 0, -b, -c8, -a, -1, -a, -c8, -b, 0, b, c8, a };
-		return t[m];
-	}
-	if (R == 12) {
-		const double t[12] = { 1, c3, h, 0, -h, -c3, -1, -c3, -h, 0, h, c3 };
-		return t[m];
-	}
-	const double t[6] = { 1, h, -h, -1, -h, h };
-	return t[m];
-}
-__host__ __device__ constexpr double sin_r(int R, int m) {
-	if (R == 6) {
-		constexpr double c3 = 0.86602540378443864676;
-		const double t[6] = { 0, c3, c3, 0, -c3, -c3 };
-		return t[m];
-	}
-	return cos_r(R, (m + 3 * R / 4) % R);     // sin x = cos(x - pi/2); R = 12, 16 are multiples of 4
-}
-
-template <int R1, int R2, int DIR, class C> __device__ __forceinline__ void dft_ct(C (&x)[R1 * R2]);
-
-template <int RAD, int DIR, class C> __device__ __forceinline__ void dft_r(C (&v)[RAD]) {
-	if constexpr (RAD == 16) dft_ct<4, 4, DIR>(v);
-	else if constexpr (RAD == 12) dft_ct<4, 3, DIR>(v);
-	else if constexpr (RAD == 8) dft8<DIR>(v);
-	else if constexpr (RAD == 6) dft_ct<2, 3, DIR>(v);
-	else if constexpr (RAD == 4) dft4<DIR>(v[0], v[1], v[2], v[3]);
-	else if constexpr (RAD == 3) dft3<DIR>(v[0], v[1], v[2]);
-	else dft2(v[0], v[1]);
-}
-
-// an R1 R2-point DFT in registers, in place: R2 DFTs of R1 points (stride
-// R2), twiddles w_R^(n2 k1), R1 DFTs of R2 points.  Input in natural order;
-// output frequency k1 + R1 k2 lands in slot k1 R2 + k2 (freq_of gives the
-// frequency of a slot), so no second array of R values is live
-template <int R1, int R2, int DIR, class C> __device__ __forceinline__ void dft_ct(C (&x)[R1 * R2]) {
-	using R = typename CT<C>::R;
-	constexpr int RR = R1 * R2;
-#pragma unroll
-	for (int n2 = 0; n2 < R2; n2++) {
-		C v[R1];
-#pragma unroll
-		for (int n1 = 0; n1 < R1; n1++) v[n1] = x[n2 + R2 * n1];
-		dft_r<R1, DIR>(v);
-#pragma unroll
-		for (int k1 = 0; k1 < R1; k1++) {
-			const int m = (n2 * k1) % RR;
-			if (m == 0) {
-				x[n2 + R2 * k1] = v[k1];
-			} else {
-				C w;
-				w.x = (R)cos_r(RR, m);
-				w.y = (R)(DIR < 0 ? -sin_r(RR, m) : sin_r(RR, m));
-				x[n2 + R2 * k1] = cmul(v[k1], w);
-			}
-		}
-	}
-#pragma unroll
-	for (int k1 = 0; k1 < R1; k1++) {
-		C v[R2];
-#pragma unroll
-		for (int n2 = 0; n2 < R2; n2++) v[n2] = x[k1 * R2 + n2];
-		dft_r<R2, DIR>(v);
-#pragma unroll
-		for (int k2 = 0; k2 < R2; k2++) x[k1 * R2 + k2] = v[k2];
-	}
-}
-
-// frequency held in slot s after dft_r<RAD> (the composite radices leave
-// their output permuted; 2, 3, 4, 8 and the sub-DFTs are in natural order)
-template <int RAD> __host__ __device__ constexpr int freq_of(int s) {
-	if (RAD == 16) return s / 4 + 4 * (s % 4);
-	if (RAD == 12) return s / 3 + 4 * (s % 3);
-	if (RAD == 6) return s / 3 + 2 * (s % 3);
-	return s;
 }
 
 // one Stockham stage of radix RAD over nl lines of length L (sub-transforms of
@@ -1033,105 +941,6 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	}
 }
 
-// The I3 chains with the whole P x P grid in shared memory (P = 48 and 96 in
-// FP32, P = 48 in FP64): one CTA per (cell, j, i) runs the wave's terms in
-// order, X[cell][j][i] += eta_i P_i . FFT2(psi2_t . IFFT2(W^_i . P_j)), each
-// chain one load of W^_i . P_j, four in-place 2-D passes over the tile and one
-// update of the partial X[cell][j][i] (in L2) instead of three global passes;
-// the assembly adds the four partials of (cell, j) in the order i = 0..3.
-template <class C> struct I3FusedP {
-	using R = typename CT<C>::R;
-	const C *What, *Pg; C *X; const R *psi2T; const int *idx; const double *scale;
-	int N, nt, t0;
-	WaveUnits un;
-	C *Y;                                 // chains of the pairs, as k_any_i3_rows_b leaves them
-	const int *kind;                      // null: every cell complex
-	Plan pl;
-};
-// RF (kind 0): the CTA (cell, j, pr), pr < 2, runs the packed chain of the
-// combos 2pr, 2pr + 1 into the real partial X[cell][j][pr] (partials 2, 3 stay
-// zero; the CTAs pr >= 2 are idle)
-template <class C, bool RF> __device__ __forceinline__ void i3_fused(const I3FusedP<C> &p, unsigned char *sm) {
-	using R = typename CT<C>::R;
-	const int P = 2 * p.N, PPi = P * P;
-	const long PP = (long)P * P;
-	Tile<C> T(sm, P, P);
-	const unsigned mgP = magic_div((unsigned)P);
-	const long cji = blockIdx.x;                  // (cell 4 + j) 4 + h
-	const long cell = cji / 16;
-	const int j3 = (int)((cji / 4) % 4), h = (int)(cji % 4);
-	load_tw(T.tw, P, p.pl);
-	C *X = p.X + ((cell * 4 + j3) * 4 + h) * PP;
-	const C *G = p.What + (cell * 4 + (RF ? 2 * h : h)) * PP;
-	for (int tt = 0; tt < p.nt; tt++) {
-		const long ct = cell * p.nt + tt;
-		const int t = p.un.term(p.t0 + tt);
-		const bool keep = p.un.pair(p.t0 + tt);
-		const R sc = (R)p.scale[t];
-		const R *ps = p.psi2T + (long)p.idx[t] * PP;
-		const C *Pj = p.Pg + (ct * 4 + (RF ? j3 / 2 : j3)) * PP;
-		C *yk = p.Y + (ct * 16 + (RF ? 2 * j3 : 4 * j3) + h) * PP;
-		{
-			batched<Two<C>>(PPi, [&](int i) {
-				Two<C> v;
-				v.a = RF ? mk<C>(G[i].x, G[i + PP].x) : G[i];
-				v.b = Pj[i];
-				return v;
-			}, [&](int i, const Two<C> &v) {
-				const int l = fdiv(i, mgP), k = i - l * P;
-				T.a[T.at(l, k)] = RF ? cscale(v.a, (j3 & 1) ? v.b.y : v.b.x) : cmul(v.a, v.b);
-			});
-			__syncthreads();
-			C *r = fft_lines<+1>(T.a, T.b, P, T.pitch, 1, p.pl, T.tw);               // rows
-			r = fft_lines<+1>(r, r == T.a ? T.b : T.a, P, 1, T.pitch, p.pl, T.tw);     // columns
-			batched<R>(PPi, [&](int i) { return ps[i]; }, [&](int i, const R &f0) {
-				const int k = fdiv(i, mgP), l = i - k * P;                   // transposed table: element (l, k)
-				const R f = sc * f0;
-				C x = r[T.at(l, k)];
-				x.x *= f;
-				x.y *= f;
-				r[T.at(l, k)] = x;
-			});
-			__syncthreads();
-			r = fft_lines<-1>(r, r == T.a ? T.b : T.a, P, 1, T.pitch, p.pl, T.tw);     // columns
-			r = fft_lines<-1>(r, r == T.a ? T.b : T.a, P, T.pitch, 1, p.pl, T.tw);     // rows
-			const C *Pa = p.Pg + (ct * 4 + h) * PP;
-			const R eta = h == 0 ? (R)1 : (R)-1;
-			batched<Two<C>>(PPi, [&](int i) {
-				Two<C> v;
-				v.a = Pa[i];
-				v.b = X[i];
-				return v;
-			}, [&](int i, const Two<C> &v) {
-				const int l = fdiv(i, mgP), k = i - l * P;
-				C x = v.b;
-				const C y0 = r[T.at(l, k)];
-				if (keep) yk[i] = y0;
-				if (RF) {                                  // eta_2h P_2h Re + eta_2h+1 P_2h+1 Im (eta_2h+1 = -1)
-					x.x += eta * (v.a.x * y0.x) - v.a.y * y0.y;
-				} else {
-					const C y = cmul(v.a, y0);
-					x.x += eta * y.x;
-					x.y += eta * y.y;
-				}
-				X[i] = x;
-			});
-			__syncthreads();
-		}
-	}
-}
-template <class C> __global__ void __launch_bounds__(kThreads) k_any_i3_fused(const I3FusedP<C> p) {
-	extern __shared__ __align__(16) unsigned char sm[];
-	const long cell = blockIdx.x / 16;
-	if constexpr (has_rf<C>()) {
-		if (p.kind != nullptr && p.kind[cell] == 0) {
-			if (blockIdx.x % 4 < 2) i3_fused<C, true>(p, sm);
-			return;
-		}
-	}
-	i3_fused<C, false>(p, sm);
-}
-
 // assembly rows: Zcc_j and Zcd_j (the combinations of k_assemble) for unit
 // (cell, j), inverse row transforms into Z[(cell 4 + j) 2 + {0, 1}]
 template <class C> struct AsmP {
@@ -1576,20 +1385,106 @@ template <class C> struct AnyRhs {
 		}
 	}
 
-	// whole-grid chains (k_any_i3_fused, where a grid fits a CTA) or the three
-	// passes.  The workspace's knob (0 off, 1 on), else QB_ANYN_FUSED (read per
-	// call), else the three passes: measured faster in FP32 at N = 24 (0.216
-	// against 0.316 ms per cell-evaluation) and N = 48 (0.710 against 0.807)
-	// once the passes read and store from their FFT stages, and faster still
-	// with their plans compiled in
-	bool fused_i3() const {
+	// whole-grid chains (k_i3g, N = 24 and 48) or the three passes.  The
+	// workspace's knob (0 off, 1 on), else QB_ANYN_FUSED (read per call), else the
+	// whole-grid chains: Strang steps, J = M = 16, passes against whole grid: 12
+	// cells at N = 24 3.7 / 2.1 ms (FP32), 7.3 / 3.4 ms (FP64), at N = 48 11.7 / 7.2 ms
+	// (FP32, complex form), 40 cells in FP64 92.7 / 48.7 ms.  Caller-built tables
+	// take the passes
+	bool fused_i3(const DevI3 &t) const {
 		int on = ws.anyn_fused;
 		if (on < 0) {
 			const char *e = getenv("QB_ANYN_FUSED");
 			if (e != nullptr && (strcmp(e, "0") == 0 || strcmp(e, "1") == 0)) on = e[0] - '0';
 		}
-		if (on < 0) on = 0;
-		return on == 1 && tile_bytes<C>(P, P) <= kMaxSmem;
+		return on != 0 && (N == 24 || N == 48) && t.pairM > 0;
+	}
+
+	// the whole-grid chains of every cell; returns the partials of X per (cell, j)
+	template <int RR> int i3_grid(const DevI3 &t, const double2 *W, AsmP<C> &as, const int *kind) {
+		using F = Grid16<RR, C>;
+		constexpr bool f32 = sizeof(C) == 8;
+		I3GridP<C> p{};
+		p.un.M = t.pairM;
+		p.ncells = ncells;
+		p.nunits = p.un.count(t.nterms);
+		const int res = grid_clusters(k_i3g<RR, C, f32>, F::NT, I3Grid<RR, C, f32>::SMEM);
+		// chunks a cell: as even a split of the pieces over the resident clusters as
+		// the partials (X, Z written once, read by the assembly) are worth
+		double best = 1e300;
+		for (int c = 1; c <= std::min(p.nunits, 64); c++) {
+			const double cost = (double)(((long)ncells * c + res - 1) / res) * ((p.nunits + c - 1) / c) + 0.15 * c;
+			if (cost < best) { best = cost; p.nchunk = c; }
+		}
+		const int ncl = (int)std::min<long>((long)ncells * p.nchunk, res);
+		const int nang = t.nterms / t.pairM;
+		const long nw = 4L * ncells * PP;
+		ws.i3p.ensure(sizeof(C) * ncells * 4 * p.nchunk * PP);
+		ws.i3z.ensure(sizeof(C) * 4 * ncells * 4 * p.nchunk * (N + 1) * (N + 1));
+		ws.wave1.ensure(sizeof(C) * ncl * 8 * PP);
+		ws.wave2.ensure(sizeof(C) * (nw + ncl * 4 * PP) + sizeof(float) * nw + sizeof(R) * nang * PP);
+		C *wi = ws.wave2.as<C>();
+		p.xscr = wi + nw;
+		R *psi = reinterpret_cast<R *>(p.xscr + ncl * 4 * PP);
+		float *wr = reinterpret_cast<float *>(psi + nang * PP);
+		p.kind = kind; p.src = W; p.WI = wi; p.WR = reinterpret_cast<const R *>(wr);
+		p.psi1 = Tabs<C>::i3_psi1(t); p.psi2 = psi; p.scale = t.scale.as<double>();
+		p.pscr = ws.wave1.as<C>(); p.X = ws.i3p.as<C>(); p.Z = ws.i3z.as<C>();
+		{
+			ProfScope ps("any_items", s);
+			const unsigned nb = (unsigned)((PP + 255) / 256);
+			for (long g0 = 0; g0 < 4L * ncells; g0 += 32768)
+				k_to_items<RR, C><<<dim3(nb, (unsigned)std::min(32768L, 4L * ncells - g0)), 256, 0, s>>>(ws.What.as<C>() + g0 * PP, wi + g0 * PP,
+				                                                                                          kind ? wr + g0 * PP : nullptr);
+			k_psi2_items<RR, C><<<dim3(nb, (unsigned)nang), 256, 0, s>>>(Tabs<C>::i3_psi2T(t), psi);
+			QB_CUDA(cudaGetLastError());
+		}
+		p.form = 1;
+		if constexpr (f32) {
+			if (kind != nullptr) {
+				I3GridP<C> r = p;
+				r.form = 0;
+				grid_launch(k_i3g<RR, C, true>, F::NT, I3Grid<RR, C, true>::SMEM, ncl, r);
+			}
+		}
+		grid_clusters(k_i3g<RR, C, false>, F::NT, I3Grid<RR, C, false>::SMEM);
+		grid_launch(k_i3g<RR, C, false>, F::NT, I3Grid<RR, C, false>::SMEM, ncl, p);
+		as.Zp = p.Z; as.nzp = 4 * p.nchunk; as.kind = kind;
+		return p.nchunk;
+	}
+	// clusters of 4 CTAs of a k_i3g resident on the GPU (its shared-memory attribute set)
+	template <class K> static int grid_clusters(K kern, int nt, size_t smem) {
+		static std::mutex mu;
+		static std::map<std::pair<int, const void *>, int> known;
+		int dev = 0;
+		QB_CUDA(cudaGetDevice(&dev));
+		std::lock_guard<std::mutex> lk(mu);
+		auto it = known.find({ dev, (const void *)kern });
+		if (it != known.end()) return it->second;
+		QB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		cudaLaunchConfig_t cfg = {};
+		cudaLaunchAttribute attr;
+		grid_config(cfg, attr, nt, smem, 1);
+		int n = 0;
+		QB_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+		return known[{ dev, (const void *)kern }] = std::max(1, n);
+	}
+	static void grid_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, int nt, size_t smem, int ncl) {
+		cfg.gridDim = dim3((unsigned)(4 * ncl));
+		cfg.blockDim = dim3((unsigned)nt);
+		cfg.dynamicSmemBytes = smem;
+		attr.id = cudaLaunchAttributeClusterDimension;
+		attr.val.clusterDim.x = 4; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+		cfg.attrs = &attr;
+		cfg.numAttrs = 1;
+	}
+	template <class K> void grid_launch(K kern, int nt, size_t smem, int ncl, const I3GridP<C> &p) {
+		cudaLaunchConfig_t cfg = {};
+		cudaLaunchAttribute attr;
+		grid_config(cfg, attr, nt, smem, ncl);
+		cfg.stream = s;
+		ProfScope ps("any_i3_grid", s);
+		QB_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
 	}
 
 	// partial sums of X and Z a (cell, component): the last row pass and the Z
@@ -1608,13 +1503,14 @@ template <class C> struct AnyRhs {
 	// launches (the kernels read a cell's kind; the real form leaves half of
 	// its units idle)
 	int i3_sums(const DevI3 &t, const double2 *W, AsmP<C> &as) {
-		const int nxp = fused_i3() ? 4 : partials();
-		ws.i3p.ensure(sizeof(C) * ncells * 4 * nxp * PP);
-		QB_CUDA(cudaMemsetAsync(ws.i3p.p, 0, sizeof(C) * ncells * 4 * nxp * PP, s));
 		const int *kind = nullptr;
 		if constexpr (sizeof(typename CT<C>::R) == 4) {
 			if (real_form_enabled()) kind = i3_form_kinds(ws, ncells, W, s);
 		}
+		if (fused_i3(t)) return N == 24 ? i3_grid<3>(t, W, as, kind) : i3_grid<6>(t, W, as, kind);
+		const int nxp = partials();
+		ws.i3p.ensure(sizeof(C) * ncells * 4 * nxp * PP);
+		QB_CUDA(cudaMemsetAsync(ws.i3p.p, 0, sizeof(C) * ncells * 4 * nxp * PP, s));
 		if (t.pairM > 0) {
 			as.nzp = partials();
 			ws.i3z.ensure(sizeof(C) * 4 * as.nzp * ncells * (N + 1) * (N + 1));
@@ -1647,15 +1543,15 @@ template <class C> struct AnyRhs {
 	// form) and 16 chains (8 in the real form).  A cell's terms still run in
 	// order, so the sums do not depend on the waves.
 	void i3_waves(const DevI3 &t, const double2 *W, int nxp, const int *kind) {
-		const bool fused = fused_i3(), pairs = t.pairM > 0;
+		const bool pairs = t.pairM > 0;
 		const WaveUnits un{ t.pairM };
 		const int nunits = pairs ? t.nterms / t.pairM * ((t.pairM + 1) / 2) : t.nterms;
-		const int per_term = fused && !pairs ? 4 : 20;
+		const int per_term = 20;
 		const int cpw = wave_cells(per_term);
 		const int nt = wave(nunits, per_term, cpw);
 		ws.wave1.ensure(sizeof(C) * (size_t)cpw * nt * 4 * PP);                // P_j, then the rows of Y_i
-		if (per_term == 20) ws.wave2.ensure(sizeof(C) * (size_t)cpw * nt * 16 * PP);   // chains
-		C *Pg = ws.wave1.as<C>(), *Y = per_term == 20 ? ws.wave2.as<C>() : nullptr;
+		ws.wave2.ensure(sizeof(C) * (size_t)cpw * nt * 16 * PP);   // chains
+		C *Pg = ws.wave1.as<C>(), *Y = ws.wave2.as<C>();
 		int nl4 = nl1;                                      // one tile, at most kOwn elements a thread
 		const int own = own_for_plan(pl, sizeof(C) == 16);
 		while (nl4 > 1 && (nl4 * P > own * kThreads || P % nl4)) nl4--;
@@ -1674,18 +1570,6 @@ template <class C> struct AnyRhs {
 				p.psiC = Tabs<C>::i3_psi1(t); p.un = un;
 				pad_rows(p, nc);
 				plain(Pg, (long)nc * n * 4, -1, true, kc, (long)n * 4, 4, 2, true);
-				if (fused) {
-					I3FusedP<C> f{};
-					f.What = What; f.Pg = Pg; f.X = X;
-					f.psi2T = Tabs<C>::i3_psi2T(t); f.idx = t.idx.as<int>(); f.scale = t.scale.as<double>();
-					f.N = N; f.nt = n; f.t0 = t0; f.kind = kc; f.un = un; f.Y = Y;
-					// FP32 default: radix-8 stages (the radix-16 register DFTs push this
-					// kernel to 173 registers, one CTA an SM); FP64 runs one CTA an SM anyway
-					f.pl = (ws.anyn_plan == 0 && sizeof(C) == 8) ? with_tw(make_plan(P, 1)) : pl;
-					launch(k_any_i3_fused<C>, "any_i3_fused", (long)nc * 16, tile_bytes<C>(P, P), s, f);
-					if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * partials() * (N + 1) * (N + 1), nc, n, t0, kc);
-					continue;
-				}
 				I3RowsAP<C> a{};
 				a.What = What; a.Pg = Pg; a.Y = Y; a.N = N; a.nl = nl1; a.nt = n; a.kind = kc; a.pl = pl;
 				by_plan([&](auto kern) { launch(kern, "any_i3_rows_a", blocks((long)nc * n * 16, nl1), smem(nl1, 1), s, a); },
