@@ -1421,7 +1421,7 @@ template <class C> struct AnyRhs {
 		const long nw = 4L * ncells * PP;
 		ws.i3p.ensure(sizeof(C) * ncells * 4 * p.nchunk * PP);
 		ws.i3z.ensure(sizeof(C) * 4 * ncells * 4 * p.nchunk * (N + 1) * (N + 1));
-		ws.wave1.ensure(sizeof(C) * ncl * 8 * PP);
+		ws.wave1.ensure(sizeof(C) * ncl * 8 * PP * (kind ? 2 : 1));
 		ws.wave2.ensure(sizeof(C) * (nw + ncl * 4 * PP) + sizeof(float) * nw + sizeof(R) * nang * PP);
 		C *wi = ws.wave2.as<C>();
 		p.xscr = wi + nw;
@@ -1444,11 +1444,13 @@ template <class C> struct AnyRhs {
 			if (kind != nullptr) {
 				I3GridP<C> r = p;
 				r.form = 0;
-				grid_launch(k_i3g<RR, C, true>, F::NT, I3Grid<RR, C, true>::SMEM, ncl, r);
+				r.pscr += ncl * 8 * PP;              // a cluster takes pieces of any cell: scratch of its own
+				grid_launch(k_i3g<RR, C, true>, F::NT, I3Grid<RR, C, true>::SMEM, ncl, r, ws.fork(s, 1));
 			}
 		}
 		grid_clusters(k_i3g<RR, C, false>, F::NT, I3Grid<RR, C, false>::SMEM);
-		grid_launch(k_i3g<RR, C, false>, F::NT, I3Grid<RR, C, false>::SMEM, ncl, p);
+		grid_launch(k_i3g<RR, C, false>, F::NT, I3Grid<RR, C, false>::SMEM, ncl, p, s);
+		if (kind != nullptr) ws.join(s, 1);          // the two forms run side by side: either may have few cells
 		as.Zp = p.Z; as.nzp = 4 * p.nchunk; as.kind = kind;
 		return p.nchunk;
 	}
@@ -1478,12 +1480,12 @@ template <class C> struct AnyRhs {
 		cfg.attrs = &attr;
 		cfg.numAttrs = 1;
 	}
-	template <class K> void grid_launch(K kern, int nt, size_t smem, int ncl, const I3GridP<C> &p) {
+	template <class K> void grid_launch(K kern, int nt, size_t smem, int ncl, const I3GridP<C> &p, cudaStream_t st) {
 		cudaLaunchConfig_t cfg = {};
 		cudaLaunchAttribute attr;
 		grid_config(cfg, attr, nt, smem, ncl);
-		cfg.stream = s;
-		ProfScope ps("any_i3_grid", s);
+		cfg.stream = st;
+		ProfScope ps("any_i3_grid", st);
 		QB_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
 	}
 

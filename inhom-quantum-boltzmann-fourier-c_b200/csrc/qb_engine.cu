@@ -180,25 +180,27 @@ Workspace::~Workspace() {
 	if (ev_out) cudaEventDestroy(ev_out);
 	if (ev_t) cudaEventDestroy(ev_t);
 	if (ev_i) cudaEventDestroy(ev_i);
-	if (ev_fork) cudaEventDestroy(ev_fork);
-	if (ev_join) cudaEventDestroy(ev_join);
-	if (side) cudaStreamDestroy(side);
+	for (int i = 0; i < 2; i++) {
+		if (ev_fork[i]) cudaEventDestroy(ev_fork[i]);
+		if (ev_join[i]) cudaEventDestroy(ev_join[i]);
+		if (side[i]) cudaStreamDestroy(side[i]);
+	}
 	if (stream) cudaStreamDestroy(stream);
 }
 
-cudaStream_t Workspace::fork(cudaStream_t s) {
-	if (side == nullptr) {
-		QB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-		QB_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-		QB_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+cudaStream_t Workspace::fork(cudaStream_t s, int which) {
+	if (side[which] == nullptr) {
+		QB_CUDA(cudaStreamCreateWithFlags(&side[which], cudaStreamNonBlocking));
+		QB_CUDA(cudaEventCreateWithFlags(&ev_fork[which], cudaEventDisableTiming));
+		QB_CUDA(cudaEventCreateWithFlags(&ev_join[which], cudaEventDisableTiming));
 	}
-	QB_CUDA(cudaEventRecord(ev_fork, s));
-	QB_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
-	return side;
+	QB_CUDA(cudaEventRecord(ev_fork[which], s));
+	QB_CUDA(cudaStreamWaitEvent(side[which], ev_fork[which], 0));
+	return side[which];
 }
-void Workspace::join(cudaStream_t s) {
-	QB_CUDA(cudaEventRecord(ev_join, side));
-	QB_CUDA(cudaStreamWaitEvent(s, ev_join, 0));
+void Workspace::join(cudaStream_t s, int which) {
+	QB_CUDA(cudaEventRecord(ev_join[which], side[which]));
+	QB_CUDA(cudaStreamWaitEvent(s, ev_join[which], 0));
 }
 
 // ---------------------------------------------------------------------------
@@ -687,10 +689,13 @@ template <int P, class C> struct Rhs {
 					p.zscr = ws.i3zs.as<C>();
 					launch_nyquist_kind(P / 2, ncells, W, kRealFormBound, ws.i3kind.as<int>(), ws.i3stats.as<unsigned long long>(), s);
 					kind = ws.i3kind.as<int>();
-					launch_i3wr(p, ncl, reinterpret_cast<const float *>(ws.WhatQ.as<C>() + 4 * ncells * PP), ws.i3y.as<float>(), kind, s);
+					// the two forms side by side: either may have too few cells to fill the GPU
+					launch_i3wr(p, ncl, reinterpret_cast<const float *>(ws.WhatQ.as<C>() + 4 * ncells * PP), ws.i3y.as<float>(), kind, ws.fork(s, 1));
 				}
 			}
-			launch_i3w<C>(p, ncl, ws.i3y.as<C>(), kind, s);      // FP32: the cells above the bound
+			// FP32: the cells above the bound (each cluster's scratch is used by one form only)
+			launch_i3w<C>(p, ncl, ws.i3y.as<C>(), kind, s);
+			if (kind != nullptr) ws.join(s, 1);
 		} else {
 			if constexpr (P == 32 && sizeof(C) == 8) {
 				if (ws.i3_variant == 1) {
@@ -751,7 +756,7 @@ template <int P, class C> struct Rhs {
 		reserve(ws, q, ncells, ch, parts);
 		spectra(ws, ncells, W, s);
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
-		const cudaStream_t s2 = small ? ws.fork(s) : s;
+		const cudaStream_t s2 = small ? ws.fork(s, 0) : s;
 		if (small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s2);
 		if (parts & RHS_CD) {
@@ -759,7 +764,7 @@ template <int P, class C> struct Rhs {
 			i2_sums(ws, *q.i2, ncells, W, ch.i2, s2);
 			if (!small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		}
-		if (small) ws.join(s);
+		if (small) ws.join(s, 0);
 	}
 
 	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells, cudaStream_t s) {
@@ -1159,8 +1164,11 @@ template <class C> struct Rhs<128, C> {
 					p.zscr = ws.i3zs.as<C>();
 					int *kind = ws.i3kind.as<int>();
 					launch_nyquist_kind(N, ncells, W, kRealFormBound, kind, ws.i3stats.as<unsigned long long>(), s);
-					launch_i3_full128r(p, ncl, reinterpret_cast<float *>(ws.scr128a.as<C>()), kind, s);
+					// the two forms side by side: either may have too few cells to fill the GPU
+					// (each cluster's scratch is used by one form only)
+					launch_i3_full128r(p, ncl, ws.scr128a.as<float>(), kind, ws.fork(s, 1));
 					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), ws.i3y.as<C>(), kind, s);     // cells above the bound
+					ws.join(s, 1);
 				} else {
 					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), ws.i3y.as<C>(), nullptr, s);
 				}
@@ -1226,7 +1234,7 @@ template <class C> struct Rhs<128, C> {
 		spectra(ws, ncells, W, s);
 		const int act = sizeof(C) == 16 ? active_quad_clusters() : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(*q.i3) < kForkUnits * act;
-		const cudaStream_t s2 = small ? ws.fork(s) : s;
+		const cudaStream_t s2 = small ? ws.fork(s, 0) : s;
 		if (small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s2);
 		if (parts & RHS_CD) {
@@ -1234,7 +1242,7 @@ template <class C> struct Rhs<128, C> {
 			i2_sums(ws, *q.i2, ncells, W, ch.i2, s2);
 			if (!small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		}
-		if (small) ws.join(s);
+		if (small) ws.join(s, 0);
 	}
 
 	static AsmParamsT<C> asm_params(Workspace &ws, int parts, const Chunks &ch, const QuadSet &q, int ncells, cudaStream_t s) {

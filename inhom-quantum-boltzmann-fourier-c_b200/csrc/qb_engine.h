@@ -140,12 +140,13 @@ struct Workspace {
 	// which collide on the caller's stream while the interior collides on `stream`
 	std::unique_ptr<Workspace> edge;
 	cudaEvent_t ev_t = nullptr, ev_i = nullptr;
-	// second stream of one evaluation: the I1, I2 and I4 sums of a small batch
-	// beside its I3 sums, between fork (after the caller's work so far) and join
-	cudaStream_t side = nullptr;
-	cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-	cudaStream_t fork(cudaStream_t s);
-	void join(cudaStream_t s);
+	// side streams of one evaluation, between fork (after the caller's work so far)
+	// and join: the I1, I2 and I4 sums of a small batch beside its I3 sums (0), the
+	// real form of the I3 sums beside the complex one (1)
+	cudaStream_t side[2] = { nullptr, nullptr };
+	cudaEvent_t ev_fork[2] = { nullptr, nullptr }, ev_join[2] = { nullptr, nullptr };
+	cudaStream_t fork(cudaStream_t s, int which);
+	void join(cudaStream_t s, int which);
 	explicit Workspace(int N);
 	~Workspace();
 };

@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 // kernel, so the error this form adds stays at the FP32 rounding of the
 // precision form.
 //
-// pscr: [cluster][4][P*P] real, natural order; out as k_i3_full128 (real
+// pscr: [cluster][8][P*P] reals, the first four used, natural order; out as k_i3_full128 (real
 // parts; imaginary parts written as zero).
 struct F128TmemR {
 	// 2 outputs x 4 row iterations x 8 real accumulators, then 4 x 8 complex values of Y
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128r(const I3ParamsT<flo
 			for (int it = 0; it < 4; it++) tmem_st8r(TM::addr(tbase, q, it), z);
 	}
 	tmem_wait_st();
-	float *Pall = pscr + cid * 4 * PP;
+	float *Pall = pscr + cid * 8 * PP;                     // where the complex form has this cluster's grids
 	const C *Gcell = p.Ghat + cell * p.g_cell;
 	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
 	// packed sums A_c = Z_2c + i Z_2c+1 on the frequencies -N/2 .. N/2 (both ends:

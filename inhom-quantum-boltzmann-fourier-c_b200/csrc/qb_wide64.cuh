@@ -398,7 +398,8 @@ __global__ void __launch_bounds__(512, Occ<C>::CTAS) k_i3w(const I3ParamsT<C> p,
 // i Y_2c+1 is packed the same way: two chains a unit and group.  A_c = Z_2c + i
 // Z_2c+1 is summed on the frequencies -N/2 .. N/2 of both dimensions (the
 // partner of -N/2 separates the two) in zscr and separated at the end.  WhR: the
-// real parts of W^ in thread order; pscr: [cluster][2][4][PP] reals.
+// real parts of W^ in thread order; pscr: [cluster][4][4][PP]
+// reals, the first half used.
 __global__ void __launch_bounds__(512, 2) k_i3wr(const I3ParamsT<float2> p, const float *__restrict__ WhR, float *pscr, const int *kind) {
 	using C = float2;
 	using TM = WideTmem<1>;
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(512, 2) k_i3wr(const I3ParamsT<float2> p, cons
 	const int kc = F.col_c(), ks = kc < N / 2 ? kc : (kc >= 3 * N / 2 ? kc - N : -1);
 	const int zk = kc <= H ? kc : kc - P;                    // this thread's column of C as a frequency
 	const int oz = F.row_c() * N + ks;
-	float *Pall = pscr + (long)cid * 8 * PP + t;
+	float *Pall = pscr + (long)cid * 16 * PP + t;          // where the complex form has this cluster's grids
 	Yb += t;
 	const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[j] * NN + oz;
 	const float *Wc = WhR + cell * 4 * PP + t;
