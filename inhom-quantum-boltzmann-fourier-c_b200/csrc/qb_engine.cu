@@ -3,7 +3,7 @@
 #include "qb_kernels.cuh"
 #include "qb_split128.cuh"
 #include "qb_full128.cuh"
-#include "qb_wide64.cuh"
+#include "qb_wide128.cuh"
 #include "qb_quad128.cuh"
 #include "qb_transport.cuh"
 
@@ -340,7 +340,7 @@ template <int P, int CS, class C> void launch_i3(const I3ParamsT<C> &p, long ncl
 // 2-CTA clusters, a whole grid per CTA, all 512 tensor-memory columns per CTA,
 // so exactly one CTA per SM, checked).  By default the cells whose Nyquist
 // content is at most kRealFormBound take the real forms (k_i3wr,
-// k_i3_full128r) and the others the complex kernels.  QB_I3_KERNEL selects one
+// k_i3_wide128r) and the others the complex kernels.  QB_I3_KERNEL selects one
 // kernel for every cell instead (for comparisons): "complex" the complex
 // kernels, "pair" the complex k_i3w and the pair-split k_i3_128.
 inline const char *i3_kernel_env() {
@@ -961,19 +961,29 @@ void launch_i3_full128(const I3ParamsT<float2> &p, long nclusters, float2 *pscr,
 	launch128(k_i3_full128<float2>, "i3_cluster", nclusters * 2, 2, kFull128Smem, s, p, pscr, yscr, kind);
 }
 
-// the real form: same shared memory and tensor-memory columns
-void launch_i3_full128r(const I3ParamsT<float2> &p, long nclusters, float *pscr, const int *kind, cudaStream_t s) {
+// the real form: the same cluster shape and tensor-memory columns
+void launch_i3_wide128r(const I3ParamsT<float2> &p, long nclusters, const float *WhR, const float *psi2, float *pscr, const int *kind, cudaStream_t s) {
 	static DeviceFlag init;
 	if (!init) {
 		check_tmem_coresidency();
-		set_smem(k_i3_full128r, kFull128Smem);
+		set_smem(k_i3_wide128r, kWide128Smem);
 		int per_sm = 0;
-		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_i3_full128r, F128::NT, kFull128Smem));
+		QB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_i3_wide128r, Wide128::NT, kWide128Smem));
 		if (per_sm * (int)F128TmemR::NCOLS > 512)
-			QB_FAIL("k_i3_full128r: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
+			QB_FAIL("k_i3_wide128r: " + std::to_string(per_sm) + " CTAs per SM would oversubscribe tensor memory");
 		init = true;
 	}
-	launch128(k_i3_full128r, "i3_cluster", nclusters * 2, 2, kFull128Smem, s, p, pscr, kind);
+	launch128(k_i3_wide128r, "i3_cluster", nclusters * 2, 2, kWide128Smem, s, p, WhR, psi2, pscr, kind);
+}
+// its operands: the real parts of the spectra and the psi2 tables in vector order
+void launch_wide128_order(const float2 *What, float *WhR, int ngrids, const float *psi2T, float *psi2, int ntab, cudaStream_t s) {
+	ProfScope ps("wide128_order", s);
+	const unsigned nb = Wide128::PP / 256;
+	for (int g = 0; g < ngrids; g += 32768)
+		k_w128_real<<<dim3(nb, (unsigned)std::min(32768, ngrids - g)), 256, 0, s>>>(What + (long)g * Wide128::PP, WhR + (long)g * Wide128::PP);
+	for (int g = 0; g < ntab; g += 32768)
+		k_psi128_real<<<dim3(nb, (unsigned)std::min(32768, ntab - g)), 256, 0, s>>>(psi2T + (long)g * Wide128::PP, psi2 + (long)g * Wide128::PP);
+	QB_CUDA(cudaGetLastError());
 }
 
 
@@ -1007,7 +1017,7 @@ void check_tmem_coresidency() {
 		{ (const void *)k_i3_128<2, 1, double2>, smem_i3_128<double2>(), G128::NT, (int)I3Tmem128<double2, 2>::NCOLS,
 		  "k_i3_128<f64, single integral>" },
 		{ (const void *)k_i3_full128<float2>, kFull128Smem, F128::NT, (int)F128Tmem::NCOLS, "k_i3_full128" },
-		{ (const void *)k_i3_full128r, kFull128Smem, F128::NT, (int)F128TmemR::NCOLS, "k_i3_full128r" },
+		{ (const void *)k_i3_wide128r, kWide128Smem, Wide128::NT, (int)F128TmemR::NCOLS, "k_i3_wide128r" },
 	};
 	for (const TmemKernel &k : dftmma_tmem_kernels()) ks.push_back(k);
 	for (const TmemKernel &k : fno_tmem_kernels()) ks.push_back(k);
@@ -1119,6 +1129,12 @@ template <class C> struct Rhs<128, C> {
 	// pair-split FP32 kernel; the whole-grid FP32 kernels leave one partial of the
 	// Z sums per CTA of their 2-CTA clusters
 	static constexpr int kZRanks = sizeof(C) == 8 ? 2 : 1;
+	// psi2 tables of a term list: one an angle, or one a term of caller-built tables
+	static int psi_tables(const DevI3 &t) { return t.pairM > 0 ? t.nterms / t.pairM : t.nterms; }
+	// W^ in quad order (FP64), or its real parts and the psi2 tables in vector order
+	static size_t wide_bytes(const DevI3 &t, int ncells) {
+		return sizeof(C) == 16 ? sizeof(C) * 4 * ncells * PP : sizeof(float) * ((size_t)4 * ncells + psi_tables(t)) * PP;
+	}
 	static bool pairs_units() { return sizeof(C) == 16 || use_full128(); }
 	static int i3_count(const DevI3 &t) {
 		I3Units u;
@@ -1161,12 +1177,16 @@ template <class C> struct Rhs<128, C> {
 				if (use_real_form() ) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
 					ws.i3zs.ensure(sizeof(C) * ncl * 2 * 2 * (N + 1) * (N + 1));
+					ws.WhatQ.ensure(wide_bytes(t, ncells));
 					p.zscr = ws.i3zs.as<C>();
 					int *kind = ws.i3kind.as<int>();
 					launch_nyquist_kind(N, ncells, W, kRealFormBound, kind, ws.i3stats.as<unsigned long long>(), s);
 					// the two forms side by side: either may have too few cells to fill the GPU
 					// (each cluster's scratch is used by one form only)
-					launch_i3_full128r(p, ncl, ws.scr128a.as<float>(), kind, ws.fork(s, 1));
+					float *whr = ws.WhatQ.as<float>(), *psi = whr + 4 * ncells * PP;
+					const cudaStream_t s2 = ws.fork(s, 1);
+					launch_wide128_order(ws.What.as<C>(), whr, 4 * ncells, T::i3_psi2T(t), psi, psi_tables(t), s2);
+					launch_i3_wide128r(p, ncl, whr, psi, ws.scr128a.as<float>(), kind, s2);
 					launch_i3_full128(p, ncl, ws.scr128a.as<C>(), ws.i3y.as<C>(), kind, s);     // cells above the bound
 					ws.join(s, 1);
 				} else {
@@ -1177,7 +1197,7 @@ template <class C> struct Rhs<128, C> {
 		}
 		if constexpr (sizeof(C) == 16) {
 			ws.i3y.ensure(sizeof(C) * ncl * 4 * PP);
-			ws.WhatQ.ensure(sizeof(C) * 4 * ncells * PP);
+			ws.WhatQ.ensure(wide_bytes(t, ncells));
 			for (int c0 = 0; c0 < 4 * ncells; c0 += 32768)
 				launch_b_to_quad(ws.What.as<C>() + c0 * PP, ws.WhatQ.as<C>() + c0 * PP, std::min(32768, 4 * ncells - c0), s);
 			launch_i3_quad(p, ws.WhatQ.as<C>(), ws.scr128a.as<C>(), ws.i3y.as<C>(), s);
@@ -1203,7 +1223,7 @@ template <class C> struct Rhs<128, C> {
 			DevBufSet &b = ws.scratch;
 			const size_t g = sizeof(C) * (size_t)ncells * PP;
 			b.add(ws.What, 4 * g);
-			if (sizeof(C) == 16) b.add(ws.WhatQ, 4 * g);
+			if (q.i3 && (sizeof(C) == 16 || use_real_form())) b.add(ws.WhatQ, wide_bytes(*q.i3, ncells));
 			if (parts & RHS_CC) {
 				b.add(ws.i1cc, 3 * ch.i1 * g);
 				b.add(ws.fs, 3 * g);

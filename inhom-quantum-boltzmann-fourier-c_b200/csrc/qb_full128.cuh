@@ -159,7 +159,7 @@ struct F128Tmem {
 // [cluster][2][P*P]; out: [cell][chunk][4][P*P] B layout; zout:
 // [cell][chunk][rank][4][N*N].
 // kind: null (every cell) or the per-cell form of k_nyquist_kind; this kernel
-// then takes the cells of kind 1 (the real form k_i3_full128r takes kind 0).
+// then takes the cells of kind 1 (the real form k_i3_wide128r takes kind 0).
 template <class C>
 __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p, C *pscr, C *yscr, const int *kind) {
 	static_assert(sizeof(C) == 8, "the whole-grid form is FP32 only");
@@ -415,8 +415,7 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 // kernel, so the error this form adds stays at the FP32 rounding of the
 // precision form.
 //
-// pscr: [cluster][8][P*P] reals, the first four used, natural order; out as k_i3_full128 (real
-// parts; imaginary parts written as zero).
+// The kernel is k_i3_wide128r (qb_wide128.cuh).
 struct F128TmemR {
 	// 2 outputs x 4 row iterations x 8 real accumulators, then 4 x 8 complex values of Y
 	static constexpr unsigned PER_THREAD = 2 * 4 * 8;         // 64
@@ -431,263 +430,6 @@ struct F128TmemR {
 		return base + ((32u * (w & 3u)) << 16) + (w >> 2) * PER_THREAD + (unsigned)(q * 4 + it) * 8;
 	}
 };
-
-__global__ void __launch_bounds__(F128::NT, 1) k_i3_full128r(const I3ParamsT<float2> p, float *pscr, const int *kind) {
-	using C = float2;
-	using F = F128;
-	using TM = F128TmemR;
-	constexpr long PP = (long)F::P * F::P;
-	extern __shared__ __align__(16) unsigned char smem_raw[];
-	__shared__ unsigned tmem_slot;
-	C *S = reinterpret_cast<C *>(smem_raw), *tw128 = S + F::GRID, *tw64 = tw128 + 128;
-	cg::cluster_group cl = cg::this_cluster();
-	const int rank = (int)cl.block_rank();
-	const long cid = blockIdx.x / 2;
-	const int chunk = (int)(cid % p.nchunk);
-	const long cell = cid / p.nchunk;
-	if (kind[cell] != 0) return;                          // both CTAs of the cluster leave before any barrier
-	const int tid = threadIdx.x, warp = tid >> 5, tau = tid & 15, sub = tid >> 4;
-	if (warp == 0) tmem_alloc(&tmem_slot, TM::NCOLS);
-	init_tw128(tw128, tw64);
-	tmem_fence_before();
-	__syncthreads();
-	tmem_fence_after();
-	const unsigned tbase = tmem_slot;
-	C wp[8];
-	wp[0] = tw64[0];
-#pragma unroll
-	for (int q = 1; q < 8; q++) wp[q] = tw64[((tau & 7) * q) & 63];
-	{
-		const float z[8] = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
-#pragma unroll 1
-		for (int q = 0; q < 2; q++)
-#pragma unroll 1
-			for (int it = 0; it < 4; it++) tmem_st8r(TM::addr(tbase, q, it), z);
-	}
-	tmem_wait_st();
-	float *Pall = pscr + cid * 8 * PP;                     // where the complex form has this cluster's grids
-	const C *Gcell = p.Ghat + cell * p.g_cell;
-	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
-	// packed sums A_c = Z_2c + i Z_2c+1 on the frequencies -N/2 .. N/2 (both ends:
-	// separating the two real-grid parts needs the partner of -N/2)
-	constexpr int H = F::N / 2, ZA = (F::N + 1) * (F::N + 1);
-	const long slot = cell * p.nchunk + chunk;
-	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
-	for (int i = tid; i < 2 * ZA; i += F::NT) za[i] = czero<C>();
-	__syncthreads();
-#pragma unroll 1
-	for (int un = t0; un < t1; un++) {
-		const int t = p.un.term(un);
-		const bool pr = p.un.pair(un);
-		// spectra of components 2 rank (real part) and 2 rank + 1 (imaginary part)
-		{
-			const double2 *sa = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank] * F::N * F::N;
-			const double2 *sb = p.src + cell * p.src_cell + (long)p.src_comp[2 * rank + 1] * F::N * F::N;
-			const C *psi1 = p.psi1 + (long)t * F::N * F::N;
-#pragma unroll 1
-			for (int it = 0; it < 4; it += 3) {             // rows outside the zero band: 0..31, 96..127
-				const int row = it * 32 + sub, ls = F::src(row);
-				C x[8];
-#pragma unroll
-				for (int r = 0; r < 8; r++) {
-					const int ks = F::src(tau + 16 * r);
-					C v = czero<C>();
-					if (ks >= 0) {
-						const int idx = ks + F::N * ls;
-						const double2 a = sa[idx], b = sb[idx];
-						v = cmul(psi1[idx], mk<C>(a.x - b.y, a.y + b.x));
-					}
-					x[r] = v;
-				}
-				fft128_line<-1, true>(x, tau, S, row, tw128, wp);
-				const LineSlots ls_ = row_slots(row, tau);
-#pragma unroll
-				for (int e = 0; e < 8; e++) S[ls_.at_out(e)] = x[e];
-			}
-			__syncthreads();
-#pragma unroll 1
-			for (int it = 0; it < 4; it++) {
-				const int col = it * 32 + sub;
-				const LineSlots cs_ = col_slots(col, tau);
-				C x[8];
-#pragma unroll
-				for (int r = 0; r < 8; r++)
-					x[r] = (r >= 2 && r < 6) ? czero<C>() : S[cs_.at_in(r)];
-				fft128_line<-1, false>(x, tau, S, col, tw128, wp);
-#pragma unroll
-				for (int e = 0; e < 8; e++) S[cs_.at_out(e)] = x[e];
-			}
-			__syncthreads();
-			float *Pa = Pall + (long)(2 * rank) * PP, *Pb = Pa + PP;
-#pragma unroll 4
-			for (int i = tid; i < F::P * F::P; i += F::NT) {
-				const C v = S[F::at(i >> 7, i & 127)];
-				Pa[i] = v.x;
-				Pb[i] = v.y;
-			}
-		}
-		cl.sync();                                          // both CTAs' spectra of term t are in L2
-		const float *psi2 = p.psi2T + (long)p.psi2_idx[t] * PP;
-		const float sc = (float)p.psi2_scale[t];
-#pragma unroll 1
-		for (int c = 0; c < 2; c++) {                        // the combos i = 2c (real part) and 2c + 1 (imaginary part)
-			const C *G0 = Gcell + (long)(2 * c) * PP, *G1 = G0 + PP;
-			const float *P0 = Pall + (long)(2 * c) * PP, *P1 = P0 + PP;
-			const float c0 = c == 0 ? 1.f : -1.f;            // eta_2c; eta_2c+1 = -1
-#pragma unroll 1
-			for (int q = 0; q < 2; q++) {
-				const int j = 2 * rank + q;
-				const float *Pj = Pall + (long)j * PP;
-				const C *Wj = Gcell + (long)j * PP;
-				const float eta = j == 0 ? 1.f : -1.f;
-				// rows: inverse transform along k of (W^_2c + i W^_2c+1) . P_j
-#pragma unroll 1
-				for (int it = 0; it < 4; it++) {
-					const int row = it * 32 + sub;
-					const C *g0 = G0 + F::brow(row), *g1 = G1 + F::brow(row);
-					const float *pj = Pj + (long)row * F::P;
-					C x[8];
-#pragma unroll
-					for (int r = 0; r < 8; r++) {
-						const int n = tau + 16 * r;
-						const float pv = pj[n];
-						x[r] = mk<C>(pv * g0[n].x, pv * g1[n].x);
-					}
-					fft128_line<+1, true>(x, tau, S, row, tw128, wp);
-					const LineSlots ls_ = row_slots(row, tau);
-#pragma unroll
-					for (int e = 0; e < 8; e++) S[ls_.at_out(e)] = x[e];
-				}
-				__syncthreads();
-				// columns: inverse transform along l, psi2, forward transform
-#pragma unroll 1
-				for (int it = 0; it < 4; it++) {
-					const int col = it * 32 + sub;
-					const LineSlots cs_ = col_slots(col, tau);
-					C x[8];
-#pragma unroll
-					for (int r = 0; r < 8; r++) x[r] = S[cs_.at_in(r)];
-					fft128_line<+1, false>(x, tau, S, col, tw128, wp);
-					const float *ps = psi2 + (long)col * F::P;
-#pragma unroll
-					for (int e = 0; e < 8; e++) {
-						const float f = sc * ps[pos128(tau, e)];
-						x[e].x *= f;
-						x[e].y *= f;
-					}
-					fft128_dit<-1, false>(x, tau, S, col, tw128, wp);
-					const int d0 = (tau & 7) + 8 * (tau >> 3);
-#pragma unroll
-					for (int m = 0; m < 8; m++) S[(d0 + 16 * (m >> 1) + 64 * (m & 1)) * F::LDP + cs_.cx[m & 1]] = x[m];
-				}
-				__syncthreads();
-				// rows: forward transform along k; the real part is T of i = 2c, the
-				// imaginary part of 2c + 1.  Y_2c + i Y_2c+1 collects eta_j W^_j . T (W^_j
-				// real; the term of j = 2 rank waits in tensor memory) and its rows are
-				// transformed as they are complete
-#pragma unroll 1
-				for (int it = 0; it < 4; it++) {
-					const int row = it * 32 + sub;
-					const LineSlots ls_ = row_slots(row, tau);
-					C x[8];
-#pragma unroll
-					for (int r = 0; r < 8; r++) x[r] = S[ls_.at_in(r)];
-					fft128_line<-1, true>(x, tau, S, row, tw128, wp);
-					const float *p0 = P0 + (long)row * F::P, *p1 = P1 + (long)row * F::P;
-					float acc[8];
-					tmem_ld8r(TM::addr(tbase, q, it), acc);
-					tmem_wait_ld();
-#pragma unroll
-					for (int e = 0; e < 8; e++) {
-						const int n = pos128(tau, e);
-						acc[e] += c0 * (p0[n] * x[e].x) - p1[n] * x[e].y;
-					}
-					tmem_st8r(TM::addr(tbase, q, it), acc);
-					if (pr) {
-						const C *wj = Wj + F::brow(row);
-#pragma unroll
-						for (int e = 0; e < 8; e++) x[e] = cscale(x[e], eta * wj[pos128(tau, e)].x);
-						if (q == 0) {
-							tmem_st8(TM::yaddr(tbase, it), x);
-						} else {
-							C y[8];
-							tmem_ld8(TM::yaddr(tbase, it), y);
-							tmem_wait_ld();
-#pragma unroll
-							for (int e = 0; e < 8; e++) x[e] = cadd(y[e], x[e]);
-							y_row(x, tau, S, row, tw128, wp);
-						}
-					}
-					tmem_wait_st();
-				}
-				// no barrier: the next chain's first row pass writes only the
-				// rows this thread's 16-lane group has just read
-			}
-			if (!pr) continue;
-			// A_c += conj(psi1) . IFFT2(Y_2c + i Y_2c+1) on the frequencies -N/2 .. N/2
-			__syncthreads();
-			const C *ps = p.psi1 + (long)t * F::N * F::N;
-#pragma unroll 1
-			for (int it = 0; it < 4; it++) {                     // columns 0..31, 32 (one line of a warp), 96..127
-				if (it == 2 || (it == 1 && warp > 0)) continue;
-				const int col = it * 32 + sub;
-				const LineSlots cs_ = col_slots(col, tau);
-				C x[8];
-#pragma unroll
-				for (int r = 0; r < 8; r++) x[r] = S[cs_.at_in(r)];
-				fft128_line<+1, false>(x, tau, S, col, tw128, wp);
-				if (col == H + 1) continue;
-				const int zk = col <= H ? col : col - F::P;
-#pragma unroll
-				for (int e = 0; e < 8; e++) {
-					if (e > 2 && e < 6) continue;                // rows 48 .. 95
-					const int l = pos128(tau, e), zl = e < 3 ? l : l - F::P;
-					if (zl > H || (zl == H && zk == -H) || (zl == -H && zk == H)) continue;
-					// psi1 is tabulated on -N/2 .. N/2 - 1; at the upper end it is conj psi1(-k)
-					const bool up = zl == H || zk == H;
-					const int a = up ? -zl : zl, b = up ? -zk : zk;
-					C w = ps[(a < 0 ? a + F::N : a) * F::N + (b < 0 ? b + F::N : b)];
-					if (!up) w.y = -w.y;
-					C *z = za + c * ZA + (zl + H) * (F::N + 1) + zk + H;
-					*z = cfma(w, x[e], *z);
-				}
-			}
-			__syncthreads();                                     // the next chain's rows reuse S
-		}
-		cl.sync();                                          // the partner is done with this term's spectra
-	}
-	// A(k) = Z_2c(k) + i Z_2c+1(k) with both parts the transforms of real grids
-	{
-		constexpr int NN = F::N * F::N;
-		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
-		for (int i = tid; i < 2 * NN; i += F::NT) {
-			const int c = i / NN, n = i % NN;
-			int l = n / F::N, k = n % F::N;
-			l = l < H ? l : l - F::N;
-			k = k < H ? k : k - F::N;
-			const C u = za[c * ZA + (l + H) * (F::N + 1) + k + H], v = za[c * ZA + (H - l) * (F::N + 1) + H - k];
-			zo[(long)(2 * c) * NN + n] = mk<C>(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
-			zo[(long)(2 * c + 1) * NN + n] = mk<C>(0.5f * (u.y + v.y), -0.5f * (u.x - v.x));
-		}
-	}
-#pragma unroll 1
-	for (int q = 0; q < 2; q++) {
-		C *o = p.out + ((cell * p.nchunk + chunk) * 4 + 2 * rank + q) * PP;
-#pragma unroll 1
-		for (int it = 0; it < 4; it++) {
-			const int row = it * 32 + sub;
-			float acc[8];
-			tmem_ld8r(TM::addr(tbase, q, it), acc);
-			tmem_wait_ld();
-#pragma unroll
-			for (int e = 0; e < 8; e++) o[F::brow(row) + pos128(tau, e)] = mk<C>(acc[e], 0.0);
-		}
-	}
-	tmem_fence_before();
-	__syncthreads();
-	tmem_fence_after();
-	if (warp == 0) tmem_dealloc(tbase, TM::NCOLS);
-}
 
 // per cell: 0 (real form) when both
 //   - the Nyquist content of the Fourier state W ([cell][4][N*N], natural
