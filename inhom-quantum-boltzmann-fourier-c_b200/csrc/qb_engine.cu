@@ -4,6 +4,7 @@
 #include "qb_split128.cuh"
 #include "qb_full128.cuh"
 #include "qb_wide128.cuh"
+#include "qb_terms64.cuh"
 #include "qb_quad128.cuh"
 #include "qb_transport.cuh"
 
@@ -295,18 +296,37 @@ template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C 
 	QB_CUDA(cudaGetLastError());
 }
 
-template <int P, class C> void launch_i1(const I1ParamsT<C> &p, long nblocks, cudaStream_t s) {
+// wide: the kernels of qb_terms64.cuh at P = 64
+template <int P, class C> void launch_i1(const I1ParamsT<C> &p, long nblocks, cudaStream_t s, bool wide = false) {
+	ProfScope ps("i1_terms", s);
+	if constexpr (P == 64) {
+		if (wide) {
+			static DeviceFlag init;
+			if (!init) { check_tmem_coresidency(); set_smem(k_i1_terms64<C>, Terms64<C>::SMEM); init = true; }
+			k_i1_terms64<C><<<(unsigned)nblocks, Terms64<C>::NT, Terms64<C>::SMEM, s>>>(p);
+			QB_CUDA(cudaGetLastError());
+			return;
+		}
+	}
 	static DeviceFlag init;
 	if (!init) { set_smem(k_i1_terms<P, C>, smem_grids<P, C>(2)); init = true; }
-	ProfScope ps("i1_terms", s);
 	k_i1_terms<P, C><<<(unsigned)nblocks, Geo<P>::NT, smem_grids<P, C>(2), s>>>(p);
 	QB_CUDA(cudaGetLastError());
 }
 
-template <int P, class C> void launch_i2(const I2ParamsT<C> &p, long nblocks, cudaStream_t s) {
+template <int P, class C> void launch_i2(const I2ParamsT<C> &p, long nblocks, cudaStream_t s, bool wide = false) {
+	ProfScope ps("i2_terms", s);
+	if constexpr (P == 64 && sizeof(C) == 16) {
+		if (wide) {
+			static DeviceFlag init;
+			if (!init) { check_tmem_coresidency(); set_smem(k_i2_terms64<C>, Terms64<C>::SMEM); init = true; }
+			k_i2_terms64<C><<<(unsigned)nblocks, Terms64<C>::NT, Terms64<C>::SMEM, s>>>(p);
+			QB_CUDA(cudaGetLastError());
+			return;
+		}
+	}
 	static DeviceFlag init;
 	if (!init) { set_smem(k_i2_terms<P, C>, smem_grids<P, C>(2)); init = true; }
-	ProfScope ps("i2_terms", s);
 	k_i2_terms<P, C><<<(unsigned)nblocks, Geo<P>::NT, smem_grids<P, C>(2), s>>>(p);
 	QB_CUDA(cudaGetLastError());
 }
@@ -599,7 +619,8 @@ template <int P, class C> struct Rhs {
 	}
 
 	// S sums for Cc (tasks g = W_1..W_3, F = -4 W^_0 + 2) or I4 (g = W_0..W_3, F = 2 W^_0 - 1)
-	static void i1_sums(Workspace &ws, const DevI1 &t, int ncells, const double2 *W, bool cc, DevBuf &part, DevBuf &fs, int nchunk, cudaStream_t s) {
+	static void i1_sums(Workspace &ws, const DevI1 &t, int ncells, const double2 *W, bool cc, DevBuf &part, DevBuf &fs, const Chunks &ch, cudaStream_t s) {
+		const int nchunk = ch.i1;
 		const int ntask = cc ? 3 : 4;
 		part.ensure(sizeof(C) * ncells * ntask * nchunk * PP);
 		I1ParamsT<C> p{};
@@ -610,7 +631,7 @@ template <int P, class C> struct Rhs {
 		p.fa = cc ? -4.0 : 2.0; p.fb = cc ? 2.0 : -1.0;
 		p.psi2 = T::i1_psi2(t); p.phi = T::i1_phi(t);
 		p.out = part.as<C>();
-		launch_i1<P>(p, (long)ncells * ntask * nchunk, s);
+		launch_i1<P>(p, (long)ncells * ntask * nchunk, s, ch.wide12);
 		fs.ensure(sizeof(C) * ncells * ntask * PP);
 		FullParamsT<C> f{};
 		f.in = part.as<C>(); f.grid_stride = nchunk * PP; f.part_stride = PP; f.nparts = nchunk;
@@ -618,7 +639,8 @@ template <int P, class C> struct Rhs {
 		launch_fft_full<P>(f, (long)ncells * ntask, s);
 	}
 
-	static void i2_sums(Workspace &ws, const DevI2 &t, int ncells, const double2 *W, int nchunk, cudaStream_t s) {
+	static void i2_sums(Workspace &ws, const DevI2 &t, int ncells, const double2 *W, const Chunks &ch, cudaStream_t s) {
+		const int nchunk = ch.i2;
 		ws.i2p.ensure(sizeof(C) * ncells * 4 * nchunk * PP);
 		I2ParamsT<C> p{};
 		p.ntask = 4; p.nchunk = nchunk; p.nterms = t.nterms;
@@ -626,7 +648,7 @@ template <int P, class C> struct Rhs {
 		for (int k = 0; k < 4; k++) { p.f_comp[k] = k; p.g_comp[k] = k; }
 		p.psi1 = T::i2_psi1(t); p.psi2 = T::i2_psi2(t);
 		p.out = ws.i2p.as<C>();
-		launch_i2<P>(p, (long)ncells * 4 * nchunk, s);
+		launch_i2<P>(p, (long)ncells * 4 * nchunk, s, ch.wide12);
 		if (sum_i2(nchunk, ncells)) {
 			ws.i2s.ensure(sizeof(C) * ncells * 4 * PP);
 			SumSlotsT<C> r{};
@@ -758,10 +780,10 @@ template <int P, class C> struct Rhs {
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
 		const cudaStream_t s2 = small ? ws.fork(s, 0) : s;
 		if (small) i3_sums(ws, *q.i3, ncells, W, ch, s);
-		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch.i1, s2);
+		if (parts & RHS_CC) i1_sums(ws, *q.i1, ncells, W, true, ws.i1cc, ws.fs, ch, s2);
 		if (parts & RHS_CD) {
-			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch.i1, s2);
-			i2_sums(ws, *q.i2, ncells, W, ch.i2, s2);
+			i1_sums(ws, *q.i4, ncells, W, false, ws.i1i4, ws.fs4, ch, s2);
+			i2_sums(ws, *q.i2, ncells, W, ch, s2);
 			if (!small) i3_sums(ws, *q.i3, ncells, W, ch, s);
 		}
 		if (small) ws.join(s, 0);
@@ -824,7 +846,7 @@ template <class K> void set_smem_once(K kern, size_t bytes, DeviceFlag &done) {
 	if (!done) { set_smem(kern, bytes); done = true; }
 }
 
-// I3 kernel of the collision operator at N = 64: 4 components on 2 CTA pairs
+// QB_I3_KERNEL=pair at N = 64 in FP32: 4 components on 2 CTA pairs
 constexpr int kI3Pairs128 = 2;
 // its dynamic shared memory: FP64 adds the landing buffer of the bulk-copy exchange
 template <class C> constexpr size_t smem_i3_128() { return smem128<C>() + (sizeof(C) == 16 ? kLbBytes : 0); }
@@ -1011,6 +1033,9 @@ void check_tmem_coresidency() {
 		{ (const void *)k_i3w<double2>, i3w_smem<double2>(), 512, (int)WideTmem<4>::COLS, "k_i3w<f64>" },
 		{ (const void *)k_i3w<float2>, i3w_smem<float2>(), 512, (int)WideTmem<2>::COLS, "k_i3w<f32>" },
 		{ (const void *)k_i3wr, i3w_smem<float2>(), 512, (int)WideTmem<1>::COLS, "k_i3wr" },
+		{ (const void *)k_i1_terms64<double2>, Terms64<double2>::SMEM, 256, (int)Terms64<double2>::COLS, "k_i1_terms64<f64>" },
+		{ (const void *)k_i1_terms64<float2>, Terms64<float2>::SMEM, 256, (int)Terms64<float2>::COLS, "k_i1_terms64<f32>" },
+		{ (const void *)k_i2_terms64<double2>, Terms64<double2>::SMEM, 256, (int)Terms64<double2>::COLS, "k_i2_terms64<f64>" },
 		{ (const void *)k_i3_quad, Quad128::SMEM, Quad128::NT, Quad128::TCOLS, "k_i3_quad" },
 		{ (const void *)k_i3_128<4, kI3Pairs128, float2>, smem_i3_128<float2>(), G128::NT,
 		  (int)I3Tmem128<float2, 4 / kI3Pairs128>::NCOLS, "k_i3_128<f32>" },
@@ -1341,10 +1366,17 @@ __global__ void k_rk4(long n, const double2 *__restrict__ W, double c, const dou
 Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) {
 	Chunks c;
 	const int sms = num_sms();
-	if (q.i1) c.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), sms, 64);
-	if (q.i2) c.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), sms, 64);
+	// N = 32: the kernels of qb_terms64.cuh, as many CTAs as an SM holds, except in
+	// small batches: there an SM has few terms to run and the 512 threads a term of
+	// the general kernels finish them sooner (7 cells, J = 8, M = 6 between Maxwell
+	// walls: 600 us a step against 631; 64 cells, J = M = 16: 15.5 ms against 15.1)
+	c.wide12 = N == 32 && ncells * (long)i3_units >= kForkUnits * resident_i3(N, prec == 32);
+	const int c1 = !c.wide12 ? 1 : prec == 32 ? Terms64<float2>::CTAS : Terms64<double2>::CTAS;
+	const int c2 = !c.wide12 || prec == 32 ? 1 : Terms64<double2>::CTAS;
+	if (q.i1) c.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), sms * c1, 64);
+	if (q.i2) c.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), sms * c2, 64);
 	// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written
-	// and read back at HBM speed; one term takes a cluster ~36 us there: 0.15
+	// and read back at HBM speed; a unit takes a cluster tens of us: 0.15
 	if (q.i3) c.i3 = best_chunks((long)ncells, std::max(1, i3_units), resident_i3(N, prec == 32), 256, 0.15);
 	return c;
 }

@@ -162,6 +162,7 @@ void ensure_tmem_coresidency();
 // chunking of the quadrature-term sums over CTAs (picked per launch shape)
 struct Chunks {
 	int i1 = 1, i2 = 1, i3 = 1;
+	bool wide12 = false;                     // N = 32: the I1, I2 and I4 sums on the kernels of qb_terms64.cuh
 	int i3_slots = 0;                        // > 0: the I3 sums run as that many contiguous (cell, term) ranges instead of chunks
 };
 Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units);

@@ -155,7 +155,7 @@ struct F128Tmem {
 };
 
 // The chains run with i outermost for the pairs of opposite shifts (I3Units), as
-// in k_i3p.  Ghat: B layout; pscr: [cluster][4][P*P] natural; yscr:
+// in k_i3w.  Ghat: B layout; pscr: [cluster][4][P*P] natural; yscr:
 // [cluster][2][P*P]; out: [cell][chunk][4][P*P] B layout; zout:
 // [cell][chunk][rank][4][N*N].
 // kind: null (every cell) or the per-cell form of k_nyquist_kind; this kernel

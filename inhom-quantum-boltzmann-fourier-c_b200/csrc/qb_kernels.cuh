@@ -17,7 +17,8 @@
 //   I1/I4-type sums  S = sum_t phi_t . IFFT2(F . FFT2(Pad(psi2_t . g)))  (k_i1_terms)
 //   I2-type sums     Q = sum_t FFT2(Pad(psi1_t f)) . FFT2(Pad(psi2_t g))  (k_i2_terms)
 //   I3-type sums     X_r = sum_t sum_i coef_i P_{t,a_i} . FFT2(psi2_t . IFFT2(G_i . P_{t,r}))
-//                    with P_{t,c} = FFT2(Pad(psi1_t . W_c))               (k_i3)
+//                    with P_{t,c} = FFT2(Pad(psi1_t . W_c))               (k_i3q here, k_i3w in
+//                    qb_wide64.cuh and others at larger N; k_i3 for the single integrals)
 //   then outer FFT/IFFT, Extract and the Pauli combination (k_fft_full, k_assemble).
 // Moving the sums over quadrature terms inside the outer transforms is exact
 // in real arithmetic; results agree with the upstream loop order to rounding.
@@ -346,7 +347,7 @@ template <class C> struct I3ParamsT {
 	I3Units un;
 	C *zout;                                              // Z_i partials, layout given at each kernel (pairing kernels)
 	C *zscr;                                              // real forms: packed Z sums of the running cluster
-	TermRanges rg;                                        // nslots > 0: one term range per cluster (k_i3p)
+	TermRanges rg;                                        // nslots > 0: one term range per cluster
 	const double2 *src; long src_cell; int src_comp[4];   // N x N grids (FP64 state)
 	const C *Ghat; long g_cell;                           // P x P grids, G_g at Ghat + cell*g_cell + g*P*P
 	int ncombo[4]; int ca[4][4], cgi[4][4]; double ccoef[4][4];

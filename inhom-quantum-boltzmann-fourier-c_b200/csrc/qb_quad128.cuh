@@ -11,8 +11,8 @@
 // butterflies, psi2 at its four points, the butterflies back) and four 64 x 64
 // forward transforms.  Every thread owns the same eight (r, c) in all of them,
 // so the E_s of a thread wait in places only it reads: two in shared memory,
-// one in tensor memory, one in registers.  The 64 x 64 transforms are those of
-// k_i3p, in one grid of pitch 65.
+// one in tensor memory, one in registers.  The 64 x 64 transforms hold 8
+// values a thread, in one grid of pitch 65.
 //
 // Padding needs no transform of zeros: of the four points (r + 64 sl, c + 64
 // sk) exactly one is outside the zero band, that of N-grid index (r, c), with

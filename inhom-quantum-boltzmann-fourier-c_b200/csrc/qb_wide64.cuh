@@ -191,8 +191,8 @@ template <class C> constexpr size_t i3w_smem() {
 // pscr are in thread order (value r of thread t of A at 256 r + t): a warp's
 // load is four full lines, where the natural order gives eight half lines and
 // twice the cycles of the shared-memory and L1 pipe, which bounds this kernel.
-// Measured (64 cells, J = M = 16, FP64): the Strang step 17.7 ms with k_i3p (8
-// values a thread, FP64 pipe 42%, shared-memory pipe 72%), 16.2 ms with 16
+// Measured (64 cells, J = M = 16, FP64): the Strang step 17.7 ms with 8
+// values a thread (FP64 pipe 42%, shared-memory pipe 72%), 16.2 ms with 16
 // values in the natural order, 15.5 ms in thread order.
 // out: [slot][4][PP], zout: [slot][rank][4][N*N], slots of the term ranges (or
 // (cell, chunk)); pscr: [cluster][2][4][PP] (two units in turn: one cluster
