@@ -161,15 +161,15 @@ class ClockSampler:
 
 # ---------------------------------------------------------------------------
 
-def i3_flops_per_term(N):
-    """algorithmic FP64 flops of the I3 kernel per (cell, quadrature term):
-    4 padded spectra (0.75 of a full 2N x 2N FFT each: half the rows are zero)
-    + 16 (i, j) pairs x (IFFT2 + FFT2) at 5 n log2 n per transform, plus the
-    pointwise products (19 flops per padded point per pair, 6 per N-point
-    per source)."""
+def i3_flops_per_pair(N):
+    """FP64 flops of the I3 kernel per (cell, pair of terms of opposite shifts):
+    4 padded spectra and 4 extracted inverse transforms (0.75 of a full 2N x 2N
+    FFT each: half the rows are zero or not needed) + 16 (i, j) pairs x (IFFT2 +
+    FFT2) at 5 n log2 n per transform, plus the pointwise products (24 flops per
+    padded point per (i, j), 14 per N-point per component)."""
     P = 2 * N
     F = 5.0 * P * P * math.log2(P * P)
-    return 4 * 0.75 * F + 32 * F + 16 * 19 * P * P + 4 * 6 * N * N
+    return 8 * 0.75 * F + 32 * F + 16 * 24 * P * P + 4 * 14 * N * N
 
 
 def captured_traffic(kernel, wl):
@@ -274,12 +274,12 @@ def run_ours(args):
     L.qb_fp64_peak_tflops.restype = ctypes.c_double
     peak = L.qb_fp64_peak_tflops()
     per_launch_ms = kms.value / max(1, kn.value)
-    flops_launch = cells * wl["J"] * wl["M"] * i3_flops_per_term(N)
+    flops_launch = cells * wl["J"] * ((wl["M"] + 1) // 2) * i3_flops_per_pair(N)
     achieved = flops_launch / (per_launch_ms * 1e-3) / 1e12
-    i3name = "k_i3p" if N == 32 else ("k_i3_128" if N == 64 else "k_i3")
-    i3desc = {"k_i3p": "k_i3p (I3 quadrature sums, 2-CTA cluster, accumulators in tensor memory)",
-              "k_i3_128": "k_i3_128 (I3 quadrature sums, grids split over CTA pairs)",
-              "k_i3": "k_i3 (I3 quadrature sums, 4-CTA cluster)"}[i3name]
+    i3name = {32: "k_i3w", 64: "k_i3_quad"}.get(N, "k_i3q")
+    i3desc = {"k_i3w": "k_i3w (I3 quadrature sums, 2-CTA cluster, 16 values a thread, accumulators in tensor memory)",
+              "k_i3_quad": "k_i3_quad (I3 quadrature sums, 4-CTA cluster, a padded grid as four N x N grids in one CTA)",
+              "k_i3q": "k_i3q (I3 quadrature sums, four components in one CTA)"}[i3name]
     roofline = {"bound": "fp64", "kernel": i3desc, "achieved": round(achieved, 3),
                 "peak": round(peak, 3), "unit": "TFLOP/s", "frac": round(achieved / peak, 4) if peak > 0 else None,
                 "peak_source": "measured live: DFMA loop on every SM (qb_fp64_peak_tflops); MEASURED_PEAKS.json has no FP64 figure",
@@ -576,7 +576,7 @@ def run_precision_form(args, wl, qbgpu, q, B, Wall, flush, value64):
 
 def run_dftmma_sample(args, qbgpu, flush, cells=64, N=16, J=16, M=16, L=6.0, R=3.75):
     """The I3 sums of the FP32 form at N = 16 two ways: the FFT kernels
-    (k_i3, 4-CTA clusters) and DFT-GEMMs on the tensor cores (k_i3_mma32:
+    (k_i3q, one CTA) and DFT-GEMMs on the tensor cores (k_i3_mma32:
     tcgen05.mma kind::tf32, TF32 hi/lo split); C[W] of `cells` cells per
     evaluation, both against the FP64 operator.  Tensor-pipe work: every
     1-D pass is a 128 x 64 x 64 real GEMM per 4 grids, 3 products (hi/lo)."""
