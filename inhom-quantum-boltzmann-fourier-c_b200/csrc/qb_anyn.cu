@@ -277,13 +277,27 @@ template <class C> __device__ void init_tw(C *tw, int L, const Plan &pl) {
 	}
 	__syncthreads();
 }
+// (c, s) rounded to the neighbouring FP32 values of least modulus error (weighed
+// 30 to 1 against the phase error)
+__device__ float2 unit_root(double c, double s) {
+	if (fabs(c) < 1e-9 || fabs(s) < 1e-9) return make_float2((float)c, (float)s);
+	float2 best = make_float2((float)c, (float)s);
+	double cost = 1e300;
+	for (int i = -2; i <= 2; i++)
+		for (int j = -2; j <= 2; j++) {
+			const float x = __int_as_float(__float_as_int((float)c) + i), y = __int_as_float(__float_as_int((float)s) + j);
+			const double re = (double)x * c + (double)y * s - 1.0, im = (double)y * c - (double)x * s, e = 30.0 * re * re + im * im;
+			if (e < cost) { cost = e; best = make_float2(x, y); }
+		}
+	return best;
+}
 // the table of init_tw for L = P, in both precisions
 __global__ void k_any_build_tw(int L, double2 *twd, float2 *twf) {
 	for (int m = threadIdx.x; m < L; m += blockDim.x) {
 		double s, c;
 		sincospi(2.0 * m / L, &s, &c);
 		twd[m] = make_double2(c, -s);
-		twf[m] = mk<float2>(c, -s);
+		twf[m] = unit_root(c, -s);
 	}
 }
 
@@ -885,7 +899,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 // needs it to separate the two packed sums; there i < 2).  One CTA per (cell,
 // i, block of nl columns of those N + 1) adds the wave's terms in order.
 template <class C> struct I3ColsZP {
-	const C *V; C *Z; const C *psi1; int N, nl, nt, t0;
+	const C *V; double2 *Z; const C *psi1; int N, nl, nt, t0;
 	int ns;                               // Z[cell][4][ns], partials as in k_any_i3_rows_b
 	WaveUnits un;
 	const int *kind;
@@ -909,7 +923,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	load_tw(T.tw, P, p.pl);
 	const int nz = min(nl, (rf ? ZS : N) - z0);       // columns of this block
 	if (nz <= 0) return;
-	C *Z = p.Z + cis * (long)ZS * ZS;
+	double2 *Z = p.Z + cis * (long)ZS * ZS;
 	const int pitch = T.pitch;
 	const unsigned mgnl = magic_div((unsigned)nl);
 	for (int tt = first; tt < p.nt; tt += p.ns) {
@@ -934,20 +948,20 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 			const int a = up ? -l : l, b = up ? -k : k;
 			C w = ps[(long)(a < 0 ? a + N : a) * N + (b < 0 ? b + N : b)];
 			if (!up) w.y = -w.y;
-			C *z = Z + (long)zr * ZS + z0 + line;
-			*z = cfma(w, r[tat(line, l < 0 ? l + P : l, pitch)], *z);
+			zadd_mem(Z + (long)zr * ZS + z0 + line, w, r[tat(line, l < 0 ? l + P : l, pitch)]);
 		}
 		__syncthreads();
 	}
 }
 
 // assembly rows: Zcc_j and Zcd_j (the combinations of k_assemble) for unit
-// (cell, j), inverse row transforms into Z[(cell 4 + j) 2 + {0, 1}]
+// (cell, j), inverse row transforms into Z[(cell 4 + j) 2 + {0, 1}], in FP64 in
+// both precisions as in k_assemble
 template <class C> struct AsmP {
 	const C *What, *FS, *FS4, *Q, *X;    // FS [cell][3], FS4 / Q [cell][4], X [cell][4][nxp] (null: part absent)
 	int nxp;                             // partials of X per (cell, j), added in order
-	const C *Zp; int nzp; const int *kind;   // sums of k_any_i3_cols_z, nzp partials a grid (null: none), and the cells' forms
-	C *Z; int N, nl;
+	const double2 *Zp; int nzp; const int *kind;   // sums of k_any_i3_cols_z, nzp partials a grid (null: none), and the cells' forms
+	double2 *Z; int N, nl;
 	double s1, s2;
 	int mode;
 	double2 *out_cc, *out_cd;
@@ -955,11 +969,10 @@ template <class C> struct AsmP {
 	Plan pl;
 };
 template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k_any_asm_rows(const AsmP<C> p) {
-	using R = typename CT<C>::R;
 	extern __shared__ __align__(16) unsigned char sm[];
 	const int P = 2 * p.N, nl = p.nl;
 	const long PP = (long)P * P;
-	Tile<C> T(sm, P, 2 * nl);
+	Tile<double2> T(sm, P, 2 * nl);
 	const unsigned mgP = magic_div((unsigned)P), mgnl = magic_div((unsigned)nl);
 	load_tw(T.tw, P, p.pl);
 	const int bpg = P / nl;
@@ -967,44 +980,44 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	const int l0 = (int)(blockIdx.x % bpg) * nl;
 	const long cell = cj / 4;
 	const int j = (int)(cj % 4);
-	const R eta2[4] = { 2, -2, -2, -2 };
-	const R s1 = (R)p.s1, s2 = (R)p.s2;
+	const double eta2[4] = { 2, -2, -2, -2 }, s1 = p.s1, s2 = p.s2;
 	const C *Wh = p.What + cell * 4 * PP;
 	for (int i = threadIdx.x; i < nl * P; i += blockDim.x) {
 		const int li = fdiv(i, mgP), k = i - li * P;
 		const long e = (long)(l0 + li) * P + k;
-		C zc = czero<C>(), zd = czero<C>();
+		double2 zc = czero(), zd = czero();
 		if (p.FS != nullptr && j > 0) {
 			const int gi = (j % 3) + 1, hi = ((j + 1) % 3) + 1;
 			const C *FS = p.FS + cell * 3 * PP;
-			zc = csub(cmul(Wh[hi * PP + e], FS[(gi - 1) * PP + e]), cmul(Wh[gi * PP + e], FS[(hi - 1) * PP + e]));
+			zc = csub(cmul(widen(Wh[hi * PP + e]), widen(FS[(gi - 1) * PP + e])), cmul(widen(Wh[gi * PP + e]), widen(FS[(hi - 1) * PP + e])));
 		}
 		if (p.Q != nullptr) {
-			C q = czero<C>();
+			double2 q = czero();
 			for (int ii = 0; ii < 4; ii++) {
-				const C s = p.Q[(cell * 4 + ii) * PP + e];
+				const double2 s = widen(p.Q[(cell * 4 + ii) * PP + e]);
 				q.x += eta2[ii] * s.x;
 				q.y += eta2[ii] * s.y;
 			}
-			C h; h.x = -Wh[j * PP + e].x; h.y = -Wh[j * PP + e].y;
-			if (j == 0) h.x += (R)1.0;
-			const C v = cmul(h, q);
+			double2 h = widen(Wh[j * PP + e]);
+			h.x = -h.x; h.y = -h.y;
+			if (j == 0) h.x += 1.0;
+			const double2 v = cmul(h, q);
 			zd.x += s2 * v.x;
 			zd.y += s2 * v.y;
 		}
 		if (p.X != nullptr) {
-			C s = p.X[(cell * 4 + j) * p.nxp * PP + e];
-			for (int k = 1; k < p.nxp; k++) s = cadd(s, p.X[((cell * 4 + j) * p.nxp + k) * PP + e]);
+			double2 s = widen(p.X[(cell * 4 + j) * p.nxp * PP + e]);
+			for (int k = 1; k < p.nxp; k++) s = cadd(s, widen(p.X[((cell * 4 + j) * p.nxp + k) * PP + e]));
 			zd.x -= eta2[j] * s1 * s.x;
 			zd.y -= eta2[j] * s1 * s.y;
 		}
 		if (p.FS4 != nullptr) {
 			const C *F4 = p.FS4 + cell * 4 * PP;
-			C v = cadd(cscale(cmul(Wh[e], F4[j * PP + e]), eta2[j]), cscale(cmul(Wh[j * PP + e], F4[e]), (R)2.0));
+			double2 v = cadd(cscale(cmul(widen(Wh[e]), widen(F4[j * PP + e])), eta2[j]), cscale(cmul(widen(Wh[j * PP + e]), widen(F4[e])), 2.0));
 			if (j == 0) {
-				C s = czero<C>();
-				for (int c = 0; c < 4; c++) s = cadd(s, cmul(Wh[c * PP + e], F4[c * PP + e]));
-				v = csub(v, cscale(s, (R)2.0));
+				double2 s = czero();
+				for (int c = 0; c < 4; c++) s = cadd(s, cmul(widen(Wh[c * PP + e]), widen(F4[c * PP + e])));
+				v = csub(v, cscale(s, 2.0));
 			}
 			zd.x += s1 * v.x;
 			zd.y += s1 * v.y;
@@ -1013,8 +1026,8 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 		T.a[T.at(nl + li, k)] = zd;
 	}
 	__syncthreads();
-	const C *r = fft_lines_x<R1, R2, +1>(T.a, T.b, 2 * nl, T.pitch, 1, p.pl, T.tw);
-	C *z = p.Z + cj * 2 * PP + (long)l0 * P;
+	const double2 *r = fft_lines_x<R1, R2, +1>(T.a, T.b, 2 * nl, T.pitch, 1, p.pl, T.tw);
+	double2 *z = p.Z + cj * 2 * PP + (long)l0 * P;
 	for (int i = threadIdx.x; i < 2 * nl * P; i += blockDim.x) {
 		const int h = i >= nl * P ? 1 : 0, rem = i - h * nl * P, li = fdiv(rem, mgP), k = rem - li * P;
 		z[h * PP + (long)li * P + k] = r[T.at(h * nl + li, k)];
@@ -1027,7 +1040,7 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	extern __shared__ __align__(16) unsigned char sm[];
 	const int N = p.N, P = 2 * N, nl = p.nl;
 	const long PP = (long)P * P, NN = (long)N * N;
-	Tile<C> T(sm, P, 2 * nl);
+	Tile<double2> T(sm, P, 2 * nl);
 	const unsigned mgP = magic_div((unsigned)P), mgnl = magic_div((unsigned)nl);
 	load_tw(T.tw, P, p.pl);
 	const int bpg = P / nl;
@@ -1035,36 +1048,35 @@ template <class C, int R1, int R2> __global__ void __launch_bounds__(kThreads) k
 	const int k0 = (int)(blockIdx.x % bpg) * nl;
 	const long cell = cj / 4;
 	const int j = (int)(cj % 4);
-	const C *z = p.Z + cj * 2 * PP;
+	const double2 *z = p.Z + cj * 2 * PP;
 	for (int i = threadIdx.x; i < 2 * nl * P; i += blockDim.x) {
 		const int h = i >= nl * P ? 1 : 0, rem = i - h * nl * P, l = fdiv(rem, mgnl), kk = rem - l * nl;
 		T.a[T.at(h * nl + kk, l)] = z[h * PP + (long)l * P + k0 + kk];
 	}
 	__syncthreads();
-	const C *r = fft_lines_x<R1, R2, +1>(T.a, T.b, 2 * nl, T.pitch, 1, p.pl, T.tw);
+	const double2 *r = fft_lines_x<R1, R2, +1>(T.a, T.b, 2 * nl, T.pitch, 1, p.pl, T.tw);
 	for (int i = threadIdx.x; i < nl * P; i += blockDim.x) {
 		const int l = fdiv(i, mgnl), kk = i - l * nl;
 		const int ls = src_idx(l, N), ks = src_idx(k0 + kk, N);
 		if (ls < 0 || ks < 0) continue;
-		const C zc = r[T.at(kk, l)], zd = r[T.at(nl + kk, l)];
-		const double2 cc = make_double2(p.s1 * (double)zc.x, p.s1 * (double)zc.y);
-		double2 cd = make_double2((double)zd.x, (double)zd.y);
+		const double2 cc = cscale(r[T.at(kk, l)], p.s1);
+		double2 cd = r[T.at(nl + kk, l)];
 		if (p.Zp != nullptr) {                       // - eta2_j s1 Z_j
 			const int H = N / 2, ZS = N + 1, fl = (ls < H ? ls : ls - N) + H, fk = (ks < H ? ks : ks - N) + H;
 			const double f = (j == 0 ? 2.0 : -2.0) * p.s1;
 			if (has_rf<C>() && p.kind != nullptr && p.kind[cell] == 0) {
 				// A = Z_2c + i Z_2c+1, each the transform of a real grid
 				for (int k = 0; k < p.nzp; k++) {
-					const C *A = p.Zp + ((cell * 4 + (j >> 1)) * p.nzp + k) * (long)ZS * ZS;
-					const C u = A[fl * ZS + fk], v = A[(N - fl) * ZS + N - fk];
-					cd.x -= f * 0.5 * ((j & 1) ? (double)u.y + (double)v.y : (double)u.x + (double)v.x);
-					cd.y -= f * 0.5 * ((j & 1) ? (double)v.x - (double)u.x : (double)u.y - (double)v.y);
+					const double2 *A = p.Zp + ((cell * 4 + (j >> 1)) * p.nzp + k) * (long)ZS * ZS;
+					const double2 u = A[fl * ZS + fk], v = A[(N - fl) * ZS + N - fk];
+					cd.x -= f * 0.5 * ((j & 1) ? u.y + v.y : u.x + v.x);
+					cd.y -= f * 0.5 * ((j & 1) ? v.x - u.x : u.y - v.y);
 				}
 			} else {
 				for (int k = 0; k < p.nzp; k++) {
-					const C z = p.Zp[(cj * p.nzp + k) * (long)ZS * ZS + fl * ZS + fk];
-					cd.x -= f * (double)z.x;
-					cd.y -= f * (double)z.y;
+					const double2 z = p.Zp[(cj * p.nzp + k) * (long)ZS * ZS + fl * ZS + fk];
+					cd.x -= f * z.x;
+					cd.y -= f * z.y;
 				}
 			}
 		}
@@ -1420,7 +1432,7 @@ template <class C> struct AnyRhs {
 		const int nang = t.nterms / t.pairM;
 		const long nw = 4L * ncells * PP;
 		ws.i3p.ensure(sizeof(C) * ncells * 4 * p.nchunk * PP);
-		ws.i3z.ensure(sizeof(C) * 4 * ncells * 4 * p.nchunk * (N + 1) * (N + 1));
+		ws.i3z.ensure(sizeof(double2) * 4 * ncells * 4 * p.nchunk * (N + 1) * (N + 1));
 		ws.wave1.ensure(sizeof(C) * ncl * 8 * PP * (kind ? 2 : 1));
 		ws.wave2.ensure(sizeof(C) * (nw + ncl * 4 * PP) + sizeof(float) * nw + sizeof(R) * nang * PP);
 		C *wi = ws.wave2.as<C>();
@@ -1429,7 +1441,7 @@ template <class C> struct AnyRhs {
 		float *wr = reinterpret_cast<float *>(psi + nang * PP);
 		p.kind = kind; p.src = W; p.WI = wi; p.WR = reinterpret_cast<const R *>(wr);
 		p.psi1 = Tabs<C>::i3_psi1(t); p.psi2 = psi; p.scale = t.scale.as<double>();
-		p.pscr = ws.wave1.as<C>(); p.X = ws.i3p.as<C>(); p.Z = ws.i3z.as<C>();
+		p.pscr = ws.wave1.as<C>(); p.X = ws.i3p.as<C>(); p.Z = ws.i3z.as<double2>();
 		{
 			ProfScope ps("any_items", s);
 			const unsigned nb = (unsigned)((PP + 255) / 256);
@@ -1515,9 +1527,9 @@ template <class C> struct AnyRhs {
 		QB_CUDA(cudaMemsetAsync(ws.i3p.p, 0, sizeof(C) * ncells * 4 * nxp * PP, s));
 		if (t.pairM > 0) {
 			as.nzp = partials();
-			ws.i3z.ensure(sizeof(C) * 4 * as.nzp * ncells * (N + 1) * (N + 1));
-			QB_CUDA(cudaMemsetAsync(ws.i3z.p, 0, sizeof(C) * 4 * as.nzp * ncells * (N + 1) * (N + 1), s));
-			as.Zp = ws.i3z.as<C>();
+			ws.i3z.ensure(sizeof(double2) * 4 * as.nzp * ncells * (N + 1) * (N + 1));
+			QB_CUDA(cudaMemsetAsync(ws.i3z.p, 0, sizeof(double2) * 4 * as.nzp * ncells * (N + 1) * (N + 1), s));
+			as.Zp = ws.i3z.as<double2>();
 			as.kind = kind;
 		}
 		i3_waves(t, W, nxp, kind);
@@ -1526,7 +1538,7 @@ template <class C> struct AnyRhs {
 
 	// the terms of the opposite shifts of a wave: rows of Y_i (into V, the P grids'
 	// place), columns into Z
-	void other_terms(const DevI3 &t, const C *What, const C *Y, C *V, C *Z, int nc, int n, int t0, const int *kc) {
+	void other_terms(const DevI3 &t, const C *What, const C *Y, C *V, double2 *Z, int nc, int n, int t0, const int *kc) {
 		I3RowsYP<C> y{};
 		y.What = What; y.Y = Y; y.V = V; y.N = N; y.nl = nl1; y.nt = n; y.t0 = t0; y.un.M = t.pairM; y.kind = kc; y.pl = pl;
 		by_plan([&](auto kern) { launch(kern, "any_i3_rows_y", blocks((long)nc * n * 4, nl1), smem(nl1, 1), s, y); },
@@ -1588,7 +1600,7 @@ template <class C> struct AnyRhs {
 				by_plan([&](auto kern) { launch(kern, "any_i3_rows_b", blocks((long)nc * 4 * nxp, nl4), smem(nl4, 1), s, b); },
 				        k_any_i3_rows_b<C, 16, 3>, k_any_i3_rows_b<C, 16, 6>, k_any_i3_rows_b<C, 16, 12>,
 				        k_any_i3_rows_b<C, 16, 16>, k_any_i3_rows_b<C, 0, 0>);
-				if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<C>() + (long)c0 * 4 * partials() * (N + 1) * (N + 1), nc, n, t0, kc);
+				if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<double2>() + (long)c0 * 4 * partials() * (N + 1) * (N + 1), nc, n, t0, kc);
 			}
 		}
 	}
@@ -1612,13 +1624,14 @@ template <class C> struct AnyRhs {
 	}
 
 	void assemble(AsmP<C> &a) {
-		const int nl2 = pick_lines(P, nl1, 2, sizeof(C));
+		// FP64 tiles in both precisions: at most 2048 elements
+		const int nl2 = pick_lines(P, sizeof(C) == 8 ? std::max(1, nl1 / 2) : nl1, 2, sizeof(double2));
 		a.nl = nl2;
-		ws.wave1.ensure(sizeof(C) * (size_t)ncells * 8 * PP);
-		a.Z = ws.wave1.as<C>();
-		by_plan([&](auto kern) { launch(kern, "any_asm_rows", blocks((long)ncells * 4, nl2), smem(nl2, 2), s, a); },
+		ws.wave1.ensure(sizeof(double2) * (size_t)ncells * 8 * PP);
+		a.Z = ws.wave1.as<double2>();
+		by_plan([&](auto kern) { launch(kern, "any_asm_rows", blocks((long)ncells * 4, nl2), tile_bytes<double2>(P, 2 * nl2), s, a); },
 		        k_any_asm_rows<C, 16, 3>, k_any_asm_rows<C, 16, 6>, k_any_asm_rows<C, 16, 12>, k_any_asm_rows<C, 16, 16>, k_any_asm_rows<C, 0, 0>);
-		by_plan([&](auto kern) { launch(kern, "any_asm_cols", blocks((long)ncells * 4, nl2), smem(nl2, 2), s, a); },
+		by_plan([&](auto kern) { launch(kern, "any_asm_cols", blocks((long)ncells * 4, nl2), tile_bytes<double2>(P, 2 * nl2), s, a); },
 		        k_any_asm_cols<C, 16, 3>, k_any_asm_cols<C, 16, 6>, k_any_asm_cols<C, 16, 12>, k_any_asm_cols<C, 16, 16>, k_any_asm_cols<C, 0, 0>);
 	}
 };

@@ -505,7 +505,7 @@ constexpr int kSumSlots = 4;
 // summed over the slots of each cell first
 template <class C>
 void sum_slots(Workspace &ws, AsmParamsT<C> &a, int ncells, long slots, long lenx, long lenz, int zranks, cudaStream_t s) {
-	if (zranks > 0) { a.Zp = ws.i3z.as<C>(); a.nz = zranks; }
+	if (zranks > 0) { a.Zp = ws.i3z.as<double2>(); a.nz = zranks; }
 	if (slots < (long)kSumSlots * ncells || ncells > 65535) return;
 	SumSlotsT<C> p{};
 	p.rg = a.xrg; p.nx = a.nx; p.per = 1;
@@ -514,10 +514,12 @@ void sum_slots(Workspace &ws, AsmParamsT<C> &a, int ncells, long slots, long len
 	launch_sum_slots(p, ncells, s);
 	a.Xp = ws.i3s.as<C>();
 	if (zranks > 0) {
-		ws.i3zsum.ensure(sizeof(C) * ncells * lenz);
-		p.in = a.Zp; p.out = ws.i3zsum.as<C>(); p.len = (int)lenz; p.per = zranks;
-		launch_sum_slots(p, ncells, s);
-		a.Zp = ws.i3zsum.as<C>(); a.nz = 1;
+		ws.i3zsum.ensure(sizeof(double2) * ncells * lenz);
+		SumSlotsT<double2> z{};
+		z.rg = a.xrg; z.nx = a.nx; z.per = zranks;
+		z.in = a.Zp; z.out = ws.i3zsum.as<double2>(); z.len = (int)lenz;
+		launch_sum_slots(z, ncells, s);
+		a.Zp = ws.i3zsum.as<double2>(); a.nz = 1;
 	}
 	a.nx = 1;
 	a.xrg = TermRanges{};
@@ -525,9 +527,9 @@ void sum_slots(Workspace &ws, AsmParamsT<C> &a, int ncells, long slots, long len
 
 template <int P, class C> void launch_assemble(const AsmParamsT<C> &p, long ncells, cudaStream_t s) {
 	static DeviceFlag init;
-	if (!init) { set_smem(k_assemble<P, C>, smem_grids<P, C>(1)); init = true; }
+	if (!init) { set_smem(k_assemble<P, C>, smem_grids<P, double2>(1)); init = true; }
 	ProfScope ps("assemble", s);
-	k_assemble<P, C><<<(unsigned)(ncells * 4), Geo<P>::NT, smem_grids<P, C>(1), s>>>(p);
+	k_assemble<P, C><<<(unsigned)(ncells * 4), Geo<P>::NT, smem_grids<P, double2>(1), s>>>(p);
 	QB_CUDA(cudaGetLastError());
 }
 
@@ -684,8 +686,8 @@ template <int P, class C> struct Rhs {
 		}
 		ws.i3p.ensure(sizeof(C) * slots * 4 * PP);
 		if (pairs_units(ws)) {
-			ws.i3z.ensure(sizeof(C) * slots * kZRanks * 4 * NN);
-			p.zout = ws.i3z.as<C>();
+			ws.i3z.ensure(sizeof(double2) * slots * kZRanks * 4 * NN);
+			p.zout = ws.i3z.as<double2>();
 		}
 		p.src = W; p.src_cell = 4 * NN;
 		for (int r = 0; r < 4; r++) p.src_comp[r] = r;
@@ -707,8 +709,8 @@ template <int P, class C> struct Rhs {
 			if constexpr (sizeof(C) == 8) {
 				if (use_real_form()) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
-					ws.i3zs.ensure(sizeof(C) * slots * kZRanks * 2 * (N + 1) * (N + 1));
-					p.zscr = ws.i3zs.as<C>();
+					ws.i3zs.ensure(sizeof(double2) * slots * kZRanks * 2 * (N + 1) * (N + 1));
+					p.zscr = ws.i3zs.as<double2>();
 					launch_nyquist_kind(P / 2, ncells, W, kRealFormBound, ws.i3kind.as<int>(), ws.i3stats.as<unsigned long long>(), s);
 					kind = ws.i3kind.as<int>();
 					// the two forms side by side: either may have too few cells to fill the GPU
@@ -751,12 +753,12 @@ template <int P, class C> struct Rhs {
 				used = r.nslots;
 			}
 			b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
-			if (pairs_units(ws)) b.add(ws.i3z, sizeof(C) * slots * kZRanks * 4 * NN);
+			if (pairs_units(ws)) b.add(ws.i3z, sizeof(double2) * slots * kZRanks * 4 * NN);
 			if (P == 64) b.add(ws.i3y, sizeof(C) * used * 8 * PP);
-			if (P == 64 && sizeof(C) == 8 && use_real_form()) b.add(ws.i3zs, sizeof(C) * slots * kZRanks * 2 * (N + 1) * (N + 1));
+			if (P == 64 && sizeof(C) == 8 && use_real_form()) b.add(ws.i3zs, sizeof(double2) * slots * kZRanks * 2 * (N + 1) * (N + 1));
 			if (used >= (size_t)kSumSlots * ncells) {
 				b.add(ws.i3s, 4 * g);
-				if (pairs_units(ws)) b.add(ws.i3zsum, g);
+				if (pairs_units(ws)) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
 			}
 		}
 		b.reserve();
@@ -1104,8 +1106,8 @@ namespace {
 
 template <class C> void launch_assemble128(const AsmParamsT<C> &p, long ncells, cudaStream_t s) {
 	static DeviceFlag init;
-	set_smem_once(k_assemble128<C>, smem128<C>(), init);
-	launch128(k_assemble128<C>, "assemble", 2 * 4 * ncells, 2, smem128<C>(), s, p);
+	set_smem_once(k_assemble128<C>, smem128<double2>(), init);
+	launch128(k_assemble128<C>, "assemble", 2 * 4 * ncells, 2, smem128<double2>(), s, p);
 }
 
 template <class C> struct Rhs<128, C> {
@@ -1181,8 +1183,8 @@ template <class C> struct Rhs<128, C> {
 		ws.scr128a.ensure(sizeof(C) * ncl * 4 * PP);
 		if (pairs_units()) {
 			p.un.M = t.pairM;
-			ws.i3z.ensure(sizeof(C) * slots * kZRanks * 4 * NN);
-			p.zout = ws.i3z.as<C>();
+			ws.i3z.ensure(sizeof(double2) * slots * kZRanks * 4 * NN);
+			p.zout = ws.i3z.as<double2>();
 		}
 		p.src = W; p.src_cell = 4 * NN;
 		for (int r = 0; r < 4; r++) p.src_comp[r] = r;
@@ -1201,9 +1203,9 @@ template <class C> struct Rhs<128, C> {
 				ws.i3y.ensure(sizeof(C) * ncl * 2 * PP);
 				if (use_real_form() ) {
 					ws.i3kind.ensure(sizeof(int) * ncells);
-					ws.i3zs.ensure(sizeof(C) * ncl * 2 * 2 * (N + 1) * (N + 1));
+					ws.i3zs.ensure(sizeof(double2) * ncl * 2 * 2 * (N + 1) * (N + 1));
 					ws.WhatQ.ensure(wide_bytes(t, ncells));
-					p.zscr = ws.i3zs.as<C>();
+					p.zscr = ws.i3zs.as<double2>();
 					int *kind = ws.i3kind.as<int>();
 					launch_nyquist_kind(N, ncells, W, kRealFormBound, kind, ws.i3stats.as<unsigned long long>(), s);
 					// the two forms side by side: either may have too few cells to fill the GPU
@@ -1266,12 +1268,12 @@ template <class C> struct Rhs<128, C> {
 				}
 				b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
 				b.add(ws.scr128a, sizeof(C) * used * 4 * PP);
-				if (pairs_units()) b.add(ws.i3z, sizeof(C) * slots * kZRanks * 4 * NN);
+				if (pairs_units()) b.add(ws.i3z, sizeof(double2) * slots * kZRanks * 4 * NN);
 				if (sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 4 * PP);
 				else if (use_full128()) b.add(ws.i3y, sizeof(C) * used * 2 * PP);
 				if (used >= (size_t)kSumSlots * ncells) {
 					b.add(ws.i3s, 4 * g);
-					if (pairs_units()) b.add(ws.i3zsum, g);
+					if (pairs_units()) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
 				}
 			}
 			b.reserve();

@@ -63,6 +63,8 @@ template <> __device__ __forceinline__ float2 csub<float2>(float2 a, float2 b) {
 	return unpack_f2(d);
 }
 // FP64 shorthands used by code that is FP64 only
+__device__ __forceinline__ double2 widen(float2 a) { return make_double2((double)a.x, (double)a.y); }
+__device__ __forceinline__ double2 widen(double2 a) { return a; }
 __device__ __forceinline__ double2 czero() { return czero<double2>(); }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return cadd<double2>(a, b); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return csub<double2>(a, b); }

@@ -199,9 +199,9 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 	const int t0 = (int)((long)chunk * p.nterms / p.nchunk), t1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
 	// this CTA's partial of the Z sums and its Y_i (element order of the threads)
 	const long slot = cell * p.nchunk + chunk;
-	C *zbase = p.zout + (slot * 2 + rank) * 4 * (long)F::N * F::N;
+	double2 *zbase = p.zout + (slot * 2 + rank) * 4 * (long)F::N * F::N;
 	C *ybuf = yscr + (cid * 2 + rank) * (long)F::P * F::P + tid;
-	for (int i = tid; i < 4 * F::N * F::N; i += F::NT) zbase[i] = czero<C>();
+	for (int i = tid; i < 4 * F::N * F::N; i += F::NT) zbase[i] = czero();
 	__syncthreads();
 #pragma unroll 1
 	for (int un = t0; un < t1; un++) {
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 #pragma unroll
 				for (int r = 0; r < 8; r++) x[r] = S[cs_.at_in(r)];
 				fft128_line<+1, false>(x, tau, S, col, tw128, wp);
-				C *z = zbase + (long)i * F::N * F::N + ks;
+				double2 *z = zbase + (long)i * F::N * F::N + ks;
 				const C *ps = p.psi1 + (long)t * F::N * F::N + ks;
 #pragma unroll
 				for (int e = 0; e < 8; e++) {                    // rows pos128(tau, e): e = 0, 1 (0..31), 6, 7 (96..127)
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(F128::NT, 1) k_i3_full128(const I3ParamsT<C> p
 					const int o = F::src(pos128(tau, e)) * F::N;
 					C w = ps[o];
 					w.y = -w.y;
-					z[o] = cfma(w, x[e], z[o]);
+					zadd_mem(z + o, w, x[e]);
 				}
 			}
 			__syncthreads();                                     // the next chain's rows reuse S

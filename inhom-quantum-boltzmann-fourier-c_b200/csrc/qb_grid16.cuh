@@ -109,7 +109,7 @@ template <class C> struct I3GridP {
 	C *pscr;                                 // [cluster][2][4][PP]
 	C *xscr;                                 // [cluster][4][PP], X of the forms that keep it in L2
 	C *X;                                    // [cell][4][nchunk][PP] natural
-	C *Z;                                    // [cell][4][4 nchunk][(N + 1)^2]
+	double2 *Z;                                  // [cell][4][4 nchunk][(N + 1)^2]
 };
 template <int R, class C, bool RF> struct I3Grid {
 	static constexpr bool XS = R == 3 || RF; // X in shared memory
@@ -143,9 +143,9 @@ __global__ void __launch_bounds__((Grid16<R, C>::NT), (I3Grid<R, C, RF>::CTAS)) 
 		const double2 *src = p.src + (cell * 4 + j) * NN;
 		const Pt *Wc = RF ? reinterpret_cast<const Pt *>(p.WR) + cell * 4 * PP : reinterpret_cast<const Pt *>(p.WI) + cell * 4 * PP;
 		const long nzp = 4L * p.nchunk;
-		C *Zc = p.Z + (cell * 4 * nzp + chunk * 4 + j) * ZA;         // grid i at i nzp ZA
+		double2 *Zc = p.Z + (cell * 4 * nzp + chunk * 4 + j) * ZA;         // grid i at i nzp ZA
 		for (int i = threadIdx.x; i < PP; i += F::NT) X[i] = Pt{};
-		for (int i = threadIdx.x; i < NC * ZA; i += F::NT) Zc[(i / ZA) * nzp * ZA + i % ZA] = czero<C>();
+		for (int i = threadIdx.x; i < NC * ZA; i += F::NT) Zc[(i / ZA) * nzp * ZA + i % ZA] = czero();
 		const int u0 = (int)((long)chunk * p.nunits / p.nchunk), u1 = (int)((long)(chunk + 1) * p.nunits / p.nchunk);
 		__syncthreads();
 #pragma unroll 1
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__((Grid16<R, C>::NT), (I3Grid<R, C, RF>::CTAS)) 
 				__syncthreads();
 				G.template stage_b<+1>();
 				__syncthreads();
-				C *Zi = Zc + c * nzp * ZA;
+				double2 *Zi = Zc + c * nzp * ZA;
 #pragma unroll 1
 				for (int item = threadIdx.x; item < ITEMS; item += F::NT) {
 					const int u = item / P, k = F::col_of(item % P), zk = k <= H ? k : k - P;
@@ -278,8 +278,7 @@ __global__ void __launch_bounds__((Grid16<R, C>::NT), (I3Grid<R, C, RF>::CTAS)) 
 						const int a = up ? -zl : zl, b = up ? -zk : zk;
 						C w = psi1[(a < 0 ? a + N : a) * N + (b < 0 ? b + N : b)];
 						if (!up) w.y = -w.y;
-						C *z = Zi + (zl + H) * ZS + zk + H;
-						*z = cfma(w, x[(v & 3) * 4 + (v >> 2)], *z);
+						zadd_mem(Zi + (zl + H) * ZS + zk + H, w, x[(v & 3) * 4 + (v >> 2)]);
 					}
 				}
 				__syncthreads();                                 // the next chain writes rows

@@ -341,12 +341,32 @@ struct I3Units {
 	__device__ __forceinline__ bool pair(int u) const { return M > 0 && 2 * (u % per_angle()) != M - 1; }
 };
 
+// z += w y, the sums Z of both precisions: in FP64. Z is summed after the inverse
+// transform, so the rounding of an FP32 sum of many units would spread over the
+// whole velocity grid, where the energy weighs it with v^2; that of X stays where X
+// is. With Z and the last transforms (k_assemble) in FP64, N = 32, J = M = 16, FP32:
+// the energy production of Cd deviates by 2.6e-6 of the sum of |Cd| (rms of
+// 48 cells) instead of 6.3e-6, and 1000 Strang steps (mean of 8 states) by 0.9e-6 from
+// FP64 instead of 2.7e-6; term by term it was 2.7e-6 and 1.5e-6
+template <class C> __device__ __forceinline__ void zadd(double2 &z, C w, C y) {
+	z = cfma(widen(w), widen(y), z);
+}
+// the same in memory that this thread alone adds to (one order of the sums); in FP32
+// without waiting for the old value: Strang step, 32 cells at N = 64, 41.9 -> 40.0 ms,
+// 12 cells at N = 48, 8.1 -> 7.5 ms
+__device__ __forceinline__ void zadd_mem(double2 *z, double2 w, double2 y) { *z = cfma(w, y, *z); }
+__device__ __forceinline__ void zadd_mem(double2 *z, float2 w, float2 y) {
+	const double2 v = cmul(widen(w), widen(y));
+	atomicAdd(&z->x, v.x);
+	atomicAdd(&z->y, v.y);
+}
+
 template <class C> struct I3ParamsT {
 	using R = typename CT<C>::R;
 	int nchunk, nterms;                                   // nterms: terms, or units of `un` in the kernels that pair them
 	I3Units un;
-	C *zout;                                              // Z_i partials, layout given at each kernel (pairing kernels)
-	C *zscr;                                              // real forms: packed Z sums of the running cluster
+	double2 *zout;                                        // Z_i partials, layout given at each kernel (pairing kernels)
+	double2 *zscr;                                        // real forms: packed Z sums of the running cluster
 	TermRanges rg;                                        // nslots > 0: one term range per cluster
 	const double2 *src; long src_cell; int src_comp[4];   // N x N grids (FP64 state)
 	const C *Ghat; long g_cell;                           // P x P grids, G_g at Ghat + cell*g_cell + g*P*P
@@ -480,11 +500,12 @@ __global__ void __launch_bounds__(I3q<P, C>::NT, I3q<P, C>::CTAS) k_i3q(const I3
 	const int u0 = (int)((long)chunk * p.nterms / p.nchunk), u1 = (int)((long)(chunk + 1) * p.nterms / p.nchunk);
 	const R etaj = (R)(j == 0 ? 1.0 : -1.0);
 	const int zk = G::src(line);                             // the extracted column of this thread, or -1
-	C acc[8], z[4];                                          // z: the thread's four extracted rows of column zk
+	C acc[8];
+	double2 z[4];                                            // the thread's four extracted rows of column zk
 #pragma unroll
 	for (int e = 0; e < 8; e++) acc[e] = czero<C>();
 #pragma unroll
-	for (int m = 0; m < 4; m++) z[m] = czero<C>();
+	for (int m = 0; m < 4; m++) z[m] = czero();
 	// value index of the thread's m-th extracted row: T = 4: e = 0, 4 (rows below
 	// P / 4), 3, 7 (from 3P / 4 on); T = 2: e = 2 m + tau
 	auto zrow = [&](int m) { return G::src(Lp::out_pos(tau, P == 32 ? (m & 1) * 4 + (m >> 1) * 3 : 2 * m + tau)); };
@@ -583,7 +604,7 @@ __global__ void __launch_bounds__(I3q<P, C>::NT, I3q<P, C>::CTAS) k_i3q(const I3
 					C v;
 					if constexpr (P == 32) v = x[(m & 1) * 4 + (m >> 1) * 3];
 					else v = tau ? x[2 * m + 1] : x[2 * m];
-					z[m] = cfma(w, v, z[m]);
+					zadd(z[m], w, v);
 				}
 			}
 		}
@@ -594,7 +615,7 @@ __global__ void __launch_bounds__(I3q<P, C>::NT, I3q<P, C>::CTAS) k_i3q(const I3
 #pragma unroll
 	for (int e = 0; e < 8; e++) o[Lp::out_pos(tau, e)] = acc[e];
 	if (zk >= 0) {
-		C *zo = p.zout + (slot * 4 + j) * (long)NN + zk;
+		double2 *zo = p.zout + (slot * 4 + j) * (long)NN + zk;
 #pragma unroll
 		for (int m = 0; m < 4; m++) zo[zrow(m) * N] = z[m];
 	}
@@ -825,8 +846,9 @@ __global__ void __launch_bounds__(256) k_sum_slots(const SumSlotsT<C> p) {
 //         + s1 (eta2_j Wh_0 . FS4_j + 2 Wh_j . FS4_0) - d_j0 2 s1 sum_c Wh_c . FS4_c   (collision.c:95-167)
 //   Cc_j = s1 Extract(IFFT2(Zcc_j)), Cd_j = Extract(IFFT2(Zcd_j)) - eta2_j s1 Z_j
 // (Z_j: the already extracted sums of I3Units)
-// The spectra and transforms are in the working precision C; Cc and Cd are
-// widened to FP64 for the outputs.  mode 0 writes Cc and Cd; mode 1 writes
+// The inputs are in the working precision C; the sums and the inverse transforms
+// are in FP64 in both: rounding after them spreads over the whole velocity grid
+// (see zadd), before them it stays where W is.  mode 0 writes Cc and Cd; mode 1 writes
 // base + dtc (Cc + Cd + CB) in FP64 with the magnetic rotation CB of `wcur`
 // (upstream simulation.c:75-135).
 template <class C> struct AsmParamsT {
@@ -837,7 +859,7 @@ template <class C> struct AsmParamsT {
 	const C *Xp; int nx;              // [cell][nx][4][P*P] I3 partials, or null
 	TermRanges xrg;                   // xrg.nslots > 0: Xp holds [slot][4][P*P] partials of term ranges
 	bool xquad;                       // P = 128: Xp in quad order (Quad128) instead of the B layout
-	const C *Zp; int nz;              // extracted I3 sums of the opposite shifts, [slot of Xp][nz][4][N*N], or null
+	const double2 *Zp; int nz;        // extracted I3 sums of the opposite shifts, [slot of Xp][nz][4][N*N], or null
 	double s1, s2;
 	int mode;
 	double2 *out_cc, *out_cd;         // mode 0: [cell][4][N*N] (either may be null)
@@ -853,9 +875,7 @@ __device__ __forceinline__ double2 zsum(const AsmParamsT<C> &p, long cell, int j
 	double2 z = czero();
 	auto add = [&](long slot) {
 		for (int r = 0; r < p.nz; r++) {
-			const C v = p.Zp[((slot * p.nz + r) * 4 + j) * NN + q];
-			z.x += (double)v.x;
-			z.y += (double)v.y;
+			z = cadd(z, p.Zp[((slot * p.nz + r) * 4 + j) * NN + q]);
 		}
 	};
 	if (p.xrg.nslots > 0) {
@@ -870,17 +890,15 @@ __device__ __forceinline__ double2 zsum(const AsmParamsT<C> &p, long cell, int j
 
 template <int P, class C>
 __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) {
-	using G = Geo<P, C>;
-	using R = typename CT<C>::R;
+	using G = Geo<P, double2>;
 	constexpr int N = G::N, NN = N * N, PP = P * P;
 	constexpr int PER = (NN + G::NT - 1) / G::NT;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	C *S = reinterpret_cast<C *>(smem_raw), *tw = S + G::GRID;
+	double2 *S = reinterpret_cast<double2 *>(smem_raw), *tw = S + G::GRID;
 	const int j = blockIdx.x & 3;
 	const long cell = blockIdx.x >> 2;
 	init_twiddles<P>(tw);
-	const R eta2[4] = { 2, -2, -2, -2 };
-	const R s1 = (R)p.s1, s2 = (R)p.s2;
+	const double eta2[4] = { 2, -2, -2, -2 }, s1 = p.s1, s2 = p.s2;
 	const C *Wh = p.What + cell * 4 * PP;
 	double2 cc[PER], cd[PER];
 #pragma unroll
@@ -891,8 +909,8 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 		const int gi = (j % 3) + 1, hi = ((j + 1) % 3) + 1;    // j=1:(2,3) j=2:(3,1) j=3:(1,2)
 		const C *FS = p.FS + cell * 3 * PP;
 		for (int i = threadIdx.x; i < PP; i += G::NT) {
-			const C z = csub(cmul(Wh[hi * PP + i], FS[(gi - 1) * PP + i]), cmul(Wh[gi * PP + i], FS[(hi - 1) * PP + i]));
-			S[G::at(i / P, i % P)] = z;
+			S[G::at(i / P, i % P)] = csub(cmul(widen(Wh[hi * PP + i]), widen(FS[(gi - 1) * PP + i])),
+			                              cmul(widen(Wh[gi * PP + i]), widen(FS[(hi - 1) * PP + i])));
 		}
 		__syncthreads();
 		fft2_smem<P, +1>(S, tw);
@@ -900,8 +918,7 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 		for (int u = 0; u < PER; u++) {
 			const int q = threadIdx.x + u * G::NT;
 			if (q < NN) {
-				const C v = S[G::at(G::pad(q / N), G::pad(q % N))];
-				cc[u] = make_double2(p.s1 * (double)v.x, p.s1 * (double)v.y);
+				cc[u] = cscale(S[G::at(G::pad(q / N), G::pad(q % N))], s1);
 			}
 		}
 		__syncthreads();
@@ -909,41 +926,41 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 	// --- Cd ---
 	if (p.FS4 != nullptr || p.Qp != nullptr || p.Xp != nullptr) {
 		// the partial sums of all the thread's elements together (as in k_fft_full)
-		C zs[8];
+		double2 zs[8];
 #pragma unroll
-		for (int e = 0; e < 8; e++) zs[e] = czero<C>();
+		for (int e = 0; e < 8; e++) zs[e] = czero();
 		if (p.Qp != nullptr) {
 #pragma unroll 1
 			for (int ii = 0; ii < 4; ii++) {
 				const C *Q = p.Qp + ((cell * 4 + ii) * p.nq) * (long)PP + threadIdx.x;
-				C s[8];
+				double2 s[8];
 #pragma unroll
-				for (int e = 0; e < 8; e++) s[e] = czero<C>();
+				for (int e = 0; e < 8; e++) s[e] = czero();
 #pragma unroll 1
 				for (int k = 0; k < p.nq; k++)
 #pragma unroll
-					for (int e = 0; e < 8; e++) s[e] = cadd(s[e], Q[(long)k * PP + e * G::NT]);
+					for (int e = 0; e < 8; e++) s[e] = cadd(s[e], widen(Q[(long)k * PP + e * G::NT]));
 #pragma unroll
 				for (int e = 0; e < 8; e++) { zs[e].x += eta2[ii] * s[e].x; zs[e].y += eta2[ii] * s[e].y; }
 			}
 #pragma unroll
 			for (int e = 0; e < 8; e++) {
-				C h = Wh[j * PP + threadIdx.x + e * G::NT];
+				double2 h = widen(Wh[j * PP + threadIdx.x + e * G::NT]);
 				h.x = -h.x; h.y = -h.y;
-				if (j == 0) h.x += (R)1.0;
-				const C v = cmul(h, zs[e]);
+				if (j == 0) h.x += 1.0;
+				const double2 v = cmul(h, zs[e]);
 				zs[e].x = s2 * v.x;
 				zs[e].y = s2 * v.y;
 			}
 		}
 		if (p.Xp != nullptr) {
-			C s[8];
+			double2 s[8];
 #pragma unroll
-			for (int e = 0; e < 8; e++) s[e] = czero<C>();
+			for (int e = 0; e < 8; e++) s[e] = czero();
 			auto add = [&](long slot) {
 				const C *X = p.Xp + (slot * 4 + j) * (long)PP + threadIdx.x;
 #pragma unroll
-				for (int e = 0; e < 8; e++) s[e] = cadd(s[e], X[e * G::NT]);
+				for (int e = 0; e < 8; e++) s[e] = cadd(s[e], widen(X[e * G::NT]));
 			};
 			if (p.xrg.nslots > 0) {
 				const TermRanges &g = p.xrg;
@@ -960,14 +977,14 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 #pragma unroll
 		for (int e = 0; e < 8; e++) {
 			const int i = threadIdx.x + e * G::NT;
-			C z = zs[e];
+			double2 z = zs[e];
 			if (p.FS4 != nullptr) {
 				const C *F4 = p.FS4 + cell * 4 * PP;
-				C v = cadd(cscale(cmul(Wh[i], F4[j * PP + i]), eta2[j]), cscale(cmul(Wh[j * PP + i], F4[i]), (R)2.0));
+				double2 v = cadd(cscale(cmul(widen(Wh[i]), widen(F4[j * PP + i])), eta2[j]), cscale(cmul(widen(Wh[j * PP + i]), widen(F4[i])), 2.0));
 				if (j == 0) {
-					C s = czero<C>();
-					for (int c = 0; c < 4; c++) s = cadd(s, cmul(Wh[c * PP + i], F4[c * PP + i]));
-					v = csub(v, cscale(s, (R)2.0));
+					double2 s = czero();
+					for (int c = 0; c < 4; c++) s = cadd(s, cmul(widen(Wh[c * PP + i]), widen(F4[c * PP + i])));
+					v = csub(v, cscale(s, 2.0));
 				}
 				z.x += s1 * v.x; z.y += s1 * v.y;
 			}
@@ -979,8 +996,7 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 		for (int u = 0; u < PER; u++) {
 			const int q = threadIdx.x + u * G::NT;
 			if (q < NN) {
-				const C v = S[G::at(G::pad(q / N), G::pad(q % N))];
-				cd[u] = make_double2((double)v.x, (double)v.y);
+				cd[u] = S[G::at(G::pad(q / N), G::pad(q % N))];
 				if (p.Zp != nullptr) {
 					const double2 z = zsum(p, cell, j, NN, q);
 					const double f = (j == 0 ? 2.0 : -2.0) * p.s1;

@@ -665,20 +665,18 @@ __device__ __forceinline__ long quad_from_b(int h, int m, int k) { return (long)
 template <class C>
 __global__ void __launch_bounds__(512, 1) k_assemble128(const AsmParamsT<C> p) {
 	using G = G128;
-	using R = typename CT<C>::R;
 	constexpr int N = G::N, NN = N * N;
 	constexpr long PP = G::PP;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	C *S = reinterpret_cast<C *>(smem_raw), *tw128 = S + G::GRID_H, *tw64 = tw128 + 128;
+	double2 *S = reinterpret_cast<double2 *>(smem_raw), *tw128 = S + G::GRID_H, *tw64 = tw128 + 128;
 	cg::cluster_group cl = cg::this_cluster();
 	const int h = (int)cl.block_rank();
-	const C *peer = cl.map_shared_rank(S, h ^ 1);
+	const double2 *peer = cl.map_shared_rank(S, h ^ 1);
 	const long unit = blockIdx.x >> 1;
 	const int j = (int)(unit & 3);
 	const long cell = unit >> 2;
 	init_tw128(tw128, tw64);
-	const R eta2[4] = { 2, -2, -2, -2 };
-	const R s1 = (R)p.s1, s2 = (R)p.s2;
+	const double eta2[4] = { 2, -2, -2, -2 }, s1 = p.s1, s2 = p.s2;
 	const C *Wh = p.What + cell * 4 * PP;
 	double2 cc[4], cd[4];
 #pragma unroll
@@ -691,61 +689,63 @@ __global__ void __launch_bounds__(512, 1) k_assemble128(const AsmParamsT<C> p) {
 		const C *FS = p.FS + cell * 3 * PP;
 		for (int i = threadIdx.x; i < 64 * 128; i += 512) {
 			const long o = hoff + i;
-			S[(i >> 7) * G::LDP + (i & 127)] = csub(cmul(Wh[hi * PP + o], FS[(gi - 1) * PP + o]), cmul(Wh[gi * PP + o], FS[(hi - 1) * PP + o]));
+			S[(i >> 7) * G::LDP + (i & 127)] = csub(cmul(widen(Wh[hi * PP + o]), widen(FS[(gi - 1) * PP + o])),
+			                                        cmul(widen(Wh[gi * PP + o]), widen(FS[(hi - 1) * PP + o])));
 		}
 		__syncthreads();
-		C v[4];
+		double2 v[4];
 		inverse_extract(S, peer, cl, h, tw128, tw64, v);
 #pragma unroll
-		for (int u = 0; u < 4; u++) cc[u] = make_double2(p.s1 * (double)v[u].x, p.s1 * (double)v[u].y);
+		for (int u = 0; u < 4; u++) cc[u] = cscale(v[u], s1);
 	}
 	if (p.FS4 != nullptr || p.Qp != nullptr || p.Xp != nullptr) {
 		for (int i = threadIdx.x; i < 64 * 128; i += 512) {
 			const long o = hoff + i;
-			C z = czero<C>();
+			double2 z = czero();
 			if (p.Qp != nullptr) {
-				C q = czero<C>();
+				double2 q = czero();
 				for (int ii = 0; ii < 4; ii++) {
 					const C *Q = p.Qp + ((cell * 4 + ii) * p.nq) * PP + o;
-					C s = czero<C>();
-					for (int k = 0; k < p.nq; k++) s = cadd(s, Q[(long)k * PP]);
+					double2 s = czero();
+					for (int k = 0; k < p.nq; k++) s = cadd(s, widen(Q[(long)k * PP]));
 					q.x += eta2[ii] * s.x; q.y += eta2[ii] * s.y;
 				}
-				C hh; hh.x = -Wh[j * PP + o].x; hh.y = -Wh[j * PP + o].y;
-				if (j == 0) hh.x += (R)1.0;
-				const C v = cmul(hh, q);
+				double2 hh = widen(Wh[j * PP + o]);
+				hh.x = -hh.x; hh.y = -hh.y;
+				if (j == 0) hh.x += 1.0;
+				const double2 v = cmul(hh, q);
 				z.x += s2 * v.x; z.y += s2 * v.y;
 			}
 			if (p.Xp != nullptr) {
-				C s = czero<C>();
+				double2 s = czero();
 				const long xo = p.xquad ? quad_from_b(h, i >> 7, i & 127) : o;
 				if (p.xrg.nslots > 0) {
 					const TermRanges &g = p.xrg;
 					const int k0 = g.cluster_of(cell * (long)g.nterms), k1 = g.cluster_of((cell + 1) * (long)g.nterms - 1);
-					for (int k = k0; k <= k1; k++) s = cadd(s, p.Xp[(((long)k * g.maxc + (cell - g.first_cell(k))) * 4 + j) * PP + xo]);
+					for (int k = k0; k <= k1; k++) s = cadd(s, widen(p.Xp[(((long)k * g.maxc + (cell - g.first_cell(k))) * 4 + j) * PP + xo]));
 				} else {
-					for (int k = 0; k < p.nx; k++) s = cadd(s, p.Xp[((cell * p.nx + k) * 4 + j) * PP + xo]);
+					for (int k = 0; k < p.nx; k++) s = cadd(s, widen(p.Xp[((cell * p.nx + k) * 4 + j) * PP + xo]));
 				}
 				z.x -= eta2[j] * s1 * s.x; z.y -= eta2[j] * s1 * s.y;
 			}
 			if (p.FS4 != nullptr) {
 				const C *F4 = p.FS4 + cell * 4 * PP;
-				C v = cadd(cscale(cmul(Wh[o], F4[j * PP + o]), eta2[j]), cscale(cmul(Wh[j * PP + o], F4[o]), (R)2.0));
+				double2 v = cadd(cscale(cmul(widen(Wh[o]), widen(F4[j * PP + o])), eta2[j]), cscale(cmul(widen(Wh[j * PP + o]), widen(F4[o])), 2.0));
 				if (j == 0) {
-					C s = czero<C>();
-					for (int c = 0; c < 4; c++) s = cadd(s, cmul(Wh[c * PP + o], F4[c * PP + o]));
-					v = csub(v, cscale(s, (R)2.0));
+					double2 s = czero();
+					for (int c = 0; c < 4; c++) s = cadd(s, cmul(widen(Wh[c * PP + o]), widen(F4[c * PP + o])));
+					v = csub(v, cscale(s, 2.0));
 				}
 				z.x += s1 * v.x; z.y += s1 * v.y;
 			}
 			S[(i >> 7) * G::LDP + (i & 127)] = z;
 		}
 		__syncthreads();
-		C v[4];
+		double2 v[4];
 		inverse_extract(S, peer, cl, h, tw128, tw64, v);
 #pragma unroll
 		for (int u = 0; u < 4; u++) {
-			cd[u] = make_double2((double)v[u].x, (double)v[u].y);
+			cd[u] = v[u];
 			if (p.Zp != nullptr) {
 				const int idx = u * 512 + (int)threadIdx.x;
 				const double2 z = zsum(p, cell, j, NN, (32 * h + (idx >> 6)) * N + (idx & 63));

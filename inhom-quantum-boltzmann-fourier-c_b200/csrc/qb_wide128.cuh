@@ -155,8 +155,8 @@ __global__ void __launch_bounds__(512, 1) k_i3_wide128r(const I3ParamsT<float2> 
 	if (warp == 0) tmem_alloc(&tmem_slot, TM::NCOLS);
 	init_twiddles<128>(tw);
 	const long slot = cell * p.nchunk + chunk;
-	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
-	for (int i = t; i < 2 * ZA; i += 512) za[i] = czero<C>();
+	double2 *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
+	for (int i = t; i < 2 * ZA; i += 512) za[i] = czero();
 	tmem_fence_before();
 	__syncthreads();
 	tmem_fence_after();
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(512, 1) k_i3_wide128r(const I3ParamsT<float2> 
 			__syncthreads();                                 // the next chain writes rows
 			if (kc <= H || kc >= P - H) {
 				dft32<+1>(x);
-				C *A = za + c * ZA + zk + H;
+				double2 *A = za + c * ZA + zk + H;
 #pragma unroll
 				for (int v = 0; v < 32; v++) {
 					if (v > 8 && v < 24) continue;               // rows 36 .. 95
@@ -323,8 +323,7 @@ __global__ void __launch_bounds__(512, 1) k_i3_wide128r(const I3ParamsT<float2> 
 					const int a = up ? -zl : zl, b = up ? -zk : zk;
 					C w = psi1[(a < 0 ? a + N : a) * N + (b < 0 ? b + N : b)];
 					if (!up) w.y = -w.y;
-					C *z = A + (zl + H) * (N + 1);
-					*z = cfma(w, x[pos32(v)], *z);
+					zadd_mem(A + (zl + H) * (N + 1), w, x[pos32(v)]);
 				}
 			}
 		}
@@ -332,15 +331,15 @@ __global__ void __launch_bounds__(512, 1) k_i3_wide128r(const I3ParamsT<float2> 
 	}
 	// A(k) = Z_2c(k) + i Z_2c+1(k) with both parts the transforms of real grids
 	{
-		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
+		double2 *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
 		for (int i = t; i < 2 * NN; i += 512) {
 			const int c = i / NN, n = i % NN;
 			int l = n / N, k = n % N;
 			l = l < H ? l : l - N;
 			k = k < H ? k : k - N;
-			const C u = za[c * ZA + (l + H) * (N + 1) + k + H], v = za[c * ZA + (H - l) * (N + 1) + H - k];
-			zo[(long)(2 * c) * NN + n] = mk<C>(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
-			zo[(long)(2 * c + 1) * NN + n] = mk<C>(0.5f * (u.y + v.y), -0.5f * (u.x - v.x));
+			const double2 u = __ldcg(za + c * ZA + (l + H) * (N + 1) + k + H), v = __ldcg(za + c * ZA + (H - l) * (N + 1) + H - k);
+			zo[(long)(2 * c) * NN + n] = make_double2(0.5 * (u.x + v.x), 0.5 * (u.y - v.y));
+			zo[(long)(2 * c + 1) * NN + n] = make_double2(0.5 * (u.y + v.y), -0.5 * (u.x - v.x));
 		}
 	}
 #pragma unroll 1

@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(512, Occ<C>::CTAS) k_i3w(const I3ParamsT<C> p,
 		                                  : cell * p.nchunk + (int)(cid % p.nchunk);
 		const C *Wc = p.Ghat + cell * p.g_cell + t;
 		const double2 *src = p.src + cell * p.src_cell + (long)p.src_comp[j] * NN + oz;
-		C *Zo = p.zout + (slot * 2 + rank) * 4 * (long)NN + oz;
+		double2 *Zo = p.zout + (slot * 2 + rank) * 4 * (long)NN + oz;
 		{
 			const C z[4] = { czero<C>(), czero<C>(), czero<C>(), czero<C>() };
 #pragma unroll
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(512, Occ<C>::CTAS) k_i3w(const I3ParamsT<C> p,
 #pragma unroll 1
 				for (int i = g; i < 4; i += 2)
 #pragma unroll
-					for (int v = 0; v < 8; v++) Zo[i * NN + 4 * v * N] = czero<C>();
+					for (int v = 0; v < 8; v++) Zo[i * NN + 4 * v * N] = czero();
 			}
 		}
 #pragma unroll 1
@@ -361,12 +361,12 @@ __global__ void __launch_bounds__(512, Occ<C>::CTAS) k_i3w(const I3ParamsT<C> p,
 						F.inverse(y);
 						F.sync();                                // the next chain writes rows
 						if (ks >= 0) {
-							C *z = Zo + i * NN;
+							double2 *z = Zo + i * NN;
 #pragma unroll
 							for (int v = 0; v < 8; v++) {
 								C w = psi1[4 * v * N];
 								w.y = -w.y;
-								z[4 * v * N] = cfma(w, y[pos16(v < 4 ? v : v + 8)], z[4 * v * N]);
+								zadd_mem(z + 4 * v * N, w, y[pos16(v < 4 ? v : v + 8)]);
 							}
 						}
 					}
@@ -417,8 +417,8 @@ __global__ void __launch_bounds__(512, 2) k_i3wr(const I3ParamsT<float2> p, cons
 	if (warp == 0) tmem_alloc(&tmem_slot, TM::COLS);
 	init_twiddles<64>(tw);
 	const long slot = cell * p.nchunk + chunk;
-	C *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
-	for (int i = threadIdx.x; i < 2 * ZA; i += 512) za[i] = czero<C>();
+	double2 *za = p.zscr + (slot * 2 + rank) * 2 * (long)ZA;
+	for (int i = threadIdx.x; i < 2 * ZA; i += 512) za[i] = czero();
 	tmem_fence_before();
 	__syncthreads();
 	tmem_fence_after();
@@ -549,8 +549,7 @@ __global__ void __launch_bounds__(512, 2) k_i3wr(const I3ParamsT<float2> p, cons
 							const int a = up ? -zl : zl, b = up ? -zk : zk;
 							C w = ps[(a < 0 ? a + N : a) * N + (b < 0 ? b + N : b)];
 							if (!up) w.y = -w.y;
-							C *z = za + c * ZA + (zl + H) * (N + 1) + zk + H;
-							*z = cfma(w, y[pos16(v)], *z);
+							zadd_mem(za + c * ZA + (zl + H) * (N + 1) + zk + H, w, y[pos16(v)]);
 						}
 					}
 				}
@@ -560,15 +559,15 @@ __global__ void __launch_bounds__(512, 2) k_i3wr(const I3ParamsT<float2> p, cons
 	}
 	__syncthreads();                                         // za is complete
 	{
-		C *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
+		double2 *zo = p.zout + (slot * 2 + rank) * 4 * (long)NN;
 		for (int i = threadIdx.x; i < 2 * NN; i += 512) {
 			const int c = i / NN, n = i % NN;
 			int l = n / N, k = n % N;
 			l = l < H ? l : l - N;
 			k = k < H ? k : k - N;
-			const C a = za[c * ZA + (l + H) * (N + 1) + k + H], b = za[c * ZA + (H - l) * (N + 1) + H - k];
-			zo[(long)(2 * c) * NN + n] = mk<C>(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-			zo[(long)(2 * c + 1) * NN + n] = mk<C>(0.5f * (a.y + b.y), -0.5f * (a.x - b.x));
+			const double2 a = __ldcg(za + c * ZA + (l + H) * (N + 1) + k + H), b = __ldcg(za + c * ZA + (H - l) * (N + 1) + H - k);
+			zo[(long)(2 * c) * NN + n] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
+			zo[(long)(2 * c + 1) * NN + n] = make_double2(0.5 * (a.y + b.y), -0.5 * (a.x - b.x));
 		}
 	}
 	C *o = p.out + (slot * 4 + j) * (long)PP + oa;
