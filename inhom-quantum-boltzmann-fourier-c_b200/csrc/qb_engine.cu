@@ -111,37 +111,51 @@ void DevBuf::ensure(size_t n) {
 	release();
 	g_buffer_generation.fetch_add(1, std::memory_order_acq_rel);
 	QB_CUDA(cudaGetDevice(&device));
-	QB_CUDA(cudaMalloc(&p, n));
+	const cudaError_t e = cudaMalloc(&p, n);
+	if (e != cudaSuccess) {
+		p = nullptr;
+		cudaGetLastError();                      // the next launch's check must not find it again
+		QB_FAIL("cudaMalloc of " + std::to_string(n) + " bytes: " + cudaGetErrorString(e));
+	}
 	bytes = n;
 }
 
+void DevBufSet::add(DevBuf &b, size_t n) {
+	for (auto &w : want)
+		if (w.first == &b) {
+			w.second = std::max(w.second, n);
+			return;
+		}
+	want.emplace_back(&b, n);
+}
+
 void DevBufSet::reserve() {
-	bool grow = false;
-	for (auto &w : want) grow = grow || w.first->bytes < w.second;
-	if (grow) {
-		// the buffers of earlier reservations move along
-		for (DevBuf *m : members)
-			if (m->view && std::none_of(want.begin(), want.end(), [m](const auto &w) { return w.first == m; })) want.emplace_back(m, m->bytes);
-		members.clear();
-		size_t total = 0;
-		for (auto &w : want) {
-			w.second = (std::max(w.first->bytes, w.second) + 255) / 256 * 256;
-			w.first->release();
-			total += w.second;
-		}
-		whole.release();
-		whole.ensure(total);
-		char *p = static_cast<char *>(whole.p);
-		for (auto &w : want) {
-			w.first->p = p;
-			w.first->bytes = w.second;
-			w.first->device = whole.device;
-			w.first->view = true;
-			members.push_back(w.first);
-			p += w.second;
-		}
+	// the list is empty again however this ends: after a failed allocation the next
+	// evaluation, of fewer cells, asks for its own sizes alone
+	std::vector<std::pair<DevBuf *, size_t>> need;
+	need.swap(want);
+	if (std::none_of(need.begin(), need.end(), [](const auto &w) { return w.first->bytes < w.second; })) return;
+	// the buffers of earlier reservations move along
+	for (DevBuf *m : members)
+		if (m->view && std::none_of(need.begin(), need.end(), [m](const auto &w) { return w.first == m; })) need.emplace_back(m, m->bytes);
+	members.clear();
+	size_t total = 0;
+	for (auto &w : need) {
+		w.second = (std::max(w.first->bytes, w.second) + 255) / 256 * 256;
+		w.first->release();
+		total += w.second;
 	}
-	want.clear();
+	whole.release();
+	whole.ensure(total);
+	char *p = static_cast<char *>(whole.p);
+	for (auto &w : need) {
+		w.first->p = p;
+		w.first->bytes = w.second;
+		w.first->device = whole.device;
+		w.first->view = true;
+		members.push_back(w.first);
+		p += w.second;
+	}
 }
 
 void DevBuf::release() {

@@ -37,9 +37,9 @@ struct DevBuf {
 	DevBuf() = default;
 	DevBuf(const DevBuf &) = delete;
 	DevBuf &operator=(const DevBuf &) = delete;
-	DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), device(o.device), view(o.view) { o.p = nullptr; o.bytes = 0; }
+	DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), device(o.device), view(o.view) { o.p = nullptr; o.bytes = 0; o.view = false; }
 	DevBuf &operator=(DevBuf &&o) noexcept {
-		if (this != &o) { release(); p = o.p; bytes = o.bytes; device = o.device; view = o.view; o.p = nullptr; o.bytes = 0; }
+		if (this != &o) { release(); p = o.p; bytes = o.bytes; device = o.device; view = o.view; o.p = nullptr; o.bytes = 0; o.view = false; }
 		return *this;
 	}
 	void ensure(size_t n);        // grow (contents discarded)
@@ -55,8 +55,8 @@ struct DevBufSet {
 	DevBuf whole;
 	std::vector<std::pair<DevBuf *, size_t>> want;
 	std::vector<DevBuf *> members;           // every buffer that may lie in `whole`
-	void add(DevBuf &b, size_t n) { want.emplace_back(&b, n); }
-	void reserve();               // makes every added buffer as large as asked and clears the list
+	void add(DevBuf &b, size_t n);
+	void reserve();               // makes every added buffer as large as asked; clears the list, also when it throws
 };
 
 // ---- quadrature tables on the device -----------------------------------------
