@@ -1225,12 +1225,13 @@ template <class C> struct AnyRhs {
 	Workspace &ws;
 	const QuadSet &q;
 	int N, P, ncells;
+	int batch;            // cells of the whole evaluation: what the order of the sums depends on
 	long PP;
 	Plan pl;
 	int nl1;              // lines per tile of the single-tile passes
 	cudaStream_t s;
 
-	AnyRhs(Workspace &w, const QuadSet &qs, int nc, cudaStream_t st) : ws(w), q(qs), N(w.N), P(2 * w.N), ncells(nc), s(st) {
+	AnyRhs(Workspace &w, const QuadSet &qs, int nc, cudaStream_t st) : ws(w), q(qs), N(w.N), P(2 * w.N), ncells(nc), batch(nc), s(st) {
 		PP = (long)P * P;
 		pl = with_tw(make_plan(P, ws.anyn_plan));
 		// lines per tile: the workspace's knob, else QB_ANYN_LINES (read per
@@ -1273,25 +1274,27 @@ template <class C> struct AnyRhs {
 		const double mb = ws.anyn_wave_mb > 0 ? ws.anyn_wave_mb : env_mb("QB_ANYN_WAVE_MB");
 		return (mb > 0 ? mb : 64.0) * 1048576.0;
 	}
-	// terms per wave: the wave's scratch of `per_term` grids per cell for nc cells within the budget
-	int wave(int nterms, int per_term, int nc = -1) const {
-		const double per = (double)per_term * (nc < 0 ? ncells : nc) * PP * sizeof(C);
+	// terms per wave: the wave's scratch of `per_term` grids per cell within the budget
+	int wave(int nterms, int per_term) const {
+		const double per = (double)per_term * ncells * PP * sizeof(C);
 		const int nt = (int)std::max(1.0, std::floor(wave_budget() / per));
 		return std::min(nt, std::max(1, nterms));
 	}
-	// cells per wave: all of them, unless one term of the batch needs more
-	// scratch than the cap (QB_ANYN_SLICE_MB, read per call, else 4 GB); then
-	// equal slices of the batch within it.  Slices within the L2 budget were
-	// measured slower (N = 96 and 128: more, smaller launches cost more than
-	// the L2 misses they save), so the cap only bounds the scratch memory.
-	int wave_cells(int per_term) const {
-		const double mb = env_mb("QB_ANYN_SLICE_MB");
-		const double cap = (mb > 0 ? mb : 4096.0) * 1048576.0;
-		const double per = (double)per_term * PP * sizeof(C);
-		const int fit = (int)std::max(1.0, std::floor(cap / per));
-		if (fit >= ncells) return ncells;
-		const int nslices = (ncells + fit - 1) / fit;
-		return (ncells + nslices - 1) / nslices;
+	// cells of one slice of a batch (scratch_cap): per cell W^, the sums and their
+	// transforms, the partials of X and Z, the grids of the assembly, and one
+	// unit's P grids and chains or the operands of the whole-grid chains
+	int slice(int parts) const {
+		const double grid = (double)PP * sizeof(C), z = (double)(N + 1) * (N + 1) * sizeof(double2);
+		double per = 4 * grid + 8.0 * PP * sizeof(double2);
+		if (parts & RHS_CC) per += 6 * grid;
+		if (parts & RHS_CD) {
+			per += (12 + 20) * grid;
+			if (q.i3 && fused_i3(*q.i3)) per += (4.0 * grid + 16 * z) * grid_chunks(*q.i3);
+			else per += 4.0 * partials() * (grid + z);
+		}
+		const int fit = (int)std::max(1.0, std::floor(scratch_cap() / per));
+		const int k = (ncells + fit - 1) / fit;
+		return (ncells + k - 1) / k;
 	}
 
 	// kind != null: grids [cell][gpc / nsub][nsub], and the cells of kind 0
@@ -1324,8 +1327,8 @@ template <class C> struct AnyRhs {
 		p.W = W; p.w_cell = 4L * N * N; p.N = N; p.nl = nl1; p.nt = nt; p.t0 = t0; p.nsub = nsub; p.out = out; p.pl = pl;
 		return p;
 	}
-	void pad_rows(const PadRowsP<C> &p, int nc = -1) {
-		by_plan([&](auto kern) { launch(kern, "any_pad_rows", blocks((long)(nc < 0 ? ncells : nc) * p.nt * p.nsub, nl1), smem(nl1, 1), s, p); },
+	void pad_rows(const PadRowsP<C> &p) {
+		by_plan([&](auto kern) { launch(kern, "any_pad_rows", blocks((long)ncells * p.nt * p.nsub, nl1), smem(nl1, 1), s, p); },
 		        k_any_pad_rows<C, 16, 3>, k_any_pad_rows<C, 16, 6>, k_any_pad_rows<C, 16, 12>, k_any_pad_rows<C, 16, 16>,
 		        k_any_pad_rows<C, 0, 0>);
 	}
@@ -1343,29 +1346,25 @@ template <class C> struct AnyRhs {
 		const int ntask = cc ? 3 : 4;
 		Sbuf.ensure(sizeof(C) * ncells * ntask * PP);
 		QB_CUDA(cudaMemsetAsync(Sbuf.p, 0, sizeof(C) * ncells * ntask * PP, s));
-		const int cpw = wave_cells(ntask);                  // waves of terms and, if need be, slices of cells
-		const int nt = wave(t.nterms, ntask, cpw);
-		ws.wave1.ensure(sizeof(C) * (size_t)cpw * nt * ntask * PP);
+		const int nt = wave(t.nterms, ntask);               // waves of terms
+		ws.wave1.ensure(sizeof(C) * (size_t)ncells * nt * ntask * PP);
 		C *G = ws.wave1.as<C>();
-		for (int c0 = 0; c0 < ncells; c0 += cpw) {
-			const int nc = std::min(cpw, ncells - c0);
-			for (int t0 = 0; t0 < t.nterms; t0 += nt) {
-				const int n = std::min(nt, t.nterms - t0);
-				PadRowsP<C> p = pad_params(W + (long)c0 * 4 * N * N, n, t0, ntask, G);
-				for (int k = 0; k < ntask; k++) { p.comp[k] = cc ? std::min(k + 1, 3) : k; p.psel[k] = 1; }
-				p.psiA = Tabs<C>::i1_psi2(t);
-				pad_rows(p, nc);
-				I1ColsP<C> c{};
-				c.g = G; c.What = ws.What.as<C>() + (long)c0 * 4 * PP; c.N = N; c.nl = nl1; c.nt = n; c.nsub = ntask; c.fcomp = 0;
-				c.fa = cc ? -4.0 : 2.0; c.fb = cc ? 2.0 : -1.0; c.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i1_cols", blocks((long)nc * n * ntask, nl1), smem(nl1, 1), s, c); },
+		for (int t0 = 0; t0 < t.nterms; t0 += nt) {
+			const int n = std::min(nt, t.nterms - t0);
+			PadRowsP<C> p = pad_params(W, n, t0, ntask, G);
+			for (int k = 0; k < ntask; k++) { p.comp[k] = cc ? std::min(k + 1, 3) : k; p.psel[k] = 1; }
+			p.psiA = Tabs<C>::i1_psi2(t);
+			pad_rows(p);
+			I1ColsP<C> c{};
+			c.g = G; c.What = ws.What.as<C>(); c.N = N; c.nl = nl1; c.nt = n; c.nsub = ntask; c.fcomp = 0;
+			c.fa = cc ? -4.0 : 2.0; c.fb = cc ? 2.0 : -1.0; c.pl = pl;
+			by_plan([&](auto kern) { launch(kern, "any_i1_cols", blocks((long)ncells * n * ntask, nl1), smem(nl1, 1), s, c); },
 		        k_any_i1_cols<C, 16, 3>, k_any_i1_cols<C, 16, 6>, k_any_i1_cols<C, 16, 12>, k_any_i1_cols<C, 16, 16>, k_any_i1_cols<C, 0, 0>);
-				I1RowsP<C> r{};
-				r.g = G; r.S = Sbuf.as<C>() + (long)c0 * ntask * PP; r.phi = Tabs<C>::i1_phi(t); r.N = N; r.nl = nl1; r.nt = n; r.t0 = t0;
-				r.nsub = ntask; r.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i1_rows", blocks((long)nc * ntask, nl1), smem(nl1, 1), s, r); },
+			I1RowsP<C> r{};
+			r.g = G; r.S = Sbuf.as<C>(); r.phi = Tabs<C>::i1_phi(t); r.N = N; r.nl = nl1; r.nt = n; r.t0 = t0;
+			r.nsub = ntask; r.pl = pl;
+			by_plan([&](auto kern) { launch(kern, "any_i1_rows", blocks((long)ncells * ntask, nl1), smem(nl1, 1), s, r); },
 		        k_any_i1_rows<C, 16, 3>, k_any_i1_rows<C, 16, 6>, k_any_i1_rows<C, 16, 12>, k_any_i1_rows<C, 16, 16>, k_any_i1_rows<C, 0, 0>);
-			}
 		}
 		FSbuf.ensure(sizeof(C) * ncells * ntask * PP);
 		QB_CUDA(cudaMemcpyAsync(FSbuf.p, Sbuf.p, sizeof(C) * ncells * ntask * PP, cudaMemcpyDeviceToDevice, s));
@@ -1376,24 +1375,20 @@ template <class C> struct AnyRhs {
 	void i2_sums(const DevI2 &t, const double2 *W) {
 		ws.i2p.ensure(sizeof(C) * ncells * 4 * PP);
 		QB_CUDA(cudaMemsetAsync(ws.i2p.p, 0, sizeof(C) * ncells * 4 * PP, s));
-		const int cpw = wave_cells(8);                      // waves of terms and, if need be, slices of cells
-		const int nt = wave(t.nterms, 8, cpw);
-		ws.wave1.ensure(sizeof(C) * (size_t)cpw * nt * 8 * PP);
+		const int nt = wave(t.nterms, 8);                   // waves of terms
+		ws.wave1.ensure(sizeof(C) * (size_t)ncells * nt * 8 * PP);
 		C *G = ws.wave1.as<C>();
 		const int nl2 = pick_lines(P, nl1, 2, sizeof(C));
-		for (int c0 = 0; c0 < ncells; c0 += cpw) {
-			const int nc = std::min(cpw, ncells - c0);
-			for (int t0 = 0; t0 < t.nterms; t0 += nt) {
-				const int n = std::min(nt, t.nterms - t0);
-				PadRowsP<C> p = pad_params(W + (long)c0 * 4 * N * N, n, t0, 8, G);
-				for (int i = 0; i < 4; i++) { p.comp[2 * i] = i; p.psel[2 * i] = 1; p.comp[2 * i + 1] = i; p.psel[2 * i + 1] = 2; }
-				p.psiA = Tabs<C>::i2_psi1(t); p.psiB = Tabs<C>::i2_psi2(t);
-				pad_rows(p, nc);
-				I2ColsP<C> c{};
-				c.g = G; c.Q = ws.i2p.as<C>() + (long)c0 * 4 * PP; c.N = N; c.nl = nl2; c.nt = n; c.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i2_cols", blocks((long)nc * 4, nl2), smem(nl2, 2), s, c); },
+		for (int t0 = 0; t0 < t.nterms; t0 += nt) {
+			const int n = std::min(nt, t.nterms - t0);
+			PadRowsP<C> p = pad_params(W, n, t0, 8, G);
+			for (int i = 0; i < 4; i++) { p.comp[2 * i] = i; p.psel[2 * i] = 1; p.comp[2 * i + 1] = i; p.psel[2 * i + 1] = 2; }
+			p.psiA = Tabs<C>::i2_psi1(t); p.psiB = Tabs<C>::i2_psi2(t);
+			pad_rows(p);
+			I2ColsP<C> c{};
+			c.g = G; c.Q = ws.i2p.as<C>(); c.N = N; c.nl = nl2; c.nt = n; c.pl = pl;
+			by_plan([&](auto kern) { launch(kern, "any_i2_cols", blocks((long)ncells * 4, nl2), smem(nl2, 2), s, c); },
 		        k_any_i2_cols<C, 16, 3>, k_any_i2_cols<C, 16, 6>, k_any_i2_cols<C, 16, 12>, k_any_i2_cols<C, 16, 16>, k_any_i2_cols<C, 0, 0>);
-			}
 		}
 	}
 
@@ -1412,6 +1407,26 @@ template <class C> struct AnyRhs {
 		return on != 0 && (N == 24 || N == 48) && t.pairM > 0;
 	}
 
+	// chunks a cell of the whole-grid chains: as even a split of the pieces over the
+	// resident clusters as the partials are worth (X and Z of a cell and chunk, 0.9 MB in
+	// FP32 at N = 48, written and read back at HBM speed: 0.003 of a unit's 140 us).
+	// Batches beyond 512 cells split as 512 do: the slices they run in are smaller
+	int grid_chunks(const DevI3 &t) const {
+		const int res = N == 24 ? grid_resident<3>() : grid_resident<6>();
+		const int nunits = I3Units{ t.pairM }.count(t.nterms), n = std::min(batch, 512);
+		int best = 1;
+		double best_cost = 1e300;
+		for (int c = 1; c <= std::min(nunits, 64); c++) {
+			const double cost = (double)(((long)n * c + res - 1) / res) * ((nunits + c - 1) / c) + (0.15 + 0.003 * n) * c;
+			if (cost < best_cost) { best_cost = cost; best = c; }
+		}
+		return best;
+	}
+	template <int RR> static int grid_resident() {
+		constexpr bool f32 = sizeof(C) == 8;
+		return grid_clusters(k_i3g<RR, C, f32>, Grid16<RR, C>::NT, I3Grid<RR, C, f32>::SMEM);
+	}
+
 	// the whole-grid chains of every cell; returns the partials of X per (cell, j)
 	template <int RR> int i3_grid(const DevI3 &t, const double2 *W, AsmP<C> &as, const int *kind) {
 		using F = Grid16<RR, C>;
@@ -1420,14 +1435,8 @@ template <class C> struct AnyRhs {
 		p.un.M = t.pairM;
 		p.ncells = ncells;
 		p.nunits = p.un.count(t.nterms);
-		const int res = grid_clusters(k_i3g<RR, C, f32>, F::NT, I3Grid<RR, C, f32>::SMEM);
-		// chunks a cell: as even a split of the pieces over the resident clusters as
-		// the partials (X, Z written once, read by the assembly) are worth
-		double best = 1e300;
-		for (int c = 1; c <= std::min(p.nunits, 64); c++) {
-			const double cost = (double)(((long)ncells * c + res - 1) / res) * ((p.nunits + c - 1) / c) + 0.15 * c;
-			if (cost < best) { best = cost; p.nchunk = c; }
-		}
+		const int res = grid_resident<RR>();
+		p.nchunk = grid_chunks(t);
 		const int ncl = (int)std::min<long>((long)ncells * p.nchunk, res);
 		const int nang = t.nterms / t.pairM;
 		const long nw = 4L * ncells * PP;
@@ -1507,7 +1516,7 @@ template <class C> struct AnyRhs {
 	// 144 CTAs of three terms each, 40 us a launch; in four partials the step of 12 cells 12.5 -> 11.8 ms).  Three CTAs an SM; the
 	// count depends on the batch alone, so waves and slices do not change the sums
 	int partials() const {
-		const long ctas = (long)ncells * 4 * (P / nl1);
+		const long ctas = (long)batch * 4 * (P / nl1);
 		return (int)std::max(1L, std::min(8L, (3 * 148 + ctas - 1) / ctas));
 	}
 
@@ -1538,21 +1547,20 @@ template <class C> struct AnyRhs {
 
 	// the terms of the opposite shifts of a wave: rows of Y_i (into V, the P grids'
 	// place), columns into Z
-	void other_terms(const DevI3 &t, const C *What, const C *Y, C *V, double2 *Z, int nc, int n, int t0, const int *kc) {
+	void other_terms(const DevI3 &t, const C *What, const C *Y, C *V, double2 *Z, int n, int t0, const int *kind) {
 		I3RowsYP<C> y{};
-		y.What = What; y.Y = Y; y.V = V; y.N = N; y.nl = nl1; y.nt = n; y.t0 = t0; y.un.M = t.pairM; y.kind = kc; y.pl = pl;
-		by_plan([&](auto kern) { launch(kern, "any_i3_rows_y", blocks((long)nc * n * 4, nl1), smem(nl1, 1), s, y); },
+		y.What = What; y.Y = Y; y.V = V; y.N = N; y.nl = nl1; y.nt = n; y.t0 = t0; y.un.M = t.pairM; y.kind = kind; y.pl = pl;
+		by_plan([&](auto kern) { launch(kern, "any_i3_rows_y", blocks((long)ncells * n * 4, nl1), smem(nl1, 1), s, y); },
 		        k_any_i3_rows_y<C, 16, 3>, k_any_i3_rows_y<C, 16, 6>, k_any_i3_rows_y<C, 16, 12>, k_any_i3_rows_y<C, 16, 16>,
 		        k_any_i3_rows_y<C, 0, 0>);
 		I3ColsZP<C> z{};
-		z.V = V; z.Z = Z; z.psi1 = Tabs<C>::i3_psi1(t); z.ns = partials(); z.N = N; z.nl = nl1; z.nt = n; z.t0 = t0; z.un.M = t.pairM; z.kind = kc; z.pl = pl;
-		by_plan([&](auto kern) { launch(kern, "any_i3_cols_z", (long)nc * 4 * z.ns * ((N + nl1) / nl1), smem(nl1, 1), s, z); },
+		z.V = V; z.Z = Z; z.psi1 = Tabs<C>::i3_psi1(t); z.ns = partials(); z.N = N; z.nl = nl1; z.nt = n; z.t0 = t0; z.un.M = t.pairM; z.kind = kind; z.pl = pl;
+		by_plan([&](auto kern) { launch(kern, "any_i3_cols_z", (long)ncells * 4 * z.ns * ((N + nl1) / nl1), smem(nl1, 1), s, z); },
 		        k_any_i3_cols_z<C, 16, 3>, k_any_i3_cols_z<C, 16, 6>, k_any_i3_cols_z<C, 16, 12>, k_any_i3_cols_z<C, 16, 16>,
 		        k_any_i3_cols_z<C, 0, 0>);
 	}
 
-	// the I3 chains in waves of terms and, where one term of the batch
-	// overflows the scratch cap, slices of cells.  Per (cell, term): 4 grids
+	// the I3 chains in waves of terms.  Per (cell, term): 4 grids
 	// of Pg (P_0..P_3, or the packed P_0 + i P_1, P_2 + i P_3 of the real
 	// form) and 16 chains (8 in the real form).  A cell's terms still run in
 	// order, so the sums do not depend on the waves.
@@ -1561,47 +1569,41 @@ template <class C> struct AnyRhs {
 		const WaveUnits un{ t.pairM };
 		const int nunits = pairs ? t.nterms / t.pairM * ((t.pairM + 1) / 2) : t.nterms;
 		const int per_term = 20;
-		const int cpw = wave_cells(per_term);
-		const int nt = wave(nunits, per_term, cpw);
-		ws.wave1.ensure(sizeof(C) * (size_t)cpw * nt * 4 * PP);                // P_j, then the rows of Y_i
-		ws.wave2.ensure(sizeof(C) * (size_t)cpw * nt * 16 * PP);   // chains
+		const int nt = wave(nunits, per_term);
+		ws.wave1.ensure(sizeof(C) * (size_t)ncells * nt * 4 * PP);                // P_j, then the rows of Y_i
+		ws.wave2.ensure(sizeof(C) * (size_t)ncells * nt * 16 * PP);   // chains
 		C *Pg = ws.wave1.as<C>(), *Y = ws.wave2.as<C>();
 		int nl4 = nl1;                                      // one tile, at most kOwn elements a thread
 		const int own = own_for_plan(pl, sizeof(C) == 16);
 		while (nl4 > 1 && (nl4 * P > own * kThreads || P % nl4)) nl4--;
-		for (int c0 = 0; c0 < ncells; c0 += cpw) {
-			const int nc = std::min(cpw, ncells - c0);
-			const double2 *Wc = W + (long)c0 * 4 * N * N;
-			const C *What = ws.What.as<C>() + (long)c0 * 4 * PP;
-			C *X = ws.i3p.as<C>() + (long)c0 * 4 * nxp * PP;
-			const int *kc = kind ? kind + c0 : nullptr;
-			for (int t0 = 0; t0 < nunits; t0 += nt) {
-				const int n = std::min(nt, nunits - t0);
-				PadRowsP<C> p = pad_params(Wc, n, t0, 4, Pg);
-				for (int g = 0; g < 4; g++) { p.comp[g] = g; p.comp2[g] = g; p.psel[g] = 3; }
-				p.kind = kc; p.nsub_rf = 2;
-				for (int g = 0; g < 2; g++) { p.comp_rf[g] = 2 * g; p.comp2_rf[g] = 2 * g + 1; p.psel_rf[g] = 4; }
-				p.psiC = Tabs<C>::i3_psi1(t); p.un = un;
-				pad_rows(p, nc);
-				plain(Pg, (long)nc * n * 4, -1, true, kc, (long)n * 4, 4, 2, true);
-				I3RowsAP<C> a{};
-				a.What = What; a.Pg = Pg; a.Y = Y; a.N = N; a.nl = nl1; a.nt = n; a.kind = kc; a.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i3_rows_a", blocks((long)nc * n * 16, nl1), smem(nl1, 1), s, a); },
-				        k_any_i3_rows_a<C, 16, 3>, k_any_i3_rows_a<C, 16, 6>, k_any_i3_rows_a<C, 16, 12>, k_any_i3_rows_a<C, 16, 16>,
-				        k_any_i3_rows_a<C, 0, 0>);
-				I3ColsP<C> c{};
-				c.Y = Y; c.psi2T = Tabs<C>::i3_psi2T(t); c.idx = t.idx.as<int>(); c.scale = t.scale.as<double>();
-				c.N = N; c.nl = nl1; c.nt = n; c.t0 = t0; c.kind = kc; c.un = un; c.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i3_cols", blocks((long)nc * n * 16, nl1), smem(nl1, 1), s, c); },
-				        k_any_i3_cols<C, 16, 3>, k_any_i3_cols<C, 16, 6>, k_any_i3_cols<C, 16, 12>, k_any_i3_cols<C, 16, 16>,
-				        k_any_i3_cols<C, 0, 0>);
-				I3RowsBP<C> b{};
-				b.Y = Y; b.Pg = Pg; b.X = X; b.ns = nxp; b.N = N; b.nl = nl4; b.nt = n; b.t0 = t0; b.kind = kc; b.un = un; b.pl = pl;
-				by_plan([&](auto kern) { launch(kern, "any_i3_rows_b", blocks((long)nc * 4 * nxp, nl4), smem(nl4, 1), s, b); },
-				        k_any_i3_rows_b<C, 16, 3>, k_any_i3_rows_b<C, 16, 6>, k_any_i3_rows_b<C, 16, 12>,
-				        k_any_i3_rows_b<C, 16, 16>, k_any_i3_rows_b<C, 0, 0>);
-				if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<double2>() + (long)c0 * 4 * partials() * (N + 1) * (N + 1), nc, n, t0, kc);
-			}
+		const C *What = ws.What.as<C>();
+		C *X = ws.i3p.as<C>();
+		for (int t0 = 0; t0 < nunits; t0 += nt) {
+			const int n = std::min(nt, nunits - t0);
+			PadRowsP<C> p = pad_params(W, n, t0, 4, Pg);
+			for (int g = 0; g < 4; g++) { p.comp[g] = g; p.comp2[g] = g; p.psel[g] = 3; }
+			p.kind = kind; p.nsub_rf = 2;
+			for (int g = 0; g < 2; g++) { p.comp_rf[g] = 2 * g; p.comp2_rf[g] = 2 * g + 1; p.psel_rf[g] = 4; }
+			p.psiC = Tabs<C>::i3_psi1(t); p.un = un;
+			pad_rows(p);
+			plain(Pg, (long)ncells * n * 4, -1, true, kind, (long)n * 4, 4, 2, true);
+			I3RowsAP<C> a{};
+			a.What = What; a.Pg = Pg; a.Y = Y; a.N = N; a.nl = nl1; a.nt = n; a.kind = kind; a.pl = pl;
+			by_plan([&](auto kern) { launch(kern, "any_i3_rows_a", blocks((long)ncells * n * 16, nl1), smem(nl1, 1), s, a); },
+			        k_any_i3_rows_a<C, 16, 3>, k_any_i3_rows_a<C, 16, 6>, k_any_i3_rows_a<C, 16, 12>, k_any_i3_rows_a<C, 16, 16>,
+			        k_any_i3_rows_a<C, 0, 0>);
+			I3ColsP<C> c{};
+			c.Y = Y; c.psi2T = Tabs<C>::i3_psi2T(t); c.idx = t.idx.as<int>(); c.scale = t.scale.as<double>();
+			c.N = N; c.nl = nl1; c.nt = n; c.t0 = t0; c.kind = kind; c.un = un; c.pl = pl;
+			by_plan([&](auto kern) { launch(kern, "any_i3_cols", blocks((long)ncells * n * 16, nl1), smem(nl1, 1), s, c); },
+			        k_any_i3_cols<C, 16, 3>, k_any_i3_cols<C, 16, 6>, k_any_i3_cols<C, 16, 12>, k_any_i3_cols<C, 16, 16>,
+			        k_any_i3_cols<C, 0, 0>);
+			I3RowsBP<C> b{};
+			b.Y = Y; b.Pg = Pg; b.X = X; b.ns = nxp; b.N = N; b.nl = nl4; b.nt = n; b.t0 = t0; b.kind = kind; b.un = un; b.pl = pl;
+			by_plan([&](auto kern) { launch(kern, "any_i3_rows_b", blocks((long)ncells * 4 * nxp, nl4), smem(nl4, 1), s, b); },
+			        k_any_i3_rows_b<C, 16, 3>, k_any_i3_rows_b<C, 16, 6>, k_any_i3_rows_b<C, 16, 12>,
+			        k_any_i3_rows_b<C, 16, 16>, k_any_i3_rows_b<C, 0, 0>);
+			if (pairs) other_terms(t, What, Y, Pg, ws.i3z.as<double2>(), n, t0, kind);
 		}
 	}
 
@@ -1638,19 +1640,29 @@ template <class C> struct AnyRhs {
 
 template <class C>
 void any_operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *cc, double2 *cd, cudaStream_t s) {
-	AnyRhs<C> r(ws, q, ncells, s);
-	AsmP<C> a = r.prepare(W, parts);
-	a.mode = 0; a.out_cc = cc; a.out_cd = cd;
-	r.assemble(a);
+	const int per = AnyRhs<C>(ws, q, ncells, s).slice(parts);
+	for (int c0 = 0; c0 < ncells; c0 += per) {
+		const long o = 4L * ws.N * ws.N * c0;
+		AnyRhs<C> r(ws, q, std::min(per, ncells - c0), s);
+		r.batch = ncells;
+		AsmP<C> a = r.prepare(W + o, parts);
+		a.mode = 0; a.out_cc = cc ? cc + o : nullptr; a.out_cd = cd ? cd + o : nullptr;
+		r.assemble(a);
+	}
 }
 
 template <class C>
 void any_update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc,
                 double2 *out, cudaStream_t s) {
-	AnyRhs<C> r(ws, q, ncells, s);
-	AsmP<C> a = r.prepare(wcur, RHS_ALL);
-	a.mode = 1; a.base = base; a.wcur = wcur; a.B = B; a.dtc = dtc; a.out = out;
-	r.assemble(a);
+	const int per = AnyRhs<C>(ws, q, ncells, s).slice(RHS_ALL);
+	for (int c0 = 0; c0 < ncells; c0 += per) {
+		const long o = 4L * ws.N * ws.N * c0;
+		AnyRhs<C> r(ws, q, std::min(per, ncells - c0), s);
+		r.batch = ncells;
+		AsmP<C> a = r.prepare(wcur + o, RHS_ALL);
+		a.mode = 1; a.base = base ? base + o : nullptr; a.wcur = wcur + o; a.B = B ? B + 3 * c0 : nullptr; a.dtc = dtc; a.out = out + o;
+		r.assemble(a);
+	}
 }
 
 unsigned grid1d(long n) { return (unsigned)std::min<long>((n + 255) / 256, 148L * 16); }

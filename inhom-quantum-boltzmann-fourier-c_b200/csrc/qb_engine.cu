@@ -129,6 +129,18 @@ void DevBufSet::add(DevBuf &b, size_t n) {
 	want.emplace_back(&b, n);
 }
 
+size_t DevBufSet::wanted() const {
+	size_t n = 0;
+	for (const auto &w : want) n += w.second;
+	return n;
+}
+
+double scratch_cap() {
+	const char *e = getenv("QB_ANYN_SLICE_MB");
+	const double mb = e != nullptr ? atof(e) : 0.0;
+	return (mb > 0 ? mb : 4096.0) * 1048576.0;
+}
+
 void DevBufSet::reserve() {
 	// the list is empty again however this ends: after a failed allocation the next
 	// evaluation, of fewer cells, asks for its own sizes alone
@@ -301,6 +313,12 @@ int best_chunks(long units, int nterms, int slots, int max_chunks, double penalt
 	}
 	return best;
 }
+
+// the price of one more I3 partial a cell, in times of a unit on a cluster: 0.15 for
+// its part in the sums of a cell, and for every cell its grids (X and Z) written and
+// read back at HBM speed: 0.26 and 1.05 MB at N = 32 and 64 in FP32 against units of 40
+// and 90 us (0.002 and 0.0036), 80 KB at N = 16 in FP64 against 70 us (0.0004)
+double i3_partial(int N, int ncells) { return 0.15 + (N >= 32 ? 0.003 : 0.0004) * ncells; }
 
 template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C *out, cudaStream_t s, C *out2 = nullptr, float *outr = nullptr) {
 	static DeviceFlag init;
@@ -613,6 +631,27 @@ int resident_i3(int N, bool f32) {
 	}
 }
 
+// An evaluation runs over slices of its cells whose scratch keeps within the cap
+// (scratch_cap): most kernels leave a partial a (cell, chunk), so the scratch
+// of a batch grows with its cells, and no batch that its caller can hold may
+// fail for want of scratch. Slices of that size fill the GPU many times over.
+// Returns the cells of the next slice of `ncells` left, with its chunks in ch and
+// its buffers in ws.scratch, not reserved yet.
+template <class Rhs>
+int next_slice(Workspace &ws, const QuadSet &q, int ncells, int parts, Chunks &ch) {
+	const double cap = scratch_cap();
+	long k = 1;
+	for (int n = ncells;;) {
+		ch = Rhs::chunks(ws, q, n);
+		ws.scratch.want.clear();
+		Rhs::want(ws, q, n, ch, parts);
+		const double bytes = (double)ws.scratch.wanted();
+		if (bytes <= cap || n == 1) return n;
+		k = std::max(k + 1, (long)std::min((double)ncells, k * (bytes / cap)));
+		n = (int)((ncells + k - 1) / k);
+	}
+}
+
 template <int P, class C> struct Rhs {
 	static constexpr int N = P / 2;
 	static constexpr long NN = (long)N * N, PP = (long)P * P;
@@ -746,7 +785,7 @@ template <int P, class C> struct Rhs {
 	}
 
 	// the scratch of one evaluation in one allocation (each user's ensure finds it there)
-	static void reserve(Workspace &ws, const QuadSet &q, int ncells, const Chunks &ch, int parts) {
+	static void want(Workspace &ws, const QuadSet &q, int ncells, const Chunks &ch, int parts) {
 		DevBufSet &b = ws.scratch;
 		const size_t g = sizeof(C) * (size_t)ncells * PP;
 		b.add(ws.What, 4 * g);
@@ -775,15 +814,13 @@ template <int P, class C> struct Rhs {
 				if (pairs_units(ws)) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
 			}
 		}
-		b.reserve();
 	}
 
-	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, Chunks &ch, cudaStream_t s) {
-		T::prepare(q, s);
-		ch = pick_chunks(N, ncells, q, (int)(8 * sizeof(typename CT<C>::R)), q.i3 ? i3_count(ws, *q.i3) : 0);
+	static Chunks chunks(const Workspace &ws, const QuadSet &q, int ncells) {
+		Chunks ch = pick_chunks(N, ncells, q, (int)(8 * sizeof(typename CT<C>::R)), q.i3 ? i3_count(ws, *q.i3) : 0);
 		if (P == 32 && sizeof(C) == 8 && ws.i3_variant == 1 && q.i3) {
 			check_tmem_coresidency();
-			ch.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), num_sms(), 256, 0.15);      // one CTA per SM
+			ch.i3 = best_chunks((long)ncells, std::max(1, q.i3->nterms), num_sms(), 256, i3_partial(N, ncells));      // one CTA per SM
 		}
 		scale_chunks(ws, q, ch, q.i3 ? i3_count(ws, *q.i3) : 0);
 		// FP64 at N = 32: every resident cluster of k_i3w takes one contiguous range
@@ -791,7 +828,11 @@ template <int P, class C> struct Rhs {
 		const bool ranges = ws.i3_ranges >= 0 ? ws.i3_ranges == 1 : term_ranges_enabled();
 		if (P == 64 && sizeof(C) == 16 && q.i3 && q.i3->nterms > 0 && ranges)
 			ch.i3_slots = (int)std::min<long>(active_i3w_clusters<C>(), (long)ncells * i3_count(ws, *q.i3));
-		reserve(ws, q, ncells, ch, parts);
+		return ch;
+	}
+
+	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, const Chunks &ch, cudaStream_t s) {
+		ws.scratch.reserve();
 		spectra(ws, ncells, W, s);
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
 		const cudaStream_t s2 = small ? ws.fork(s, 0) : s;
@@ -822,19 +863,29 @@ template <int P, class C> struct Rhs {
 	}
 
 	static void operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *cc, double2 *cd, cudaStream_t s) {
-		Chunks ch;
-		prepare(ws, q, ncells, W, parts, ch, s);
-		AsmParamsT<C> a = asm_params(ws, parts, ch, q, ncells, s);
-		a.mode = 0; a.out_cc = cc; a.out_cd = cd;
-		launch_assemble<P>(a, ncells, s);
+		T::prepare(q, s);
+		for (int c0 = 0, n; c0 < ncells; c0 += n) {
+			const long o = 4 * NN * c0;
+			Chunks ch;
+			n = next_slice<Rhs>(ws, q, ncells - c0, parts, ch);
+			prepare(ws, q, n, W + o, parts, ch, s);
+			AsmParamsT<C> a = asm_params(ws, parts, ch, q, n, s);
+			a.mode = 0; a.out_cc = cc ? cc + o : nullptr; a.out_cd = cd ? cd + o : nullptr;
+			launch_assemble<P>(a, n, s);
+		}
 	}
 
 	static void update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc, double2 *out, cudaStream_t s) {
-		Chunks ch;
-		prepare(ws, q, ncells, wcur, RHS_ALL, ch, s);
-		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, ncells, s);
-		a.mode = 1; a.base = base; a.wcur = wcur; a.B = B; a.dtc = dtc; a.out = out;
-		launch_assemble<P>(a, ncells, s);
+		T::prepare(q, s);
+		for (int c0 = 0, n; c0 < ncells; c0 += n) {
+			const long o = 4 * NN * c0;
+			Chunks ch;
+			n = next_slice<Rhs>(ws, q, ncells - c0, RHS_ALL, ch);
+			prepare(ws, q, n, wcur + o, RHS_ALL, ch, s);
+			AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, n, s);
+			a.mode = 1; a.base = base ? base + o : nullptr; a.wcur = wcur + o; a.B = B ? B + 3 * c0 : nullptr; a.dtc = dtc; a.out = out + o;
+			launch_assemble<P>(a, n, s);
+		}
 	}
 };
 
@@ -1247,8 +1298,8 @@ template <class C> struct Rhs<128, C> {
 		}
 	}
 
-	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, Chunks &ch, cudaStream_t s) {
-		T::prepare(q, s);
+	static Chunks chunks(const Workspace &ws, const QuadSet &q, int ncells) {
+		Chunks ch;
 		const int pairs = std::max(1, num_sms() / 2);
 		if (q.i1) ch.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), pairs, 64, 0.15);
 		if (q.i2) ch.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), pairs, 64, 0.15);
@@ -1257,41 +1308,48 @@ template <class C> struct Rhs<128, C> {
 				if (q.i3->nterms > 0) ch.i3_slots = (int)std::min<long>(active_quad_clusters(), (long)ncells * i3_count(*q.i3));
 			}
 			const int act = sizeof(C) == 16 ? 1 : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
-			ch.i3 = best_chunks((long)ncells, std::max(1, i3_count(*q.i3)), act, 256, 0.15);
+			ch.i3 = best_chunks((long)ncells, std::max(1, i3_count(*q.i3)), act, 256, i3_partial(N, ncells));
 		}
 		scale_chunks(ws, q, ch, q.i3 ? i3_count(*q.i3) : 0);
-		{
-			DevBufSet &b = ws.scratch;
-			const size_t g = sizeof(C) * (size_t)ncells * PP;
-			b.add(ws.What, 4 * g);
-			if (q.i3 && (sizeof(C) == 16 || use_real_form())) b.add(ws.WhatQ, wide_bytes(*q.i3, ncells));
-			if (parts & RHS_CC) {
-				b.add(ws.i1cc, 3 * ch.i1 * g);
-				b.add(ws.fs, 3 * g);
-			}
-			if (parts & RHS_CD) {
-				b.add(ws.i1i4, 4 * ch.i1 * g);
-				b.add(ws.fs4, 4 * g);
-				b.add(ws.i2p, 4 * ch.i2 * g);
-				b.add(ws.scr128b, 4 * ch.i2 * g);
-				size_t slots = (size_t)ncells * ch.i3, used = slots;
-				if (ch.i3_slots > 0) {
-					const TermRanges r = term_ranges(ch.i3_slots, i3_count(*q.i3), ncells);
-					slots = (size_t)r.nslots * r.maxc;
-					used = r.nslots;
-				}
-				b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
-				b.add(ws.scr128a, sizeof(C) * used * 4 * PP);
-				if (pairs_units()) b.add(ws.i3z, sizeof(double2) * slots * kZRanks * 4 * NN);
-				if (sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 4 * PP);
-				else if (use_full128()) b.add(ws.i3y, sizeof(C) * used * 2 * PP);
-				if (used >= (size_t)kSumSlots * ncells) {
-					b.add(ws.i3s, 4 * g);
-					if (pairs_units()) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
-				}
-			}
-			b.reserve();
+		return ch;
+	}
+
+	// the scratch of one evaluation in one allocation (each user's ensure finds it there)
+	static void want(Workspace &ws, const QuadSet &q, int ncells, const Chunks &ch, int parts) {
+		DevBufSet &b = ws.scratch;
+		const size_t g = sizeof(C) * (size_t)ncells * PP;
+		b.add(ws.What, 4 * g);
+		if (q.i3 && (sizeof(C) == 16 || use_real_form())) b.add(ws.WhatQ, wide_bytes(*q.i3, ncells));
+		if (parts & RHS_CC) {
+			b.add(ws.i1cc, 3 * ch.i1 * g);
+			b.add(ws.fs, 3 * g);
 		}
+		if (parts & RHS_CD) {
+			b.add(ws.i1i4, 4 * ch.i1 * g);
+			b.add(ws.fs4, 4 * g);
+			b.add(ws.i2p, 4 * ch.i2 * g);
+			b.add(ws.scr128b, 4 * ch.i2 * g);
+			size_t slots = (size_t)ncells * ch.i3, used = slots;
+			if (ch.i3_slots > 0) {
+				const TermRanges r = term_ranges(ch.i3_slots, i3_count(*q.i3), ncells);
+				slots = (size_t)r.nslots * r.maxc;
+				used = r.nslots;
+			}
+			b.add(ws.i3p, sizeof(C) * slots * 4 * PP);
+			b.add(ws.scr128a, sizeof(C) * used * 4 * PP);
+			if (pairs_units()) b.add(ws.i3z, sizeof(double2) * slots * kZRanks * 4 * NN);
+			if (sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 4 * PP);
+			else if (use_full128()) b.add(ws.i3y, sizeof(C) * used * 2 * PP);
+			if (sizeof(C) == 8 && use_real_form()) b.add(ws.i3zs, sizeof(double2) * used * 2 * 2 * (N + 1) * (N + 1));
+			if (used >= (size_t)kSumSlots * ncells) {
+				b.add(ws.i3s, 4 * g);
+				if (pairs_units()) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
+			}
+		}
+	}
+
+	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, const Chunks &ch, cudaStream_t s) {
+		ws.scratch.reserve();
 		spectra(ws, ncells, W, s);
 		const int act = sizeof(C) == 16 ? active_quad_clusters() : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(*q.i3) < kForkUnits * act;
@@ -1323,19 +1381,29 @@ template <class C> struct Rhs<128, C> {
 	}
 
 	static void operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *cc, double2 *cd, cudaStream_t s) {
-		Chunks ch;
-		prepare(ws, q, ncells, W, parts, ch, s);
-		AsmParamsT<C> a = asm_params(ws, parts, ch, q, ncells, s);
-		a.mode = 0; a.out_cc = cc; a.out_cd = cd;
-		launch_assemble128(a, ncells, s);
+		T::prepare(q, s);
+		for (int c0 = 0, n; c0 < ncells; c0 += n) {
+			const long o = 4 * NN * c0;
+			Chunks ch;
+			n = next_slice<Rhs>(ws, q, ncells - c0, parts, ch);
+			prepare(ws, q, n, W + o, parts, ch, s);
+			AsmParamsT<C> a = asm_params(ws, parts, ch, q, n, s);
+			a.mode = 0; a.out_cc = cc ? cc + o : nullptr; a.out_cd = cd ? cd + o : nullptr;
+			launch_assemble128(a, n, s);
+		}
 	}
 
 	static void update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc, double2 *out, cudaStream_t s) {
-		Chunks ch;
-		prepare(ws, q, ncells, wcur, RHS_ALL, ch, s);
-		AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, ncells, s);
-		a.mode = 1; a.base = base; a.wcur = wcur; a.B = B; a.dtc = dtc; a.out = out;
-		launch_assemble128(a, ncells, s);
+		T::prepare(q, s);
+		for (int c0 = 0, n; c0 < ncells; c0 += n) {
+			const long o = 4 * NN * c0;
+			Chunks ch;
+			n = next_slice<Rhs>(ws, q, ncells - c0, RHS_ALL, ch);
+			prepare(ws, q, n, wcur + o, RHS_ALL, ch, s);
+			AsmParamsT<C> a = asm_params(ws, RHS_ALL, ch, q, n, s);
+			a.mode = 1; a.base = base ? base + o : nullptr; a.wcur = wcur + o; a.B = B ? B + 3 * c0 : nullptr; a.dtc = dtc; a.out = out + o;
+			launch_assemble128(a, n, s);
+		}
 	}
 };
 
@@ -1391,9 +1459,7 @@ Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) 
 	const int c2 = !c.wide12 || prec == 32 ? 1 : Terms64<double2>::CTAS;
 	if (q.i1) c.i1 = best_chunks((long)ncells * 7, std::max(1, q.i1->nterms), sms * c1, 64);
 	if (q.i2) c.i2 = best_chunks((long)ncells * 4, std::max(1, q.i2->nterms), sms * c2, 64);
-	// an I3 partial is 4 padded grids per cluster (256 KB at N = 32) written
-	// and read back at HBM speed; a unit takes a cluster tens of us: 0.15
-	if (q.i3) c.i3 = best_chunks((long)ncells, std::max(1, i3_units), resident_i3(N, prec == 32), 256, 0.15);
+	if (q.i3) c.i3 = best_chunks((long)ncells, std::max(1, i3_units), resident_i3(N, prec == 32), 256, i3_partial(N, ncells));
 	return c;
 }
 

@@ -56,8 +56,12 @@ struct DevBufSet {
 	std::vector<std::pair<DevBuf *, size_t>> want;
 	std::vector<DevBuf *> members;           // every buffer that may lie in `whole`
 	void add(DevBuf &b, size_t n);
+	size_t wanted() const;        // bytes on the list
 	void reserve();               // makes every added buffer as large as asked; clears the list, also when it throws
 };
+
+// bytes of scratch that one slice of an evaluation may take: QB_ANYN_SLICE_MB (read per call), else 4 GB
+double scratch_cap();
 
 // ---- quadrature tables on the device -----------------------------------------
 // I1-type (I1 and I4):  S = sum_t phi_t . IFFT2(F . FFT2(Pad(psi2_t . g)))
