@@ -1467,12 +1467,14 @@ void prepare_f32_tables(const QuadSet &q, cudaStream_t s) { Tab<float2>::prepare
 
 void collision_operators(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, double2 *out_cc, double2 *out_cd, cudaStream_t s) {
 	if (anyn_route(ws.N)) { anyn_operators(ws, q, ncells, W, parts, out_cc, out_cd, s); return; }
+	if (ncells < 1) QB_FAIL("collision operator: at least one cell");
 	if (ws.prec == 32) by_n<OpsRun<float2>::F>(ws.N, ws, q, ncells, W, parts, out_cc, out_cd, s);
 	else by_n<OpsRun<double2>::F>(ws.N, ws, q, ncells, W, parts, out_cc, out_cd, s);
 }
 
 void collision_update(Workspace &ws, const QuadSet &q, int ncells, const double2 *base, const double2 *wcur, const double *B, double dtc, double2 *out, cudaStream_t s) {
 	if (anyn_route(ws.N)) { anyn_update(ws, q, ncells, base, wcur, B, dtc, out, s); return; }
+	if (ncells < 1) QB_FAIL("collision operator: at least one cell");
 	if (ws.prec == 32) by_n<UpdRun<float2>::F>(ws.N, ws, q, ncells, base, wcur, B, dtc, out, s);
 	else by_n<UpdRun<double2>::F>(ws.N, ws, q, ncells, base, wcur, B, dtc, out, s);
 }
