@@ -1517,7 +1517,7 @@ template <class C> struct AnyRhs {
 	// count depends on the batch alone, so waves and slices do not change the sums
 	int partials() const {
 		const long ctas = (long)batch * 4 * (P / nl1);
-		return (int)std::max(1L, std::min(8L, (3 * 148 + ctas - 1) / ctas));
+		return (int)std::max(1L, std::min(8L, (3 * num_sms() + ctas - 1) / ctas));
 	}
 
 	// returns the partials of X per (cell, j).  FP32: the cells of kind 0 (no

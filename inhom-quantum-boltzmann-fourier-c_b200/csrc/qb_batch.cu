@@ -133,22 +133,21 @@ Sched autotune(qb::Workspace &ws, const qb::Quad &q, int N, int prec, int g, con
 	std::vector<Sched> cand(1);
 	if (qb::anyn_route(N)) {
 		// the any-N engine: radix schedules (fewest stages, radix 8 first, radix 3
-		// first, radix 4 only), tile heights (lines per tile), wave budgets, and the
-		// three-pass I3 chains against the whole-grid ones (both forced; the
-		// default picks by precision)
+		// first, radix 4 only), tile heights (lines per tile), wave budgets, and at
+		// N = 24 and 48 the three-pass I3 chains against the whole-grid ones, the
+		// default there
 		// (the engine's defaults: tiles of about 4096 elements in FP32, 2048 in
 		// FP64; a 64 MB wave budget)
 		const int P = 2 * N, dl = std::max(1, (prec == 32 ? 4096 : 2048) / P);
 		for (int v : { 1, 2, 3 }) { Sched c; c.plan = v; cand.push_back(c); }
 		for (int nl : { dl / 2, 2 * dl }) if (nl >= 1 && nl <= P) { Sched c; c.lines = nl; cand.push_back(c); }
 		for (float mb : { 24.0f, 128.0f }) { Sched c; c.wave_mb = mb; cand.push_back(c); }
-		for (int f : { 0, 1 }) { Sched c; c.fused = f; cand.push_back(c); }
+		if (N == 24 || N == 48) { Sched c; c.fused = 0; cand.push_back(c); }
 	} else {
-		cand.resize(5);
-		cand[1].s12 = 0.5f;
-		cand[2].s12 = 2.0f;
-		cand[3].s3 = 0.5f;
-		cand[4].s3 = 2.0f;
+		for (float f : { 0.5f, 2.0f }) { Sched c; c.s12 = f; cand.push_back(c); }
+		// the I3 sums in FP64 at N = 32 and 64 run as term ranges, without chunks
+		if (prec == 32 || N < 32)
+			for (float f : { 0.5f, 2.0f }) { Sched c; c.s3 = f; cand.push_back(c); }
 		if (N == 32 && prec == 64) { Sched c; c.ranges = 0; cand.push_back(c); }
 		if (N == 16 && prec == 32) { Sched c; c.variant = 1; cand.push_back(c); }
 	}

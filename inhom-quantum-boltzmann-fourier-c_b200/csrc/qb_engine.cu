@@ -263,6 +263,7 @@ struct DeviceInt {
 	DeviceInt &operator=(int x) { v[cur_dev()].store(x, std::memory_order_release); return *this; }
 };
 
+}  // namespace
 int num_sms() {
 	static DeviceInt sms{0};
 	if (sms == 0) {
@@ -273,6 +274,7 @@ int num_sms() {
 	}
 	return sms;
 }
+namespace {
 
 // before the first launch of any tensor-memory kernel on a device (defined below)
 void check_tmem_coresidency();

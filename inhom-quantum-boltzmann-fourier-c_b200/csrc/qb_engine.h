@@ -24,6 +24,8 @@ void fail(const char *file, int line, const std::string &msg);
 #define QB_CUDA(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) ::qb::fail(__FILE__, __LINE__, std::string(#call) + ": " + cudaGetErrorString(e_)); } while (0)
 bool supported_n(int N);      // grid sizes with kernels: the fixed sizes 8, 16, 32, 64 and the any-N engine's
 
+int num_sms();                // of the current device
+
 // ---- device buffers ---------------------------------------------------------
 // Process-wide count of device-buffer reallocations and releases: a captured
 // CUDA graph holds raw buffer addresses, so it is replayed only while this
