@@ -215,12 +215,16 @@ Workspace::~Workspace() {
 	if (stream) cudaStreamDestroy(stream);
 }
 
-cudaStream_t Workspace::fork(cudaStream_t s, int which) {
-	if (side[which] == nullptr) {
-		QB_CUDA(cudaStreamCreateWithFlags(&side[which], cudaStreamNonBlocking));
-		QB_CUDA(cudaEventCreateWithFlags(&ev_fork[which], cudaEventDisableTiming));
-		QB_CUDA(cudaEventCreateWithFlags(&ev_join[which], cudaEventDisableTiming));
+void Workspace::create_sides() {
+	for (int i = 0; i < 2; i++) {
+		if (side[i] != nullptr) continue;
+		QB_CUDA(cudaEventCreateWithFlags(&ev_fork[i], cudaEventDisableTiming));
+		QB_CUDA(cudaEventCreateWithFlags(&ev_join[i], cudaEventDisableTiming));
+		QB_CUDA(cudaStreamCreateWithFlags(&side[i], cudaStreamNonBlocking));
 	}
+}
+cudaStream_t Workspace::fork(cudaStream_t s, int which) {
+	create_sides();
 	QB_CUDA(cudaEventRecord(ev_fork[which], s));
 	QB_CUDA(cudaStreamWaitEvent(side[which], ev_fork[which], 0));
 	return side[which];
@@ -534,6 +538,10 @@ template <class C> void launch_sum_slots(const SumSlotsT<C> &p, int ncells, cuda
 // partials a cell from which the sums get their own launch: below, the
 // assembly reads them faster than the launch costs
 constexpr int kSumSlots = 4;
+// cells whose sums may get it: the batch's own, or those of a smaller one that its
+// `slots` partials serve too (a smaller batch finds its scratch in that of a larger
+// one, also in a stream that is being captured, where nothing can be allocated)
+size_t summed_cells(size_t slots, int ncells) { return std::min<size_t>(ncells, std::max<size_t>(1, slots / kSumSlots)); }
 // the partial sums of X (a.Xp, lenx values a slot) and of Z (ws.i3z, zranks x
 // lenz values a slot; zranks = 0: none) as the assembly takes them: as they are, or
 // summed over the slots of each cell first
@@ -800,7 +808,7 @@ template <int P, class C> struct Rhs {
 			b.add(ws.i1i4, 4 * ch.i1 * g);
 			b.add(ws.fs4, 4 * g);
 			b.add(ws.i2p, 4 * ch.i2 * g);
-			if (sum_i2(ch.i2, ncells)) b.add(ws.i2s, 4 * g);
+			b.add(ws.i2s, 4 * sizeof(C) * PP * summed_cells((size_t)ncells * ch.i2, ncells));
 			size_t slots = (size_t)ncells * ch.i3, used = slots;
 			if (ch.i3_slots > 0) {
 				const TermRanges r = term_ranges(ch.i3_slots, i3_count(ws, *q.i3), ncells);
@@ -811,10 +819,9 @@ template <int P, class C> struct Rhs {
 			if (pairs_units(ws)) b.add(ws.i3z, sizeof(double2) * slots * kZRanks * 4 * NN);
 			if (P == 64) b.add(ws.i3y, sizeof(C) * used * 8 * PP);
 			if (P == 64 && sizeof(C) == 8 && use_real_form()) b.add(ws.i3zs, sizeof(double2) * slots * kZRanks * 2 * (N + 1) * (N + 1));
-			if (used >= (size_t)kSumSlots * ncells) {
-				b.add(ws.i3s, 4 * g);
-				if (pairs_units(ws)) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
-			}
+			const size_t sc = summed_cells(used, ncells);
+			b.add(ws.i3s, 4 * sizeof(C) * PP * sc);
+			if (pairs_units(ws)) b.add(ws.i3zsum, 4 * sizeof(double2) * NN * sc);
 		}
 	}
 
@@ -835,6 +842,7 @@ template <int P, class C> struct Rhs {
 
 	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, const Chunks &ch, cudaStream_t s) {
 		ws.scratch.reserve();
+		ws.create_sides();
 		spectra(ws, ncells, W, s);
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(ws, *q.i3) < kForkUnits * resident_i3(N, sizeof(C) == 8);
 		const cudaStream_t s2 = small ? ws.fork(s, 0) : s;
@@ -1343,15 +1351,15 @@ template <class C> struct Rhs<128, C> {
 			if (sizeof(C) == 16) b.add(ws.i3y, sizeof(C) * used * 4 * PP);
 			else if (use_full128()) b.add(ws.i3y, sizeof(C) * used * 2 * PP);
 			if (sizeof(C) == 8 && use_real_form()) b.add(ws.i3zs, sizeof(double2) * used * 2 * 2 * (N + 1) * (N + 1));
-			if (used >= (size_t)kSumSlots * ncells) {
-				b.add(ws.i3s, 4 * g);
-				if (pairs_units()) b.add(ws.i3zsum, sizeof(double2) * 4 * (size_t)ncells * NN);
-			}
+			const size_t sc = summed_cells(used, ncells);
+			b.add(ws.i3s, 4 * sizeof(C) * PP * sc);
+			if (pairs_units()) b.add(ws.i3zsum, 4 * sizeof(double2) * NN * sc);
 		}
 	}
 
 	static void prepare(Workspace &ws, const QuadSet &q, int ncells, const double2 *W, int parts, const Chunks &ch, cudaStream_t s) {
 		ws.scratch.reserve();
+		ws.create_sides();
 		spectra(ws, ncells, W, s);
 		const int act = sizeof(C) == 16 ? active_quad_clusters() : use_full128() ? active_i3_full128_clusters() : active_i3_clusters128<float2>();
 		const bool small = (parts & RHS_CD) && (long)ncells * i3_count(*q.i3) < kForkUnits * act;

@@ -151,6 +151,7 @@ struct Workspace {
 	// real form of the I3 sums beside the complex one (1)
 	cudaStream_t side[2] = { nullptr, nullptr };
 	cudaEvent_t ev_fork[2] = { nullptr, nullptr }, ev_join[2] = { nullptr, nullptr };
+	void create_sides();                     // by the first evaluation, whether it forks or not
 	cudaStream_t fork(cudaStream_t s, int which);
 	void join(cudaStream_t s, int which);
 	explicit Workspace(int N);
