@@ -879,7 +879,8 @@ struct qb_fno {
 	qb::DevBuf GO, GH;
 	int use_tc = 0;                               // pointwise maps and truncated DFTs on the tensor cores (BF16, FP32 accumulation)
 	qb::DevBuf kerr;                              // error word of the bounded MMA waits
-	qb::DevBuf twn, twm, tscr, uscr;                   // tensor-core DFTs: the 4 twiddle matrices, stage scratch
+	qb::DevBuf twn;                               // the N-th roots of unity of the FP32 transforms
+	qb::DevBuf twm, tscr, uscr;                   // tensor-core DFTs: the 4 twiddle matrices, stage scratch
 	const float *Bm1 = nullptr, *Bm2 = nullptr, *BmA = nullptr, *BmB = nullptr;
 
 	// the twiddle matrices of the two-stage DFT and inverse (FP32 [Nn][K], from FP64)
@@ -925,22 +926,10 @@ struct qb_fno {
 		launch(name, k_fno_tc<Ld, Ep, Bb>, grid, fnotc::kThreads, (size_t)fnotc::kSmem, s, ld, ep, bm, K, Nn, kerr.as<int>());
 	}
 
-	// the N-th roots of unity of the FP32 transforms (from FP64)
-	const float2 *roots(cudaStream_t s) {
-		if (twn.p == nullptr) {
-			std::vector<float2> h(N);
-			for (int j = 0; j < N; j++) h[j] = make_float2((float)std::cos(2.0 * M_PI * j / N), (float)std::sin(2.0 * M_PI * j / N));
-			twn.ensure(sizeof(float2) * N);
-			QB_CUDA(cudaMemcpyAsync(twn.p, h.data(), sizeof(float2) * N, cudaMemcpyHostToDevice, s));
-			QB_CUDA(cudaStreamSynchronize(s));
-		}
-		return twn.as<float2>();
-	}
-
 	// H[fld] = scale DFT(f[fld]) for the B w fields
 	void dft(int B, const float *f, float2 *Hout, float scale, cudaStream_t s) {
 		if (!use_tc) {
-			launch("fno_dft", k_fno_dft, (unsigned)(B * w), 256, dft_smem(), s, N, m, f, roots(s), Hout, scale);
+			launch("fno_dft", k_fno_dft, (unsigned)(B * w), 256, dft_smem(), s, N, m, f, twn.as<float2>(), Hout, scale);
 			return;
 		}
 		ensure_err(s);
@@ -953,7 +942,7 @@ struct qb_fno {
 	// out[fld] (=, +=) scale Re IDFT(O[fld]), then times dgelu(u) when u is given
 	void idft(int B, const float2 *O, float *out, float scale, int accumulate, const float *u, cudaStream_t s) {
 		if (!use_tc) {
-			launch("fno_idft", k_fno_idft, (unsigned)(B * w), 256, idft_smem(), s, N, m, O, roots(s), out, scale, accumulate, u);
+			launch("fno_idft", k_fno_idft, (unsigned)(B * w), 256, idft_smem(), s, N, m, O, twn.as<float2>(), out, scale, accumulate, u);
 			return;
 		}
 		ensure_err(s);
@@ -1170,6 +1159,10 @@ qb_fno *qb_fno_create(int N, int width, int modes, int layers, unsigned long lon
 		QB_CUDA(cudaMemset(n->am.p, 0, sizeof(float) * np));
 		QB_CUDA(cudaMemset(n->av.p, 0, sizeof(float) * np));
 		QB_CUDA(cudaMemset(n->grads.p, 0, sizeof(float) * np));
+		std::vector<float2> tw(N);
+		for (int j = 0; j < N; j++) tw[j] = make_float2((float)std::cos(2.0 * M_PI * j / N), (float)std::sin(2.0 * M_PI * j / N));
+		n->twn.ensure(sizeof(float2) * N);
+		QB_CUDA(cudaMemcpy(n->twn.p, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
 		net = n.release();
 	});
 	return net;

@@ -27,3 +27,22 @@ def test_capture_after_a_larger_batch(N, prec, large, small):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out[0], direct[0]) and torch.equal(out[1], direct[1])
+
+
+@pytest.mark.gpu
+def test_capture_fp32_surrogate_after_tensor_cores():
+    """the FP32 transforms of a network that ran on the tensor cores before"""
+    net = qbgpu.FNO(16, width=8, modes=4, layers=2, seed=3)
+    W = torch.from_numpy(qbgpu.gaussian_mixture_state(16, L, seed=3, ncells=4)).cuda()
+    direct = net.forward(W)
+    net = qbgpu.FNO(16, width=8, modes=4, layers=2, seed=3)
+    net.set_tensor_cores(True)
+    net.forward(W)
+    net.set_tensor_cores(False)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = net.forward(W)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, direct)
