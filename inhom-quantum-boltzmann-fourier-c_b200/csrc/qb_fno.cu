@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(fnomma::kThreads) k_fno_pointwise_mma(int B, i
 
 // ---------------------------------------------------------------------------
 // A grouped row GEMM on the tensor cores (BF16 operands, FP32 accumulation)
-// for the separable truncated DFTs and the mode mixing: for each of the
+// for the separable truncated DFTs: for each of the
 // bm.groups() groups and 128-row tiles of its bm.rows() rows,
 // D[row][n] = sum_k A[row][k] Bg[n][k], k < K <= 128, n < Nn <= 128, with A
 // read through the loader ld(g, row, k), Bg through bm(g, n, k) (rebuilt when a
@@ -757,35 +757,6 @@ struct BMat {
 	__device__ int groups() const { return 1; }
 	__device__ float operator()(int, int n, int k) const { return Bm[(long)n * K + k]; }
 };
-// mode mixing, one group per mode k: rows b (cells), A = [in_re | in_im] of the
-// summed channels, outputs [out_re | out_im]; forward out_o = sum_i R[i][o] in_i,
-// backward (conj) out_i = sum_o conj(R[i][o]) in_o (R[i][o][k] = Rr + i Ri)
-struct BMix {
-	const float *Rr, *Ri; int w, K, nb, conj;
-	__device__ long rows() const { return nb; }
-	__device__ int groups() const { return K; }
-	__device__ float operator()(int g, int n, int k) const {
-		const int c = n % w, j = k % w;           // output channel c, summed channel j
-		const long ri = conj ? ((long)c * w + j) * K + g : ((long)j * w + c) * K + g;
-		const float rr = Rr[ri], rim = conj ? -Ri[ri] : Ri[ri];
-		// out_re = sum rr in_re - rim in_im, out_im = sum rim in_re + rr in_im
-		if (n < w) return k < w ? rr : -rim;
-		return k < w ? rim : rr;
-	}
-};
-struct LdMix {
-	const float2 *in; int w, K;
-	__device__ float operator()(int g, long row, int k) const {
-		const float2 v = in[(row * w + (k % w)) * (long)K + g];
-		return k < w ? v.x : v.y;
-	}
-};
-struct EpMix {
-	float2 *out; int w, K;
-	__device__ void operator()(int g, long row, const float (&d)[fnotc::kMaxN]) const {
-		for (int c = 0; c < w; c++) out[(row * w + c) * (long)K + g] = make_float2(d[c], d[w + c]);
-	}
-};
 struct LdDft1 { const float *f; int N; __device__ float operator()(int, long row, int k) const { return f[row * N + k]; } };
 struct EpDft1 {
 	float *T; int N, m;
@@ -850,8 +821,7 @@ std::vector<qb::TmemKernel> qb::fno_tmem_kernels() {
 	         { (const void *)k_fno_tc<LdDft1, EpDft1, BMat>, fnotc::kSmem, fnotc::kThreads, fnotc::kCols, "k_fno_tc<dft 1>" },
 	         { (const void *)k_fno_tc<LdDft2, EpDft2, BMat>, fnotc::kSmem, fnotc::kThreads, fnotc::kCols, "k_fno_tc<dft 2>" },
 	         { (const void *)k_fno_tc<LdIdftA, EpIdftA, BMat>, fnotc::kSmem, fnotc::kThreads, fnotc::kCols, "k_fno_tc<idft A>" },
-	         { (const void *)k_fno_tc<LdIdftB, EpIdftB, BMat>, fnotc::kSmem, fnotc::kThreads, fnotc::kCols, "k_fno_tc<idft B>" },
-	         { (const void *)k_fno_tc<LdMix, EpMix, BMix>, fnotc::kSmem, fnotc::kThreads, fnotc::kCols, "k_fno_tc<mix>" } };
+	         { (const void *)k_fno_tc<LdIdftB, EpIdftB, BMat>, fnotc::kSmem, fnotc::kThreads, fnotc::kCols, "k_fno_tc<idft B>" } };
 }
 
 namespace {
@@ -955,17 +925,11 @@ struct qb_fno {
 		const long nw = (long)B * w * P;
 		if (u != nullptr) launch("fno_gelu_bwd", k_fno_gelu_bwd, grid_for(nw), 256, 0, s, nw, u, out);
 	}
-	// mode mixing: out[b][c][k] = sum over the other channel of R (or conj R, backward) times in.
-	// On the tensor cores a mode's B matrix is rebuilt per 128-cell tile, which
-	// pays only when the batch fills the tiles (at 64 cells the FP32 kernel is faster)
+	// mode mixing: out[b][c][k] = sum over the other channel of R (or conj R, backward) times in;
+	// FP32 in both modes (on the tensor cores, with a mode's matrix built for
+	// each 128 cells, 117 us against 48 for 256 cells, 706 against 318 for 2048)
 	void mix(int B, const float2 *in, const float *Rr, const float *Ri, float2 *out, int conj, cudaStream_t s) {
-		if (!use_tc || B < 128) {
-			launch("fno_mix", k_fno_mix, grid_for(2L * K * ((w + 3) / 4) * ((B + 3) / 4)), 128, 0, s, B, w, K, in, Rr, Ri, out, conj);
-			return;
-		}
-		ensure_err(s);
-		row_gemm("fno_mix_tc", LdMix{ in, w, K }, EpMix{ out, w, K }, BMix{ Rr, Ri, w, K, B, conj }, (long)K * ((B + 127) / 128), 2 * w,
-		         2 * w, s);
+		launch("fno_mix", k_fno_mix, grid_for(2L * K * ((w + 3) / 4) * ((B + 3) / 4)), 128, 0, s, B, w, K, in, Rr, Ri, out, conj);
 	}
 	void ensure_err(cudaStream_t s) {
 		if (kerr.p == nullptr) {
