@@ -357,8 +357,8 @@ template <int P, class C> void launch_i2(const I2ParamsT<C> &p, long nblocks, cu
 	if constexpr (P == 64 && sizeof(C) == 16) {
 		if (wide) {
 			static DeviceFlag init;
-			if (!init) { check_tmem_coresidency(); set_smem(k_i2_terms64<C>, Terms64<C>::SMEM); init = true; }
-			k_i2_terms64<C><<<(unsigned)nblocks, Terms64<C>::NT, Terms64<C>::SMEM, s>>>(p);
+			if (!init) { check_tmem_coresidency(); set_smem(k_i2_terms64, Terms64<C>::SMEM); init = true; }
+			k_i2_terms64<<<(unsigned)nblocks, Terms64<C>::NT, Terms64<C>::SMEM, s>>>(p);
 			QB_CUDA(cudaGetLastError());
 			return;
 		}
@@ -1112,7 +1112,7 @@ void check_tmem_coresidency() {
 		{ (const void *)k_i3wr, i3w_smem<float2>(), 512, (int)WideTmem<1>::COLS, "k_i3wr" },
 		{ (const void *)k_i1_terms64<double2>, Terms64<double2>::SMEM, 256, (int)Terms64<double2>::COLS, "k_i1_terms64<f64>" },
 		{ (const void *)k_i1_terms64<float2>, Terms64<float2>::SMEM, 256, (int)Terms64<float2>::COLS, "k_i1_terms64<f32>" },
-		{ (const void *)k_i2_terms64<double2>, Terms64<double2>::SMEM, 256, (int)Terms64<double2>::COLS, "k_i2_terms64<f64>" },
+		{ (const void *)k_i2_terms64, Terms64<double2>::SMEM, 256, (int)Terms64<double2>::COLS, "k_i2_terms64<f64>" },
 		{ (const void *)k_i3_quad, Quad128::SMEM, Quad128::NT, Quad128::TCOLS, "k_i3_quad" },
 		{ (const void *)k_i3_128<4, kI3Pairs128, float2>, smem_i3_128<float2>(), G128::NT,
 		  (int)I3Tmem128<float2, 4 / kI3Pairs128>::NCOLS, "k_i3_128<f32>" },

@@ -107,10 +107,8 @@ __device__ __forceinline__ void fft128_line(C (&x)[8], int tau, C *S, int line, 
 // 64-point transforms E and O, the butterfly Z[k] = E[k] + w^k O[k],
 // Z[k + 64] = E[k] - w^k O[k] is split between the lane pair: lanes 0-7 take
 // k = (tau & 7) + 16 j, lanes 8-15 k = (tau & 7) + 16 j + 8, one shuffle of four
-// values each way.  Output i of lane tau is Z[dpos128(tau, i)].  Applied after
-// fft128_line it needs no reordering in between.
-__device__ __forceinline__ int dpos128(int tau, int i) { return (tau & 7) + 16 * (i >> 1) + 8 * (tau >> 3) + 64 * (i & 1); }
-
+// values each way.  Output i of lane tau is Z[(tau & 7) + 16 (i >> 1) + 8 (tau >> 3) +
+// 64 (i & 1)].  Applied after fft128_line it needs no reordering in between.
 template <int DIR, bool ROW, class C>
 __device__ __forceinline__ void fft128_dit(C (&x)[8], int tau, C *S, int line, const C *tw128, const C (&wp)[8]) {
 	const int h = tau >> 3, t = tau & 7;
@@ -139,7 +137,7 @@ __device__ __forceinline__ void y_row(C (&x)[8], int tau, C *S, int row, const C
 	fft128_dit<+1, true>(x, tau, S, row, tw128, wp);
 	const int m = ((row >> 6) & 1) << 3, k0 = (tau & 7) + 8 * (tau >> 3);
 #pragma unroll
-	for (int i = 0; i < 8; i++)                     // positions dpos128(tau, i)
+	for (int i = 0; i < 8; i++)                     // the positions of fft128_dit
 		S[row * F128::LDP + 64 * (i & 1) + ((k0 + 16 * (i >> 1)) ^ m ^ ((i & 1) << 3))] = x[i];
 }
 

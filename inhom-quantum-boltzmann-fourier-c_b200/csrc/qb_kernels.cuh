@@ -78,14 +78,6 @@ template <class C> struct MulCplx {           // psi (complex N x N) .* v   (Mul
 	const C *psi;
 	__device__ __forceinline__ C operator()(int idx, double2 v) const { return cmul(psi[idx], mk<C>(v.x, v.y)); }
 };
-template <class C> struct MulCplxPair {       // psi .* (v + i b): two grids packed in one transform
-	const C *psi;
-	const double2 *b;
-	__device__ __forceinline__ C operator()(int idx, double2 v) const {
-		const double2 w = b[idx];
-		return cmul(psi[idx], mk<C>(v.x - w.y, v.y + w.x));
-	}
-};
 
 // lane's 8 inputs of padded row `prow` of Pad(mul . src)
 template <int P, class C, class Mul>
@@ -652,12 +644,6 @@ __device__ __forceinline__ void tmem_st(unsigned taddr, double2 v) {
 	const unsigned c = (unsigned)__double2loint(v.y), d = (unsigned)__double2hiint(v.y);
 	asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
-__device__ __forceinline__ void tmem_ld(unsigned taddr, float2 &v) {
-	unsigned a, b;
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(taddr) : "memory");
-	v.x = __uint_as_float(a);
-	v.y = __uint_as_float(b);
-}
 __device__ __forceinline__ void tmem_st(unsigned taddr, float2 v) {
 	asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)) : "memory");
 }
@@ -720,23 +706,6 @@ __device__ __forceinline__ void tmem_st4(unsigned taddr, const double2 (&v)[4]) 
 		r[4 * e] = (unsigned)__double2loint(v[e].x); r[4 * e + 1] = (unsigned)__double2hiint(v[e].x);
 		r[4 * e + 2] = (unsigned)__double2loint(v[e].y); r[4 * e + 3] = (unsigned)__double2hiint(v[e].y);
 	}
-	asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-	             :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-
-// eight FP64 reals (16 columns) in one load or store
-__device__ __forceinline__ void tmem_ld8r(unsigned taddr, double (&v)[8]) {
-	unsigned r[16];
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-	             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-	             : "r"(taddr) : "memory");
-#pragma unroll
-	for (int e = 0; e < 8; e++) v[e] = __hiloint2double((int)r[2 * e + 1], (int)r[2 * e]);
-}
-__device__ __forceinline__ void tmem_st8r(unsigned taddr, const double (&v)[8]) {
-	unsigned r[16];
-#pragma unroll
-	for (int e = 0; e < 8; e++) { r[2 * e] = (unsigned)__double2loint(v[e]); r[2 * e + 1] = (unsigned)__double2hiint(v[e]); }
 	asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
 	             :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }

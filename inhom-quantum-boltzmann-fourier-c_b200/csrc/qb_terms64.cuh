@@ -8,9 +8,7 @@
 // transform do not fit 128 registers; FP32: three CTAs, accumulators in registers.
 // Measured (Strang step, 64 cells, J = M = 16, the sums alone): I1 and I4 in FP64 1009 ->
 // 666 us, I2 357 -> 280 us; I1 and I4 in FP32 734 -> 418 us. Both are bound by the
-// shared-memory pipe and the latency of its barriers. I2 in FP32 stays with k_i2_terms:
-// on 16 values a thread 1000 steps (8 cells, J = M = 16, all sums here) drift 9.5e-6
-// from FP64 against 7.2e-6 with the general kernels; I1 and I4 here alone: 6.2e-6.
+// shared-memory pipe and the latency of its barriers. I2 in FP32 stays with k_i2_terms.
 #pragma once
 #include "qb_wide64.cuh"
 
@@ -148,9 +146,9 @@ __global__ void __launch_bounds__(Terms64<C>::NT, Terms64<C>::CTAS) k_i1_terms64
 	if (t < 32) tmem_dealloc(tmem_slot, T::COLS);
 }
 
-// the sums of k_i2_terms at P = 64
-template <class C>
-__global__ void __launch_bounds__(Terms64<C>::NT, Terms64<C>::CTAS) k_i2_terms64(const I2ParamsT<C> p) {
+// the sums of k_i2_terms at P = 64 in FP64
+__global__ void __launch_bounds__(Terms64<double2>::NT, Terms64<double2>::CTAS) k_i2_terms64(const I2ParamsT<double2> p) {
+	using C = double2;
 	using T = Terms64<C>;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	__shared__ unsigned tmem_slot;
