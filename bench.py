@@ -161,15 +161,20 @@ class ClockSampler:
 
 # ---------------------------------------------------------------------------
 
-def i3_flops_per_pair(N):
-    """FP64 flops of the I3 kernel per (cell, pair of terms of opposite shifts):
-    4 padded spectra and 4 extracted inverse transforms (0.75 of a full 2N x 2N
-    FFT each: half the rows are zero or not needed) + 16 (i, j) pairs x (IFFT2 +
-    FFT2) at 5 n log2 n per transform, plus the pointwise products (24 flops per
-    padded point per (i, j), 14 per N-point per component)."""
+def i3_flops_per_angle(N, M):
+    """FP64 flops of the I3 kernel per (cell, angle): M // 2 pairs of terms of
+    opposite shifts and, of an odd M, the middle node alone.  A pair: 4 padded
+    spectra and 4 extracted inverse transforms (0.75 of a full 2N x 2N FFT each:
+    half the rows are zero or not needed) + 16 (i, j) pairs x (IFFT2 + FFT2) at
+    5 n log2 n per transform, plus the pointwise products (24 flops per padded
+    point per (i, j), 14 per N-point per component).  The middle node has no
+    extracted transforms and no products W^_j . T_ij (16 flops per padded point,
+    6 per N-point)."""
     P = 2 * N
     F = 5.0 * P * P * math.log2(P * P)
-    return 8 * 0.75 * F + 32 * F + 16 * 24 * P * P + 4 * 14 * N * N
+    pair = 8 * 0.75 * F + 32 * F + 16 * 24 * P * P + 4 * 14 * N * N
+    single = 4 * 0.75 * F + 32 * F + 16 * 16 * P * P + 4 * 6 * N * N
+    return (M // 2) * pair + (M % 2) * single
 
 
 def captured_traffic(kernel, wl):
@@ -274,7 +279,7 @@ def run_ours(args):
     L.qb_fp64_peak_tflops.restype = ctypes.c_double
     peak = L.qb_fp64_peak_tflops()
     per_launch_ms = kms.value / max(1, kn.value)
-    flops_launch = cells * wl["J"] * ((wl["M"] + 1) // 2) * i3_flops_per_pair(N)
+    flops_launch = cells * wl["J"] * i3_flops_per_angle(N, wl["M"])
     achieved = flops_launch / (per_launch_ms * 1e-3) / 1e12
     i3name = {32: "k_i3w", 64: "k_i3_quad"}.get(N, "k_i3q")
     i3desc = {"k_i3w": "k_i3w (I3 quadrature sums, 2-CTA cluster, 16 values a thread, accumulators in tensor memory)",
