@@ -336,7 +336,7 @@ template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C 
 
 // wide: the kernels of qb_terms64.cuh at P = 64
 template <int P, class C> void launch_i1(const I1ParamsT<C> &p, long nblocks, cudaStream_t s, bool wide = false) {
-	ProfScope ps("i1_terms", s);
+	ProfScope ps(wide ? "i1_terms64" : "i1_terms", s);
 	if constexpr (P == 64) {
 		if (wide) {
 			static DeviceFlag init;
@@ -353,7 +353,7 @@ template <int P, class C> void launch_i1(const I1ParamsT<C> &p, long nblocks, cu
 }
 
 template <int P, class C> void launch_i2(const I2ParamsT<C> &p, long nblocks, cudaStream_t s, bool wide = false) {
-	ProfScope ps("i2_terms", s);
+	ProfScope ps(wide && sizeof(C) == 16 ? "i2_terms64" : "i2_terms", s);
 	if constexpr (P == 64 && sizeof(C) == 16) {
 		if (wide) {
 			static DeviceFlag init;
@@ -1462,8 +1462,10 @@ Chunks pick_chunks(int N, int ncells, const QuadSet &q, int prec, int i3_units) 
 	const int sms = num_sms();
 	// N = 32: the kernels of qb_terms64.cuh, as many CTAs as an SM holds, except in
 	// small batches: there an SM has few terms to run and the 512 threads a term of
-	// the general kernels finish them sooner (7 cells, J = 8, M = 6 between Maxwell
-	// walls: 600 us a step against 631; 64 cells, J = M = 16: 15.5 ms against 15.1)
+	// the general kernels finish them sooner. Cc and Cd with the general kernels over
+	// the time with these, for J x M = 16 x 16, 8 x 6, 32 x 32 and 4 x 4: FP64, from
+	// the line to 12 times as many cells 0.995 to 1.17, below half of it 0.96 to 1.02;
+	// FP32 0.91 to 1.17 above (median 1.02) and 1.00 to 1.17 below
 	c.wide12 = N == 32 && ncells * (long)i3_units >= kForkUnits * resident_i3(N, prec == 32);
 	const int c1 = !c.wide12 ? 1 : prec == 32 ? Terms64<float2>::CTAS : Terms64<double2>::CTAS;
 	const int c2 = !c.wide12 || prec == 32 ? 1 : Terms64<double2>::CTAS;
