@@ -1408,8 +1408,9 @@ template <class C> struct AnyRhs {
 	}
 
 	// chunks a cell of the whole-grid chains: as even a split of the pieces over the
-	// resident clusters as the partials are worth (X and Z of a cell and chunk, 0.9 MB in
-	// FP32 at N = 48, written and read back at HBM speed: 0.003 of a unit's 140 us).
+	// resident clusters as the partials are worth (0.15 of a unit in the sums of a cell,
+	// or X and Z of every cell and chunk, 0.9 MB in FP32 at N = 48, written and read
+	// back at HBM speed: 0.003 of a unit's 140 us).
 	// Batches beyond 512 cells split as 512 do: the slices they run in are smaller
 	int grid_chunks(const DevI3 &t) const {
 		const int res = N == 24 ? grid_resident<3>() : grid_resident<6>();
@@ -1417,7 +1418,7 @@ template <class C> struct AnyRhs {
 		int best = 1;
 		double best_cost = 1e300;
 		for (int c = 1; c <= std::min(nunits, 64); c++) {
-			const double cost = (double)(((long)n * c + res - 1) / res) * ((nunits + c - 1) / c) + (0.15 + 0.003 * n) * c;
+			const double cost = (double)(((long)n * c + res - 1) / res) * ((nunits + c - 1) / c) + std::max(0.15, 0.003 * n) * c;
 			if (cost < best_cost) { best_cost = cost; best = c; }
 		}
 		return best;

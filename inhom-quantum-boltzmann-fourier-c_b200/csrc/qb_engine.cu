@@ -321,10 +321,11 @@ int best_chunks(long units, int nterms, int slots, int max_chunks, double penalt
 }
 
 // the price of one more I3 partial a cell, in times of a unit on a cluster: 0.15 for
-// its part in the sums of a cell, and for every cell its grids (X and Z) written and
-// read back at HBM speed: 0.26 and 1.05 MB at N = 32 and 64 in FP32 against units of 40
-// and 90 us (0.002 and 0.0036), 80 KB at N = 16 in FP64 against 70 us (0.0004)
-double i3_partial(int N, int ncells) { return 0.15 + (N >= 32 ? 0.003 : 0.0004) * ncells; }
+// its part in the sums of a cell, or in large batches what its grids (X and Z) of every
+// cell, written and read back at HBM speed, come to: 0.26 and 1.05 MB at N = 32 and
+// 64 in FP32 against units of 40 and 90 us (0.002 and 0.0036 a cell), 80 KB at N = 16
+// in FP64 against 70 us (0.0004)
+double i3_partial(int N, int ncells) { return std::max(0.15, (N >= 32 ? 0.003 : 0.0004) * ncells); }
 
 template <int P, class C> void launch_pad_fft(int ngrids, const double2 *src, C *out, cudaStream_t s, C *out2 = nullptr, float *outr = nullptr) {
 	static DeviceFlag init;
@@ -569,9 +570,9 @@ void sum_slots(Workspace &ws, AsmParamsT<C> &a, int ncells, long slots, long len
 
 template <int P, class C> void launch_assemble(const AsmParamsT<C> &p, long ncells, cudaStream_t s) {
 	static DeviceFlag init;
-	if (!init) { set_smem(k_assemble<P, C>, smem_grids<P, double2>(1)); init = true; }
+	if (!init) { set_smem(k_assemble<P, C>, smem_grids<P, typename Asm<P, C>::A>(1)); init = true; }
 	ProfScope ps("assemble", s);
-	k_assemble<P, C><<<(unsigned)(ncells * 4), Geo<P>::NT, smem_grids<P, double2>(1), s>>>(p);
+	k_assemble<P, C><<<(unsigned)(ncells * 4), Geo<P>::NT, smem_grids<P, typename Asm<P, C>::A>(1), s>>>(p);
 	QB_CUDA(cudaGetLastError());
 }
 

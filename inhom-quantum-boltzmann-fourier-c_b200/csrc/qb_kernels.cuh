@@ -23,6 +23,7 @@
 // Moving the sums over quadrature terms inside the outer transforms is exact
 // in real arithmetic; results agree with the upstream loop order to rounding.
 #pragma once
+#include <type_traits>
 #include <cooperative_groups.h>
 #include "qb_fft.cuh"
 
@@ -816,7 +817,7 @@ __global__ void __launch_bounds__(256) k_sum_slots(const SumSlotsT<C> p) {
 //   Cc_j = s1 Extract(IFFT2(Zcc_j)), Cd_j = Extract(IFFT2(Zcd_j)) - eta2_j s1 Z_j
 // (Z_j: the already extracted sums of I3Units)
 // The inputs are in the working precision C; the sums and the inverse transforms
-// are in FP64 in both: rounding after them spreads over the whole velocity grid
+// are in FP64 in both (Asm): rounding after them spreads over the whole velocity grid
 // (see zadd), before them it stays where W is.  mode 0 writes Cc and Cd; mode 1 writes
 // base + dtc (Cc + Cd + CB) in FP64 with the magnetic rotation CB of `wcur`
 // (upstream simulation.c:75-135).
@@ -857,17 +858,25 @@ __device__ __forceinline__ double2 zsum(const AsmParamsT<C> &p, long cell, int j
 	return z;
 }
 
+// the assembly's type: FP64, but FP32 in the FP32 form at N = 8, where a step of
+// launches costs 13 us more in FP64 (11 cells, J = M = 4: 153 against 133 us a
+// midpoint step) and the FP32 form was never further from FP64 than term by term
+template <int P, class C> struct Asm { using A = typename std::conditional<P == 16, C, double2>::type; };
+
 template <int P, class C>
 __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) {
-	using G = Geo<P, double2>;
+	using A = typename Asm<P, C>::A;
+	using G = Geo<P, A>;
+	using R = typename CT<A>::R;
 	constexpr int N = G::N, NN = N * N, PP = P * P;
 	constexpr int PER = (NN + G::NT - 1) / G::NT;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	double2 *S = reinterpret_cast<double2 *>(smem_raw), *tw = S + G::GRID;
+	A *S = reinterpret_cast<A *>(smem_raw), *tw = S + G::GRID;
 	const int j = blockIdx.x & 3;
 	const long cell = blockIdx.x >> 2;
 	init_twiddles<P>(tw);
-	const double eta2[4] = { 2, -2, -2, -2 }, s1 = p.s1, s2 = p.s2;
+	const R eta2[4] = { 2, -2, -2, -2 }, s1 = (R)p.s1, s2 = (R)p.s2;
+	auto in = [](C v) { return mk<A>(v.x, v.y); };
 	const C *Wh = p.What + cell * 4 * PP;
 	double2 cc[PER], cd[PER];
 #pragma unroll
@@ -878,8 +887,8 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 		const int gi = (j % 3) + 1, hi = ((j + 1) % 3) + 1;    // j=1:(2,3) j=2:(3,1) j=3:(1,2)
 		const C *FS = p.FS + cell * 3 * PP;
 		for (int i = threadIdx.x; i < PP; i += G::NT) {
-			S[G::at(i / P, i % P)] = csub(cmul(widen(Wh[hi * PP + i]), widen(FS[(gi - 1) * PP + i])),
-			                              cmul(widen(Wh[gi * PP + i]), widen(FS[(hi - 1) * PP + i])));
+			S[G::at(i / P, i % P)] = csub(cmul(in(Wh[hi * PP + i]), in(FS[(gi - 1) * PP + i])),
+			                              cmul(in(Wh[gi * PP + i]), in(FS[(hi - 1) * PP + i])));
 		}
 		__syncthreads();
 		fft2_smem<P, +1>(S, tw);
@@ -887,7 +896,7 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 		for (int u = 0; u < PER; u++) {
 			const int q = threadIdx.x + u * G::NT;
 			if (q < NN) {
-				cc[u] = cscale(S[G::at(G::pad(q / N), G::pad(q % N))], s1);
+				cc[u] = cscale(widen(S[G::at(G::pad(q / N), G::pad(q % N))]), p.s1);
 			}
 		}
 		__syncthreads();
@@ -895,41 +904,41 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 	// --- Cd ---
 	if (p.FS4 != nullptr || p.Qp != nullptr || p.Xp != nullptr) {
 		// the partial sums of all the thread's elements together (as in k_fft_full)
-		double2 zs[8];
+		A zs[8];
 #pragma unroll
-		for (int e = 0; e < 8; e++) zs[e] = czero();
+		for (int e = 0; e < 8; e++) zs[e] = czero<A>();
 		if (p.Qp != nullptr) {
 #pragma unroll 1
 			for (int ii = 0; ii < 4; ii++) {
 				const C *Q = p.Qp + ((cell * 4 + ii) * p.nq) * (long)PP + threadIdx.x;
-				double2 s[8];
+				A s[8];
 #pragma unroll
-				for (int e = 0; e < 8; e++) s[e] = czero();
+				for (int e = 0; e < 8; e++) s[e] = czero<A>();
 #pragma unroll 1
 				for (int k = 0; k < p.nq; k++)
 #pragma unroll
-					for (int e = 0; e < 8; e++) s[e] = cadd(s[e], widen(Q[(long)k * PP + e * G::NT]));
+					for (int e = 0; e < 8; e++) s[e] = cadd(s[e], in(Q[(long)k * PP + e * G::NT]));
 #pragma unroll
 				for (int e = 0; e < 8; e++) { zs[e].x += eta2[ii] * s[e].x; zs[e].y += eta2[ii] * s[e].y; }
 			}
 #pragma unroll
 			for (int e = 0; e < 8; e++) {
-				double2 h = widen(Wh[j * PP + threadIdx.x + e * G::NT]);
+				A h = in(Wh[j * PP + threadIdx.x + e * G::NT]);
 				h.x = -h.x; h.y = -h.y;
-				if (j == 0) h.x += 1.0;
-				const double2 v = cmul(h, zs[e]);
+				if (j == 0) h.x += (R)1.0;
+				const A v = cmul(h, zs[e]);
 				zs[e].x = s2 * v.x;
 				zs[e].y = s2 * v.y;
 			}
 		}
 		if (p.Xp != nullptr) {
-			double2 s[8];
+			A s[8];
 #pragma unroll
-			for (int e = 0; e < 8; e++) s[e] = czero();
+			for (int e = 0; e < 8; e++) s[e] = czero<A>();
 			auto add = [&](long slot) {
 				const C *X = p.Xp + (slot * 4 + j) * (long)PP + threadIdx.x;
 #pragma unroll
-				for (int e = 0; e < 8; e++) s[e] = cadd(s[e], widen(X[e * G::NT]));
+				for (int e = 0; e < 8; e++) s[e] = cadd(s[e], in(X[e * G::NT]));
 			};
 			if (p.xrg.nslots > 0) {
 				const TermRanges &g = p.xrg;
@@ -946,14 +955,14 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 #pragma unroll
 		for (int e = 0; e < 8; e++) {
 			const int i = threadIdx.x + e * G::NT;
-			double2 z = zs[e];
+			A z = zs[e];
 			if (p.FS4 != nullptr) {
 				const C *F4 = p.FS4 + cell * 4 * PP;
-				double2 v = cadd(cscale(cmul(widen(Wh[i]), widen(F4[j * PP + i])), eta2[j]), cscale(cmul(widen(Wh[j * PP + i]), widen(F4[i])), 2.0));
+				A v = cadd(cscale(cmul(in(Wh[i]), in(F4[j * PP + i])), eta2[j]), cscale(cmul(in(Wh[j * PP + i]), in(F4[i])), (R)2.0));
 				if (j == 0) {
-					double2 s = czero();
-					for (int c = 0; c < 4; c++) s = cadd(s, cmul(widen(Wh[c * PP + i]), widen(F4[c * PP + i])));
-					v = csub(v, cscale(s, 2.0));
+					A s = czero<A>();
+					for (int c = 0; c < 4; c++) s = cadd(s, cmul(in(Wh[c * PP + i]), in(F4[c * PP + i])));
+					v = csub(v, cscale(s, (R)2.0));
 				}
 				z.x += s1 * v.x; z.y += s1 * v.y;
 			}
@@ -965,7 +974,7 @@ __global__ void __launch_bounds__(Geo<P>::NT) k_assemble(const AsmParamsT<C> p) 
 		for (int u = 0; u < PER; u++) {
 			const int q = threadIdx.x + u * G::NT;
 			if (q < NN) {
-				cd[u] = S[G::at(G::pad(q / N), G::pad(q % N))];
+				cd[u] = widen(S[G::at(G::pad(q / N), G::pad(q % N))]);
 				if (p.Zp != nullptr) {
 					const double2 z = zsum(p, cell, j, NN, q);
 					const double f = (j == 0 ? 2.0 : -2.0) * p.s1;
