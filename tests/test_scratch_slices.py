@@ -37,6 +37,23 @@ def test_slices_give_the_same(N, prec, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,prec", [(16, 64), (32, 32), (48, 32)])
+def test_slices_in_a_captured_step(N, prec, monkeypatch):
+    """a Strang step in slices: launched, captured and replayed the same"""
+    monkeypatch.setenv("QB_ANYN_SLICE_MB", "1")
+    cells = 6
+    q, ws = qbgpu.Quad(N, 4, 3, L, R), qbgpu.Workspace(N, precision=prec)
+    W = torch.from_numpy(qbgpu.gaussian_mixture_state(N, L, seed=2, ncells=cells)).cuda()
+    outs, out = [], torch.empty_like(W)
+    for _ in range(4):
+        out.zero_()
+        qbgpu.inhom_step(ws, q, W, 0.1, 0.005, out=out)
+        outs.append(out.clone())
+    assert ws.graph_replays == 2
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("N,prec,cells,J,M", [(24, 64, 1500, 8, 8), (32, 32, 2048, 16, 16), (64, 32, 300, 8, 8), (64, 64, 600, 2, 2), (96, 32, 260, 2, 2)])
 def test_scratch_of_large_batches(N, prec, cells, J, M):
     q, W = qbgpu.Quad(N, J, M, L, R), fourier(N, cells, 4)
