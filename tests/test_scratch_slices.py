@@ -44,10 +44,11 @@ def test_slices_in_a_captured_step(N, prec, monkeypatch):
     cells = 6
     q, ws = qbgpu.Quad(N, 4, 3, L, R), qbgpu.Workspace(N, precision=prec)
     W = torch.from_numpy(qbgpu.gaussian_mixture_state(N, L, seed=2, ncells=cells)).cuda()
+    B = torch.zeros((cells, 3), dtype=torch.float64, device="cuda")         # one set of pointers: graphs are kept by them
     outs, out = [], torch.empty_like(W)
     for _ in range(4):
         out.zero_()
-        qbgpu.inhom_step(ws, q, W, 0.1, 0.005, out=out)
+        qbgpu.inhom_step(ws, q, W, 0.1, 0.005, B, out=out)
         outs.append(out.clone())
     assert ws.graph_replays == 2
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
